@@ -10,6 +10,7 @@ import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libgq_b200.so")
+NATIVE_PATH = os.path.join(_HERE, "_gq_torch.so")
 
 ERRORS = {-1: "unsupported GGML type", -2: "bad shape (K not a multiple of 256, negative size, or M over the limit)",
           -3: "bad argument (null or misaligned pointer, inconsistent sizes)", -4: "workspace too small",
@@ -73,6 +74,23 @@ def lib() -> ctypes.CDLL:
             fn.restype, fn.argtypes = res, args
         _lib = L
     return _lib
+
+
+_native = None
+
+
+def native():
+    """The extension module with the native call path (csrc/gq_torch.cpp); raises where it is missing, as lib() does."""
+    global _native
+    if _native is None:
+        lib()
+        if not os.path.exists(NATIVE_PATH):
+            raise GqError(f"{NATIVE_PATH} is missing: build it with `python -m hyperqwen_rtx4080s32_b200.build`")
+        from . import _gq_torch
+
+        _gq_torch.set_error_type(GqError)
+        _native = _gq_torch
+    return _native
 
 
 def check(rc: int, what: str) -> int:

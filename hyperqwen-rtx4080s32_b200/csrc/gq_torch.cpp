@@ -1,0 +1,164 @@
+// Native call path of a packed run: the Python extension module `_gq_torch`.
+//
+// GGUFLinearMethod.apply is called once per linear layer and token step.  Going through the torch custom op and ctypes
+// costs 46 us of host time per call on an idle GPU (boxing nine arguments, three of them lists of tensors, a Python
+// kernel, two allocations from Python and a ctypes call with fifteen arguments), six times what the GPU needs for a small
+// layer.  A Run keeps what does not change between calls — the packed buffer, the descriptor tables, the split per
+// row count — and does the call's host work here: output and scratch from torch's caching allocator on the current
+// stream, then the C ABI of include/gq_b200.h.
+//
+// forward() answers None for whatever is not the plain case (dtype, layout, device, autograd, torch dispatch modes, a
+// call of zero rows); the caller then takes the general path, which also states the errors.
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <pybind11/pybind11.h>
+#include <pybind11/stl.h>
+#include <torch/csrc/utils/pybind.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <string>
+#include <vector>
+#include "../../include/gq_b200.h"
+
+namespace py = pybind11;
+
+namespace {
+
+const char *error_text(int rc) {
+    switch (rc) {
+        case GQ_ERR_TYPE: return "unsupported GGML type";
+        case GQ_ERR_SHAPE: return "bad shape (K not a multiple of 256, negative size, or M over the limit)";
+        case GQ_ERR_ARG: return "bad argument (null or misaligned pointer, inconsistent sizes)";
+        case GQ_ERR_WORKSPACE: return "workspace too small";
+        case GQ_ERR_CUDA: return "CUDA runtime error";
+        case GQ_ERR_LIMIT: return "size beyond a fixed maximum";
+        default: return "unknown error";
+    }
+}
+PyObject *g_error = PyExc_RuntimeError;      // GqError of _lib.py, kept for the life of the process
+
+void check(int64_t rc, const char *what) {
+    if (rc >= 0) return;
+    std::string msg = std::string(what) + " failed (" + std::to_string(rc) + "): " + error_text((int)rc);
+    if (rc == GQ_ERR_CUDA) msg += std::string(": ") + gq_last_cuda_error();
+    PyErr_SetString(g_error, msg.c_str());
+    throw py::error_already_set();
+}
+
+inline bool plain_cuda(const at::Tensor &t, int device) {
+    return t.is_cuda() && t.layout() == at::kStrided && t.get_device() == device && !t.requires_grad();
+}
+
+class Run {
+  public:
+    Run(at::Tensor packed, std::vector<at::Tensor> descs, std::vector<int64_t> splits, std::vector<int64_t> n_outs, std::vector<int64_t> types,
+        int64_t nb, std::vector<int64_t> split_of_rows, int64_t decode_rows, int64_t pre_rows)
+        : packed_(std::move(packed)), descs_(std::move(descs)), splits_(std::move(splits)), K_(nb * 256), decode_rows_(decode_rows),
+          pre_rows_(pre_rows), device_(packed_.get_device()) {
+        std::vector<int32_t> t32(types.begin(), types.end());
+        check(info_ = gq_run_info((int)t32.size(), t32.data()), "gq_run_info");
+        for (int64_t n : n_outs) n_total_ += n;
+        one_ = index_of(1);
+        for (int64_t s : split_of_rows) by_rows_.push_back(index_of(s));
+        TORCH_CHECK((int64_t)by_rows_.size() > decode_rows_, "split_of_rows covers 0..decode_rows");
+    }
+
+    // x [..., K] -> [..., n_total]; None: not the plain case
+    PyObject *forward(py::handle x) { return call(x, 0, nullptr, nullptr, nullptr, 0.0f); }
+    PyObject *forward_silu_mul(py::handle x) { return call(x, 1, nullptr, nullptr, nullptr, 0.0f); }
+    PyObject *forward_add_rms_norm(py::handle x, const at::Tensor &weight, c10::optional<at::Tensor> residual,
+                                   c10::optional<at::Tensor> residual_out, double eps) {
+        return call(x, 2, &weight, residual.has_value() ? &*residual : nullptr, residual_out.has_value() ? &*residual_out : nullptr, (float)eps);
+    }
+
+  private:
+    int index_of(int64_t split) const {
+        int one = 0;
+        for (size_t i = 0; i < splits_.size(); ++i) {
+            if (splits_[i] == split) return (int)i;
+            if (splits_[i] == 1) one = (int)i;
+        }
+        return one;
+    }
+    static PyObject *none() { Py_RETURN_NONE; }
+
+    PyObject *call(py::handle xh, int pre, const at::Tensor *weight, const at::Tensor *residual, const at::Tensor *residual_out, float eps) {
+        if (!THPVariable_CheckExact(xh.ptr()) || c10::impl::dispatch_mode_enabled()) return none();
+        const at::Tensor &x = THPVariable_Unpack(xh.ptr());
+        const int64_t width = pre == 1 ? 2 * K_ : K_, nd = x.dim();
+        if (nd < 1 || !plain_cuda(x, device_) || x.scalar_type() != at::kBFloat16 || x.size(-1) != width || x.stride(-1) != 1) return none();
+        int64_t m = 1, ldx = width;
+        if (nd == 2) { m = x.size(0); ldx = x.stride(0); if (m == 1 && ldx < width) ldx = width; }
+        else { if (!x.is_contiguous()) return none(); for (int64_t i = 0; i + 1 < nd; ++i) m *= x.size(i); }
+        if (m <= 0 || n_total_ == 0 || ldx < width) return none();
+        if (pre) {
+            if (m > pre_rows_) return none();
+            if (pre == 2) {
+                if (!plain_cuda(*weight, device_) || weight->scalar_type() != at::kBFloat16 || weight->numel() != K_ || !weight->is_contiguous()) return none();
+                if ((residual == nullptr) != (residual_out == nullptr)) return none();
+                if (residual) {
+                    for (const at::Tensor *r : {residual, residual_out})
+                        if (!plain_cuda(*r, device_) || r->scalar_type() != at::kBFloat16 || r->dim() != 2 || r->size(0) != m || r->size(1) != K_ ||
+                            r->stride(1) != 1) return none();
+                    if (residual->stride(0) != residual_out->stride(0)) return none();
+                }
+            }
+        }
+        const bool wide = m > decode_rows_;
+        if (wide && ((ldx & 7) || (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15))) return none();
+        c10::cuda::CUDAGuard guard((c10::DeviceIndex)device_);
+        void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device_).stream();
+        at::DimVector sizes(x.sizes().begin(), x.sizes().end());
+        sizes.back() = n_total_;
+        at::Tensor y = at::detail::empty_cuda(sizes, at::kBFloat16, x.device(), c10::nullopt);
+        auto *alloc = c10::cuda::CUDACachingAllocator::get();
+        if (wide) {
+            const int64_t n_desc = descs_[one_].size(0), need = gq_prefill_workspace_bytes(m, K_, n_total_, n_desc);
+            check(need, "gq_prefill_workspace_bytes");
+            c10::DataPtr ws = alloc->allocate((size_t)need + 1024);
+            const uintptr_t base = (reinterpret_cast<uintptr_t>(ws.get()) + 1023) & ~(uintptr_t)1023;
+            check(gq_gemm_prefill(x.data_ptr(), m, K_, ldx, packed_.data_ptr(), (const int32_t *)descs_[one_].data_ptr(), n_desc, info_, y.data_ptr(),
+                                  n_total_, n_total_, (void *)base, need, stream), "gq_gemm_prefill");
+        } else {
+            const int i = by_rows_[m];
+            const int split = (int)splits_[i];
+            const at::Tensor &d = descs_[i];
+            const int64_t need = gq_workspace_bytes(m, K_, n_total_, split);
+            check(need, "gq_workspace_bytes");
+            c10::DataPtr ws = alloc->allocate((size_t)need);
+            if (pre)
+                check(gq_gemv_grouped_pre(x.data_ptr(), m, K_, ldx, pre, weight ? weight->data_ptr() : nullptr, residual ? residual->data_ptr() : nullptr,
+                                          residual_out ? residual_out->data_ptr() : nullptr, residual ? residual->stride(0) : 0, eps, packed_.data_ptr(),
+                                          (const int32_t *)d.data_ptr(), d.size(0), split, info_, y.data_ptr(), n_total_, n_total_, ws.get(), need, stream),
+                      "gq_gemv_grouped_pre");
+            else
+                check(gq_gemv_grouped(x.data_ptr(), m, K_, ldx, packed_.data_ptr(), (const int32_t *)d.data_ptr(), d.size(0), split, info_, y.data_ptr(),
+                                      n_total_, n_total_, ws.get(), need, stream), "gq_gemv_grouped");
+        }
+        return THPVariable_Wrap(std::move(y));
+    }
+
+    at::Tensor packed_;
+    std::vector<at::Tensor> descs_;
+    std::vector<int64_t> splits_;
+    std::vector<int> by_rows_;       // rows -> index into descs_
+    int64_t K_, n_total_ = 0, decode_rows_, pre_rows_;
+    int device_, info_ = 0, one_ = 0;
+};
+
+}  // namespace
+
+PYBIND11_MODULE(_gq_torch, m) {
+    m.def("set_error_type", [](py::object e) { g_error = e.release().ptr(); });
+    py::class_<Run>(m, "Run")
+        .def(py::init<at::Tensor, std::vector<at::Tensor>, std::vector<int64_t>, std::vector<int64_t>, std::vector<int64_t>, int64_t, std::vector<int64_t>,
+                      int64_t, int64_t>())
+        .def("forward", [](Run &r, py::handle x) { return py::reinterpret_steal<py::object>(r.forward(x)); })
+        .def("forward_silu_mul", [](Run &r, py::handle x) { return py::reinterpret_steal<py::object>(r.forward_silu_mul(x)); })
+        .def("forward_add_rms_norm", [](Run &r, py::handle x, const at::Tensor &w, c10::optional<at::Tensor> res, c10::optional<at::Tensor> out, double eps) {
+            return py::reinterpret_steal<py::object>(r.forward_add_rms_norm(x, w, res, out, eps));
+        });
+}

@@ -240,6 +240,11 @@ class GGUFLinearMethod:
                 [tiles[sid] for sid in run], [layer.gguf_tiles_rows[sid] for sid in run], [layer.gguf_tiles_types[sid] for sid in run])
             tiles.update(zip(run, views))
             layer.gguf_groups[run[0]] = (packed, descs, splits, run, nb, block_bytes)
+        # the native call path of a layer that is one run (every layer whose shards are all tiled)
+        layer.gguf_native = None
+        if len(runs) == 1 and len(runs[0]) == len(order):
+            layer.gguf_native = ops.NativeRun(layer.gguf_groups[order[0]], [layer.gguf_tiles_rows[sid] for sid in order],
+                                              [layer.gguf_tiles_types[sid] for sid in order])
 
     def check_status(self, device=None) -> None:
         """Raise if any kernel of the path has reported a bounded wait that ran out on the device since the last
@@ -256,11 +261,18 @@ class GGUFLinearMethod:
         """apply of pre(x), pre being ops.PreSiluMul / ops.PreAddRMSNorm (or None): the op in front of the layer is folded
         into the launch for up to 16 rows.  An addition to the reference's method, whose apply takes the finished
         activation (gguf-tiles-all-types.patch:203-262)."""
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, x.shape[-1])
+        native = layer.__dict__.get("gguf_native")
         if pre is not None and getattr(pre, "residual", None) is not None:
             pre.residual = pre.residual.reshape(-1, pre.residual.shape[-1])
             pre.residual_out = pre.residual_out.reshape(-1, pre.residual_out.shape[-1])
+        if native is not None:
+            out = native(layer.gguf_groups, x, pre)
+            if out is not None:
+                if bias is not None:
+                    out.add_(bias)
+                return out
+        lead = x.shape[:-1]
+        x2 = x.reshape(-1, x.shape[-1])
         tiles = getattr(layer, "gguf_tiles", None)
         groups = getattr(layer, "gguf_groups", None)
         if not tiles or not groups:

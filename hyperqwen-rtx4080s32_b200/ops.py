@@ -17,7 +17,7 @@ import numpy as np
 import torch
 
 from . import formats as F
-from ._lib import DESC_WORDS, MAX_GEMV_ROWS, GqError, check, lib
+from ._lib import DESC_WORDS, MAX_GEMV_ROWS, GqError, check, lib, native
 
 TILE_TYPES = F.SUPPORTED_TYPES   # every supported type is held tile-major (the reference: GLUON_TILE_TYPES)
 GEMV_MAX_ROWS = MAX_GEMV_ROWS    # the grouped kernel's own limit (the C ABI accepts up to 64 rows)
@@ -40,10 +40,18 @@ def _i64_array(vals: Sequence[int]):
     return (ctypes.c_int64 * len(vals))(*[int(v) for v in vals])
 
 
+_SM_COUNT: dict[int, int] = {}
+
+
 def sm_count(device=None) -> int:
-    if torch.cuda.is_available():
-        return torch.cuda.get_device_properties(device if device is not None else torch.cuda.current_device()).multi_processor_count
-    return 148
+    if not torch.cuda.is_available():
+        return 148
+    index = torch.device(device).index if device is not None and not isinstance(device, int) else device
+    if index is None:
+        index = torch.cuda.current_device()
+    if index not in _SM_COUNT:
+        _SM_COUNT[index] = torch.cuda.get_device_properties(index).multi_processor_count
+    return _SM_COUNT[index]
 
 
 # ---- host-only helpers (usable without a GPU) -----------------------------------------------------
@@ -79,8 +87,14 @@ def grouped_split_for(n_tiles: int, nb: int, m: int | None = None, block_bytes: 
     return int(lib().gq_split_for(int(n_tiles), int(nb), int(m or 0), int(block_bytes or 0), int(sms or sm_count())))
 
 
+_RUN_INFO: dict[tuple[int, ...], int] = {}      # bounded by the combinations of types a model's merged layers have
+
+
 def run_info(wtypes: Sequence[int]) -> int:
-    return check(lib().gq_run_info(len(wtypes), _i32_array(wtypes)), "gq_run_info")
+    key = tuple(wtypes)
+    if key not in _RUN_INFO:
+        _RUN_INFO[key] = check(lib().gq_run_info(len(key), _i32_array(key)), "gq_run_info")
+    return _RUN_INFO[key]
 
 
 def device_status(device=None, clear: bool = True) -> int:
@@ -391,6 +405,40 @@ def mul_mat_tiles_grouped(x: torch.Tensor, packed: torch.Tensor, descs: list[tor
         return out
     prefill_gemm(x, packed, descs[desc_splits.index(1)], n_total, out=out, wtypes=weight_types)
     return out
+
+
+# ---- native call path ------------------------------------------------------------------------------
+
+class NativeRun:
+    """A packed run's calls without the torch dispatcher and ctypes (csrc/gq_torch.cpp): the same entry points of the C ABI,
+    chosen by the same rules.  Answers None for a call it does not take; the caller then goes through
+    mul_mat_tiles_grouped.  Copies and pickles of the layer that holds one start without it."""
+    __slots__ = ("group", "_run")
+
+    def __init__(self, group=None, n_outs=(), wtypes=()):
+        self.group, self._run = group, None
+        if group is None:
+            return
+        packed, descs, splits, _, nb, block_bytes = group
+        n_tiles = sum(-(-int(n) // 64) for n in n_outs)
+        split = grouped_split_for(n_tiles, nb, block_bytes=block_bytes, sms=sm_count(packed.device))      # the same for every row count
+        self._run = native().Run(packed, descs, splits, [int(n) for n in n_outs], [int(t) for t in wtypes], nb, [split] * (DECODE_MAX_ROWS + 1),
+                                 DECODE_MAX_ROWS, PRE_MAX_ROWS)
+
+    def __reduce__(self):
+        return NativeRun, ()
+
+    def __call__(self, groups, x: torch.Tensor, pre) -> torch.Tensor | None:
+        if self._run is None or _FUSED_AR is not None or _NEXT_WEIGHTS or torch.compiler.is_compiling() or len(groups) != 1:
+            return None
+        for group in groups.values():
+            if group is not self.group:
+                return None
+        if pre is None:
+            return self._run.forward(x)
+        if pre.kind == 1:
+            return self._run.forward_silu_mul(x)
+        return self._run.forward_add_rms_norm(x, pre.weight, pre.residual, pre.residual_out, pre.eps)
 
 
 # ---- torch custom op (traceable boundary) ----------------------------------------------------------
