@@ -7,6 +7,7 @@
 #include <atomic>
 #include <mutex>
 #include <unordered_map>
+#include <vector>
 #include "../../include/gq_b200.h"
 #include "gq_decode.cuh"
 #include "gq_decode8.cuh"
@@ -61,33 +62,9 @@ extern "C" int gq_slab_map(int type, int32_t *map) {
 }
 
 // ---------------------------------------------------------------------------------------------------
-// repack / un-repack: one CTA per (16-row slab, k-block); the slab's raw image goes through shared memory
+// un-repack: one CTA per (16-row slab, k-block); the slab's raw image goes through shared memory
 // ---------------------------------------------------------------------------------------------------
 #define GQ_MAX_SLAB (16 * 272)
-
-__global__ void __launch_bounds__(256) repack_kernel(int type, int B, const uint8_t *__restrict__ raw, int64_t n_out, int nb,
-                                                     int64_t row_stride, uint8_t *__restrict__ out) {
-    __shared__ __align__(16) uint8_t img[GQ_MAX_SLAB];
-    const int slab = blockIdx.x, kb = blockIdx.y;
-    const int64_t row0 = (int64_t)slab * 16;
-    for (int i = threadIdx.x; i < 16 * B; i += 256) {
-        const int r = i / B, b = i - r * B;
-        img[i] = (row0 + r < n_out) ? raw[(row0 + r) * row_stride + (int64_t)kb * B + b] : (uint8_t)0;
-    }
-    __syncthreads();
-    // packed address: tile = slab / 4, slab-in-tile = slab % 4
-    uint8_t *dst = out + (((int64_t)(slab >> 2) * nb + kb) * 4 + (slab & 3)) * (int64_t)(16 * B);
-    for (int w = threadIdx.x; w < 4 * B; w += 256) {
-        uint32_t v = 0;
-#pragma unroll
-        for (int z = 0; z < 4; ++z) {
-            int row, byte;
-            gq_slab_src(type, 4 * w + z, &row, &byte);
-            v |= (uint32_t)img[row * B + byte] << (8 * z);
-        }
-        reinterpret_cast<uint32_t *>(dst)[w] = v;
-    }
-}
 
 // fills img[16][B] (raw order) from a packed slab
 __device__ __forceinline__ void slab_to_raw_image(int type, int B, const uint8_t *__restrict__ src, uint8_t *img) {
@@ -116,10 +93,6 @@ __global__ void __launch_bounds__(256) unrepack_kernel(int type, int B, const ui
     }
 }
 
-// ---------------------------------------------------------------------------------------------------
-// bit-exact dequantiser (fp32 in the format reference's operation order: (d*sc) first, then *q, then -(dmin*m);
-// explicit round-to-nearest multiplies and subtracts so nothing is fused)
-// ---------------------------------------------------------------------------------------------------
 // The codebook grids live in global memory, not in constant memory: the kernels copy them into shared memory with one
 // index per thread, which the constant cache would serve one address at a time.
 __device__ uint32_t c_iq3s_grid[512];
@@ -139,110 +112,8 @@ __device__ __forceinline__ void report_status(int *status, int code) {
 // time limit of the waits on data from another GPU (the fused and the separate all-reduce), nanoseconds
 static std::atomic<unsigned long long> g_peer_wait_ns{GQ_WAIT_LIMIT_NS};
 
+#include "gq_load.cuh"
 #include "gq_prefill.cuh"
-
-__device__ __forceinline__ float h2f(const uint8_t *p) { return __half2float(__ushort_as_half((unsigned short)(p[0] | (p[1] << 8)))); }
-
-__device__ __forceinline__ void scale_min_k4(const uint8_t *s, int j, int &sc, int &mn) {
-    if (j < 4) { sc = s[j] & 63; mn = s[j + 4] & 63; }
-    else { sc = (s[j + 4] & 0xF) | ((s[j - 4] >> 6) << 4); mn = (s[j + 4] >> 4) | ((s[j] >> 6) << 4); }
-}
-
-// weight w (0..255) of the raw 256-weight segment b
-__device__ float deq_one(int type, const uint8_t *b, int w) {
-    switch (type) {
-        case GQ_Q4_0: { const uint8_t *k = b + 18 * (w >> 5); const int j = w & 31;
-            const int q = (j < 16 ? (k[2 + j] & 0xF) : (k[2 + j - 16] >> 4)) - 8; return __fmul_rn(h2f(k), (float)q); }
-        case GQ_IQ4_NL: { const uint8_t *k = b + 18 * (w >> 5); const int j = w & 31;
-            const int q = c_iq4_kvalues[j < 16 ? (k[2 + j] & 0xF) : (k[2 + j - 16] >> 4)]; return __fmul_rn(h2f(k), (float)q); }
-        case GQ_Q5_0: { const uint8_t *k = b + 22 * (w >> 5); const int j = w & 31;
-            const uint32_t qh = k[2] | (k[3] << 8) | (k[4] << 16) | ((uint32_t)k[5] << 24);
-            const int lo = j < 16 ? (k[6 + j] & 0xF) : (k[6 + j - 16] >> 4);
-            const int q = (lo | (((qh >> j) & 1) << 4)) - 16; return __fmul_rn(h2f(k), (float)q); }
-        case GQ_Q8_0: { const uint8_t *k = b + 34 * (w >> 5); return __fmul_rn((float)(int8_t)k[2 + (w & 31)], h2f(k)); }
-        case GQ_Q2_K: { const int n = w >> 7, t = (w >> 5) & 3, l = w & 31, g = w >> 4;
-            const float dl = __fmul_rn(h2f(b + 80), (float)(b[g] & 0xF)), ml = __fmul_rn(h2f(b + 82), (float)(b[g] >> 4));
-            const int q = (b[16 + 32 * n + l] >> (2 * t)) & 3; return __fsub_rn(__fmul_rn(dl, (float)q), ml); }
-        case GQ_Q3_K: { const int nn = w >> 7, j = (w >> 5) & 3, l = w & 31, i = w >> 4; const uint8_t *s = b + 96;
-            const int lo = (s[i % 8] >> (4 * (i / 8))) & 0xF, hi = (s[8 + i % 4] >> (2 * (i / 4))) & 3;
-            const float dl = __fmul_rn(h2f(b + 108), (float)((lo | (hi << 4)) - 32));
-            const int q = (int)((b[32 + 32 * nn + l] >> (2 * j)) & 3) - (((b[l] >> (4 * nn + j)) & 1) ? 0 : 4);
-            return __fmul_rn(dl, (float)q); }
-        case GQ_Q4_K: { const int ib = w >> 5, p = w & 31; int sc, mn; scale_min_k4(b + 4, ib, sc, mn);
-            const float dl = __fmul_rn(h2f(b), (float)sc), dm = __fmul_rn(h2f(b + 2), (float)mn);
-            const int q = (b[16 + 32 * (ib >> 1) + p] >> (4 * (ib & 1))) & 0xF; return __fsub_rn(__fmul_rn(dl, (float)q), dm); }
-        case GQ_Q5_K: { const int ib = w >> 5, p = w & 31; int sc, mn; scale_min_k4(b + 4, ib, sc, mn);
-            const float dl = __fmul_rn(h2f(b), (float)sc), dm = __fmul_rn(h2f(b + 2), (float)mn);
-            const int q = ((b[48 + 32 * (ib >> 1) + p] >> (4 * (ib & 1))) & 0xF) | (((b[16 + p] >> ib) & 1) << 4);
-            return __fsub_rn(__fmul_rn(dl, (float)q), dm); }
-        case GQ_Q6_K: { const int h = w >> 7, t = (w >> 5) & 3, p = w & 31;
-            const int q = (int)(((b[64 * h + 32 * (t & 1) + p] >> (4 * (t >> 1))) & 0xF) | (((b[128 + 32 * h + p] >> (2 * t)) & 3) << 4)) - 32;
-            const float dl = __fmul_rn(h2f(b + 208), (float)(int8_t)b[192 + (w >> 4)]); return __fmul_rn(dl, (float)q); }
-        case GQ_IQ3_S: { const int ib = w >> 5, j = w & 31, k = j >> 2, e = j & 3;
-            const int s = (b[106 + (ib >> 1)] >> (4 * (ib & 1))) & 0xF; const float db = __fmul_rn(h2f(b), (float)(1 + 2 * s));
-            const int idx = b[2 + 8 * ib + k] | (((b[66 + ib] >> k) & 1) << 8);
-            const float mag = (float)((c_iq3s_grid[idx] >> (8 * e)) & 0xFF);
-            const float v = __fmul_rn(db, mag); return ((b[74 + 4 * ib + (j >> 3)] >> (j & 7)) & 1) ? -v : v; }
-        case GQ_IQ3_XXS: { const int ib = w >> 5, j = w & 31; const uint8_t *q = b + 66 + 4 * ib;
-            const uint32_t sw = q[0] | (q[1] << 8) | (q[2] << 16) | ((uint32_t)q[3] << 24);
-            const float db = __fmul_rn(__fmul_rn(h2f(b), 0.5f + (float)(sw >> 28)), 0.5f);
-            const uint32_t f = (sw >> (7 * (j >> 3))) & 0x7Fu, mask = f | (((uint32_t)__popc(f) & 1u) << 7);
-            const float mag = (float)((c_iq3xxs_grid[b[2 + 8 * ib + (j >> 2)]] >> (8 * (j & 3))) & 0xFF);
-            const float v = __fmul_rn(db, mag); return ((mask >> (j & 7)) & 1) ? -v : v; }
-        case GQ_IQ2_XXS: { const int ib = w >> 5, j = w & 31, l = j >> 3; const uint8_t *q = b + 2 + 8 * ib;
-            const uint32_t sw = q[4] | (q[5] << 8) | (q[6] << 16) | ((uint32_t)q[7] << 24);
-            const float db = __fmul_rn(__fmul_rn(h2f(b), 0.5f + (float)(sw >> 28)), 0.25f);
-            const uint32_t f = (sw >> (7 * l)) & 0x7Fu, mask = f | (((uint32_t)__popc(f) & 1u) << 7);
-            const float mag = (float)((c_iq2xxs_grid[2 * q[l] + ((j >> 2) & 1)] >> (8 * (j & 3))) & 0xFF);
-            const float v = __fmul_rn(db, mag); return ((mask >> (j & 7)) & 1) ? -v : v; }
-        case GQ_IQ2_XS: { const int g = w >> 3, j = w & 7; const uint32_t hw = b[2 + 2 * g] | (b[3 + 2 * g] << 8);
-            const int sc = (b[66 + (g >> 2)] >> (4 * ((g >> 1) & 1))) & 0xF;
-            const float db = __fmul_rn(__fmul_rn(h2f(b), 0.5f + (float)sc), 0.25f);
-            const uint32_t f = hw >> 9, mask = f | (((uint32_t)__popc(f) & 1u) << 7);
-            const float mag = (float)((c_iq2xs_grid[2 * (hw & 511u) + (j >> 2)] >> (8 * (j & 3))) & 0xFF);
-            const float v = __fmul_rn(db, mag); return ((mask >> j) & 1) ? -v : v; }
-        case GQ_IQ2_S: { const int g = w >> 3, j = w & 7;
-            const uint32_t idx = b[2 + g] | (((uint32_t)(b[66 + (g >> 2)] >> (2 * (g & 3))) & 3u) << 8);
-            const int sc = (b[74 + (g >> 2)] >> (4 * ((g >> 1) & 1))) & 0xF;
-            const float db = __fmul_rn(__fmul_rn(h2f(b), 0.5f + (float)sc), 0.25f);
-            const float mag = (float)((c_iq2s_grid[2 * idx + (j >> 2)] >> (8 * (j & 3))) & 0xFF);
-            const float v = __fmul_rn(db, mag); return ((b[34 + g] >> j) & 1) ? -v : v; }
-        case GQ_IQ1_M: { const int g = w >> 3, j = w & 7;
-            const uint32_t s0 = b[48] | (b[49] << 8), s1 = b[50] | (b[51] << 8), s2 = b[52] | (b[53] << 8), s3 = b[54] | (b[55] << 8);
-            const uint32_t dv = (s0 >> 12) | ((s1 >> 8) & 0xF0u) | ((s2 >> 4) & 0xF00u) | (s3 & 0xF000u);
-            const float d = __half2float(__ushort_as_half((unsigned short)dv));
-            const uint32_t nib = (b[32 + (g >> 1)] >> (4 * (g & 1))) & 0xFu, idx = b[g] | ((nib & 7u) << 8);
-            const uint32_t sw = (g >> 3) == 0 ? s0 : (g >> 3) == 1 ? s1 : (g >> 3) == 2 ? s2 : s3;
-            const float dl = __fmul_rn(d, (float)(2 * ((sw >> (3 * ((g >> 1) & 3))) & 7u) + 1));
-            const int byte = (int)((c_iq1_grid[2 * idx + (j >> 2)] >> (8 * (j & 3))) & 0xFF);
-            const float gv = (float)(byte - 16) * 0.125f;
-            return __fmul_rn(dl, gv + ((nib & 8u) ? -0.125f : 0.125f)); }
-        case GQ_IQ4_XS: { const int ib = w >> 5, j = w & 31; const uint32_t sh = b[2] | (b[3] << 8);
-            const int ls = (int)(((b[4 + (ib >> 1)] >> (4 * (ib & 1))) & 0xF) | (((sh >> (2 * ib)) & 3) << 4)) - 32;
-            const float dl = __fmul_rn(h2f(b), (float)ls);
-            const int q = c_iq4_kvalues[j < 16 ? (b[8 + 16 * ib + j] & 0xF) : (b[8 + 16 * ib + j - 16] >> 4)];
-            return __fmul_rn(dl, (float)q); }
-    }
-    return 0.0f;
-}
-
-__global__ void __launch_bounds__(256) dequant_kernel(int type, int B, const uint8_t *__restrict__ tiles, int64_t n_out, int nb,
-                                                      void *__restrict__ out, int out_dtype, int64_t ld) {
-    __shared__ __align__(16) uint8_t img[GQ_MAX_SLAB];
-    const int slab = blockIdx.x, kb = blockIdx.y;
-    const uint8_t *src = tiles + (((int64_t)(slab >> 2) * nb + kb) * 4 + (slab & 3)) * (int64_t)(16 * B);
-    slab_to_raw_image(type, B, src, img);
-    __syncthreads();
-    const int64_t row0 = (int64_t)slab * 16;
-    for (int i = threadIdx.x; i < 16 * 256; i += 256) {
-        const int r = i >> 8, w = i & 255;
-        if (row0 + r >= n_out) continue;
-        const float v = deq_one(type, img + r * B, w);
-        const int64_t o = (row0 + r) * ld + (int64_t)kb * 256 + w;
-        if (out_dtype == 0) reinterpret_cast<float *>(out)[o] = v;
-        else reinterpret_cast<__nv_bfloat16 *>(out)[o] = __float2bfloat16_rn(v);
-    }
-}
 
 // ---------------------------------------------------------------------------------------------------
 // activation preparation: bf16 row -> fp16 row scaled by a power of two (so any bf16 magnitude fits fp16
@@ -1298,6 +1169,34 @@ static int ensure_tables() {
     return GQ_OK;
 }
 
+static int device_sms() {
+    static std::atomic<int> cached[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    int v = cached[dev].load();
+    if (v <= 0) {
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
+        cached[dev].store(v);
+    }
+    return v;
+}
+
+// opts a kernel in, once per device, to the dynamic shared memory it is launched with (more than 48 KB needs it)
+template <auto KERNEL>
+static int allow_smem(int bytes) {
+    if (bytes <= 48 * 1024) return GQ_OK;
+    static std::atomic<unsigned long long> done_mask{0};
+    int dev = 0;
+    GQ_CUDA(cudaGetDevice(&dev));
+    if (dev < 64 && ((done_mask.load() >> dev) & 1ull)) return GQ_OK;
+    GQ_CUDA(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    if (dev < 64) done_mask.fetch_or(1ull << dev);
+    return GQ_OK;
+}
+#define GQ_EACH_TYPE(X)                                                                                                     \
+    X(GQ_Q4_0) X(GQ_Q5_0) X(GQ_Q8_0) X(GQ_Q2_K) X(GQ_Q3_K) X(GQ_Q4_K) X(GQ_Q5_K) X(GQ_Q6_K) X(GQ_IQ4_NL) X(GQ_IQ3_S) X(GQ_IQ4_XS) \
+    X(GQ_IQ3_XXS) X(GQ_IQ2_XXS) X(GQ_IQ2_XS) X(GQ_IQ2_S) X(GQ_IQ1_M)
+
 static int check_tensor_args(int type, int64_t n_out, int64_t K) {
     if (!gq_type_bytes(type)) return GQ_ERR_TYPE;
     if (n_out < 0 || K <= 0 || K % GQ_QK || K / GQ_QK > 65535) return GQ_ERR_SHAPE;
@@ -1312,8 +1211,15 @@ extern "C" int gq_repack(int type, const void *raw_dev, int64_t n_out, int64_t K
     if (!raw_dev || !out_dev || ((uintptr_t)out_dev & 15) || raw_row_stride < (int64_t)nb * B) return GQ_ERR_ARG;
     const int64_t slabs = ((n_out + 63) / 64) * 4;
     if (slabs > 0x7fffffff) return GQ_ERR_LIMIT;
-    repack_kernel<<<dim3((unsigned)slabs, (unsigned)nb), 256, 0, (cudaStream_t)stream>>>(type, B, (const uint8_t *)raw_dev, n_out, nb,
-                                                                                     raw_row_stride, (uint8_t *)out_dev);
+    switch (type) {
+#define GQ_ONE(T) case T: {                                                                                                        \
+            if (int rc = allow_smem<repack_kernel<T>>(16 * stage_pitch(repack_kc<T>() * gq_type_bytes(T)))) return rc;                \
+            repack_kernel<T><<<dim3((unsigned)slabs, (unsigned)((nb + repack_kc<T>() - 1) / repack_kc<T>())), GQ_LOAD_THREADS,        \
+                               16 * stage_pitch(repack_kc<T>() * gq_type_bytes(T)), (cudaStream_t)stream>>>(                         \
+                (const uint8_t *)raw_dev, n_out, nb, raw_row_stride, (uint8_t *)out_dev); break; }
+        GQ_EACH_TYPE(GQ_ONE)
+#undef GQ_ONE
+    }
     GQ_LAUNCHED();
     return GQ_OK;
 }
@@ -1341,8 +1247,49 @@ extern "C" int gq_dequant(int type, const void *tiles_dev, int64_t n_out, int64_
     if (int rc = ensure_tables()) return rc;
     const int64_t slabs = ((n_out + 63) / 64) * 4;
     if (slabs > 0x7fffffff) return GQ_ERR_LIMIT;
-    dequant_kernel<<<dim3((unsigned)slabs, (unsigned)nb), 256, 0, (cudaStream_t)stream>>>(type, B, (const uint8_t *)tiles_dev, n_out, nb, out_dev,
-                                                                                      out_dtype, ld);
+    // a CTA walks as many of its slab's k-blocks as leave about six CTAs per SM: the codebook table it fills is then shared
+    // by up to a whole row of k-blocks
+    const int groups = (nb + GQ_LOAD_WARPS - 1) / GQ_LOAD_WARPS;
+    int64_t parts = (6 * (int64_t)device_sms() + slabs - 1) / slabs;
+    if (parts > groups) parts = groups;
+    const int kc = (int)((groups + parts - 1) / parts) * GQ_LOAD_WARPS;
+    const dim3 grid((unsigned)slabs, (unsigned)((nb + kc - 1) / kc));
+    switch (type) {
+#define GQ_ONE_DT(T, BF) {                                                                                                          \
+            if (int rc = allow_smem<dequant_kernel<T, BF>>(dequant_smem<T, BF>())) return rc;                                        \
+            dequant_kernel<T, BF><<<grid, GQ_LOAD_THREADS, dequant_smem<T, BF>(), (cudaStream_t)stream>>>((const uint8_t *)tiles_dev, \
+                                                                                                        n_out, nb, kc, out_dev, ld); }
+#define GQ_ONE(T) case T: if (out_dtype == 0) GQ_ONE_DT(T, false) else GQ_ONE_DT(T, true) break;
+        GQ_EACH_TYPE(GQ_ONE)
+#undef GQ_ONE
+#undef GQ_ONE_DT
+    }
+    GQ_LAUNCHED();
+    return GQ_OK;
+}
+
+extern "C" int gq_dequant_rows(int type, const void *raw_dev, int64_t n_rows, int64_t K, int64_t raw_row_stride, const void *ids_dev, int ids_bytes,
+                               int64_t n_ids, void *out_dev, int out_dtype, int64_t ld, void *stream) {
+    if (int rc = check_tensor_args(type, n_rows, K)) return rc;
+    const int B = gq_type_bytes(type);
+    const int nb = (int)(K / GQ_QK);
+    if (n_ids < 0) return GQ_ERR_SHAPE;
+    if (n_ids == 0) return GQ_OK;
+    if (!raw_dev || !ids_dev || !out_dev || raw_row_stride < (int64_t)nb * B || ld < K || (out_dtype != 0 && out_dtype != 1) ||
+        (ids_bytes != 4 && ids_bytes != 8)) return GQ_ERR_ARG;
+    if ((n_ids + 15) / 16 > 0x7fffffff) return GQ_ERR_LIMIT;
+    if (int rc = ensure_tables()) return rc;
+    const dim3 grid((unsigned)((n_ids + 15) / 16), (unsigned)((nb + GQ_LOAD_WARPS - 1) / GQ_LOAD_WARPS));
+    switch (type) {
+#define GQ_ONE_DT(T, BF) {                                                                                                          \
+            if (int rc = allow_smem<dequant_rows_kernel<T, BF>>(dequant_rows_smem<T>())) return rc;                                  \
+            dequant_rows_kernel<T, BF><<<grid, GQ_LOAD_THREADS, dequant_rows_smem<T>(), (cudaStream_t)stream>>>(                     \
+                (const uint8_t *)raw_dev, n_rows, nb, raw_row_stride, ids_dev, ids_bytes == 8, n_ids, out_dev, ld); }
+#define GQ_ONE(T) case T: if (out_dtype == 0) GQ_ONE_DT(T, false) else GQ_ONE_DT(T, true) break;
+        GQ_EACH_TYPE(GQ_ONE)
+#undef GQ_ONE
+#undef GQ_ONE_DT
+    }
     GQ_LAUNCHED();
     return GQ_OK;
 }
@@ -1354,36 +1301,82 @@ extern "C" int64_t gq_desc_rows(int n_shards, const int64_t *n_outs, int split) 
     return tiles * split;
 }
 
-extern "C" int64_t gq_build_descs(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split, int32_t *desc_host) {
-    if (n_shards <= 0 || !types || !n_outs || !desc_host) return GQ_ERR_ARG;
+// One row of the table, computed from its index alone (host and device).  first_tile / base16 / col0 are the shard's.
+struct DescShard {
+    int type, n_tiles, n_out, col0, base16;
+};
+__host__ __device__ inline void desc_row(const DescShard &s, int64_t nb, int split, int tile, int part, int32_t *r) {
+    r[0] = (int32_t)(s.base16 + (int64_t)tile * nb * 4 * gq_type_bytes(s.type));       // 64 * bytes / 16
+    r[1] = s.type;
+    r[2] = s.col0 + tile * 64;
+    r[3] = s.n_out - tile * 64 < 64 ? s.n_out - tile * 64 : 64;
+    r[4] = (int32_t)((part * nb) / split);
+    r[5] = (int32_t)(((part + 1) * nb) / split);
+    r[6] = part;
+    r[7] = 0;
+}
+// the shards of a run back to back, checked against what a row's 32-bit fields can hold; returns the number of rows
+static int64_t desc_shards(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split, DescShard *out) {
+    if (n_shards <= 0 || !types || !n_outs) return GQ_ERR_ARG;
     if (K <= 0 || K % GQ_QK) return GQ_ERR_SHAPE;
     const int64_t nb = K / GQ_QK;
     if (split < 1 || split > nb) return GQ_ERR_ARG;
-    int64_t base = 0, col0 = 0, row = 0;
+    int64_t base16 = 0, col0 = 0, rows = 0;
     for (int i = 0; i < n_shards; ++i) {
         const int B = gq_type_bytes(types[i]);
         if (!B) return GQ_ERR_TYPE;
         if (n_outs[i] < 0) return GQ_ERR_SHAPE;
-        const int64_t n_tiles = (n_outs[i] + 63) / 64, tile_kb_bytes = 64 * (int64_t)B;
-        for (int64_t ti = 0; ti < n_tiles; ++ti)
-            for (int s = 0; s < split; ++s) {
-                const int64_t o = base + ti * nb * tile_kb_bytes;
-                if ((o >> 4) > 0x7fffffff || col0 + ti * 64 > 0x7fffffff) return GQ_ERR_LIMIT;
-                int32_t *r = desc_host + row * GQ_DESC_WORDS;
-                r[0] = (int32_t)(o >> 4);
-                r[1] = types[i];
-                r[2] = (int32_t)(col0 + ti * 64);
-                r[3] = (int32_t)(n_outs[i] - ti * 64 < 64 ? n_outs[i] - ti * 64 : 64);
-                r[4] = (int32_t)((s * nb) / split);
-                r[5] = (int32_t)(((s + 1) * nb) / split);
-                r[6] = s;
-                r[7] = 0;
-                ++row;
-            }
-        base += n_tiles * nb * tile_kb_bytes;
+        const int64_t n_tiles = (n_outs[i] + 63) / 64;
+        // the largest values are those of the shard's last tile; an empty shard writes none
+        if (n_tiles && (base16 + (n_tiles - 1) * nb * 4 * B > 0x7fffffff || col0 + (n_tiles - 1) * 64 > 0x7fffffff)) return GQ_ERR_LIMIT;
+        if (n_tiles) out[i] = {types[i], (int)n_tiles, (int)n_outs[i], (int)col0, (int)base16};
+        else out[i] = {types[i], 0, 0, 0, 0};
+        base16 += n_tiles * nb * 4 * B;
         col0 += n_outs[i];
+        rows += n_tiles * split;
     }
-    return row;
+    return rows;
+}
+
+extern "C" int64_t gq_build_descs(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split, int32_t *desc_host) {
+    if (n_shards <= 0 || !desc_host) return GQ_ERR_ARG;
+    std::vector<DescShard> sh((size_t)n_shards);
+    const int64_t rows = desc_shards(n_shards, types, n_outs, K, split, sh.data());
+    if (rows < 0) return rows;
+    for (const DescShard &s : sh)
+        for (int t = 0; t < s.n_tiles; ++t)
+            for (int p = 0; p < split; ++p, desc_host += GQ_DESC_WORDS) desc_row(s, K / GQ_QK, split, t, p, desc_host);
+    return rows;
+}
+
+struct DescShards {
+    DescShard s[GQ_MAX_DEVICE_SHARDS];
+    int n;
+};
+__global__ void __launch_bounds__(256) build_descs_kernel(const DescShards sh, int nb, int split, int rows, int32_t *__restrict__ desc) {
+    const int row = blockIdx.x * 256 + threadIdx.x;
+    if (row >= rows) return;
+    int tile = row / split, i = 0;
+    while (i + 1 < sh.n && tile >= sh.s[i].n_tiles) tile -= sh.s[i++].n_tiles;
+    __align__(16) int32_t r[GQ_DESC_WORDS];
+    desc_row(sh.s[i], nb, split, tile, row % split, r);
+    int4 *o = reinterpret_cast<int4 *>(desc + (int64_t)row * GQ_DESC_WORDS);
+    o[0] = make_int4(r[0], r[1], r[2], r[3]);
+    o[1] = make_int4(r[4], r[5], r[6], r[7]);
+}
+
+extern "C" int64_t gq_build_descs_device(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split, int32_t *desc_dev,
+                                         void *stream) {
+    if (n_shards > GQ_MAX_DEVICE_SHARDS) return GQ_ERR_LIMIT;
+    if (!desc_dev || ((uintptr_t)desc_dev & 15)) return GQ_ERR_ARG;
+    DescShards sh;
+    const int64_t rows = desc_shards(n_shards, types, n_outs, K, split, sh.s);
+    if (rows <= 0) return rows;
+    if (rows > 0x7ffffff0) return GQ_ERR_LIMIT;
+    sh.n = n_shards;
+    build_descs_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, (cudaStream_t)stream>>>(sh, (int)(K / GQ_QK), split, (int)rows, desc_dev);
+    GQ_LAUNCHED();
+    return rows;
 }
 
 extern "C" int gq_split_for(int64_t n_tiles, int64_t nb, int64_t M, int avg_bytes_per_256, int sm_count) {
@@ -1845,18 +1838,6 @@ static int prefill_split(int64_t n_desc, int64_t M, int64_t nb, int nbt, int sms
         if (cost < best_cost - 1e-9) { best_cost = cost; best = S; }
     }
     return best;
-}
-
-static int device_sms() {
-    static std::atomic<int> cached[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    int v = cached[dev].load();
-    if (v <= 0) {
-        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
-        cached[dev].store(v);
-    }
-    return v;
 }
 
 static int64_t pf_ws_layout(int64_t M, int64_t K, int nbt, int split, int64_t n_total, void *base, int **status, float **ex, uint8_t **xp,

@@ -33,7 +33,7 @@ enum GqType {
 #endif
 
 // bytes of one row's 256-weight segment (0: unsupported type)
-GQ_HD inline int gq_type_bytes(int type) {
+GQ_HD constexpr int gq_type_bytes(int type) {
     switch (type) {
         case GQ_Q4_0: return 144;
         case GQ_Q5_0: return 176;
@@ -56,7 +56,7 @@ GQ_HD inline int gq_type_bytes(int type) {
 }
 
 // number of 512-byte lane-ordered chunks at the head of a slab
-GQ_HD inline int gq_type_chunks(int type) {
+GQ_HD constexpr int gq_type_chunks(int type) {
     switch (type) {
         case GQ_Q4_0: case GQ_IQ4_NL: case GQ_Q4_K: case GQ_IQ4_XS: case GQ_Q5_0: return 4;
         case GQ_Q5_K: return 5;
@@ -71,7 +71,7 @@ GQ_HD inline int gq_type_chunks(int type) {
 
 // Codebook types keep a table of grid entries in shared memory while a kernel decodes them.  Kind index of a type
 // (-1: not a codebook type), and the table's bytes in the integer form (form 1: magnitudes as bytes) and in the fp16 form (form 0).
-GQ_HD inline int gq_cb_kind(int type) {
+GQ_HD constexpr int gq_cb_kind(int type) {
     switch (type) {
         case GQ_IQ3_S: return 0;
         case GQ_IQ3_XXS: return 1;
@@ -83,7 +83,7 @@ GQ_HD inline int gq_cb_kind(int type) {
     }
 }
 #define GQ_CB_KINDS 6
-GQ_HD inline int gq_cb_bytes(int kind, int form) {
+GQ_HD constexpr int gq_cb_bytes(int kind, int form) {
     switch (kind) {
         case 0: return form ? 2048 : 4096;     // IQ3_S: 512 entries of 4 bytes / of two fp16 pairs
         case 1: return form ? 1024 : 2048;     // IQ3_XXS: 256 entries of 4 bytes / of two fp16 pairs

@@ -149,10 +149,33 @@ class Run {
     int device_, info_ = 0, one_ = 0;
 };
 
+// rows `ids` of a raw table -> weights; None: not the plain case
+PyObject *dequantize_rows(py::handle rawh, int64_t type, py::handle idsh, bool bf16) {
+    if (!THPVariable_CheckExact(rawh.ptr()) || !THPVariable_CheckExact(idsh.ptr()) || c10::impl::dispatch_mode_enabled()) Py_RETURN_NONE;
+    const at::Tensor &raw = THPVariable_Unpack(rawh.ptr()), &ids = THPVariable_Unpack(idsh.ptr());
+    const int B = gq_bytes_per_256((int)type);
+    if (!raw.is_cuda() || raw.scalar_type() != at::kByte || raw.dim() != 2 || raw.stride(1) != 1 || raw.size(0) == 0 || B == 0 || raw.size(1) == 0 ||
+        raw.size(1) % B || !ids.is_cuda() || ids.get_device() != raw.get_device() || !ids.is_contiguous() || ids.numel() == 0 ||
+        (ids.scalar_type() != at::kLong && ids.scalar_type() != at::kInt)) Py_RETURN_NONE;
+    const int device = raw.get_device();
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+    void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
+    const int64_t K = raw.size(1) / B * 256;
+    at::DimVector sizes(ids.sizes().begin(), ids.sizes().end());
+    sizes.push_back(K);
+    at::Tensor out = at::detail::empty_cuda(sizes, bf16 ? at::kBFloat16 : at::kFloat, raw.device(), c10::nullopt);
+    check(gq_dequant_rows((int)type, raw.data_ptr(), raw.size(0), K, raw.stride(0), ids.data_ptr(), ids.scalar_type() == at::kLong ? 8 : 4, ids.numel(),
+                          out.data_ptr(), bf16 ? 1 : 0, K, stream), "gq_dequant_rows");
+    return THPVariable_Wrap(std::move(out));
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_gq_torch, m) {
     m.def("set_error_type", [](py::object e) { g_error = e.release().ptr(); });
+    m.def("dequantize_rows", [](py::handle raw, int64_t type, py::handle ids, bool bf16) {
+        return py::reinterpret_steal<py::object>(dequantize_rows(raw, type, ids, bf16));
+    });
     py::class_<Run>(m, "Run")
         .def(py::init<at::Tensor, std::vector<at::Tensor>, std::vector<int64_t>, std::vector<int64_t>, std::vector<int64_t>, int64_t, std::vector<int64_t>,
                       int64_t, int64_t>())

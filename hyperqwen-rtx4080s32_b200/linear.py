@@ -210,11 +210,12 @@ class GGUFLinearMethod:
         gguf_tiles / gguf_tiles_rows / gguf_tiles_types keyed by shard id (or "__all__"), the names the plugin reads."""
         if self._is_token_embedding(layer):
             return
-        packed = [(key, ops.repack_tiles(raw, raw.shape[0], wtype), raw.shape[0], wtype, drop)
-                  for key, raw, wtype, drop in self._weight_tensors(layer)
-                  if wtype in ops.TILE_TYPES and raw.numel() > 0]
-        if not packed:
+        weights = [w for w in self._weight_tensors(layer) if w[2] in ops.TILE_TYPES and w[1].numel() > 0]
+        if not weights:
             return
+        tiled = ops.repack_shards([raw for _, raw, _, _ in weights], [wtype for _, _, wtype, _ in weights])
+        packed = [(key, tiles, raw.shape[0], wtype, drop) for (key, raw, wtype, drop), tiles in zip(weights, tiled)]
+        del weights
         for _, _, _, _, drop in packed:
             drop()
         layer.gguf_tiles = {key: tiles for key, tiles, _, _, _ in packed}

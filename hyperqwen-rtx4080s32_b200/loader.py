@@ -153,17 +153,10 @@ def load_gguf(path: str, device="cuda", strict: bool = True) -> LoadedModel:
 
 def embedding_lookup(raw: torch.Tensor, wtype: int, ids: torch.Tensor, dtype=torch.bfloat16) -> torch.Tensor:
     """Rows `ids` of a quantized embedding table raw uint8 [vocab, row_bytes] (kept raw, as the plugin keeps it:
-    gguf-tiles-all-types.patch:80-89) dequantised to [len(ids), K]: the rows are gathered as bytes, repacked and
-    dequantised by the same kernels that serve the weights — bit-identical to gguf.quants.dequantize of those rows."""
+    gguf-tiles-all-types.patch:80-89) dequantised to [*ids.shape, K]: one launch gathers the rows' bytes and decodes
+    them with the decoders that serve the weights — bit-identical to gguf.quants.dequantize of those rows."""
     from . import ops
 
     if int(wtype) not in F.SUPPORTED_TYPES:
         raise ValueError(f"GGML type {wtype} is not a type the kernels decode")
-    k = raw.shape[1] // F.BYTES_PER_256[int(wtype)] * F.QK
-    flat = ids.reshape(-1).to(raw.device)
-    rows = raw.index_select(0, flat)
-    n = int(rows.shape[0])
-    if n == 0:
-        return torch.empty((*ids.shape, k), dtype=dtype, device=raw.device)
-    w = ops.dequantize_tiles(ops.repack_tiles(rows, n, int(wtype)), n, k, int(wtype), dtype=dtype)
-    return w.reshape(*ids.shape, k)
+    return ops.dequantize_rows(raw, int(wtype), ids, dtype=dtype)

@@ -21,6 +21,7 @@ from ._lib import DESC_WORDS, MAX_GEMV_ROWS, GqError, check, lib, native
 
 TILE_TYPES = F.SUPPORTED_TYPES   # every supported type is held tile-major (the reference: GLUON_TILE_TYPES)
 GEMV_MAX_ROWS = MAX_GEMV_ROWS    # the grouped kernel's own limit (the C ABI accepts up to 64 rows)
+MAX_DEVICE_SHARDS = 8            # GQ_MAX_DEVICE_SHARDS
 DECODE_MAX_ROWS = 32             # row-count dispatch threshold: above it the tcgen05 kernel takes over
 
 def _stream_ptr(t: torch.Tensor) -> int:
@@ -82,6 +83,21 @@ def build_descs(wtypes: Sequence[int], n_outs: Sequence[int], k: int, split: int
     return out
 
 
+def build_descs_on(device, wtypes: Sequence[int], n_outs: Sequence[int], k: int, splits: Sequence[int]) -> list[torch.Tensor]:
+    """The descriptor tables of several splits on a device, written there by a kernel (no copy, no synchronisation)."""
+    device = torch.device(device)
+    if device.type != "cuda" or len(wtypes) > MAX_DEVICE_SHARDS:
+        return [torch.from_numpy(build_descs(wtypes, n_outs, k, s)).to(device) for s in splits]
+    types, rows = _i32_array(wtypes), _i64_array(n_outs)
+    tiles = sum(-(-int(n) // 64) for n in n_outs)
+    descs = list(torch.empty((tiles * sum(splits), DESC_WORDS), dtype=torch.int32, device=device).split([tiles * s for s in splits]))
+    with torch.cuda.device(device):
+        for s, d in zip(splits, descs):
+            got = check(lib().gq_build_descs_device(len(wtypes), types, rows, int(k), int(s), d.data_ptr(), _stream_ptr(d)), "gq_build_descs_device")
+            assert got == d.shape[0]
+    return descs
+
+
 def grouped_split_for(n_tiles: int, nb: int, m: int | None = None, block_bytes: int | None = None, sms: int | None = None) -> int:
     """Split-K of a grouped launch (reference: grouped_split_for, gguf-plugin/gluon/tiles_grouped.py:237-250)."""
     return int(lib().gq_split_for(int(n_tiles), int(nb), int(m or 0), int(block_bytes or 0), int(sms or sm_count())))
@@ -112,8 +128,9 @@ def set_peer_wait_limit(seconds: float) -> None:
 
 # ---- load time -----------------------------------------------------------------------------------
 
-def repack_tiles(raw: torch.Tensor, n_out: int, wtype: int) -> torch.Tensor:
-    """raw uint8 [n_out, nb * bytes_per_256] (any row stride) -> tiles uint8 [ceil(n_out/64), nb, 64 * bytes_per_256]."""
+def repack_tiles(raw: torch.Tensor, n_out: int, wtype: int, out: torch.Tensor | None = None) -> torch.Tensor:
+    """raw uint8 [n_out, nb * bytes_per_256] (any row stride) -> tiles uint8 [ceil(n_out/64), nb, 64 * bytes_per_256],
+    written into the flat uint8 buffer `out` of exactly that size if one is given (16-byte aligned)."""
     _need_cuda(raw, "raw")
     if raw.dtype != torch.uint8 or raw.dim() != 2 or raw.shape[0] != n_out:
         raise GqError(f"raw must be uint8 [n_out, row_bytes], got {raw.dtype} {tuple(raw.shape)}")
@@ -122,7 +139,10 @@ def repack_tiles(raw: torch.Tensor, n_out: int, wtype: int) -> torch.Tensor:
         raise GqError(f"row bytes {raw.shape[1]} are not whole {bb}-byte k-blocks of type {wtype}")
     nb = raw.shape[1] // bb
     n_tiles = -(-n_out // 64)
-    out = torch.empty((n_tiles, nb, 64 * bb), dtype=torch.uint8, device=raw.device)
+    if out is None:
+        out = torch.empty((n_tiles, nb, 64 * bb), dtype=torch.uint8, device=raw.device)
+    else:
+        out = out.view(n_tiles, nb, 64 * bb)
     with torch.cuda.device(raw.device):
         check(lib().gq_repack(int(wtype), raw.data_ptr(), n_out, nb * 256, raw.stride(0), out.data_ptr(), _stream_ptr(raw)), "gq_repack")
     return out
@@ -153,6 +173,48 @@ def dequantize_tiles(tiles: torch.Tensor, n_out: int, k: int, wtype: int, dtype=
     return out
 
 
+def repack_shards(raws: Sequence[torch.Tensor], wtypes: Sequence[int]) -> list[torch.Tensor]:
+    """repack_tiles of each shard, the shards' tiles back to back in one buffer: pack_tiles then has nothing to copy."""
+    for raw in raws:
+        _need_cuda(raw, "raw")
+    if len(raws) == 1 or any(r.device != raws[0].device for r in raws):
+        return [repack_tiles(r, r.shape[0], t) for r, t in zip(raws, wtypes)]
+    sizes = [packed_bytes(t, r.shape[0], r.shape[1] // F.BYTES_PER_256[int(t)] * F.QK) for r, t in zip(raws, wtypes)]
+    buf = torch.empty(sum(sizes), dtype=torch.uint8, device=raws[0].device)
+    return [repack_tiles(r, r.shape[0], t, out=o) for r, t, o in zip(raws, wtypes, buf.split(sizes))]
+
+
+def dequantize_rows(raw: torch.Tensor, wtype: int, ids: torch.Tensor, dtype=torch.float32) -> torch.Tensor:
+    """Rows `ids` (int32 or int64, any shape) of a raw uint8 table [rows, row_bytes] -> [*ids.shape, K], in one launch; the
+    values are those of dequantize_tiles.  An id outside the table is reported through device_status."""
+    out = native().dequantize_rows(raw, int(wtype), ids, dtype is torch.bfloat16) if dtype in (torch.float32, torch.bfloat16) else None
+    if out is not None:
+        return out
+    _need_cuda(raw, "raw")
+    if dtype not in (torch.float32, torch.bfloat16):
+        raise GqError("dequantize_rows produces float32 or bfloat16")
+    bb = F.BYTES_PER_256[int(wtype)]
+    if raw.dtype != torch.uint8 or raw.dim() != 2 or raw.shape[1] % bb:
+        raise GqError(f"raw must be uint8 [rows, whole {bb}-byte k-blocks], got {raw.dtype} {tuple(raw.shape)}")
+    k = raw.shape[1] // bb * F.QK
+    rows = raw.index_select(0, ids.reshape(-1).to(raw.device))       # layouts and index types the kernel does not read
+    n = int(rows.shape[0])
+    if n == 0:
+        return torch.empty((*ids.shape, k), dtype=dtype, device=raw.device)
+    return dequantize_tiles(repack_tiles(rows, n, int(wtype)), n, k, int(wtype), dtype=dtype).reshape(*ids.shape, k)
+
+
+def _adjacent(tiles: Sequence[torch.Tensor]) -> bool:
+    """Whether the tensors lie back to back in one storage."""
+    first = tiles[0]
+    at = first.data_ptr()
+    for t in tiles:
+        if not t.is_contiguous() or t.data_ptr() != at or t.untyped_storage().data_ptr() != first.untyped_storage().data_ptr():
+            return False
+        at += t.numel()
+    return True
+
+
 def pack_tiles(shards: Sequence[tuple[torch.Tensor, int, int]]):
     """[(tiles, n_out, type)] -> (packed uint8 buffer, meta): the shards' tiles back to back in one buffer."""
     nb = None
@@ -160,7 +222,13 @@ def pack_tiles(shards: Sequence[tuple[torch.Tensor, int, int]]):
         if t.shape[0] != -(-n_out // 64) or (nb is not None and t.shape[1] != nb):
             raise GqError("shards of a run must share K and hold ceil(n_out/64) tiles")
         nb = int(t.shape[1])
-    packed = shards[0][0].reshape(-1) if len(shards) == 1 else torch.cat([t.reshape(-1) for t, _, _ in shards])
+    tiles = [t for t, _, _ in shards]
+    if len(shards) == 1:
+        packed = tiles[0].reshape(-1)
+    elif _adjacent(tiles):
+        packed = tiles[0].as_strided((sum(t.numel() for t in tiles),), (1,))
+    else:
+        packed = torch.cat([t.reshape(-1) for t in tiles])
     meta = {"nb": nb, "n_outs": [int(n) for _, n, _ in shards], "types": [int(w) for _, _, w in shards],
             "n_total": sum(int(n) for _, n, _ in shards)}
     return packed, meta
@@ -180,8 +248,9 @@ def prepare_grouped_layer(tiles_list: Sequence[torch.Tensor], n_outs: Sequence[i
     n_tiles = sum(-(-int(n) // 64) for n in n_outs)
     block_bytes = int(round(sum(int(n) * F.BYTES_PER_256[int(w)] for n, w in zip(n_outs, wtypes)) / max(1, n_total)))
     sms = sm_count(packed.device)
-    splits = sorted({grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sms) for m in ms} | {1})
-    descs = [torch.from_numpy(build_descs(wtypes, n_outs, nb * 256, s)).to(packed.device) for s in splits]
+    # the library's policy looks at the run's shape only: one question answers every row count
+    splits = sorted({grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sms) for m in list(ms)[:1]} | {1})
+    descs = build_descs_on(packed.device, wtypes, n_outs, nb * 256, splits)
     return packed, views, descs, splits, nb, block_bytes
 
 

@@ -70,6 +70,13 @@ int gq_unrepack(int type, const void *tiles_dev, int64_t n_out, int64_t K, void 
  * (gguf-plugin/gluon/iq3s_tile_dequant.py:22-63). */
 int gq_dequant(int type, const void *tiles_dev, int64_t n_out, int64_t K, void *out_dev, int out_dtype, int64_t ld, void *stream);
 
+/* Rows of a raw (not packed) table -> dequantised weights [n_ids, K], row stride ld elements: the quantized embedding lookup.
+ * raw_dev uint8 [n_rows, raw_row_stride], ids_dev int32 or int64 (ids_bytes 4 or 8); out_dtype as gq_dequant.  An id outside
+ * [0, n_rows) is not read: its output row is unspecified and the device's status word (gq_device_status) becomes 2.
+ * Reference: the plugin keeps the embedding raw and gathers its rows (gguf-plugin/patches/gguf-tiles-all-types.patch:80-89). */
+int gq_dequant_rows(int type, const void *raw_dev, int64_t n_rows, int64_t K, int64_t raw_row_stride, const void *ids_dev, int ids_bytes,
+                    int64_t n_ids, void *out_dev, int out_dtype, int64_t ld, void *stream);
+
 /* Descriptor table of a run of shards that share K and sit back to back in one packed buffer
  * (shard i's tiles start at byte offset sum_{j<i} gq_packed_bytes(j)).  One row of GQ_DESC_WORDS int32
  * per (64-row tile, k-range): {tile byte offset / 16, type, first output column, valid rows, kb0, kb1,
@@ -78,6 +85,11 @@ int gq_dequant(int type, const void *tiles_dev, int64_t n_out, int64_t K, void *
  * Reference: descriptors / prepare_grouped_layer (gguf-plugin/gluon/tiles_grouped.py:253-299). */
 int64_t gq_desc_rows(int n_shards, const int64_t *n_outs, int split);
 int64_t gq_build_descs(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split, int32_t *desc_host);
+
+/* The same table written on the device (desc_dev has room for gq_desc_rows rows, 16-byte aligned) by a kernel on `stream`, so
+ * that loading a layer copies and waits for nothing.  Up to GQ_MAX_DEVICE_SHARDS shards, GQ_ERR_LIMIT beyond. */
+#define GQ_MAX_DEVICE_SHARDS 8
+int64_t gq_build_descs_device(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split, int32_t *desc_dev, void *stream);
 
 /* Split-K of a grouped launch: n_tiles output tiles, nb k-blocks, M batch rows, avg_bytes_per_256 of
  * the run, on a device with sm_count SMs.  Always in [1, nb] and at most 8 (the split then stays inside
