@@ -170,17 +170,6 @@ static int64_t ws_layout(int64_t M, int64_t K, int64_t n_total, int split, void 
 #define GQ_PREP_THREADS 512
 #define GQ_PREP_VECS 5      // 16-byte loads a thread keeps in registers: rows up to 512 * 5 * 8 = 20480 activations are read once
 
-__device__ __forceinline__ float amax8(const uint4 &v) {
-    const __nv_bfloat162 *b = reinterpret_cast<const __nv_bfloat162 *>(&v);
-    float a = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float2 f = __bfloat1622float2(b[j]);
-        a = fmaxf(a, fmaxf(fabsf(f.x), fabsf(f.y)));
-    }
-    return a;
-}
-
 // eight activations (half a 16-weight run) -> fp16 at `scale`, stored into the staged tile; the run's fp32 sum is
 // completed with the neighbouring lane, which holds the other half
 __device__ __forceinline__ void prep_store8(const uint4 &v, int64_t vec, float scale, int M, int m, uint8_t *__restrict__ xt) {
@@ -1818,72 +1807,85 @@ extern "C" int gq_allreduce_push(const void *in_dev, void *out_dev, int64_t n_by
 }
 
 // ---- prefill ----------------------------------------------------------------------------------------
-static int prefill_nb(int64_t M) { return M <= 64 ? 64 : M <= 128 ? 128 : 256; }
+// Dynamic shared memory of a CTA: two CTAs (SETS = 1) or one fill the SM, so that no third user of tensor memory joins them:
+// the CTAs of a cluster wait for one another while they hold theirs.
+#define GQ_PF_SMEM_1 (112 * 1024)
+#define GQ_PF_SMEM_2 (226 * 1024)
 
-// Split-K of a prefill launch: one CTA per (pair of 64-row tiles, NB batch rows) is resident per SM, so a launch of
-// few CTAs (o / down / qkv at a few hundred rows) leaves SMs idle; its k-blocks are then cut into S balanced parts
-// (grid.z), S chosen to minimise waves x (k-blocks per CTA + a fixed cost per wave).  Larger launches keep S = 1.
-static int prefill_split(int64_t n_desc, int64_t M, int64_t nb, int nbt, int sms) {
-    const int64_t ctas = ((n_desc + 1) / 2) * ((M + nbt - 1) / nbt);
+// How a prefill launch is cut: N batch rows per CTA (a multiple of 16, tiles balanced), the cluster split of K, and which of
+// the two kernels (SETS) runs it.
+struct PrefillPlan {
+    int sets, N, tiles, split;
+};
+// SETS = 1 (two CTAs per SM) holds tiles of up to 128 batch rows, SETS = 2 up to 256; a wider batch takes as many equal tiles
+// as it needs, since every further tile decodes the weights again.  K is split while that shortens the launch: a wave costs
+// about six k-blocks of start-up and drain on top of its own, and a CTA keeps at least four k-blocks (at least eight in the
+// run, so short K is never split).
+static PrefillPlan prefill_plan(int64_t n_desc, int64_t M, int64_t nb, int sms) {
+    PrefillPlan p;
     if (sms <= 0) sms = 148;
-    if (nbt <= 64) sms *= 2;       // the 64-row variant is built for two CTAs per SM
-    int best = 1;
-    double best_cost = 1e300;
-    // the fp32 partials cost a write and a read of S x M x n_total x 4 bytes: worth it only while a launch fills less than
-    // half of the GPU (measured: down at 512 rows, 80 CTAs on 148 SMs, gains nothing from a split; at 64 rows it halves)
-    if (ctas * 2 > sms) return 1;
-    for (int S = 1; S <= 8 && (int64_t)S * 4 <= nb; ++S) {
-        const int64_t waves = (ctas * S + sms - 1) / sms;
-        const double cost = (double)waves * ((double)nb / S + 6.0) + (S > 1 ? 2.0 : 0.0);
-        if (cost < best_cost - 1e-9) { best_cost = cost; best = S; }
+    p.tiles = (int)((M + 255) / 256);
+    p.N = (int)(((M + p.tiles - 1) / p.tiles + 15) & ~15);
+    p.sets = p.N <= 128 ? 1 : 2;
+    const int64_t slots = p.sets == 1 ? 2 * (int64_t)sms : sms, ctas = ((n_desc + 1) / 2) * p.tiles;
+    p.split = 1;
+    double best = 1e300;
+    for (int S = 1; S <= 8 && (S == 1 || (int64_t)S * 4 <= nb); ++S) {
+        // clusters leave some slots unused
+        const int64_t usable = slots * (100 - 3 * (S - 1)) / 100;
+        const int64_t waves = (ctas * S + usable - 1) / usable;
+        const double cost = (double)waves * ((double)((nb + S - 1) / S) + 6.0) + (S > 1 ? 2.0 : 0.0);
+        if (cost < best - 1e-9) { best = cost; p.split = S; }
     }
-    return best;
+    return p;
 }
 
-static int64_t pf_ws_layout(int64_t M, int64_t K, int nbt, int split, int64_t n_total, void *base, int **status, float **ex, uint8_t **xp,
-                            float **partials) {
-    const int64_t mt = (M + nbt - 1) / nbt;
+static int64_t pf_ws_layout(int64_t K, const PrefillPlan &pl, void *base, int **status, float **ex, uint8_t **xp) {
+    const int64_t rows = (int64_t)pl.tiles * pl.N;
     int64_t off = 256;
-    const int64_t o_ex = off; off = align256(off + M * 4);
+    const int64_t o_ex = off; off = align256(off + rows * 4);
     off = (off + 1023) & ~(int64_t)1023;
-    const int64_t o_xp = off; off += mt * nbt * K * 2;
-    const int64_t o_p = off; if (split > 1) off = align256(off + (int64_t)split * M * n_total * 4);
-    if (base) { uint8_t *b = (uint8_t *)base; *status = (int *)b; *ex = (float *)(b + o_ex); *xp = b + o_xp; *partials = (float *)(b + o_p); }
+    const int64_t o_xp = off; off += rows * K * 2;
+    if (base) { uint8_t *b = (uint8_t *)base; *status = (int *)b; *ex = (float *)(b + o_ex); *xp = b + o_xp; }
     return off;
 }
 
 extern "C" int64_t gq_prefill_workspace_bytes(int64_t M, int64_t K, int64_t n_total, int64_t n_desc) {
     if (M < 0 || K <= 0 || K % GQ_QK || n_total < 0 || n_desc < 0) return GQ_ERR_SHAPE;
-    const int nbt = prefill_nb(M);
-    return pf_ws_layout(M, K, nbt, prefill_split(n_desc, M, K / GQ_QK, nbt, device_sms()), n_total, nullptr, nullptr, nullptr, nullptr, nullptr);
+    if (M == 0) return 256;
+    return pf_ws_layout(K, prefill_plan(n_desc, M, K / GQ_QK, device_sms()), nullptr, nullptr, nullptr, nullptr);
 }
 
-template <int NB>
-static int launch_prefill(PrefillParams &p, const __nv_bfloat16 *x, int64_t ldx, float *ex, uint8_t *xp, cudaStream_t st) {
-    const int mt = (p.M + NB - 1) / NB;
-    const size_t smem_base = 1024 + (size_t)GQ_PF_STAGES * (GQ_PF_A_BYTES + NB * 128) + 128;
-    // the tables of the run's codebook types sit side by side; the opt-in covers every combination that fits a CTA at all
-    const size_t smem = smem_base + (size_t)gq_cb_region_sum(p.cb_mask);
-    const size_t smem_all = smem_base + (size_t)gq_cb_region_sum(63), smem_max = smem_all < 232448 ? smem_all : 232448;
-    if (smem > smem_max) return GQ_ERR_LIMIT;
-    static std::atomic<unsigned long long> done_mask{0};
-    int dev = 0;
-    GQ_CUDA(cudaGetDevice(&dev));
-    if (dev >= 64 || !((done_mask.load() >> dev) & 1ull)) {
-        GQ_CUDA(cudaFuncSetAttribute(gemm_prefill_kernel<NB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
-        GQ_CUDA(cudaFuncSetAttribute(gemm_prefill_kernel<NB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
-        if (dev < 64) done_mask.fetch_or(1ull << dev);
+template <int SETS>
+static int launch_prefill(PrefillParams &p, const PrefillPlan &pl, int maxb, cudaStream_t st) {
+    const int total = SETS == 1 ? GQ_PF_SMEM_1 : GQ_PF_SMEM_2, tables = gq_cb_region_sum(p.cb_mask), bbytes = pl.N * 128;
+    p.wstage_bytes = 128 * maxb;
+    // the activation ring takes four slices (one k-block), the weight ring the rest; a run whose widest type leaves no two
+    // weight stages beside them takes activation stages away, down to two
+    int left = total - 1024 - tables;
+    p.bstages = 4;
+    while (p.bstages > 2 && (left - p.bstages * bbytes) / p.wstage_bytes < 2) --p.bstages;
+    p.wstages = (left - p.bstages * bbytes) / p.wstage_bytes;
+    if (p.wstages < 1) return GQ_ERR_LIMIT;
+    if (p.wstages > GQ_PF_MAX_STAGES) p.wstages = GQ_PF_MAX_STAGES;
+    left -= p.wstages * p.wstage_bytes + p.bstages * bbytes;
+    while (p.bstages < GQ_PF_SLOTS * SETS && left >= bbytes) { ++p.bstages; left -= bbytes; }
+    if (int rc = allow_smem<gemm_prefill_kernel<SETS>>(total)) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (pl.split > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = (unsigned)pl.split; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1;
+        ++na;
     }
-    prep_x_prefill_kernel<NB><<<(unsigned)(mt * NB), 256, 0, st>>>(x, ldx, p.K, p.M, ex, xp, p.status);
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+    cfg.gridDim = dim3((unsigned)((p.n_desc + 1) / 2 * pl.split), (unsigned)pl.tiles); cfg.blockDim = dim3(32 * (8 * SETS + 3));
+    cfg.dynamicSmemBytes = (size_t)total; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = na;
+    GQ_CUDA(cudaLaunchKernelEx(&cfg, gemm_prefill_kernel<SETS>, p));
     GQ_LAUNCHED();
-    if (p.split > 1) gemm_prefill_kernel<NB, true><<<dim3((unsigned)((p.n_desc + 1) / 2), (unsigned)mt, (unsigned)p.split), GQ_PF_THREADS, smem, st>>>(p);
-    else gemm_prefill_kernel<NB, false><<<dim3((unsigned)((p.n_desc + 1) / 2), (unsigned)mt), GQ_PF_THREADS, smem, st>>>(p);
-    GQ_LAUNCHED();
-    if (p.split > 1) {
-        const int64_t n = (int64_t)p.M * p.n_total;
-        sum_partials_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p.partials, p.split, p.M, p.n_total, p.y, p.ldy);
-        GQ_LAUNCHED();
-    }
     return GQ_OK;
 }
 
@@ -1898,22 +1900,27 @@ extern "C" int gq_gemm_prefill(const void *x_dev, int64_t M, int64_t K, int64_t 
     if (n_desc > 0x7ffffffe || M > (int64_t)65535 * 64) return GQ_ERR_LIMIT;
     const int maxb = run_info & 0xFFFF;
     if (maxb < 56 || maxb > 272 || (maxb & 1)) return GQ_ERR_ARG;
-    const int nbt = prefill_nb(M);
-    const int split = prefill_split(n_desc, M, K / GQ_QK, nbt, device_sms());
-    int *status; float *ex; uint8_t *xp; float *partials;
-    const int64_t need = pf_ws_layout(M, K, nbt, split, n_total, workspace_dev, &status, &ex, &xp, &partials);
+    const PrefillPlan pl = prefill_plan(n_desc, M, K / GQ_QK, device_sms());
+    int *status; float *ex; uint8_t *xp;
+    const int64_t need = pf_ws_layout(K, pl, workspace_dev, &status, &ex, &xp);
     if (workspace_bytes < need) return GQ_ERR_WORKSPACE;
+    if ((n_desc + 1) / 2 * pl.split > 0x7fffffff) return GQ_ERR_LIMIT;
     if (int rc = ensure_tables()) return rc;
-    PrefillParams p;
+    PrefillParams p = {};
     p.packed = (const uint8_t *)packed_dev; p.desc = desc_dev; p.n_desc = (int)n_desc; p.xp = xp; p.ex = ex;
-    p.y = (__nv_bfloat16 *)y_dev; p.ldy = ldy; p.M = (int)M; p.K = (int)K; p.nb = (int)(K / GQ_QK); p.status = status;
-    p.split = split; p.partials = partials; p.n_total = n_total; p.cb_mask = (run_info >> 22) & 63;
+    p.y = (__nv_bfloat16 *)y_dev; p.ldy = ldy; p.M = (int)M; p.nb = (int)(K / GQ_QK); p.N = pl.N; p.status = status;
+    p.split = pl.split; p.cb_mask = (run_info >> 22) & 63;
     cudaStream_t st = (cudaStream_t)stream;
-    switch (nbt) {
-        case 64: return launch_prefill<64>(p, (const __nv_bfloat16 *)x_dev, ldx, ex, xp, st);
-        case 128: return launch_prefill<128>(p, (const __nv_bfloat16 *)x_dev, ldx, ex, xp, st);
-        default: return launch_prefill<256>(p, (const __nv_bfloat16 *)x_dev, ldx, ex, xp, st);
+    {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.gridDim = dim3((unsigned)(pl.tiles * pl.N)); cfg.blockDim = dim3(GQ_PF_PREP_THREADS); cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 1;
+        GQ_CUDA(cudaLaunchKernelEx(&cfg, prep_x_prefill_kernel, (const __nv_bfloat16 *)x_dev, ldx, (int)K, (int)M, pl.N, ex, xp, status));
+        GQ_LAUNCHED();
     }
+    return pl.sets == 1 ? launch_prefill<1>(p, pl, maxb, st) : launch_prefill<2>(p, pl, maxb, st);
 }
 
 extern "C" int gq_device_status(int clear, void *stream) {

@@ -1,47 +1,52 @@
-// Large-batch (prefill) path: fused dequantise -> shared memory -> tcgen05 MMA with the accumulator in tensor
-// memory.  Replaces the reference's wide forms and its dequantise-then-cuBLAS path
-// (gguf-plugin/gluon/interface.py:159-188, gguf-plugin/gluon/tiles.py:141-149): the dequantised weights never
-// touch HBM.
+// Large-batch (prefill) path: packed weights are dequantised in registers, stored into TENSOR MEMORY as the A operand of
+// tcgen05.mma, and multiplied there; the accumulator lives in tensor memory too.  Replaces the reference's wide forms and its
+// dequantise-then-cuBLAS path (gguf-plugin/gluon/interface.py:159-188, gguf-plugin/gluon/tiles.py:141-149): the dequantised
+// weights touch neither HBM nor shared memory.
 //
-// One CTA computes a 128 (weight rows: two 64-row tiles of the packed run) x NB (batch rows) output tile:
-//   warp 0      producer of the activation operand: one bulk copy per 64-wide k-slice of a tile the preparation
-//               kernel already stored in the MMA's shared-memory layout (K-major, 128-byte swizzle)
-//   warp 1      allocates tensor memory, issues tcgen05.mma (one elected thread), commits to the stage barriers
-//   warps 2-9   dequantisers: each owns a 16-row slab, reads its lane-ordered chunks straight from global memory,
-//               turns them into fp16 weights (exact integer x fp16 scale, minus the fp16 minimum) and stores
-//               them into the K-major swizzled A stage; afterwards they drain the accumulator (tcgen05.ld),
-//               apply the activation row scale and store bf16.
-// Weights sit on the MMA's M side (D rows = output features), batch rows on N, as in the small-batch kernel.
-// With a split-K factor S > 1 (grid.z; for launches that would otherwise leave SMs without a CTA) a CTA walks one
-// balanced part of the k-blocks and stores fp32 partial outputs, which sum_partials_kernel adds in split order.
-// (Streaming the packed tiles through a shared-memory ring with bulk copies instead of loading them straight into
-// registers one k-block ahead was measured 8-15 % slower at every batch size: the ring costs an A / B stage at 256
-// batch rows, and the loads from it sit at the head of every k-block instead of overlapping the previous one.)
+// Why tensor memory.  The lane-ordered slab layout was made for mma.sync fragments: lane 4g + t holds rows g and g + 8,
+// weights 4t .. 4t+3 of a 16-weight run.  tcgen05.st.16x256b writes exactly that fragment — a run is one 256-bit row segment
+// of sixteen TMEM lanes — so a slab's 64-wide k-slice is ONE store instruction of sixteen registers, without a swizzle, bank
+// conflicts or a proxy fence, and the tensor core reads A at no shared-memory bandwidth: an MMA of M = 128, K = 16 takes
+// 12 / 17 / 32 / 63 / 125 cycles at N = 16 / 32 / 64 / 128 / 256, with A in shared memory 40 / 40 / 48 / 63 / 125.
+//
+// One CTA computes a 128 (weight rows: two 64-row tiles of the packed run) x N (batch rows, a multiple of 16 up to 256) tile
+// over a range of k-blocks:
+//   dequantiser warps   SETS groups of eight; a warp owns a 16-row slab and every SETS-th k-block.  It loads the slab from
+//                       the weight ring, releases the stage at once, and stores four k-slices into its set's four A slots
+//   weight producer     one thread; a k-block of both tiles per stage, bulk copies
+//   activation producer one thread; a 64-wide k-slice per stage, in the MMA's shared-memory layout (K-major, 128-byte
+//                       swizzle) as the preparation kernel stored it
+//   MMA issuer          one warp; four tcgen05.mma (M = 128, K = 16, A in TMEM, B in shared memory) per k-slice
+// Two shapes: SETS = 1 for N <= 128, two CTAs per SM of 256 TMEM columns (128 accumulator + four A slots of 32 columns each);
+// SETS = 2 for N <= 256, one CTA per SM with all 512 columns (256 + 2 x 4 x 32).  Either way sixteen dequantiser warps share
+// an SM.  Weights sit on the MMA's M side (D rows = output features), batch rows on N, as in the small-batch kernel.
+//
+// Split-K: the S CTAs of a tile form a thread-block cluster.  When their accumulators are done each CTA sends column part r
+// of its own to CTA r through distributed shared memory (which the rings no longer need) and adds the S parts of its own
+// columns in split order: no fp32 partials in HBM, no second kernel, the additions in a fixed order.
 // Every wait is bounded; a wait that runs out sets the status word, and the CTA still frees its tensor memory.
 #pragma once
 #include "gq_decode.cuh"
 
-// (included after the two __constant__ format tables c_iq3s_grid / c_iq3xxs_grid / c_iq2*_grid / c_iq4_kvalues are declared)
+// (included after the codebook tables and gq_load.cuh)
 namespace gq {
 
-#define GQ_PF_STAGES 4
-#define GQ_PF_A_BYTES (128 * 128)            // 128 rows x 64 fp16
-#define GQ_PF_DEQ_WARPS 8
-#define GQ_PF_THREADS (32 * (2 + GQ_PF_DEQ_WARPS))
+#define GQ_PF_SLOTS 4                        // A slots of a set: the four 64-wide k-slices of a k-block
+#define GQ_PF_MAX_STAGES 6                   // upper bound of the weight ring
 
 struct PrefillParams {
     const uint8_t *packed;
     const int32_t *desc;      // split-1 descriptor table: one row per 64-row tile
     int n_desc;
-    const uint8_t *xp;        // [m_tile][K/64][NB rows][128 B]: fp16 activations in MMA layout
-    const float *ex;          // [M] row scales
+    const uint8_t *xp;        // [m_tile][K/64][N rows][128 B]: fp16 activations in MMA layout
+    const float *ex;          // [m_tiles * N] row scales
     __nv_bfloat16 *y;
     int64_t ldy;
-    int M, K, nb;
+    int M, nb, N;             // N: batch rows of a CTA's tile
     int *status;
-    int split;                // split-K factor (grid.z); > 1: fp32 partials instead of y
-    float *partials;          // [split][M][n_total]
-    int64_t n_total;
+    int split;                // CTAs of a cluster, each with its part of the k-blocks
+    int wstages, bstages;     // ring depths
+    int wstage_bytes;         // both tiles of the widest type of the run
     int cb_mask;              // the codebook types of the run (bit gq_cb_kind): their tables sit side by side in shared memory
 };
 
@@ -54,24 +59,45 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
     const uint32_t hi = 64u | (1u << 14) | (2u << 29);
     return ((uint64_t)hi << 32) | lo;
 }
-
-template <int NB>
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
-    // instruction descriptor: D fp32, A and B fp16, both K-major, N = NB, M = 128
-    constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NB >> 3) << 17) | (8u << 24);
+// instruction descriptor: D fp32, A and B fp16, both K-major
+__device__ __forceinline__ uint32_t umma_idesc(int m, int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24); }
+// D[128, N] (+)= A[128, 16] (tensor memory) . B[16, N] (shared memory)
+__device__ __forceinline__ void umma_ts_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
         :
-        : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+// one thread of the warp, chosen so that the compiler knows the branch to be uniform
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.b32 %0, 1, 0, p;\n}" : "=r"(p));
+    return p != 0;
 }
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// sixteen lanes (rows) x 32 columns of tensor memory from the fragments of four 16-weight runs
+__device__ __forceinline__ void tmem_st_16x256b_x4(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]),
+                 "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
 
-// ---- one 64-wide k-slice (run pairs 2J, 2J+1) of one slab: decode, scale, store into the A stage ----------
+// ---- run pair P of one slab: decode, scale -> fp16 weights as the registers of two 16x256b store units ----------
 template <int TYPE, int P>
-__device__ __forceinline__ void pf_store_pair(const Dec<TYPE> &dec, uint8_t *a_stage, int row0, int g, int t) {
+__device__ __forceinline__ void pf_pair(const Dec<TYPE> &dec, uint32_t *o) {
     uint32_t a[2][4];
     dec.template pair<P>(a);
     float d0, d1;
@@ -89,188 +115,208 @@ __device__ __forceinline__ void pf_store_pair(const Dec<TYPE> &dec, uint8_t *a_s
         const uint32_t sc[2] = {h2_as_u32(__float2half2_rn(s0 * d0)), h2_as_u32(__float2half2_rn(s1 * d1))};
         const uint32_t mn[2] = {h2_as_u32(__float2half2_rn(-m0)), h2_as_u32(__float2half2_rn(-m1))};
         constexpr float off = Dec<TYPE>::template offs<2 * P>();   // both runs of a pair share the field position
-        constexpr int chunk0 = 4 * (P & 1);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             uint32_t w01 = a[u][h], w23 = a[u][2 + h];
             if constexpr (off != 0.0f) { w01 = hsub2(w01, h2k(off)); w23 = hsub2(w23, h2k(off)); }
             if constexpr (Dec<TYPE>::HAS_MIN) { w01 = hfma2(w01, sc[h], mn[h]); w23 = hfma2(w23, sc[h], mn[h]); }
             else { w01 = hmul2(w01, sc[h]); w23 = hmul2(w23, sc[h]); }
-            // A-tile row of weight row g + 8h of the slab: 2g + h.  Interleaving the two rows a lane owns gives the
-            // sixteen lanes of a half-warp (g = 0..3 or 4..7, one h) four different swizzle phases, so their 8-byte
-            // stores hit all 32 banks once; with row = g + 8h rows g and g + 8 shared a phase (2-way conflicts)
-            const int row = row0 + 2 * g + h;
-            const int chunk = chunk0 + 2 * u + (t >> 1);
-            uint8_t *dst = a_stage + row * 128 + ((chunk ^ (row & 7)) << 4) + ((t & 1) << 3);
-            *reinterpret_cast<uint2 *>(dst) = make_uint2(w01, w23);
+            // 32-bit column 2t, 2t + 1 of row g + 8h of the run's eight columns
+            o[4 * u + 2 * h] = w01;
+            o[4 * u + 2 * h + 1] = w23;
         }
     }
 }
 
-// the dequantiser loop of one warp for a tile of TYPE: for every k-block, four k-slices through the stage ring
-template <int TYPE>
-__device__ __forceinline__ bool pf_dequant(const uint8_t *tile_base, int slab, int row0, int nb, uint8_t *smem_a0, int stage_bytes,   // tile_base: first k-block of this CTA's part
-                                           uint64_t *a_full, uint64_t *freeb, const DecAux &aux, int lane) {
-    const int Bt = gq_type_bytes(TYPE);
-    const int g = lane >> 2, t = lane & 3;
-    int st = 0, round = 0;
-    Dec<TYPE> nxt;
-    nxt.load(tile_base + slab * 16 * Bt, lane, aux);
-    for (int kb = 0; kb < nb; ++kb) {
-        Dec<TYPE> cur = nxt;
-        if (kb + 1 < nb) nxt.load(tile_base + (int64_t)(kb + 1) * 64 * Bt + slab * 16 * Bt, lane, aux);
-#define GQ_PF_SLICE(J)                                                                                   \
-        {                                                                                                \
-            if (round > 0 && !mbar_wait(freeb + st, (round - 1) & 1)) return false;                     \
-            uint8_t *a_stage = smem_a0 + (size_t)st * stage_bytes;                                       \
-            pf_store_pair<TYPE, 2 * (J)>(cur, a_stage, row0, g, t);                                      \
-            pf_store_pair<TYPE, 2 * (J) + 1>(cur, a_stage, row0, g, t);                                  \
-            fence_proxy_async();                                                                         \
-            __syncwarp();                                                                                \
-            if (lane == 0) mbar_arrive(a_full + st);                                                     \
-            if (++st == GQ_PF_STAGES) { st = 0; ++round; }                                               \
-        }
-        GQ_PF_SLICE(0) GQ_PF_SLICE(1) GQ_PF_SLICE(2) GQ_PF_SLICE(3)
-#undef GQ_PF_SLICE
-    }
-    return true;
-}
+struct PfRings {
+    uint8_t *wring;
+    int wstage_bytes, wstages;
+    uint64_t *wfull, *wfree, *afull, *afree;
+};
 
-// a slab with no tile behind it (odd number of tiles in the run): its rows stay zero; it only keeps the barriers moving
-__device__ __forceinline__ bool pf_idle(int nb, uint64_t *a_full, uint64_t *freeb, int lane) {
-    int st = 0, round = 0;
-    for (int i = 0; i < 4 * nb; ++i) {
-        if (round > 0 && !mbar_wait(freeb + st, (round - 1) & 1)) return false;
+// the dequantiser loop of one warp for a tile of TYPE: k-blocks set, set + SETS, ... of this CTA's nkb
+template <int TYPE, int SETS>
+__device__ __forceinline__ bool pf_dequant(const PfRings &r, int slab_off, int set, int nkb, uint32_t ta, const DecAux &aux, int lane) {
+    int ws = set % r.wstages, wround = set / r.wstages;
+    for (int kb = set, use = 0; kb < nkb; kb += SETS, ++use) {
+        if (!mbar_wait(r.wfull + ws, wround & 1)) return false;
+        Dec<TYPE> dec;
+        dec.load(r.wring + (size_t)ws * r.wstage_bytes + slab_off, lane, aux);
         __syncwarp();
-        if (lane == 0) mbar_arrive(a_full + st);
-        if (++st == GQ_PF_STAGES) { st = 0; ++round; }
+        if (lane == 0) mbar_arrive(r.wfree + ws);          // everything the decoder needs is in registers
+        ws += SETS;
+        while (ws >= r.wstages) { ws -= r.wstages; ++wround; }
+        const auto slice = [&](auto j_) -> bool {
+            constexpr int J = decltype(j_)::value;
+            uint32_t o[16];
+            pf_pair<TYPE, 2 * J>(dec, o);
+            pf_pair<TYPE, 2 * J + 1>(dec, o + 8);
+            if (use > 0 && !mbar_wait(r.afree + J, (use - 1) & 1)) return false;
+            __syncwarp();
+            tc_fence_after();
+            tmem_st_16x256b_x4(ta + 32 * J, o);
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(r.afull + J);
+            return true;
+        };
+        if (!slice(std::integral_constant<int, 0>{}) || !slice(std::integral_constant<int, 1>{}) || !slice(std::integral_constant<int, 2>{}) ||
+            !slice(std::integral_constant<int, 3>{})) return false;
     }
     return true;
 }
 
-template <int NB, bool SPLITK>
-__global__ void __launch_bounds__(GQ_PF_THREADS, NB <= 64 ? 2 : 1) gemm_prefill_kernel(const PrefillParams p) {
+// eight accumulator columns (batch rows n0..n0+7) of the lane's feature row to y.  Two neighbouring lanes hold
+// neighbouring columns of y: they trade values so that each stores both of one batch row (four bytes instead of two).
+__device__ __forceinline__ void pf_store8(const PrefillParams &p, const float (&v)[8], int n0, int64_t col, bool row_ok, bool pair_ok, int lane) {
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+        const bool odd = lane & 1;
+        const float got = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+        if (pair_ok) {
+            const int n = n0 + j + (odd ? 1 : 0);
+            if (n < p.M) *reinterpret_cast<__nv_bfloat162 *>(p.y + (int64_t)n * p.ldy + col - (odd ? 1 : 0)) =
+                odd ? __floats2bfloat162_rn(got, v[j + 1]) : __floats2bfloat162_rn(v[j], got);
+        } else if (row_ok) {
+            if (n0 + j < p.M) p.y[(int64_t)(n0 + j) * p.ldy + col] = __float2bfloat16_rn(v[j]);
+            if (n0 + j + 1 < p.M) p.y[(int64_t)(n0 + j + 1) * p.ldy + col] = __float2bfloat16_rn(v[j + 1]);
+        }
+    }
+}
+
+template <int SETS>
+__global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_prefill_kernel(const __grid_constant__ PrefillParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    // layout: [stages x (A 16 KB | B NB*128)] [barriers] [tmem slot] [codebook tables of the run's types]
+    // layout: [activation ring][weight ring][codebook tables of the run's types]; the reduction of a split reuses the rings
+    __shared__ __align__(8) uint64_t bars[2 * GQ_PF_MAX_STAGES + 2 * GQ_PF_SLOTS * SETS + 1];
+    __shared__ uint32_t tmem_slot;
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    constexpr int B_BYTES = NB * 128;
-    constexpr int STAGE = GQ_PF_A_BYTES + B_BYTES;
-    uint64_t *a_full = reinterpret_cast<uint64_t *>(smem + GQ_PF_STAGES * STAGE);
-    uint64_t *b_full = a_full + GQ_PF_STAGES;
-    uint64_t *freeb = b_full + GQ_PF_STAGES;
-    uint64_t *done = freeb + GQ_PF_STAGES;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
-    uint2 *grid_s = reinterpret_cast<uint2 *>(smem + GQ_PF_STAGES * STAGE + 128);
+    const int bbytes = p.N * 128, N = p.N;
+    uint8_t *wring = smem + p.bstages * bbytes;
+    uint8_t *tables = wring + p.wstages * p.wstage_bytes;
+    uint64_t *wfull = bars, *wfree = bars + GQ_PF_MAX_STAGES;
+    uint64_t *afull = bars + 2 * GQ_PF_MAX_STAGES, *afree = afull + GQ_PF_SLOTS * SETS, *done = afree + GQ_PF_SLOTS * SETS;
+    constexpr uint32_t TMEM_COLS = 256u * SETS, D_COLS = 128u * SETS;      // the A slots follow the accumulator
+    constexpr int DEQ = 8 * SETS;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int pair = blockIdx.x, mt = blockIdx.y, z = SPLITK ? (int)blockIdx.z : 0;
-    const int kb0 = SPLITK ? (int)(((int64_t)z * p.nb) / p.split) : 0, kb1 = SPLITK ? (int)(((int64_t)(z + 1) * p.nb) / p.split) : p.nb;
-    const int nkb = kb1 - kb0, nslices = 4 * nkb;
+    const int part = (int)blockIdx.x % p.split, pair = (int)blockIdx.x / p.split, mt = blockIdx.y;      // a cluster: consecutive blockIdx.x
+    const int kb0 = (int)(((int64_t)part * p.nb) / p.split), nkb = (int)(((int64_t)(part + 1) * p.nb) / p.split) - kb0;
 
     // the two 64-row tiles of this CTA
     const int32_t *d0 = p.desc + (int64_t)(2 * pair) * GQ_DESC_WORDS;
     const bool has1 = 2 * pair + 1 < p.n_desc;
     const int32_t *d1 = has1 ? d0 + GQ_DESC_WORDS : d0;
+    const int type0 = d0[1], type1 = d1[1];
+    const int wb0 = 64 * gq_type_bytes(type0), wb1 = has1 ? 64 * gq_type_bytes(type1) : 0;
 
-    // a codebook type the call's run_info did not announce has no table space: report and leave (nothing is allocated yet)
+    // a codebook type the call's run_info did not announce has no table space, a wider type no stage: report and leave
+    // (nothing is allocated yet; the CTAs of a cluster work on the same tiles, so a cluster leaves as one)
     {
-        const int k0 = gq_cb_kind(d0[1]), k1 = gq_cb_kind(d1[1]);
-        if ((k0 >= 0 && !((p.cb_mask >> k0) & 1)) || (k1 >= 0 && !((p.cb_mask >> k1) & 1))) {
+        const int k0 = gq_cb_kind(type0), k1 = gq_cb_kind(type1);
+        if ((k0 >= 0 && !((p.cb_mask >> k0) & 1)) || (k1 >= 0 && !((p.cb_mask >> k1) & 1)) || 2 * wb0 > p.wstage_bytes || 2 * wb1 > p.wstage_bytes) {
             if (threadIdx.x == 0) { pdl_wait(); report_status(p.status, GQ_DEV_BAD_SHAPE); }      // after the preparation kernel has cleared the word
             return;
         }
     }
     if (threadIdx.x == 0) {
-        for (int s = 0; s < GQ_PF_STAGES; ++s) {
-            mbar_init(a_full + s, GQ_PF_DEQ_WARPS);
-            mbar_init(b_full + s, 1);
-            mbar_init(freeb + s, 1);
-        }
+        const uint32_t slabs = has1 ? 8 : 4;
+        for (int s = 0; s < p.wstages; ++s) { mbar_init(wfull + s, 1); mbar_init(wfree + s, slabs); }
+        for (int s = 0; s < GQ_PF_SLOTS * SETS; ++s) { mbar_init(afull + s, slabs + 1); mbar_init(afree + s, 1); }
         mbar_init(done, 1);
         fence_barrier_init();
     }
-    // the codebook tables of the two tiles' types, each at its place among the tables of the run's types
-    for (int which = 0; which < 2; ++which) {
-        const int ty = which ? d1[1] : d0[1], kind = gq_cb_kind(ty);
-        if (kind < 0 || (which && d1[1] == d0[1])) continue;
-        uint8_t *tb = reinterpret_cast<uint8_t *>(grid_s) + gq_cb_offset(p.cb_mask, kind);
-        uint32_t *t32 = reinterpret_cast<uint32_t *>(tb);
-        uint2 *t64 = reinterpret_cast<uint2 *>(tb);
-        switch (ty) {
-            case GQ_IQ3_S: for (int i = threadIdx.x; i < 512; i += blockDim.x) t64[i] = iq3s_grid_entry(c_iq3s_grid[i]); break;
-            case GQ_IQ3_XXS: for (int i = threadIdx.x; i < 256; i += blockDim.x) t64[i] = iq3s_grid_entry(c_iq3xxs_grid[i]); break;
-            case GQ_IQ2_XXS: for (int i = threadIdx.x; i < 512; i += blockDim.x) t32[i] = prmt(c_iq2xxs_grid[i], 0u, 0x3120u); break;
-            case GQ_IQ2_XS: for (int i = threadIdx.x; i < 1024; i += blockDim.x) t32[i] = prmt(c_iq2xs_grid[i], 0u, 0x3120u); break;
-            case GQ_IQ2_S: for (int i = threadIdx.x; i < 2048; i += blockDim.x) t32[i] = prmt(c_iq2s_grid[i], 0u, 0x3120u); break;
-            case GQ_IQ1_M: for (int i = threadIdx.x; i < 4096; i += blockDim.x) t32[i] = prmt(c_iq1_grid[i], 0u, 0x3120u); break;
-        }
-    }
-    if (!has1) {
-        // rows 64..127 of every A stage are never written: clear them once
-        for (int s = 0; s < GQ_PF_STAGES; ++s)
-            for (int i = threadIdx.x; i < 64 * 128 / 16; i += blockDim.x)
-                reinterpret_cast<uint4 *>(smem + (size_t)s * STAGE + 64 * 128)[i] = make_uint4(0, 0, 0, 0);
-        fence_proxy_async();
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)NB) : "memory");
+    if (warp == DEQ + 2) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    // the codebook tables of the two tiles' types, each at its place among the tables of the run's types
+    if (gq_cb_kind(type0) >= 0) fill_codebook(type0, tables + gq_cb_offset(p.cb_mask, gq_cb_kind(type0)), threadIdx.x, blockDim.x);
+    if (gq_cb_kind(type1) >= 0 && type1 != type0)
+        fill_codebook(type1, tables + gq_cb_offset(p.cb_mask, gq_cb_kind(type1)), threadIdx.x, blockDim.x);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem = tmem_slot;
     bool ok = true;
 
-    if (warp == 0) {
-        // ---- activation producer ----
+    if (warp == DEQ) {
+        // ---- weight producer: does not depend on the kernel in front of this one ----
         if (lane == 0) {
-            const uint8_t *src = p.xp + ((int64_t)mt * (p.K / 64) + 4 * (int64_t)kb0) * B_BYTES;
-            for (int i = 0, st = 0, round = 0; i < nslices; ++i) {
-                if (round > 0 && !mbar_wait(freeb + st, (round - 1) & 1)) { ok = false; break; }
-                mbar_expect_tx(b_full + st, B_BYTES);
-                bulk_g2s(smem + (size_t)st * STAGE + GQ_PF_A_BYTES, src + (int64_t)i * B_BYTES, B_BYTES, b_full + st);
-                if (++st == GQ_PF_STAGES) { st = 0; ++round; }
+            const uint8_t *s0 = p.packed + (int64_t)d0[0] * 16 + (int64_t)kb0 * wb0;
+            const uint8_t *s1 = p.packed + (int64_t)d1[0] * 16 + (int64_t)kb0 * wb1;
+            for (int kb = 0, st = 0, round = 0; kb < nkb; ++kb) {
+                if (round > 0 && !mbar_wait_parked(wfree + st, (round - 1) & 1)) { ok = false; break; }
+                uint8_t *dst = wring + (size_t)st * p.wstage_bytes;
+                mbar_expect_tx(wfull + st, (uint32_t)(wb0 + wb1));
+                bulk_g2s(dst, s0 + (int64_t)kb * wb0, (uint32_t)wb0, wfull + st);
+                if (wb1) bulk_g2s(dst + wb0, s1 + (int64_t)kb * wb1, (uint32_t)wb1, wfull + st);
+                if (++st == p.wstages) { st = 0; ++round; }
             }
         }
-    } else if (warp == 1) {
-        // ---- MMA issuer ----
+        __syncwarp();
+    } else if (warp == DEQ + 1) {
+        // ---- activation producer.  Slice i takes stage i % bstages; the MMAs of slice i - bstages have read it when that
+        // slice's A slot comes free (bstages <= 4 SETS, so the slot cannot have been used again by then).  The copy completes on
+        // the barrier of the slice's A slot, so that the MMA issuer waits once per slice ----
         if (lane == 0) {
-            for (int i = 0, st = 0, round = 0; i < nslices; ++i) {
-                if (!mbar_wait(a_full + st, round & 1) || !mbar_wait(b_full + st, round & 1)) { ok = false; break; }
-                tc_fence_after();
-                const uint32_t a_addr = smem_u32(smem + (size_t)st * STAGE);
-                const uint64_t ad = umma_desc(a_addr), bd = umma_desc(a_addr + GQ_PF_A_BYTES);
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk) umma_f16<NB>(tmem_base, ad + 2 * kk, bd + 2 * kk, (i > 0 || kk > 0) ? 1u : 0u);
-                umma_commit(freeb + st);          // the stage may be overwritten once these MMAs have read it
-                if (++st == GQ_PF_STAGES) { st = 0; ++round; }
+            pdl_wait();
+            const uint8_t *src = p.xp + ((int64_t)mt * p.nb + kb0) * 4 * bbytes;
+            for (int i = 0, st = 0; i < 4 * nkb; ++i) {
+                const int o = i - p.bstages;
+                if (o >= 0 && !mbar_wait_parked(afree + ((o >> 2) % SETS) * GQ_PF_SLOTS + (o & 3), ((o >> 2) / SETS) & 1)) { ok = false; break; }
+                uint64_t *full = afull + ((i >> 2) % SETS) * GQ_PF_SLOTS + (i & 3);
+                mbar_expect_tx(full, (uint32_t)bbytes);
+                bulk_g2s(smem + (size_t)st * bbytes, src + (int64_t)i * bbytes, (uint32_t)bbytes, full);
+                if (++st == p.bstages) st = 0;
             }
-            umma_commit(done);
+            pdl_trigger();
         }
-    } else {
-        // ---- dequantisers, then epilogue ----
-        const int slab = warp - 2;                 // 0..7: rows 16*slab .. 16*slab+15 of the 128
-        const int32_t *dd = (slab < 4) ? d0 : d1;
-        DecAux aux;
-        aux.grid = reinterpret_cast<const uint2 *>(reinterpret_cast<const uint8_t *>(grid_s) + (gq_cb_kind(dd[1]) >= 0 ? gq_cb_offset(p.cb_mask, gq_cb_kind(dd[1])) : 0));
-        {
-            uint32_t tb[4];
+        __syncwarp();
+    } else if (warp == DEQ + 2) {
+        // ---- MMA issuer: the warp waits as one and a thread chosen by elect.sync issues, so that addresses and descriptors
+        // stay in uniform registers (issued from a `lane == 0` branch an MMA cost the thread a hundred cycles) ----
+        const uint32_t idesc = umma_idesc(128, N);
+        const uint64_t bdesc0 = umma_desc(smem_u32(smem));
+        const uint32_t bstep = (uint32_t)bbytes >> 4, bwrap = bstep * (uint32_t)p.bstages;
+        uint32_t boff = 0;
+        for (int kb = 0; kb < nkb && ok; ++kb) {
+            const int set = kb % SETS;
+            const uint32_t parity = (uint32_t)(kb / SETS) & 1u;
+            uint64_t *full = afull + GQ_PF_SLOTS * set, *free = afree + GQ_PF_SLOTS * set;
+            const uint32_t ta = tmem + D_COLS + 32u * GQ_PF_SLOTS * set;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                tb[j] = 0;
+                if (!mbar_wait(full + j, parity)) { ok = false; break; }
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint64_t bd = bdesc0 + boff;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) tb[j] |= (uint32_t)(uint8_t)(c_iq4_kvalues[4 * j + i] + 128) << (8 * i);
+                    for (int kk = 0; kk < 4; ++kk) umma_ts_f16(tmem, ta + 32 * j + 8 * kk, bd + 2 * kk, idesc, (j > 0 || kk > 0) ? 1u : (uint32_t)(kb > 0));
+                    umma_commit(free + j);        // the slot and the activation stage may be overwritten once these MMAs have read them
+                    if (j == 3 && kb + 1 == nkb) umma_commit(done);
+                }
+                boff += bstep;
+                if (boff == bwrap) boff = 0;
             }
-            aux.iq4 = {tb[0], tb[1], tb[2], tb[3]};
+            __syncwarp();
         }
-        if (slab >= 4 && !has1) {
-            ok = pf_idle(nkb, a_full, freeb, lane);
-        } else {
-            const uint8_t *tile_base = p.packed + (int64_t)dd[0] * 16 + (int64_t)kb0 * 64 * gq_type_bytes(dd[1]);
-            const int sl = slab & 3, row0 = 16 * slab;
-#define GQ_PF(T) case T: ok = pf_dequant<T>(tile_base, sl, row0, nkb, smem, STAGE, a_full, freeb, aux, lane); break;
-            switch (dd[1]) {
+    } else {
+        // ---- dequantisers: warp w reaches the TMEM lanes of partition w % 4, which hold slabs 2 (w % 4) and + 1 ----
+        const int w = warp & 7, slab = 2 * (w & 3) + (w >> 2), set = warp >> 3;
+        const int type = slab < 4 ? type0 : type1;
+        if (slab < 4 || has1) {
+            DecAux aux;
+            aux.grid = reinterpret_cast<const uint2 *>(tables + (gq_cb_kind(type) >= 0 ? gq_cb_offset(p.cb_mask, gq_cb_kind(type)) : 0));
+            aux.iq4 = iq4_table_biased();
+            PfRings r;
+            r.wring = wring; r.wstage_bytes = p.wstage_bytes; r.wstages = p.wstages;
+            r.wfull = wfull; r.wfree = wfree; r.afull = afull + GQ_PF_SLOTS * set; r.afree = afree + GQ_PF_SLOTS * set;
+            const int slab_off = (slab < 4 ? 0 : wb0) + (slab & 3) * 16 * gq_type_bytes(type);
+            const uint32_t ta = tmem + D_COLS + 32u * GQ_PF_SLOTS * set + ((uint32_t)(16 * slab) << 16);
+#define GQ_PF(T) case T: ok = pf_dequant<T, SETS>(r, slab_off, set, nkb, ta, aux, lane); break;
+            switch (type) {
                 GQ_PF(GQ_Q4_0) GQ_PF(GQ_Q5_0) GQ_PF(GQ_Q8_0) GQ_PF(GQ_Q2_K) GQ_PF(GQ_Q3_K) GQ_PF(GQ_Q4_K)
                 GQ_PF(GQ_Q5_K) GQ_PF(GQ_Q6_K) GQ_PF(GQ_IQ4_NL) GQ_PF(GQ_IQ3_S) GQ_PF(GQ_IQ4_XS) GQ_PF(GQ_IQ3_XXS)
                 GQ_PF(GQ_IQ2_XXS) GQ_PF(GQ_IQ2_XS) GQ_PF(GQ_IQ2_S) GQ_PF(GQ_IQ1_M)
@@ -278,38 +324,68 @@ __global__ void __launch_bounds__(GQ_PF_THREADS, NB <= 64 ? 2 : 1) gemm_prefill_
 #undef GQ_PF
         }
         if (ok && !mbar_wait(done, 0)) ok = false;
+        __syncwarp();
         tc_fence_after();
-        if (ok) {
-            // TMEM lane group of this warp = warp % 4; the two warps of a lane group split the NB columns
-            const int lg = warp & 3, half = (warp - 2) >> 2;
-            const int feat = 32 * lg + lane;                       // row of the 128-row tile pair
-            const int32_t *dt = (feat < 64) ? d0 : d1;
-            const int ra = feat & 63;                              // row of the A tile -> weight row of the packed tile
-            const int r = (ra & ~15) | ((ra & 15) >> 1) | ((ra & 1) << 3);
-            const bool row_ok = (feat < 64 || has1) && r < dt[3];
-            const int64_t col = (int64_t)dt[2] + r;
+        pdl_wait();       // y may be read, and ex is written, by what runs in front
+    }
+
+    // ---- epilogue: warps 0 .. DEQ-1; lane l of partition q is row 32 q + l of the pair of tiles ----
+    const int q = warp & 3, e = warp >> 2, feat = 32 * q + lane;
+    const int32_t *dt = (feat < 64) ? d0 : d1;
+    const int rt = feat & 63;
+    const bool row_ok = (feat < 64 || has1) && rt < dt[3];
+    const int64_t col = (int64_t)dt[2] + rt;
+    const bool pair_ok = (feat < 64 || has1) && (rt | 1) < dt[3] && !(p.ldy & 1) && !((reinterpret_cast<uintptr_t>(p.y) + 2 * (uintptr_t)(col - (lane & 1))) & 3);
+    const uint32_t td = tmem + ((uint32_t)(32 * q) << 16);
+    if (p.split == 1) {
+        if (warp < DEQ && ok) {
 #pragma unroll 1
-            for (int c0 = half * (NB / 2); c0 < (half + 1) * (NB / 2); c0 += 32) {
-                uint32_t v[32];
-                const uint32_t taddr = tmem_base + ((uint32_t)(32 * lg) << 16) + (uint32_t)c0;
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                      "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-                      "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-                      "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(taddr)
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int c = 8 * e; c < N; c += 8 * (DEQ / 4)) {
+                uint32_t a[8];
+                tmem_ld_32x32b_x8(td + c, a);
+                const float4 e0 = *reinterpret_cast<const float4 *>(p.ex + mt * N + c), e1 = *reinterpret_cast<const float4 *>(p.ex + mt * N + c + 4);
+                tmem_wait_ld();
+                const float es[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+                float v[8];
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const int n = mt * NB + c0 + j;
-                    if (row_ok && n < p.M) {
-                        const float val = __uint_as_float(v[j]) * p.ex[n];
-                        if constexpr (SPLITK) p.partials[((int64_t)z * p.M + n) * p.n_total + col] = val;
-                        else p.y[(int64_t)n * p.ldy + col] = __float2bfloat16_rn(val);
-                    }
+                for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(a[j]) * es[j];
+                pf_store8(p, v, mt * N + c, col, row_ok, pair_ok, lane);
+            }
+        }
+    } else {
+        // columns [r ch, (r + 1) ch) are summed and stored by CTA r of the cluster; slot s of its buffer, [ch][128] fp32, is CTA s's part
+        const int S = p.split, ch = ((N + S - 1) / S + 7) & ~7;
+        float *buf = reinterpret_cast<float *>(smem);
+        cluster_sync_all();                 // every CTA of the cluster has finished with its rings
+        if (warp < DEQ) {
+            const uint32_t mine = smem_u32(buf) + (uint32_t)(part * ch * 128 + feat) * 4;
+#pragma unroll 1
+            for (int c = 8 * e; c < N; c += 8 * (DEQ / 4)) {
+                const int r = c / ch;
+                uint32_t a[8];
+                tmem_ld_32x32b_x8(td + c, a);
+                tmem_wait_ld();
+                const uint32_t dst = map_to_rank(mine, (uint32_t)r) + (uint32_t)(c - r * ch) * 512;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) st_cluster_f32(dst + 512 * j, __uint_as_float(a[j]));
+            }
+            __syncwarp();
+        }
+        const bool any_bad = __syncthreads_or(!ok);
+        cluster_sync_all();
+        const int c1 = (part + 1) * ch < N ? (part + 1) * ch : N;
+        if (warp < DEQ && !any_bad) {
+#pragma unroll 1
+            for (int c = part * ch + 8 * e; c < c1; c += 8 * (DEQ / 4)) {
+                float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                for (int s = 0; s < S; ++s) {
+                    const float *b = buf + (s * ch + (c - part * ch)) * 128 + feat;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[j] += b[128 * j];
                 }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] *= p.ex[mt * N + c + j];
+                pf_store8(p, v, mt * N + c, col, row_ok, pair_ok, lane);
             }
         }
     }
@@ -320,64 +396,81 @@ __global__ void __launch_bounds__(GQ_PF_THREADS, NB <= 64 ? 2 : 1) gemm_prefill_
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) {
+    if (warp == DEQ + 2) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)NB) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
     }
 }
 
+__device__ __forceinline__ float amax8(const uint4 &v) {
+    const __nv_bfloat162 *b = reinterpret_cast<const __nv_bfloat162 *>(&v);
+    float a = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float2 f = __bfloat1622float2(b[j]);
+        a = fmaxf(a, fmaxf(fabsf(f.x), fabsf(f.y)));
+    }
+    return a;
+}
+
 // activation preparation for the prefill path: bf16 row -> fp16 scaled by an exact power of two, stored in the
-// MMA's shared-memory layout (tiles of NB rows x 64 k, K-major, 16-byte chunks XOR-swizzled by row % 8) so the
-// kernel's producer moves a whole k-slice with one bulk copy
-template <int NB>
-__global__ void __launch_bounds__(256) prep_x_prefill_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int K, int M, float *__restrict__ ex,
-                                                             uint8_t *__restrict__ xp, int *status) {
-    __shared__ float red[8];
-    __shared__ float s_scale;
-    const int m = blockIdx.x;
+// MMA's shared-memory layout (tiles of N rows x 64 k, K-major, 16-byte chunks XOR-swizzled by row % 8) so the
+// kernel's producer moves a whole k-slice with one bulk copy.  One CTA per row of the padded batch; the row is read once and
+// kept in registers between the maximum and the conversion (rows up to 512 * 5 * 8 = 20480 activations).
+#define GQ_PF_PREP_THREADS 512
+#define GQ_PF_PREP_VECS 5
+__global__ void __launch_bounds__(GQ_PF_PREP_THREADS) prep_x_prefill_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int K, int M, int N,
+                                                                            float *__restrict__ ex, uint8_t *__restrict__ xp, int *status) {
+    __shared__ float red[GQ_PF_PREP_THREADS / 32];
+    const int m = blockIdx.x, r = m % N, nvec = K >> 3;
+    uint8_t *dst = xp + (int64_t)(m / N) * (K / 64) * (N * 128) + r * 128;
+    const int phase = r & 7;
+    pdl_trigger();    // the kernel behind this one may start fetching weights
+    pdl_wait();       // whatever ran before (possibly still reading this workspace) has finished
     if (m == 0 && threadIdx.x == 0) *status = 0;
-    const int mt = m / NB, r = m % NB;
-    uint8_t *tile0 = xp + (int64_t)mt * (K / 64) * (NB * 128);
+    const auto put = [&](int c, const uint4 &o) { *reinterpret_cast<uint4 *>(dst + (int64_t)(c >> 3) * (N * 128) + (((c & 7) ^ phase) << 4)) = o; };
     if (m >= M) {
         // rows past the batch inside the last tile: zeros (their outputs are never stored)
-        for (int c = threadIdx.x; c < K / 8; c += 256) {
-            const int slice = c >> 3, chunk = c & 7;
-            *reinterpret_cast<uint4 *>(tile0 + (int64_t)slice * (NB * 128) + r * 128 + ((chunk ^ (r & 7)) << 4)) = make_uint4(0, 0, 0, 0);
-        }
+        for (int c = threadIdx.x; c < nvec; c += GQ_PF_PREP_THREADS) put(c, make_uint4(0, 0, 0, 0));
         return;
     }
-    const __nv_bfloat16 *xr = x + (int64_t)m * ldx;
+    const uint4 *xr = reinterpret_cast<const uint4 *>(x + (int64_t)m * ldx);
+    uint4 v[GQ_PF_PREP_VECS];
     float amax = 0.0f;
-    for (int c = threadIdx.x; c < K / 8; c += 256) {
-        const uint4 v = *reinterpret_cast<const uint4 *>(xr + 8 * c);
-        const __nv_bfloat162 *b = reinterpret_cast<const __nv_bfloat162 *>(&v);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(b[j]); amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y))); }
+    for (int i = 0; i < GQ_PF_PREP_VECS; ++i) {
+        const int c = threadIdx.x + i * GQ_PF_PREP_THREADS;
+        v[i] = c < nvec ? __ldg(xr + c) : make_uint4(0u, 0u, 0u, 0u);
     }
+#pragma unroll
+    for (int i = 0; i < GQ_PF_PREP_VECS; ++i) amax = fmaxf(amax, amax8(v[i]));
+    for (int c = threadIdx.x + GQ_PF_PREP_VECS * GQ_PF_PREP_THREADS; c < nvec; c += GQ_PF_PREP_THREADS) amax = fmaxf(amax, amax8(__ldg(xr + c)));
 #pragma unroll
     for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float a = red[0];
-        for (int i = 1; i < 8; ++i) a = fmaxf(a, red[i]);
-        int e = 9;
-        if (a > 0.0f && a < 3.0e38f) { e = (int)((__float_as_uint(a) >> 23) & 0xFF) - 127; if (e < -100) e = -100; }
-        s_scale = __uint_as_float((uint32_t)(127 + 9 - e) << 23);
-        ex[m] = __uint_as_float((uint32_t)(127 - 9 + e) << 23);
-    }
-    __syncthreads();
-    const float scale = s_scale;
-    for (int c = threadIdx.x; c < K / 8; c += 256) {
-        const uint4 v = *reinterpret_cast<const uint4 *>(xr + 8 * c);
-        const __nv_bfloat162 *b = reinterpret_cast<const __nv_bfloat162 *>(&v);
+    float a = red[0];
+#pragma unroll
+    for (int i = 1; i < GQ_PF_PREP_THREADS / 32; ++i) a = fmaxf(a, red[i]);
+    // scale = 2^(9 - e), amax * scale in [512, 1024); identity for a zero, tiny or non-finite row
+    int e = 9;
+    if (a > 0.0f && a < 3.0e38f) { e = (int)((__float_as_uint(a) >> 23) & 0xFF) - 127; if (e < -100) e = -100; }
+    const float scale = __uint_as_float((uint32_t)(127 + 9 - e) << 23);
+    if (threadIdx.x == 0) ex[m] = __uint_as_float((uint32_t)(127 - 9 + e) << 23);
+    const auto convert = [&](int c, const uint4 &w) {
+        const __nv_bfloat162 *b = reinterpret_cast<const __nv_bfloat162 *>(&w);
         uint4 o;
         uint32_t *oo = reinterpret_cast<uint32_t *>(&o);
 #pragma unroll
         for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(b[j]); oo[j] = h2_as_u32(__floats2half2_rn(f.x * scale, f.y * scale)); }
-        const int slice = c >> 3, chunk = c & 7;
-        *reinterpret_cast<uint4 *>(tile0 + (int64_t)slice * (NB * 128) + r * 128 + ((chunk ^ (r & 7)) << 4)) = o;
+        put(c, o);
+    };
+#pragma unroll
+    for (int i = 0; i < GQ_PF_PREP_VECS; ++i) {
+        const int c = threadIdx.x + i * GQ_PF_PREP_THREADS;
+        if (c < nvec) convert(c, v[i]);
     }
+    for (int c = threadIdx.x + GQ_PF_PREP_VECS * GQ_PF_PREP_THREADS; c < nvec; c += GQ_PF_PREP_THREADS) convert(c, __ldg(xr + c));
 }
 
 }  // namespace gq

@@ -1,0 +1,31 @@
+"""The tcgen05 path where its cuts end: batch tiles of 16-row steps up to 128 (two CTAs per SM) and 256, several balanced
+tiles, K split over a cluster, runs with an odd number of tiles and outputs whose rows are not four-byte aligned."""
+import numpy as np
+import pytest
+import torch
+
+from hyperqwen_rtx4080s32_b200 import formats as F
+from hyperqwen_rtx4080s32_b200 import ops, synth
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+TOL = 6e-3      # bf16 output rounding (2^-8 of the value) plus the fp16 rounding of the weights
+
+
+@pytest.mark.parametrize("m", [33, 48, 49, 127, 128, 129, 144, 255, 256, 257, 513, 520])
+@pytest.mark.parametrize("parts,k", [([(64, F.Q4_K), (64, F.Q8_0), (70, F.IQ3_S)], 512), ([(129, F.IQ1_M), (33, F.Q2_K)], 2048), ([(200, F.Q6_K)], 4352)])
+def test_tiles_splits_and_ragged_outputs(m, parts, k):
+    n_outs, types = [n for n, _ in parts], [t for _, t in parts]
+    raws = [synth.random_blocks(n, k, t, seed=300 + i) for i, (n, t) in enumerate(parts)]
+    tiles = [ops.repack_tiles(r.cuda(), n, t) for r, (n, t) in zip(raws, parts)]
+    packed, _, descs, splits, _, _ = ops.prepare_grouped_layer(tiles, n_outs, types)
+    d1, n = descs[splits.index(1)], sum(n_outs)
+    x = synth.activations(m, k, device="cuda")
+    ref = np.concatenate([oracle.matmul_f64(x.float().cpu().numpy(), r.numpy(), t) for r, t in zip(raws, types)], axis=1)
+    y = ops.prefill_gemm(x, packed, d1, n, wtypes=types)
+    assert oracle.rel_err(y.float().cpu().numpy(), ref) < TOL
+    for pad in (0, 1):      # a view at an odd column, in rows of even and odd stride
+        wide = torch.full((m, n + 6 + pad), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.prefill_gemm(x, packed, d1, n, out=wide[:, 3:3 + n], wtypes=types)
+        assert torch.equal(wide[:, 3:3 + n], y) and bool(torch.isnan(wide[:, :3]).all()) and bool(torch.isnan(wide[:, 3 + n:]).all())
+    assert ops.device_status() == 0
