@@ -27,6 +27,7 @@
 // Every wait is bounded; a wait that runs out sets the status word, and the CTA still frees its tensor memory.
 #pragma once
 #include "gq_decode.cuh"
+#include "gq_scale16.cuh"
 
 // (included after the codebook tables and gq_load.cuh)
 namespace gq {
@@ -93,37 +94,32 @@ __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&v)[
                  : "memory");
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
 
-// ---- run pair P of one slab: decode, scale -> fp16 weights as the registers of two 16x256b store units ----------
-template <int TYPE, int P>
-__device__ __forceinline__ void pf_pair(const Dec<TYPE> &dec, uint32_t *o) {
-    uint32_t a[2][4];
-    dec.template pair<P>(a);
-    float d0, d1;
-    dec.kscale(d0, d1);
+// ---- k-slice J (runs 4J .. 4J+3) of one slab: decode, scale -> fp16 weights as the registers of one 16x256b.x4 store --------
+template <int TYPE, int J>
+__device__ __forceinline__ void pf_slice(const Dec<TYPE> &dec, uint32_t (&o)[16]) {
+    uint32_t s[2][4], m[2][4], a[2][2][4];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        float s0, s1, m0 = 0.f, m1 = 0.f;
-        if constexpr (Dec<TYPE>::GROUP == 32) {
-            dec.template scale<P>(s0, s1);
-            if constexpr (Dec<TYPE>::HAS_MIN) dec.template minterm<P>(m0, m1);
-        } else {
-            if (u == 0) { dec.template scale<2 * P>(s0, s1); if constexpr (Dec<TYPE>::HAS_MIN) dec.template minterm<2 * P>(m0, m1); }
-            else { dec.template scale<2 * P + 1>(s0, s1); if constexpr (Dec<TYPE>::HAS_MIN) dec.template minterm<2 * P + 1>(m0, m1); }
-        }
-        const uint32_t sc[2] = {h2_as_u32(__float2half2_rn(s0 * d0)), h2_as_u32(__float2half2_rn(s1 * d1))};
-        const uint32_t mn[2] = {h2_as_u32(__float2half2_rn(-m0)), h2_as_u32(__float2half2_rn(-m1))};
-        constexpr float off = Dec<TYPE>::template offs<2 * P>();   // both runs of a pair share the field position
+    for (int h = 0; h < 2; ++h) {
+        hscales<J>(dec, h, s[h]);
+        if constexpr (Dec<TYPE>::HAS_MIN) hmins<J>(dec, h, m[h]);
+    }
+    dec.template pair<2 * J>(a[0]);
+    dec.template pair<2 * J + 1>(a[1]);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        // both runs of a pair share the field position
+        constexpr float off0 = Dec<TYPE>::template offs<4 * J>(), off1 = Dec<TYPE>::template offs<4 * J + 2>();
+        const uint32_t off = r < 2 ? h2k(off0) : h2k(off1);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            uint32_t w01 = a[u][h], w23 = a[u][2 + h];
-            if constexpr (off != 0.0f) { w01 = hsub2(w01, h2k(off)); w23 = hsub2(w23, h2k(off)); }
-            if constexpr (Dec<TYPE>::HAS_MIN) { w01 = hfma2(w01, sc[h], mn[h]); w23 = hfma2(w23, sc[h], mn[h]); }
-            else { w01 = hmul2(w01, sc[h]); w23 = hmul2(w23, sc[h]); }
+            uint32_t w01 = a[r >> 1][r & 1][h], w23 = a[r >> 1][r & 1][2 + h];
+            if constexpr (off0 != 0.0f) { w01 = hsub2(w01, off); w23 = hsub2(w23, off); }
+            if constexpr (Dec<TYPE>::HAS_MIN) { w01 = hfma2(w01, s[h][r], m[h][r]); w23 = hfma2(w23, s[h][r], m[h][r]); }
+            else { w01 = hmul2(w01, s[h][r]); w23 = hmul2(w23, s[h][r]); }
             // 32-bit column 2t, 2t + 1 of row g + 8h of the run's eight columns
-            o[4 * u + 2 * h] = w01;
-            o[4 * u + 2 * h + 1] = w23;
+            o[4 * r + 2 * h] = w01;
+            o[4 * r + 2 * h + 1] = w23;
         }
     }
 }
@@ -149,8 +145,7 @@ __device__ __forceinline__ bool pf_dequant(const PfRings &r, int slab_off, int s
         const auto slice = [&](auto j_) -> bool {
             constexpr int J = decltype(j_)::value;
             uint32_t o[16];
-            pf_pair<TYPE, 2 * J>(dec, o);
-            pf_pair<TYPE, 2 * J + 1>(dec, o + 8);
+            pf_slice<TYPE, J>(dec, o);
             if (use > 0 && !mbar_wait(r.afree + J, (use - 1) & 1)) return false;
             __syncwarp();
             tc_fence_after();
@@ -353,21 +348,22 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
             }
         }
     } else {
-        // columns [r ch, (r + 1) ch) are summed and stored by CTA r of the cluster; slot s of its buffer, [ch][128] fp32, is CTA s's part
+        // columns [r ch, (r + 1) ch) are summed and stored by CTA r of the cluster; slot s of its buffer is CTA s's part, as
+        // [ch / 4][128 rows] of four columns each: 16-byte stores and loads, one per lane side by side
         const int S = p.split, ch = ((N + S - 1) / S + 7) & ~7;
-        float *buf = reinterpret_cast<float *>(smem);
+        float4 *buf = reinterpret_cast<float4 *>(smem);
         cluster_sync_all();                 // every CTA of the cluster has finished with its rings
         if (warp < DEQ) {
-            const uint32_t mine = smem_u32(buf) + (uint32_t)(part * ch * 128 + feat) * 4;
+            const uint32_t mine = smem_u32(buf) + (uint32_t)(part * (ch >> 2) * 128 + feat) * 16;
 #pragma unroll 1
             for (int c = 8 * e; c < N; c += 8 * (DEQ / 4)) {
                 const int r = c / ch;
                 uint32_t a[8];
                 tmem_ld_32x32b_x8(td + c, a);
                 tmem_wait_ld();
-                const uint32_t dst = map_to_rank(mine, (uint32_t)r) + (uint32_t)(c - r * ch) * 512;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) st_cluster_f32(dst + 512 * j, __uint_as_float(a[j]));
+                const uint32_t dst = map_to_rank(mine, (uint32_t)r) + (uint32_t)((c - r * ch) >> 2) * 2048;
+                st_cluster_f4(dst, __uint_as_float(a[0]), __uint_as_float(a[1]), __uint_as_float(a[2]), __uint_as_float(a[3]));
+                st_cluster_f4(dst + 2048, __uint_as_float(a[4]), __uint_as_float(a[5]), __uint_as_float(a[6]), __uint_as_float(a[7]));
             }
             __syncwarp();
         }
@@ -379,12 +375,15 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
             for (int c = part * ch + 8 * e; c < c1; c += 8 * (DEQ / 4)) {
                 float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 for (int s = 0; s < S; ++s) {
-                    const float *b = buf + (s * ch + (c - part * ch)) * 128 + feat;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] += b[128 * j];
+                    const float4 *b = buf + ((s * ch + (c - part * ch)) >> 2) * 128 + feat;
+                    const float4 x = b[0], y = b[128];
+                    v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+                    v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
                 }
+                const float4 e0 = *reinterpret_cast<const float4 *>(p.ex + mt * N + c), e1 = *reinterpret_cast<const float4 *>(p.ex + mt * N + c + 4);
+                const float es[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] *= p.ex[mt * N + c + j];
+                for (int j = 0; j < 8; ++j) v[j] *= es[j];
                 pf_store8(p, v, mt * N + c, col, row_ok, pair_ok, lane);
             }
         }
