@@ -49,6 +49,11 @@ GQ_HD inline float s8f(uint32_t word, int byte) { return (float)(int)(int8_t)((w
 #define GQ_MAGIC_B4 0x54005400u   // 64 + field
 #define GQ_MAGIC_B6 0x4C004C00u   // 16 + field
 
+// Multipliers that carry bits 0, 1 (GQ_SIGN01) or 2, 3 (GQ_SIGN23) of a value of up to eight bits to bits 15 and 31, the signs
+// of an fp16 pair: the two shifted copies do not overlap, so nothing carries.
+#define GQ_SIGN01 0x40008000u
+#define GQ_SIGN23 0x10002000u
+
 // the IQ4 codebook as unsigned bytes (value + 128) in four registers, filled by the kernel from the
 // generated table
 struct Iq4Table { uint32_t t0, t1, t2, t3; };
@@ -675,9 +680,9 @@ struct Dec<GQ_IQ3_S> {
         const uint32_t hw = (ib < 4) ? qh[h].x : qh[h].y;
         const uint32_t idx = or_and(idxb, shl_c<8 - (8 * (ib & 3) + 4 * u)>(hw), 0x100u);
         const uint2 e = grid[idx];
-        const uint32_t nib = (w4(sg[h], R >> 2) >> (8 * (R & 3))) & 0xFu;
-        a01 = xor_and(e.x, nib * 0x40008000u, 0x80008000u);
-        a23 = xor_and(e.y, (nib >> 2) * 0x40008000u, 0x80008000u);
+        const uint32_t nib = (w4(sg[h], R >> 2) >> (8 * (R & 3))) & 0xFFu;
+        a01 = xor_and(e.x, nib * GQ_SIGN01, 0x80008000u);
+        a23 = xor_and(e.y, nib * GQ_SIGN23, 0x80008000u);
     }
     template <int P>
     GQ_HD void pair(uint32_t (&a)[2][4]) const {
@@ -734,8 +739,8 @@ struct Dec<GQ_IQ3_XXS> {
         const uint32_t f = (sw[h][R >> 1] >> (14 * (R & 1) + sh0)) & 0x7Fu;
         const uint32_t mask = f | (popc32(f) << 7);          // bit 7: the parity (higher bits fall outside the nibble)
         const uint32_t nib = (mask >> shn) & 0xFu;
-        a01 = xor_and(e.x, nib * 0x40008000u, 0x80008000u);
-        a23 = xor_and(e.y, (nib >> 2) * 0x40008000u, 0x80008000u);
+        a01 = xor_and(e.x, nib * GQ_SIGN01, 0x80008000u);
+        a23 = xor_and(e.y, nib * GQ_SIGN23, 0x80008000u);
     }
     template <int P>
     GQ_HD void pair(uint32_t (&a)[2][4]) const {
@@ -762,8 +767,8 @@ struct Dec<GQ_IQ3_XXS> {
 GQ_HD inline uint32_t pick_alt_bytes16(uint32_t a, uint32_t b, int tp) { return prmt(a, b, 0x6420u + 0x1111u * (uint32_t)tp); }
 // the lane's word e of a grid entry and its four sign bits -> the fp16 pairs (w0, w1), (w2, w3)
 GQ_HD inline void iq2_pairs(uint32_t e, uint32_t nib, uint32_t &a01, uint32_t &a23) {
-    a01 = xor_and(hsub2(prmt(e, GQ_MAGICB, 0x5250u), h2k(1024)), nib * 0x40008000u, 0x80008000u);
-    a23 = xor_and(hsub2(prmt(e, GQ_MAGICB, 0x5351u), h2k(1024)), (nib >> 2) * 0x40008000u, 0x80008000u);
+    a01 = xor_and(hsub2(prmt(e, GQ_MAGICB, 0x5250u), h2k(1024)), nib * GQ_SIGN01, 0x80008000u);
+    a23 = xor_and(hsub2(prmt(e, GQ_MAGICB, 0x5351u), h2k(1024)), nib * GQ_SIGN23, 0x80008000u);
 }
 GQ_HD inline float odd_scale_f32(uint32_t s) { return u32_as_f32(0x4B000001u + 2u * s) - 8388608.0f; }    // 2 s + 1
 

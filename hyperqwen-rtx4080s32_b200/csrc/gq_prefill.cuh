@@ -98,7 +98,8 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 // ---- k-slice J (runs 4J .. 4J+3) of one slab: decode, scale -> fp16 weights as the registers of one 16x256b.x4 store --------
 template <int TYPE, int J>
 __device__ __forceinline__ void pf_slice(const Dec<TYPE> &dec, uint32_t (&o)[16]) {
-    uint32_t s[2][4], m[2][4], a[2][2][4];
+    uint32_t s[2][2], m[2][2], a[2][2][4];
+    constexpr int G = Dec<TYPE>::GROUP;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         hscales<J>(dec, h, s[h]);
@@ -106,22 +107,21 @@ __device__ __forceinline__ void pf_slice(const Dec<TYPE> &dec, uint32_t (&o)[16]
     }
     dec.template pair<2 * J>(a[0]);
     dec.template pair<2 * J + 1>(a[1]);
+    const auto run = [&](auto r_) {
+        constexpr int R = decltype(r_)::value;
+        constexpr float off = Dec<TYPE>::template offs<4 * J + R>();
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        // both runs of a pair share the field position
-        constexpr float off0 = Dec<TYPE>::template offs<4 * J>(), off1 = Dec<TYPE>::template offs<4 * J + 2>();
-        const uint32_t off = r < 2 ? h2k(off0) : h2k(off1);
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint32_t w01 = a[r >> 1][r & 1][h], w23 = a[r >> 1][r & 1][2 + h];
-            if constexpr (off0 != 0.0f) { w01 = hsub2(w01, off); w23 = hsub2(w23, off); }
-            if constexpr (Dec<TYPE>::HAS_MIN) { w01 = hfma2(w01, s[h][r], m[h][r]); w23 = hfma2(w23, s[h][r], m[h][r]); }
-            else { w01 = hmul2(w01, s[h][r]); w23 = hmul2(w23, s[h][r]); }
-            // 32-bit column 2t, 2t + 1 of row g + 8h of the run's eight columns
-            o[4 * r + 2 * h] = w01;
-            o[4 * r + 2 * h + 1] = w23;
-        }
-    }
+            for (int k = 0; k < 2; ++k) {
+                __half2 w = u32_as_h2(a[R >> 1][R & 1][2 * k + h]);
+                if constexpr (off != 0.0f) w = __hsub2(w, u32_as_h2(h2k(off)));
+                if constexpr (Dec<TYPE>::HAS_MIN) w = __hfma2(w, scale_of<G, R>(s[h]), scale_of<G, R>(m[h]));
+                else w = __hmul2(w, scale_of<G, R>(s[h]));
+                o[4 * R + 2 * h + k] = h2_as_u32(w);       // 32-bit column 2t + k of row g + 8h of the run's eight columns
+            }
+    };
+    run(std::integral_constant<int, 0>{}); run(std::integral_constant<int, 1>{}); run(std::integral_constant<int, 2>{}); run(std::integral_constant<int, 3>{});
 }
 
 struct PfRings {
