@@ -1809,35 +1809,47 @@ extern "C" int gq_allreduce_push(const void *in_dev, void *out_dev, int64_t n_by
 // ---- prefill ----------------------------------------------------------------------------------------
 // Dynamic shared memory of a CTA: two CTAs (SETS = 1) or one fill the SM, so that no third user of tensor memory joins them:
 // the CTAs of a cluster wait for one another while they hold theirs.
-#define GQ_PF_SMEM_1 (112 * 1024)
-#define GQ_PF_SMEM_2 (226 * 1024)
+#define GQ_PF_SMEM_1 (111 * 1024)
+#define GQ_PF_SMEM_2 (225 * 1024)
 
 // How a prefill launch is cut: N batch rows per CTA (a multiple of 16, tiles balanced), the cluster split of K, and which of
-// the two kernels (SETS) runs it.
+// the kernel's shapes runs it.
 struct PrefillPlan {
-    int sets, N, tiles, split;
+    int sets, wide, N, tiles, split;
 };
-// SETS = 1 (two CTAs per SM) holds tiles of up to 128 batch rows, SETS = 2 up to 256; a wider batch takes as many equal tiles
-// as it needs, since every further tile decodes the weights again.  K is split while that shortens the launch: a wave costs
-// about six k-blocks of start-up and drain on top of its own, and a CTA keeps at least four k-blocks (at least eight in the
-// run, so short K is never split).
-static PrefillPlan prefill_plan(int64_t n_desc, int64_t M, int64_t nb, int sms) {
+static PrefillPlan prefill_shape(int64_t M, int64_t tiles) {
     PrefillPlan p;
-    if (sms <= 0) sms = 148;
-    p.tiles = (int)((M + 255) / 256);
-    p.N = (int)(((M + p.tiles - 1) / p.tiles + 15) & ~15);
+    const int64_t rows = (M + tiles - 1) / tiles;
+    p.tiles = (int)tiles;
+    p.wide = rows > 256;
+    p.N = (int)(p.wide ? (rows + 31) & ~31 : (rows + 15) & ~15);
     p.sets = p.N <= 128 ? 1 : 2;
-    const int64_t slots = p.sets == 1 ? 2 * (int64_t)sms : sms, ctas = ((n_desc + 1) / 2) * p.tiles;
     p.split = 1;
-    double best = 1e300;
-    for (int S = 1; S <= 8 && (S == 1 || (int64_t)S * 4 <= nb); ++S) {
-        // clusters leave some slots unused
-        const int64_t usable = slots * (100 - 3 * (S - 1)) / 100;
-        const int64_t waves = (ctas * S + usable - 1) / usable;
-        const double cost = (double)waves * ((double)((nb + S - 1) / S) + 6.0) + (S > 1 ? 2.0 : 0.0);
-        if (cost < best - 1e-9) { best = cost; p.split = S; }
-    }
     return p;
+}
+// CTAs of one batch tile and one part of K: two 64-row tiles each, in pairs where the MMAs span a pair
+static int64_t prefill_ctas(int64_t n_desc, const PrefillPlan &p) { return p.sets == 1 ? (n_desc + 1) / 2 : (n_desc + 3) / 4 * 2; }
+// Every batch tile decodes the weights again, so there are as few as fit (384 rows each) up to what 256-row tiles would need;
+// K is split over a cluster, at least four k-blocks to a CTA and eight in the run.  Both are chosen by the cycles that the waves
+// of the launch take: a k-block costs a CTA its MMAs (7.8 N cycles) or its share of the decoding (2700 cycles alone on an SM,
+// 4200 where two CTAs share one), whichever is longer, and a wave its start-up and its drain (5000 cycles and 25 a batch row).
+static PrefillPlan prefill_plan(int64_t n_desc, int64_t M, int64_t nb, int sms) {
+    PrefillPlan best = prefill_shape(M, (M + 255) / 256);
+    if (sms <= 0) sms = 148;
+    double best_cost = 1e300;
+    for (int64_t tiles = (M + 383) / 384; tiles <= (M + 255) / 256; ++tiles) {
+        PrefillPlan p = prefill_shape(M, tiles);
+        const int64_t slots = p.sets == 1 ? 2 * (int64_t)sms : sms, ctas = prefill_ctas(n_desc, p) * tiles;
+        const double mma = 7.8 * p.N + 300.0, decode = p.sets == 1 ? 4200.0 : 2700.0, per_kb = mma > decode ? mma : decode;
+        for (int S = 1; S * p.sets <= 8 && (S == 1 || (int64_t)S * 4 <= nb); ++S) {
+            // clusters leave some slots unused
+            const int64_t usable = slots * (100 - 3 * (S - 1)) / 100;
+            const int64_t waves = (ctas * S + usable - 1) / usable;
+            const double cost = (double)waves * ((double)((nb + S - 1) / S) * per_kb + 5000.0 + 25.0 * p.N + (S > 1 ? 6000.0 : 0.0));
+            if (cost < best_cost * (1.0 - 1e-9)) { best_cost = cost; best = p; best.split = S; }
+        }
+    }
+    return best;
 }
 
 static int64_t pf_ws_layout(int64_t K, const PrefillPlan &pl, void *base, int **status, float **ex, uint8_t **xp) {
@@ -1856,9 +1868,9 @@ extern "C" int64_t gq_prefill_workspace_bytes(int64_t M, int64_t K, int64_t n_to
     return pf_ws_layout(K, prefill_plan(n_desc, M, K / GQ_QK, device_sms()), nullptr, nullptr, nullptr, nullptr);
 }
 
-template <int SETS>
+template <int SETS, bool WIDE>
 static int launch_prefill(PrefillParams &p, const PrefillPlan &pl, int maxb, cudaStream_t st) {
-    const int total = SETS == 1 ? GQ_PF_SMEM_1 : GQ_PF_SMEM_2, tables = gq_cb_region_sum(p.cb_mask), bbytes = pl.N * 128;
+    const int total = SETS == 1 ? GQ_PF_SMEM_1 : GQ_PF_SMEM_2, tables = gq_cb_region_sum(p.cb_mask), bbytes = pl.N * 128 / SETS;
     p.wstage_bytes = 128 * maxb;
     // the activation ring takes four slices (one k-block), the weight ring the rest; a run whose widest type leaves no two
     // weight stages beside them takes activation stages away, down to two
@@ -1866,25 +1878,26 @@ static int launch_prefill(PrefillParams &p, const PrefillPlan &pl, int maxb, cud
     p.bstages = 4;
     while (p.bstages > 2 && (left - p.bstages * bbytes) / p.wstage_bytes < 2) --p.bstages;
     p.wstages = (left - p.bstages * bbytes) / p.wstage_bytes;
-    if (p.wstages < 1) return GQ_ERR_LIMIT;
     if (p.wstages > GQ_PF_MAX_STAGES) p.wstages = GQ_PF_MAX_STAGES;
+    p.wstages -= p.wstages % SETS;        // each set walks stages of its own
+    if (p.wstages < 1) return GQ_ERR_LIMIT;
     left -= p.wstages * p.wstage_bytes + p.bstages * bbytes;
-    while (p.bstages < GQ_PF_SLOTS * SETS && left >= bbytes) { ++p.bstages; left -= bbytes; }
-    if (int rc = allow_smem<gemm_prefill_kernel<SETS>>(total)) return rc;
+    while (p.bstages < GQ_PF_SLOTS * (WIDE ? 1 : SETS) && left >= bbytes) { ++p.bstages; left -= bbytes; }
+    if (int rc = allow_smem<gemm_prefill_kernel<SETS, WIDE>>(total)) return rc;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     int na = 0;
-    if (pl.split > 1) {
+    if (pl.split * SETS > 1) {
         attr[na].id = cudaLaunchAttributeClusterDimension;
-        attr[na].val.clusterDim.x = (unsigned)pl.split; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1;
+        attr[na].val.clusterDim.x = (unsigned)(pl.split * SETS); attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1;
         ++na;
     }
     attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
-    cfg.gridDim = dim3((unsigned)((p.n_desc + 1) / 2 * pl.split), (unsigned)pl.tiles); cfg.blockDim = dim3(32 * (8 * SETS + 3));
+    cfg.gridDim = dim3((unsigned)(pl.split * SETS), (unsigned)(prefill_ctas(p.n_desc, pl) / SETS), (unsigned)pl.tiles); cfg.blockDim = dim3(32 * (8 * SETS + 3));
     cfg.dynamicSmemBytes = (size_t)total; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = na;
-    GQ_CUDA(cudaLaunchKernelEx(&cfg, gemm_prefill_kernel<SETS>, p));
+    GQ_CUDA(cudaLaunchKernelEx(&cfg, gemm_prefill_kernel<SETS, WIDE>, p));
     GQ_LAUNCHED();
     return GQ_OK;
 }
@@ -1904,12 +1917,17 @@ extern "C" int gq_gemm_prefill(const void *x_dev, int64_t M, int64_t K, int64_t 
     int *status; float *ex; uint8_t *xp;
     const int64_t need = pf_ws_layout(K, pl, workspace_dev, &status, &ex, &xp);
     if (workspace_bytes < need) return GQ_ERR_WORKSPACE;
-    if ((n_desc + 1) / 2 * pl.split > 0x7fffffff) return GQ_ERR_LIMIT;
+    if (prefill_ctas(n_desc, pl) / pl.sets > 65535) return GQ_ERR_LIMIT;
     if (int rc = ensure_tables()) return rc;
     PrefillParams p = {};
     p.packed = (const uint8_t *)packed_dev; p.desc = desc_dev; p.n_desc = (int)n_desc; p.xp = xp; p.ex = ex;
     p.y = (__nv_bfloat16 *)y_dev; p.ldy = ldy; p.M = (int)M; p.nb = (int)(K / GQ_QK); p.N = pl.N; p.status = status;
     p.split = pl.split; p.cb_mask = (run_info >> 22) & 63;
+    for (int t = 0; t < 32; ++t) {
+        const int kind = gq_cb_kind(t);
+        p.half_bytes[t] = (uint8_t)(gq_type_bytes(t) / 2);
+        p.cb_at[t] = (uint16_t)(kind < 0 ? 0 : (p.cb_mask >> kind) & 1 ? gq_cb_offset(p.cb_mask, kind) / 16 + 2 : 1);
+    }
     cudaStream_t st = (cudaStream_t)stream;
     {
         cudaLaunchConfig_t cfg = {};
@@ -1917,10 +1935,11 @@ extern "C" int gq_gemm_prefill(const void *x_dev, int64_t M, int64_t K, int64_t 
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.gridDim = dim3((unsigned)(pl.tiles * pl.N)); cfg.blockDim = dim3(GQ_PF_PREP_THREADS); cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 1;
-        GQ_CUDA(cudaLaunchKernelEx(&cfg, prep_x_prefill_kernel, (const __nv_bfloat16 *)x_dev, ldx, (int)K, (int)M, pl.N, ex, xp, status));
+        GQ_CUDA(cudaLaunchKernelEx(&cfg, prep_x_prefill_kernel, (const __nv_bfloat16 *)x_dev, ldx, (int)K, (int)M, pl.N, pl.sets == 1 ? 0 : pl.wide ? pl.N / 2 : pl.N, ex, xp, status));
         GQ_LAUNCHED();
     }
-    return pl.sets == 1 ? launch_prefill<1>(p, pl, maxb, st) : launch_prefill<2>(p, pl, maxb, st);
+    if (pl.wide) return launch_prefill<2, true>(p, pl, maxb, st);
+    return pl.sets == 1 ? launch_prefill<1, false>(p, pl, maxb, st) : launch_prefill<2, false>(p, pl, maxb, st);
 }
 
 extern "C" int gq_device_status(int clear, void *stream) {

@@ -9,7 +9,7 @@
 // conflicts or a proxy fence, and the tensor core reads A at no shared-memory bandwidth: an MMA of M = 128, K = 16 takes
 // 12 / 17 / 32 / 63 / 125 cycles at N = 16 / 32 / 64 / 128 / 256, with A in shared memory 40 / 40 / 48 / 63 / 125.
 //
-// One CTA computes a 128 (weight rows: two 64-row tiles of the packed run) x N (batch rows, a multiple of 16 up to 256) tile
+// One CTA computes a 128 (weight rows: two 64-row tiles of the packed run) x N (batch rows, a multiple of 16 up to 384) tile
 // over a range of k-blocks:
 //   dequantiser warps   SETS groups of eight; a warp owns a 16-row slab and every SETS-th k-block.  It loads the slab from
 //                       the weight ring, releases the stage at once, and stores four k-slices into its set's four A slots
@@ -17,9 +17,13 @@
 //   activation producer one thread; a 64-wide k-slice per stage, in the MMA's shared-memory layout (K-major, 128-byte
 //                       swizzle) as the preparation kernel stored it
 //   MMA issuer          one warp; four tcgen05.mma (M = 128, K = 16, A in TMEM, B in shared memory) per k-slice
-// Two shapes: SETS = 1 for N <= 128, two CTAs per SM of 256 TMEM columns (128 accumulator + four A slots of 32 columns each);
-// SETS = 2 for N <= 256, one CTA per SM with all 512 columns (256 + 2 x 4 x 32).  Either way sixteen dequantiser warps share
-// an SM.  Weights sit on the MMA's M side (D rows = output features), batch rows on N, as in the small-batch kernel.
+// Three shapes, all with sixteen dequantiser warps on an SM: SETS = 1 for N <= 128, two CTAs per SM of 256 TMEM columns (128
+// accumulator + a ring of four A slots of 32 columns); SETS = 2 for N <= 256, one CTA with all 512 columns (256 + a ring of four
+// slots per set); and WIDE for N <= 384 (384 + one ring that the two sets fill in turn), where a weight is decoded once for half
+// as many rows again and the tensor core needs 3000 cycles a k-block against 1300 of decoding.  The SETS = 2 shapes run as CTA
+// pairs (cta_group::2): the MMAs span both CTAs' 128 rows and each CTA holds half of the batch rows, because the activation
+// slices are read once per 128 weight rows otherwise, 65 bytes a cycle and SM out of the L2, which is more than it gives.
+// Weights sit on the MMA's M side (D rows = output features), batch rows on N, as in the small-batch kernel.
 //
 // Split-K: the S CTAs of a tile form a thread-block cluster.  When their accumulators are done each CTA sends column part r
 // of its own to CTA r through distributed shared memory (which the rings no longer need) and adds the S parts of its own
@@ -32,7 +36,7 @@
 // (included after the codebook tables and gq_load.cuh)
 namespace gq {
 
-#define GQ_PF_SLOTS 4                        // A slots of a set: the four 64-wide k-slices of a k-block
+#define GQ_PF_SLOTS 4                        // A slots of a ring: the four 64-wide k-slices of a k-block
 #define GQ_PF_MAX_STAGES 6                   // upper bound of the weight ring
 
 struct PrefillParams {
@@ -49,6 +53,10 @@ struct PrefillParams {
     int wstages, bstages;     // ring depths
     int wstage_bytes;         // both tiles of the widest type of the run
     int cb_mask;              // the codebook types of the run (bit gq_cb_kind): their tables sit side by side in shared memory
+    // per GGML type, read from the parameter bank: the size functions of gq_layout.h are switches, and at the start of a CTA every
+    // jump is an instruction-cache miss (they and the divisions of a flat block index cost 2500 .. 4000 cycles per CTA)
+    uint8_t half_bytes[32];   // bytes_per_256 / 2
+    uint16_t cb_at[32];       // 0: no codebook; 1: one the run did not announce; else offset of its table / 16 + 2
 };
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -62,13 +70,21 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
 }
 // instruction descriptor: D fp32, A and B fp16, both K-major
 __device__ __forceinline__ uint32_t umma_idesc(int m, int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24); }
-// D[128, N] (+)= A[128, 16] (tensor memory) . B[16, N] (shared memory)
+// D[128 CG, N] (+)= A[128 CG, 16] (tensor memory) . B[16, N] (shared memory); CG = 2: of both CTAs of a pair, half of B's rows each
+template <int CG>
 __device__ __forceinline__ void umma_ts_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-        :
-        : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
+    if constexpr (CG == 1)
+        asm volatile(
+            "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+            :
+            : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}"
+            :
+            : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+            : "memory");
 }
 // one thread of the warp, chosen so that the compiler knows the branch to be uniform
 __device__ __forceinline__ bool elect_one() {
@@ -76,9 +92,34 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.b32 %0, 1, 0, p;\n}" : "=r"(p));
     return p != 0;
 }
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+// arrive on `bar` when the MMAs issued so far are done; CG = 2: on the barrier at the same place in both CTAs of the pair (`ctas`: their bits)
+template <int CG>
+__device__ __forceinline__ void umma_commit(uint64_t *bar, uint16_t ctas) {
+    if constexpr (CG == 1)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(ctas)
+                     : "memory");
 }
+template <int CG>
+__device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t cols) {
+    if constexpr (CG == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+}
+template <int CG>
+__device__ __forceinline__ void tmem_dealloc(uint32_t tmem, uint32_t cols) {
+    if constexpr (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+}
+// an arrival on a barrier of the cluster, by its shared::cluster address.  No fence at cluster scope (release.cluster costs a
+// memory barrier of hundreds of cycles, measured 1.6x on the whole kernel): what it announces is tensor memory, ordered by
+// tcgen05.fence, or bulk copies, which their own barrier has completed.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory"); }
 // sixteen lanes (rows) x 32 columns of tensor memory from the fragments of four 16-weight runs
 __device__ __forceinline__ void tmem_st_16x256b_x4(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]),
@@ -127,14 +168,19 @@ __device__ __forceinline__ void pf_slice(const Dec<TYPE> &dec, uint32_t (&o)[16]
 struct PfRings {
     uint8_t *wring;
     int wstage_bytes, wstages;
-    uint64_t *wfull, *wfree, *afull, *afree;
+    uint64_t *wfull, *wfree, *afree;
+    uint32_t afull;                  // shared::cluster address: in a CTA pair, of the CTA that issues the MMAs
 };
 
-// the dequantiser loop of one warp for a tile of TYPE: k-blocks set, set + SETS, ... of this CTA's nkb
-template <int TYPE, int SETS>
+// the dequantiser loop of one warp for a tile of TYPE: k-blocks set, set + SETS, ... of this CTA's nkb; k-block kb fills the
+// A ring kb % RINGS once the MMAs of k-block kb - RINGS have read it.  Barriers are waited on phase by phase: wfull because the
+// weight ring has a multiple of SETS stages, afree because it belongs to a set's k-blocks, not to the ring.
+template <int TYPE, int SETS, int RINGS>
 __device__ __forceinline__ bool pf_dequant(const PfRings &r, int slab_off, int set, int nkb, uint32_t ta, const DecAux &aux, int lane) {
     int ws = set % r.wstages, wround = set / r.wstages;
-    for (int kb = set, use = 0; kb < nkb; kb += SETS, ++use) {
+    for (int kb = set; kb < nkb; kb += SETS) {
+        const int prev = kb - RINGS;
+        uint64_t *afree = r.afree + GQ_PF_SLOTS * ((kb + SETS - RINGS) % SETS);
         if (!mbar_wait(r.wfull + ws, wround & 1)) return false;
         Dec<TYPE> dec;
         dec.load(r.wring + (size_t)ws * r.wstage_bytes + slab_off, lane, aux);
@@ -146,14 +192,14 @@ __device__ __forceinline__ bool pf_dequant(const PfRings &r, int slab_off, int s
             constexpr int J = decltype(j_)::value;
             uint32_t o[16];
             pf_slice<TYPE, J>(dec, o);
-            if (use > 0 && !mbar_wait(r.afree + J, (use - 1) & 1)) return false;
+            if (prev >= 0 && !mbar_wait(afree + J, (prev / SETS) & 1)) return false;
             __syncwarp();
             tc_fence_after();
             tmem_st_16x256b_x4(ta + 32 * J, o);
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(r.afull + J);
+            if (lane == 0) mbar_arrive_cluster(r.afull + 8 * J);
             return true;
         };
         if (!slice(std::integral_constant<int, 0>{}) || !slice(std::integral_constant<int, 1>{}) || !slice(std::integral_constant<int, 2>{}) ||
@@ -180,107 +226,143 @@ __device__ __forceinline__ void pf_store8(const PrefillParams &p, const float (&
     }
 }
 
-template <int SETS>
+template <int SETS, bool WIDE>
 __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_prefill_kernel(const __grid_constant__ PrefillParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // layout: [activation ring][weight ring][codebook tables of the run's types]; the reduction of a split reuses the rings
     __shared__ __align__(8) uint64_t bars[2 * GQ_PF_MAX_STAGES + 2 * GQ_PF_SLOTS * SETS + 1];
     __shared__ uint32_t tmem_slot;
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    const int bbytes = p.N * 128, N = p.N;
+    const int N = p.N, bbytes = N * 128 / SETS;          // a CTA of a pair holds half of the batch rows of a slice
     uint8_t *wring = smem + p.bstages * bbytes;
     uint8_t *tables = wring + p.wstages * p.wstage_bytes;
+    constexpr int RINGS = WIDE ? 1 : SETS, CG = SETS;
     uint64_t *wfull = bars, *wfree = bars + GQ_PF_MAX_STAGES;
-    uint64_t *afull = bars + 2 * GQ_PF_MAX_STAGES, *afree = afull + GQ_PF_SLOTS * SETS, *done = afree + GQ_PF_SLOTS * SETS;
-    constexpr uint32_t TMEM_COLS = 256u * SETS, D_COLS = 128u * SETS;      // the A slots follow the accumulator
+    uint64_t *afull = bars + 2 * GQ_PF_MAX_STAGES, *afree = afull + GQ_PF_SLOTS * RINGS, *done = afree + GQ_PF_SLOTS * SETS;
+    constexpr uint32_t TMEM_COLS = 256u * SETS, D_COLS = TMEM_COLS - 32u * GQ_PF_SLOTS * RINGS;      // the A slots follow the accumulator
     constexpr int DEQ = 8 * SETS;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int part = (int)blockIdx.x % p.split, pair = (int)blockIdx.x / p.split, mt = blockIdx.y;      // a cluster: consecutive blockIdx.x
-    const int kb0 = (int)(((int64_t)part * p.nb) / p.split), nkb = (int)(((int64_t)(part + 1) * p.nb) / p.split) - kb0;
+    // grid (CG * split, units, batch tiles): a cluster is the parts of one unit, CG groups of two tiles each
+    const int half = (int)blockIdx.x % CG, part = (int)blockIdx.x / CG, unit = blockIdx.y, mt = blockIdx.z;
+    const int kb0 = (int)((uint32_t)(part * p.nb) / (uint32_t)p.split), nkb = (int)((uint32_t)((part + 1) * p.nb) / (uint32_t)p.split) - kb0;
+    const uint32_t leader = (uint32_t)(part * CG);       // cluster rank of the CTA that issues the pair's MMAs
+    __shared__ __align__(16) float s_ex[SETS == 1 ? 128 : 384];
 
-    // the two 64-row tiles of this CTA
-    const int32_t *d0 = p.desc + (int64_t)(2 * pair) * GQ_DESC_WORDS;
-    const bool has1 = 2 * pair + 1 < p.n_desc;
+    // the two 64-row tiles of this CTA (neither, in the second CTA of a last pair; only one, in the last CTA with any)
+    const int first = 2 * (unit * CG + half);
+    const bool has0 = first < p.n_desc, has1 = first + 1 < p.n_desc;
+    const int32_t *d0 = p.desc + (int64_t)(has0 ? first : p.n_desc - 1) * GQ_DESC_WORDS;
     const int32_t *d1 = has1 ? d0 + GQ_DESC_WORDS : d0;
-    const int type0 = d0[1], type1 = d1[1];
-    const int wb0 = 64 * gq_type_bytes(type0), wb1 = has1 ? 64 * gq_type_bytes(type1) : 0;
+    int types[2 * CG];                  // of all tiles of the pair, requested together (a load from global memory costs 700 cycles)
+#pragma unroll
+    for (int t = 0; t < 2 * CG; ++t) types[t] = p.desc[(int64_t)min(2 * unit * CG + t, p.n_desc - 1) * GQ_DESC_WORDS + 1];
+    const int off0 = d0[0], off1 = d1[0];
+    const int type0 = CG > 1 && half && has0 ? types[2 * CG - 2] : types[0], type1 = !has1 ? type0 : CG > 1 && half ? types[2 * CG - 1] : types[1];
+    const int wb0 = has0 ? 128 * p.half_bytes[type0 & 31] : 0, wb1 = has1 ? 128 * p.half_bytes[type1 & 31] : 0;
 
     // a codebook type the call's run_info did not announce has no table space, a wider type no stage: report and leave
-    // (nothing is allocated yet; the CTAs of a cluster work on the same tiles, so a cluster leaves as one)
-    {
-        const int k0 = gq_cb_kind(type0), k1 = gq_cb_kind(type1);
-        if ((k0 >= 0 && !((p.cb_mask >> k0) & 1)) || (k1 >= 0 && !((p.cb_mask >> k1) & 1)) || 2 * wb0 > p.wstage_bytes || 2 * wb1 > p.wstage_bytes) {
-            if (threadIdx.x == 0) { pdl_wait(); report_status(p.status, GQ_DEV_BAD_SHAPE); }      // after the preparation kernel has cleared the word
-            return;
-        }
+    // (nothing is allocated yet; every CTA of a cluster looks at all of its tiles, so a cluster leaves as one)
+    bool bad = false;
+#pragma unroll
+    for (int t = 0; t < 2 * CG; ++t) {
+        const int hb = p.half_bytes[types[t] & 31];
+        bad |= hb == 0 || 256 * hb > p.wstage_bytes || p.cb_at[types[t] & 31] == 1;
     }
-    if (threadIdx.x == 0) {
-        const uint32_t slabs = has1 ? 8 : 4;
-        for (int s = 0; s < p.wstages; ++s) { mbar_init(wfull + s, 1); mbar_init(wfree + s, slabs); }
-        for (int s = 0; s < GQ_PF_SLOTS * SETS; ++s) { mbar_init(afull + s, slabs + 1); mbar_init(afree + s, 1); }
+    if (bad) {
+        if (threadIdx.x == 0) { pdl_wait(); report_status(p.status, GQ_DEV_BAD_SHAPE); }      // after the preparation kernel has cleared the word
+        return;
+    }
+    const uint8_t *wsrc0 = p.packed + (int64_t)off0 * 16 + (int64_t)kb0 * wb0, *wsrc1 = p.packed + (int64_t)off1 * 16 + (int64_t)kb0 * wb1;
+    const auto load_weights = [&](int kb, int st) {
+        uint8_t *dst = wring + (size_t)st * p.wstage_bytes;
+        mbar_expect_tx(wfull + st, (uint32_t)(wb0 + wb1));
+        bulk_g2s(dst, wsrc0 + (int64_t)kb * wb0, (uint32_t)wb0, wfull + st);
+        if (wb1) bulk_g2s(dst + wb0, wsrc1 + (int64_t)kb * wb1, (uint32_t)wb1, wfull + st);
+    };
+    if (threadIdx.x == 32 * DEQ) {
+        const uint32_t slabs = has1 ? 8 : has0 ? 4 : 0;
+        // an A slot is full when all slabs of the pair are stored and each CTA's rows of the activation slice are there; the
+        // second CTA's own barrier sees its copy only, and its relay warp passes that on
+        const int in_pair = p.n_desc - 2 * unit * CG;
+        const uint32_t pair_slabs = (uint32_t)(in_pair < 2 * CG ? in_pair : 2 * CG) * 4;
+        for (int s = 0; s < p.wstages; ++s) { mbar_init(wfull + s, 1); mbar_init(wfree + s, slabs ? slabs : 1); }
+        for (int s = 0; s < GQ_PF_SLOTS * RINGS; ++s) mbar_init(afull + s, half ? 1 : pair_slabs + CG);
+        for (int s = 0; s < GQ_PF_SLOTS * SETS; ++s) mbar_init(afree + s, 1);
         mbar_init(done, 1);
         fence_barrier_init();
+        fence_proxy_async();
+        // the first weights do not wait for anything: on their way while the rest is set up
+        if (has0)
+            for (int kb = 0; kb < SETS && kb < nkb; ++kb) load_weights(kb, kb);
     }
-    if (warp == DEQ + 2) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+    __syncwarp();
+    if (warp == DEQ + 2) tmem_alloc<CG>(&tmem_slot, TMEM_COLS);
     // the codebook tables of the two tiles' types, each at its place among the tables of the run's types
-    if (gq_cb_kind(type0) >= 0) fill_codebook(type0, tables + gq_cb_offset(p.cb_mask, gq_cb_kind(type0)), threadIdx.x, blockDim.x);
-    if (gq_cb_kind(type1) >= 0 && type1 != type0)
-        fill_codebook(type1, tables + gq_cb_offset(p.cb_mask, gq_cb_kind(type1)), threadIdx.x, blockDim.x);
+    const int cb0 = p.cb_at[type0 & 31], cb1 = p.cb_at[type1 & 31];
+    if (cb0) fill_codebook(type0, tables + 16 * (cb0 - 2), threadIdx.x, blockDim.x);
+    if (cb1 && type1 != type0) fill_codebook(type1, tables + 16 * (cb1 - 2), threadIdx.x, blockDim.x);
     tc_fence_before();
-    __syncthreads();
+    __syncwarp();
+    if constexpr (CG > 1) cluster_sync_all();      // the other CTA's barriers exist before anything arrives on them
+    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     bool ok = true;
 
     if (warp == DEQ) {
-        // ---- weight producer: does not depend on the kernel in front of this one ----
-        if (lane == 0) {
-            const uint8_t *s0 = p.packed + (int64_t)d0[0] * 16 + (int64_t)kb0 * wb0;
-            const uint8_t *s1 = p.packed + (int64_t)d1[0] * 16 + (int64_t)kb0 * wb1;
-            for (int kb = 0, st = 0, round = 0; kb < nkb; ++kb) {
+        // ---- weight producer (the rest of the k-blocks): does not depend on the kernel in front of this one ----
+        if (lane == 0 && has0) {
+            for (int kb = SETS, st = SETS % p.wstages, round = SETS / p.wstages; kb < nkb; ++kb) {
                 if (round > 0 && !mbar_wait_parked(wfree + st, (round - 1) & 1)) { ok = false; break; }
-                uint8_t *dst = wring + (size_t)st * p.wstage_bytes;
-                mbar_expect_tx(wfull + st, (uint32_t)(wb0 + wb1));
-                bulk_g2s(dst, s0 + (int64_t)kb * wb0, (uint32_t)wb0, wfull + st);
-                if (wb1) bulk_g2s(dst + wb0, s1 + (int64_t)kb * wb1, (uint32_t)wb1, wfull + st);
+                load_weights(kb, st);
                 if (++st == p.wstages) { st = 0; ++round; }
             }
         }
         __syncwarp();
     } else if (warp == DEQ + 1) {
         // ---- activation producer.  Slice i takes stage i % bstages; the MMAs of slice i - bstages have read it when that
-        // slice's A slot comes free (bstages <= 4 SETS, so the slot cannot have been used again by then).  The copy completes on
+        // slice's A slot comes free (bstages <= 4 RINGS, so the slot cannot have been used again by then).  The copy completes on
         // the barrier of the slice's A slot, so that the MMA issuer waits once per slice ----
         if (lane == 0) {
             pdl_wait();
-            const uint8_t *src = p.xp + ((int64_t)mt * p.nb + kb0) * 4 * bbytes;
+            const uint8_t *src = p.xp + (((int64_t)mt * p.nb + kb0) * 4 * CG + half) * bbytes;
             for (int i = 0, st = 0; i < 4 * nkb; ++i) {
                 const int o = i - p.bstages;
                 if (o >= 0 && !mbar_wait_parked(afree + ((o >> 2) % SETS) * GQ_PF_SLOTS + (o & 3), ((o >> 2) / SETS) & 1)) { ok = false; break; }
-                uint64_t *full = afull + ((i >> 2) % SETS) * GQ_PF_SLOTS + (i & 3);
+                uint64_t *full = afull + ((i >> 2) % RINGS) * GQ_PF_SLOTS + (i & 3);
                 mbar_expect_tx(full, (uint32_t)bbytes);
-                bulk_g2s(smem + (size_t)st * bbytes, src + (int64_t)i * bbytes, (uint32_t)bbytes, full);
+                bulk_g2s(smem + (size_t)st * bbytes, src + (int64_t)i * CG * bbytes, (uint32_t)bbytes, full);
                 if (++st == p.bstages) st = 0;
             }
             pdl_trigger();
         }
         __syncwarp();
+    } else if (warp == DEQ + 2 && half) {
+        // ---- relay of the pair's second CTA: its activation rows are there -> the issuing CTA's barrier ----
+        for (int kb = 0; kb < nkb && ok; ++kb) {
+            const int slot0 = GQ_PF_SLOTS * (kb % RINGS);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (!mbar_wait(afull + slot0 + j, (uint32_t)(kb / RINGS) & 1u)) { ok = false; break; }
+                if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(afull + slot0 + j), leader));
+            }
+            __syncwarp();
+        }
     } else if (warp == DEQ + 2) {
         // ---- MMA issuer: the warp waits as one and a thread chosen by elect.sync issues, so that addresses and descriptors
         // stay in uniform registers (issued from a `lane == 0` branch an MMA cost the thread a hundred cycles) ----
-        const uint32_t idesc = umma_idesc(128, N);
+        const int nmma = WIDE ? N >> 1 : N;           // an MMA takes up to 256 batch rows: the wide tile is two of them
+        const uint32_t idesc = umma_idesc(128 * CG, nmma);
+        const uint16_t ctas = (uint16_t)(3u << leader);
         const uint64_t bdesc0 = umma_desc(smem_u32(smem));
         const uint32_t bstep = (uint32_t)bbytes >> 4, bwrap = bstep * (uint32_t)p.bstages;
         uint32_t boff = 0;
         for (int kb = 0; kb < nkb && ok; ++kb) {
-            const int set = kb % SETS;
-            const uint32_t parity = (uint32_t)(kb / SETS) & 1u;
-            uint64_t *full = afull + GQ_PF_SLOTS * set, *free = afree + GQ_PF_SLOTS * set;
-            const uint32_t ta = tmem + D_COLS + 32u * GQ_PF_SLOTS * set;
+            const int ring = kb % RINGS;
+            const uint32_t parity = (uint32_t)(kb / RINGS) & 1u;
+            uint64_t *full = afull + GQ_PF_SLOTS * ring, *free = afree + GQ_PF_SLOTS * (kb % SETS);
+            const uint32_t ta = tmem + D_COLS + 32u * GQ_PF_SLOTS * ring;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if (!mbar_wait(full + j, parity)) { ok = false; break; }
@@ -288,9 +370,13 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
                 if (elect_one()) {
                     const uint64_t bd = bdesc0 + boff;
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) umma_ts_f16(tmem, ta + 32 * j + 8 * kk, bd + 2 * kk, idesc, (j > 0 || kk > 0) ? 1u : (uint32_t)(kb > 0));
-                    umma_commit(free + j);        // the slot and the activation stage may be overwritten once these MMAs have read them
-                    if (j == 3 && kb + 1 == nkb) umma_commit(done);
+                    for (int kk = 0; kk < 4; ++kk) {
+                        const uint32_t acc = (j > 0 || kk > 0) ? 1u : (uint32_t)(kb > 0);
+                        umma_ts_f16<CG>(tmem, ta + 32 * j + 8 * kk, bd + 2 * kk, idesc, acc);
+                        if constexpr (WIDE) umma_ts_f16<CG>(tmem + nmma, ta + 32 * j + 8 * kk, bd + 8 / CG * nmma + 2 * kk, idesc, acc);      // 128 bytes a row
+                    }
+                    // the slot and the activation stage may be overwritten once these MMAs have read them
+                    umma_commit<CG>(j == 3 && kb + 1 == nkb ? done : free + j, ctas);
                 }
                 boff += bstep;
                 if (boff == bwrap) boff = 0;
@@ -299,18 +385,20 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
         }
     } else {
         // ---- dequantisers: warp w reaches the TMEM lanes of partition w % 4, which hold slabs 2 (w % 4) and + 1 ----
-        const int w = warp & 7, slab = 2 * (w & 3) + (w >> 2), set = warp >> 3;
+        const int w = warp & 7, slab = 2 * (w & 3) + (w >> 2), set = warp >> 3, ring = set % RINGS;
         const int type = slab < 4 ? type0 : type1;
-        if (slab < 4 || has1) {
+        if (slab < 4 ? has0 : has1) {
             DecAux aux;
-            aux.grid = reinterpret_cast<const uint2 *>(tables + (gq_cb_kind(type) >= 0 ? gq_cb_offset(p.cb_mask, gq_cb_kind(type)) : 0));
+            const int cb = slab < 4 ? cb0 : cb1;
+            aux.grid = reinterpret_cast<const uint2 *>(tables + (cb ? 16 * (cb - 2) : 0));
             aux.iq4 = iq4_table_biased();
             PfRings r;
             r.wring = wring; r.wstage_bytes = p.wstage_bytes; r.wstages = p.wstages;
-            r.wfull = wfull; r.wfree = wfree; r.afull = afull + GQ_PF_SLOTS * set; r.afree = afree + GQ_PF_SLOTS * set;
-            const int slab_off = (slab < 4 ? 0 : wb0) + (slab & 3) * 16 * gq_type_bytes(type);
-            const uint32_t ta = tmem + D_COLS + 32u * GQ_PF_SLOTS * set + ((uint32_t)(16 * slab) << 16);
-#define GQ_PF(T) case T: ok = pf_dequant<T, SETS>(r, slab_off, set, nkb, ta, aux, lane); break;
+            r.wfull = wfull; r.wfree = wfree; r.afree = afree;
+            r.afull = map_to_rank(smem_u32(afull + GQ_PF_SLOTS * ring), CG > 1 ? leader : cluster_ctarank());
+            const int slab_off = (slab < 4 ? 0 : wb0) + (slab & 3) * 32 * p.half_bytes[type & 31];
+            const uint32_t ta = tmem + D_COLS + 32u * GQ_PF_SLOTS * ring + ((uint32_t)(16 * slab) << 16);
+#define GQ_PF(T) case T: ok = pf_dequant<T, SETS, RINGS>(r, slab_off, set, nkb, ta, aux, lane); break;
             switch (type) {
                 GQ_PF(GQ_Q4_0) GQ_PF(GQ_Q5_0) GQ_PF(GQ_Q8_0) GQ_PF(GQ_Q2_K) GQ_PF(GQ_Q3_K) GQ_PF(GQ_Q4_K)
                 GQ_PF(GQ_Q5_K) GQ_PF(GQ_Q6_K) GQ_PF(GQ_IQ4_NL) GQ_PF(GQ_IQ3_S) GQ_PF(GQ_IQ4_XS) GQ_PF(GQ_IQ3_XXS)
@@ -318,19 +406,21 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
             }
 #undef GQ_PF
         }
+        pdl_wait();       // y may be read, and ex is written, by what runs in front
+        for (int i = threadIdx.x; i < N; i += 32 * DEQ) s_ex[i] = p.ex[mt * N + i];
         if (ok && !mbar_wait(done, 0)) ok = false;
         __syncwarp();
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * DEQ) : "memory");
         tc_fence_after();
-        pdl_wait();       // y may be read, and ex is written, by what runs in front
     }
 
     // ---- epilogue: warps 0 .. DEQ-1; lane l of partition q is row 32 q + l of the pair of tiles ----
     const int q = warp & 3, e = warp >> 2, feat = 32 * q + lane;
     const int32_t *dt = (feat < 64) ? d0 : d1;
     const int rt = feat & 63;
-    const bool row_ok = (feat < 64 || has1) && rt < dt[3];
+    const bool tile_ok = feat < 64 ? has0 : has1, row_ok = tile_ok && rt < dt[3];
     const int64_t col = (int64_t)dt[2] + rt;
-    const bool pair_ok = (feat < 64 || has1) && (rt | 1) < dt[3] && !(p.ldy & 1) && !((reinterpret_cast<uintptr_t>(p.y) + 2 * (uintptr_t)(col - (lane & 1))) & 3);
+    const bool pair_ok = tile_ok && (rt | 1) < dt[3] && !(p.ldy & 1) && !((reinterpret_cast<uintptr_t>(p.y) + 2 * (uintptr_t)(col - (lane & 1))) & 3);
     const uint32_t td = tmem + ((uint32_t)(32 * q) << 16);
     if (p.split == 1) {
         if (warp < DEQ && ok) {
@@ -338,7 +428,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
             for (int c = 8 * e; c < N; c += 8 * (DEQ / 4)) {
                 uint32_t a[8];
                 tmem_ld_32x32b_x8(td + c, a);
-                const float4 e0 = *reinterpret_cast<const float4 *>(p.ex + mt * N + c), e1 = *reinterpret_cast<const float4 *>(p.ex + mt * N + c + 4);
+                const float4 e0 = *reinterpret_cast<const float4 *>(s_ex + c), e1 = *reinterpret_cast<const float4 *>(s_ex + c + 4);
                 tmem_wait_ld();
                 const float es[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
                 float v[8];
@@ -348,7 +438,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
             }
         }
     } else {
-        // columns [r ch, (r + 1) ch) are summed and stored by CTA r of the cluster; slot s of its buffer is CTA s's part, as
+        // columns [r ch, (r + 1) ch) are summed and stored by the CTA of part r; slot s of its buffer is part s's share, as
         // [ch / 4][128 rows] of four columns each: 16-byte stores and loads, one per lane side by side
         const int S = p.split, ch = ((N + S - 1) / S + 7) & ~7;
         float4 *buf = reinterpret_cast<float4 *>(smem);
@@ -361,7 +451,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
                 uint32_t a[8];
                 tmem_ld_32x32b_x8(td + c, a);
                 tmem_wait_ld();
-                const uint32_t dst = map_to_rank(mine, (uint32_t)r) + (uint32_t)((c - r * ch) >> 2) * 2048;
+                const uint32_t dst = map_to_rank(mine, (uint32_t)(r * CG + half)) + (uint32_t)((c - r * ch) >> 2) * 2048;
                 st_cluster_f4(dst, __uint_as_float(a[0]), __uint_as_float(a[1]), __uint_as_float(a[2]), __uint_as_float(a[3]));
                 st_cluster_f4(dst + 2048, __uint_as_float(a[4]), __uint_as_float(a[5]), __uint_as_float(a[6]), __uint_as_float(a[7]));
             }
@@ -380,7 +470,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
                     v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
                     v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
                 }
-                const float4 e0 = *reinterpret_cast<const float4 *>(p.ex + mt * N + c), e1 = *reinterpret_cast<const float4 *>(p.ex + mt * N + c + 4);
+                const float4 e0 = *reinterpret_cast<const float4 *>(s_ex + c), e1 = *reinterpret_cast<const float4 *>(s_ex + c + 4);
                 const float es[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[j] *= es[j];
@@ -394,10 +484,12 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
         for (int i = 0; i < 100; ++i) __nanosleep(10000);
     }
     tc_fence_before();
-    __syncthreads();
+    __syncwarp();
+    if constexpr (CG > 1) cluster_sync_all();      // tensor memory is given back by both CTAs, after both have read theirs
+    else __syncthreads();
     if (warp == DEQ + 2) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+        tmem_dealloc<CG>(tmem, TMEM_COLS);
     }
 }
 
@@ -414,14 +506,18 @@ __device__ __forceinline__ float amax8(const uint4 &v) {
 
 // activation preparation for the prefill path: bf16 row -> fp16 scaled by an exact power of two, stored in the
 // MMA's shared-memory layout (tiles of N rows x 64 k, K-major, 16-byte chunks XOR-swizzled by row % 8) so the
-// kernel's producer moves a whole k-slice with one bulk copy.  One CTA per row of the padded batch; the row is read once and
-// kept in registers between the maximum and the conversion (rows up to 512 * 5 * 8 = 20480 activations).
-#define GQ_PF_PREP_THREADS 512
+// kernel's producer moves a whole k-slice with one bulk copy.  For CTA pairs a slice holds the rows of the first CTA, then
+// those of the second: of every `nmma` rows that an MMA takes, the first half is the first CTA's.  One CTA per row of the padded batch; the row is read once and
+// kept in registers between the maximum and the conversion (the first 128 * 5 * 8 = 5120 activations).  128 threads of few
+// registers, so that these CTAs fit beside those of a matrix kernel: they are in place when the kernel in front ends, and the
+// matrix kernel behind them gets its SMs, fetches weights and decodes while they run (with 512 threads a CTA kept it off its SM).
+#define GQ_PF_PREP_THREADS 128
 #define GQ_PF_PREP_VECS 5
-__global__ void __launch_bounds__(GQ_PF_PREP_THREADS) prep_x_prefill_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int K, int M, int N,
+__global__ void __launch_bounds__(GQ_PF_PREP_THREADS, 10) prep_x_prefill_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int K, int M, int N, int nmma,
                                                                             float *__restrict__ ex, uint8_t *__restrict__ xp, int *status) {
     __shared__ float red[GQ_PF_PREP_THREADS / 32];
-    const int m = blockIdx.x, r = m % N, nvec = K >> 3;
+    const int m = blockIdx.x, n = m % N, nvec = K >> 3, hn = nmma >> 1;
+    const int r = nmma ? (n % nmma) / hn * (N >> 1) + n / nmma * hn + n % hn : n;
     uint8_t *dst = xp + (int64_t)(m / N) * (K / 64) * (N * 128) + r * 128;
     const int phase = r & 7;
     pdl_trigger();    // the kernel behind this one may start fetching weights
