@@ -1342,46 +1342,66 @@ struct DescShards {
     DescShard s[GQ_MAX_DEVICE_SHARDS];
     int n;
 };
-__global__ void __launch_bounds__(256) build_descs_kernel(const DescShards sh, int nb, int split, int rows, int32_t *__restrict__ desc) {
+struct DescSplits {
+    int split[GQ_MAX_DEVICE_SPLITS], n;
+};
+__global__ void __launch_bounds__(256) build_descs_kernel(const DescShards sh, const DescSplits sp, int nb, int tiles, int rows, int32_t *__restrict__ desc) {
     const int row = blockIdx.x * 256 + threadIdx.x;
     if (row >= rows) return;
-    int tile = row / split, i = 0;
+    int r0 = row, i = 0, k = 0;
+    while (k + 1 < sp.n && r0 >= tiles * sp.split[k]) r0 -= tiles * sp.split[k++];      // the table, then the row in it
+    const int split = sp.split[k];
+    int tile = r0 / split;
+    const int part = r0 - tile * split;
     while (i + 1 < sh.n && tile >= sh.s[i].n_tiles) tile -= sh.s[i++].n_tiles;
     __align__(16) int32_t r[GQ_DESC_WORDS];
-    desc_row(sh.s[i], nb, split, tile, row % split, r);
+    desc_row(sh.s[i], nb, split, tile, part, r);
     int4 *o = reinterpret_cast<int4 *>(desc + (int64_t)row * GQ_DESC_WORDS);
     o[0] = make_int4(r[0], r[1], r[2], r[3]);
     o[1] = make_int4(r[4], r[5], r[6], r[7]);
 }
 
-extern "C" int64_t gq_build_descs_device(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split, int32_t *desc_dev,
-                                         void *stream) {
-    if (n_shards > GQ_MAX_DEVICE_SHARDS) return GQ_ERR_LIMIT;
-    if (!desc_dev || ((uintptr_t)desc_dev & 15)) return GQ_ERR_ARG;
+extern "C" int64_t gq_build_descs_device(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int n_splits, const int32_t *splits,
+                                         int32_t *desc_dev, void *stream) {
+    if (n_shards > GQ_MAX_DEVICE_SHARDS || n_splits > GQ_MAX_DEVICE_SPLITS) return GQ_ERR_LIMIT;
+    if (!desc_dev || ((uintptr_t)desc_dev & 15) || n_splits <= 0 || !splits) return GQ_ERR_ARG;
     DescShards sh;
-    const int64_t rows = desc_shards(n_shards, types, n_outs, K, split, sh.s);
-    if (rows <= 0) return rows;
+    DescSplits sp;
+    const int64_t tiles = desc_shards(n_shards, types, n_outs, K, 1, sh.s);
+    if (tiles < 0) return tiles;
+    int64_t rows = 0;
+    for (int i = 0; i < n_splits; ++i) {
+        if (splits[i] < 1 || splits[i] > K / GQ_QK) return GQ_ERR_ARG;
+        sp.split[i] = splits[i];
+        rows += tiles * splits[i];
+    }
+    if (rows == 0) return 0;
     if (rows > 0x7ffffff0) return GQ_ERR_LIMIT;
-    sh.n = n_shards;
-    build_descs_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, (cudaStream_t)stream>>>(sh, (int)(K / GQ_QK), split, (int)rows, desc_dev);
+    sh.n = n_shards; sp.n = n_splits;
+    build_descs_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, (cudaStream_t)stream>>>(sh, sp, (int)(K / GQ_QK), (int)tiles, (int)rows, desc_dev);
     GQ_LAUNCHED();
     return rows;
 }
 
 extern "C" int gq_split_for(int64_t n_tiles, int64_t nb, int64_t M, int avg_bytes_per_256, int sm_count) {
-    (void)M; (void)avg_bytes_per_256;
+    (void)avg_bytes_per_256;
     if (n_tiles <= 0 || nb <= 0) return 1;
     if (sm_count <= 0) sm_count = 148;
-    // from sweeps on B200 (Q4_K / Q2_K / IQ3_S / IQ4_XS; 80-, 112-, 272- and 544-tile layers at K 5120 and 17408): the
+    // from sweeps on B200 (Q4_K / Q2_K / IQ3_S / IQ4_XS; 80- to 544-tile layers at K 5120 and 17408): the
     // largest split that (a) leaves a CTA at least three k-blocks, (b) stays inside one thread-block cluster (8), and
-    // (c) keeps the launch in one wave of four CTAs per SM — counting that clusters cannot use every slot: a launch
-    // of clusters of S fills at most about 1 - 0.03 (S - 1) of them before a second wave starts
-    const int64_t slots = 4 * (int64_t)sm_count;
+    // (c) keeps the launch in one wave of the CTAs that the kernel for M rows has resident on an SM (four to 8 rows, three to 16,
+    // two above) — counting that clusters cannot use every slot: a launch of clusters of S fills at most about 1 - 0.03 (S - 1)
+    // of them before a second wave starts.  (With four for every M, 80 tiles at K 5120 ran as 480 CTAs: Q4_K 14.2 us at 16 rows
+    // and 23.8 at 27, with the splits of this rule, 4 and 3, 10.4 and 16.7.)
+    const int64_t per_sm = M <= 8 ? 4 : M <= 16 ? 3 : 2, slots = per_sm * sm_count;
     int64_t s_max = nb / 3;
     if (s_max > 8) s_max = 8;
     int64_t s = 1;
     for (int64_t c = 2; c <= s_max; ++c)
         if (c * n_tiles * 100 <= slots * (100 - 3 * (c - 1))) s = c;
+    // 9 .. 16 rows, one CTA short of what an SM holds: two parts in a wave and a quarter are 13 - 20 % faster (272 tiles: Q4_K
+    // 25.8 -> 22.4 us, IQ3_S 34.6 -> 28.0)
+    if (per_sm == 3 && s == 1 && s_max >= 2 && n_tiles * 3 < slots * 2) s = 2;
     if (s > nb) s = nb;
     return (int)s;
 }

@@ -11,6 +11,7 @@ from __future__ import annotations
 import contextlib
 
 import ctypes
+import functools
 from typing import Sequence
 
 import numpy as np
@@ -21,7 +22,7 @@ from ._lib import DESC_WORDS, MAX_GEMV_ROWS, GqError, check, lib, native
 
 TILE_TYPES = F.SUPPORTED_TYPES   # every supported type is held tile-major (the reference: GLUON_TILE_TYPES)
 GEMV_MAX_ROWS = MAX_GEMV_ROWS    # the grouped kernel's own limit (the C ABI accepts up to 64 rows)
-MAX_DEVICE_SHARDS = 8            # GQ_MAX_DEVICE_SHARDS
+MAX_DEVICE_SHARDS = MAX_DEVICE_SPLITS = 8     # GQ_MAX_DEVICE_SHARDS, GQ_MAX_DEVICE_SPLITS
 DECODE_MAX_ROWS = 32             # row-count dispatch threshold: above it the tcgen05 kernel takes over
 
 def _stream_ptr(t: torch.Tensor) -> int:
@@ -86,21 +87,30 @@ def build_descs(wtypes: Sequence[int], n_outs: Sequence[int], k: int, split: int
 def build_descs_on(device, wtypes: Sequence[int], n_outs: Sequence[int], k: int, splits: Sequence[int]) -> list[torch.Tensor]:
     """The descriptor tables of several splits on a device, written there by a kernel (no copy, no synchronisation)."""
     device = torch.device(device)
-    if device.type != "cuda" or len(wtypes) > MAX_DEVICE_SHARDS:
+    if device.type != "cuda" or len(wtypes) > MAX_DEVICE_SHARDS or len(splits) > MAX_DEVICE_SPLITS:
         return [torch.from_numpy(build_descs(wtypes, n_outs, k, s)).to(device) for s in splits]
-    types, rows = _i32_array(wtypes), _i64_array(n_outs)
     tiles = sum(-(-int(n) // 64) for n in n_outs)
-    descs = list(torch.empty((tiles * sum(splits), DESC_WORDS), dtype=torch.int32, device=device).split([tiles * s for s in splits]))
+    buf = torch.empty((tiles * sum(splits), DESC_WORDS), dtype=torch.int32, device=device)
     with torch.cuda.device(device):
-        for s, d in zip(splits, descs):
-            got = check(lib().gq_build_descs_device(len(wtypes), types, rows, int(k), int(s), d.data_ptr(), _stream_ptr(d)), "gq_build_descs_device")
-            assert got == d.shape[0]
-    return descs
+        check(lib().gq_build_descs_device(len(wtypes), _i32_array(wtypes), _i64_array(n_outs), int(k), len(splits), _i32_array(splits),
+                                          buf.data_ptr(), _stream_ptr(buf)), "gq_build_descs_device")
+    return list(buf.split([tiles * s for s in splits]))
 
 
 def grouped_split_for(n_tiles: int, nb: int, m: int | None = None, block_bytes: int | None = None, sms: int | None = None) -> int:
     """Split-K of a grouped launch (reference: grouped_split_for, gguf-plugin/gluon/tiles_grouped.py:237-250)."""
-    return int(lib().gq_split_for(int(n_tiles), int(nb), int(m or 0), int(block_bytes or 0), int(sms or sm_count())))
+    return _split_for(int(n_tiles), int(nb), int(m or 0), int(block_bytes or 0), int(sms or sm_count()))
+
+
+@functools.lru_cache(maxsize=1024)      # a question per call otherwise; a model has a few dozen of them
+def _split_for(n_tiles: int, nb: int, m: int, block_bytes: int, sms: int) -> int:
+    return int(lib().gq_split_for(n_tiles, nb, m, block_bytes, sms))
+
+
+ROW_CLASSES = (8, 16, 32, 64)    # the row counts that end a form of the grouped kernel: the split policy knows no finer ones
+
+
+_ROW_CLASS = [next(c for c in ROW_CLASSES if m <= c) for m in range(GEMV_MAX_ROWS + 1)]
 
 
 _RUN_INFO: dict[tuple[int, ...], int] = {}      # bounded by the combinations of types a model's merged layers have
@@ -248,8 +258,7 @@ def prepare_grouped_layer(tiles_list: Sequence[torch.Tensor], n_outs: Sequence[i
     n_tiles = sum(-(-int(n) // 64) for n in n_outs)
     block_bytes = int(round(sum(int(n) * F.BYTES_PER_256[int(w)] for n, w in zip(n_outs, wtypes)) / max(1, n_total)))
     sms = sm_count(packed.device)
-    # the library's policy looks at the run's shape only: one question answers every row count
-    splits = sorted({grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sms) for m in list(ms)[:1]} | {1})
+    splits = sorted({grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sms) for m in {_ROW_CLASS[m] for m in ms}} | {1})
     descs = build_descs_on(packed.device, wtypes, n_outs, nb * 256, splits)
     return packed, views, descs, splits, nb, block_bytes
 
@@ -490,9 +499,10 @@ class NativeRun:
             return
         packed, descs, splits, _, nb, block_bytes = group
         n_tiles = sum(-(-int(n) // 64) for n in n_outs)
-        split = grouped_split_for(n_tiles, nb, block_bytes=block_bytes, sms=sm_count(packed.device))      # the same for every row count
-        self._run = native().Run(packed, descs, splits, [int(n) for n in n_outs], [int(t) for t in wtypes], nb, [split] * (DECODE_MAX_ROWS + 1),
-                                 DECODE_MAX_ROWS, PRE_MAX_ROWS)
+        sms = sm_count(packed.device)
+        split = {m: grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sms) for m in ROW_CLASSES}
+        self._run = native().Run(packed, descs, splits, [int(n) for n in n_outs], [int(t) for t in wtypes], nb,
+                                 [split[c] for c in _ROW_CLASS[:DECODE_MAX_ROWS + 1]], DECODE_MAX_ROWS, PRE_MAX_ROWS)
 
     def __reduce__(self):
         return NativeRun, ()

@@ -86,13 +86,16 @@ int gq_dequant_rows(int type, const void *raw_dev, int64_t n_rows, int64_t K, in
 int64_t gq_desc_rows(int n_shards, const int64_t *n_outs, int split);
 int64_t gq_build_descs(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split, int32_t *desc_host);
 
-/* The same table written on the device (desc_dev has room for gq_desc_rows rows, 16-byte aligned) by a kernel on `stream`, so
- * that loading a layer copies and waits for nothing.  Up to GQ_MAX_DEVICE_SHARDS shards, GQ_ERR_LIMIT beyond. */
+/* The tables of several splits written on the device, back to back (desc_dev has room for the gq_desc_rows of all of them,
+ * 16-byte aligned), by one kernel on `stream`, so that loading a layer copies and waits for nothing.  Returns the number of
+ * rows.  Up to GQ_MAX_DEVICE_SHARDS shards and GQ_MAX_DEVICE_SPLITS splits, GQ_ERR_LIMIT beyond. */
 #define GQ_MAX_DEVICE_SHARDS 8
-int64_t gq_build_descs_device(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split, int32_t *desc_dev, void *stream);
+#define GQ_MAX_DEVICE_SPLITS 8
+int64_t gq_build_descs_device(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int n_splits, const int32_t *splits,
+                              int32_t *desc_dev, void *stream);
 
-/* Split-K of a grouped launch: n_tiles output tiles, nb k-blocks, M batch rows, avg_bytes_per_256 of
- * the run, on a device with sm_count SMs.  Always in [1, nb] and at most 8 (the split then stays inside
+/* Split-K of a grouped launch: n_tiles output tiles, nb k-blocks, M batch rows (it matters whether there are up to 8, up to
+ * 16 or more), avg_bytes_per_256 of the run, on a device with sm_count SMs.  Always in [1, nb] and at most 8 (the split then stays inside
  * one thread-block cluster); any other value in [1, nb] is also valid for the calls below.
  * Reference: grouped_split_for (gguf-plugin/gluon/tiles_grouped.py:209-250), re-derived for 148 SMs. */
 int gq_split_for(int64_t n_tiles, int64_t nb, int64_t M, int avg_bytes_per_256, int sm_count);
