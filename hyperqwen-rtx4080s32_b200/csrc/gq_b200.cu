@@ -746,7 +746,15 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
             for (int j = 0; j < 4; ++j) tot[j] = bf[nt][j];
         } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) tot[j] = (j < 2 ? d0 : d1) * fmaf((float)(aH[nt][j] + bH[nt][j]), 256.0f, (float)(aL[nt][j] + bL[nt][j]));
+            for (int j = 0; j < 4; ++j) {
+                if constexpr (D::SCHEME == GQ_FOLD) {
+                    // the even and the odd k-steps together: below 2^24 (128 weights of at most 180, and 4 * 45, times 255), exact as float
+                    const int h = (aH[nt][j] << D::ODD_SHIFT) + bH[nt][j], l = (aL[nt][j] << D::ODD_SHIFT) + bL[nt][j];
+                    tot[j] = (j < 2 ? d0 : d1) * (fmaf((float)h, 256.0f, (float)l) * (1.0f / (1 << D::ODD_SHIFT)));
+                } else {
+                    tot[j] = (j < 2 ? d0 : d1) * fmaf((float)aH[nt][j], 256.0f, (float)aL[nt][j]);
+                }
+            }
         }
         if constexpr (D::NCORR > 0) {
             const uint8_t *sb = xs + (nt * 8 + g) * GQ_X8_ROW + GQ_X8_SUMS + 8 * t;
@@ -889,7 +897,8 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
     const int stage_bytes = wmax + xbytes;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)stages * stage_bytes);
     uint64_t *empty = full + stages;
-    uint2 *grid_s = reinterpret_cast<uint2 *>(empty + stages);
+    uint64_t *parts = empty + stages;          // push-form split-K: per consumer warp, the other splits' sums have landed
+    uint2 *grid_s = reinterpret_cast<uint2 *>(parts + GQ_CONSUMER_WARPS);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int32_t *d = p.desc + (int64_t)blockIdx.x * GQ_DESC_WORDS;
@@ -915,6 +924,8 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, GQ_CONSUMER_WARPS); }
+        if (p.cluster_push)
+            for (int w = 0; w < GQ_CONSUMER_WARPS; ++w) mbar_init(parts + w, 1);
         fence_barrier_init();
     }
     __syncthreads();
@@ -944,7 +955,8 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
         }
         asm volatile("bar.sync 1, %0;" ::"n"(32 * GQ_CONSUMER_WARPS) : "memory");
     }
-    // push-form split-K: a CTA may store into the split-0 CTA's shared memory only once that CTA is known to run;
+    // push-form split-K: a CTA may store into the split-0 CTA's shared memory only once that CTA is known to run and has
+    // initialised its barriers;
     // every thread enters this rendezvous here and collects it just before its first remote store (or before the
     // closing barrier), long after everyone has arrived
     const bool push = p.cluster && p.cluster_push;
@@ -988,9 +1000,9 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
             }
         }
         if (!p.cluster) return;
-        if (push) cluster_wait();
-        cluster_sync_all();     // the reduction's cluster barriers need every thread of every CTA
-        if (!push) cluster_sync_all();
+        if (push) { cluster_wait(); return; }
+        cluster_sync_all();     // the pull form's cluster barriers need every thread of every CTA
+        cluster_sync_all();
         return;
     }
 
@@ -1050,18 +1062,22 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
     float4 *red = reinterpret_cast<float4 *>(reinterpret_cast<uint8_t *>(grid_s) + p.cb_bytes);
     if (push) {
         cluster_wait();         // the rendezvous entered at the start: every CTA of the cluster is running
-        // split-K inside a cluster, push form: the CTAs of splits 1.. store their accumulators into their slot of the
-        // split-0 CTA's scratch through distributed shared memory; one cluster barrier (release / acquire) later that
-        // CTA adds the slots from its own shared memory, in split order, and writes bf16 once.  No partial sums in
-        // HBM, no second kernel, fixed order of the additions.
+        // split-K inside a cluster, push form: the warps of splits 1.. store their accumulators into their slot of the split-0
+        // CTA's scratch through distributed shared memory; that CTA's warp of the same columns adds the slots from its own shared
+        // memory, in split order, and writes bf16 once.  No partial sums in HBM, no second kernel, fixed order of the additions.
+        // The stores are st.async, whose bytes the receiving warp's mbarrier counts: neither side needs a fence or a barrier at
+        // cluster scope, and the senders leave at once.
         if (split_idx != 0) {
             const uint32_t dst = map_to_rank(smem_u32(red), 0u) + (uint32_t)((split_idx - 1) * GQ_CONSUMER_WARPS * MT * 512);
+            const uint32_t bar = map_to_rank(smem_u32(parts + warp), 0u);
 #pragma unroll
             for (int nt = 0; nt < MT; ++nt)
-                st_cluster_f4(dst + (uint32_t)(((warp * MT + nt) * 32 + lane) * 16), acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
+                st_async_f4(dst + (uint32_t)(((warp * MT + nt) * 32 + lane) * 16), acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3], bar);
+            return;
         }
-        cluster_sync_all();
-        if (split_idx != 0) return;
+        if (lane == 0) mbar_expect_tx(parts + warp, (uint32_t)((p.split - 1) * MT * 512));
+        __syncwarp();
+        if (!mbar_wait(parts + warp, 0)) { ok = false; if (lane == 0) report_status(p.status, GQ_DEV_TIMEOUT); }
         for (int s = 1; s < p.split; ++s) {
 #pragma unroll
             for (int nt = 0; nt < MT; ++nt) {
@@ -1415,7 +1431,7 @@ template <int MT, int MINB, int FORM, int ONLY>
 static int launch_gemv(const GemvParams &p, int64_t n_desc, cudaStream_t stream) {
     constexpr int xbytes = gq_stage_xbytes<MT, FORM>();
     const int stage_bytes = p.wbytes_max + xbytes;
-    const size_t smem = (size_t)p.stages * stage_bytes + (size_t)p.stages * 16 + (size_t)p.cb_bytes +
+    const size_t smem = (size_t)p.stages * stage_bytes + (size_t)p.stages * 16 + 8 * GQ_CONSUMER_WARPS + (size_t)p.cb_bytes +
                         (size_t)GQ_CONSUMER_WARPS * MT * 512 * (p.cluster_push ? p.split - 1 : 1);
     if (smem > 232448) return GQ_ERR_LIMIT;
     // opt in once per device to the largest dynamic shared memory a CTA can have
@@ -1539,7 +1555,7 @@ static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ld
         const int xb = !form ? 8 * mt * GQ_XROW_BYTES : mt == 1 ? gq_stage_xbytes<1, 1>() : mt == 2 ? gq_stage_xbytes<2, 1>() : gq_stage_xbytes<4, 1>();
         const int stage_bytes = p.wbytes_max + xb;
         // (an SM has 228 KB of shared memory and the system keeps 1 KB of it per resident CTA)
-        const int fixed = 64 + p.cb_bytes + 1024, red1 = GQ_CONSUMER_WARPS * mt * 512;
+        const int fixed = 64 + 8 * GQ_CONSUMER_WARPS + p.cb_bytes + 1024, red1 = GQ_CONSUMER_WARPS * mt * 512;
         // split-K in a cluster: the push form of the reduction needs a scratch slot per other split in every CTA; it
         // is used when that costs no resident CTA (the ring then has three stages; its depth does not matter)
         if (p.cluster) {

@@ -383,13 +383,16 @@ struct Dec8<GQ_Q2_K> {
             dd[h] = ld4(slab + 1024 + 256 + 4 * row);
         }
     }
-    // run R = 8n + 2j + u of row half H: bit pair j of word (n, 2H + u), times the run's scale
+    // run R = 8n + 2j + u of row half H: bit pair j of word (n, 2H + u), times the run's scale.  The odd bit pairs stay two bits
+    // up (at most 4 * 45 = 180): their k-steps have accumulators of their own, ODD_SHIFT says by how much those are too large
     template <int R, int H>
     GQ_HD uint32_t quad() const {
         constexpr int n = R >> 3, j = (R >> 1) & 3, u = R & 1;
-        const uint32_t f = (w4(q[n], 2 * H + u) >> (2 * j)) & 0x03030303u;
+        const uint32_t w = w4(q[n], 2 * H + u);
+        const uint32_t f = (j >> 1 ? w >> 4 : w) & ((j & 1) ? 0x0c0c0c0cu : 0x03030303u);
         return f * (uint32_t)ubyte<(R & 3)>(w4(sc[H], R >> 2));
     }
+    static constexpr int ODD_SHIFT = 2;
     template <int S>
     GQ_HD void step(uint32_t (&a)[4]) const {
         a[0] = quad<2 * S, 0>(); a[1] = quad<2 * S, 1>(); a[2] = quad<2 * S + 1, 0>(); a[3] = quad<2 * S + 1, 1>();
@@ -416,6 +419,7 @@ struct Dec8<GQ_Q3_K> {
     static constexpr int SCHEME = GQ_FOLD;
     static constexpr bool A_SIGNED = false;
     static constexpr int NCORR = 1;
+    static constexpr int ODD_SHIFT = 0;
     uint4 q[3];
     uint32_t sv[2][4];   // the sixteen 6-bit scales of a row as bytes (raw value, 0..63)
     uint32_t ss[2][4];   // the same minus 32, as int8 bytes
