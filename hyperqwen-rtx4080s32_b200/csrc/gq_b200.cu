@@ -138,7 +138,7 @@ __host__ __device__ inline int64_t align256(int64_t v) { return (v + 255) & ~(in
 
 // The same row in the integer form used for 1..16 batch rows: per k-block and batch row the activations as 16-bit
 // fixed point (x * 2^e, e chosen per row and k-block so that the largest magnitude lands in [2^14, 2^15)), split into
-// a signed high-byte plane (256 B) and an unsigned low-byte plane (256 B), then the sixteen 16-weight run sums
+// two signed bytes, x = 256 hi + lo: a plane of high bytes (256 B) and one of low bytes (256 B), then the sixteen 16-weight run sums
 // (times 2^-6) as fp16 hi parts (32 B) and lo parts (32 B).  Inside a plane the bytes are ordered for the lane that
 // reads them: 16-byte unit 4*i + t holds, for runs 4i..4i+3, the quad 4t..4t+3 with bytes in the order (0,2,1,3).
 // 576 = 64 mod 128, so the two rows a quarter-warp reads with one 16-byte load each sit in different banks.
@@ -320,8 +320,10 @@ __device__ __forceinline__ void prep8_store(const float (&v)[8], int kb, int m, 
     bad = __any_sync(0xffffffffu, bad);
     // scale = 2^(14 - e) with 2^e <= amax < 2^(e+1); a zero block keeps scale 1; a block holding a NaN or an infinity
     // gets a NaN scale, so that every output of that batch row is NaN as it would be in floating point
+    // (255 * 2^7, the largest 8-bit significand at that scale, is one more than two signed bytes hold: such a block takes half
+    // the scale, and what it holds exactly begins at 2^-6 of its largest value instead of 2^-7)
     int e = 14;
-    if (amax > 0.0f) { e = (int)((__float_as_uint(amax) >> 23) & 0xFF) - 127; if (e < -100) e = -100; }
+    if (amax > 0.0f) { e = (int)(((__float_as_uint(amax) + 0x00010000u) >> 23) & 0xFF) - 127; if (e < -100) e = -100; }
     const float scale = __uint_as_float((uint32_t)(127 + 14 - e) << 23);
     const float inv = bad ? __uint_as_float(0x7fc00000u) : __uint_as_float((uint32_t)(127 - 14 + e) << 23);
     int xi[8], sum = 0;
@@ -333,8 +335,10 @@ __device__ __forceinline__ void prep8_store(const float (&v)[8], int kb, int m, 
 #pragma unroll
     for (int qd = 0; qd < 2; ++qd) {
         const int *q = xi + 4 * qd;
-        const uint32_t hi = ((uint32_t)(q[0] >> 8) & 0xFFu) | (((uint32_t)(q[2] >> 8) & 0xFFu) << 8) | (((uint32_t)(q[1] >> 8) & 0xFFu) << 16) |
-                            (((uint32_t)(q[3] >> 8) & 0xFFu) << 24);
+        uint32_t h4[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) h4[j] = (uint32_t)((q[j] + 128) >> 8) & 0xFFu;
+        const uint32_t hi = h4[0] | (h4[2] << 8) | (h4[1] << 16) | (h4[3] << 24);
         const uint32_t lo = ((uint32_t)q[0] & 0xFFu) | (((uint32_t)q[2] & 0xFFu) << 8) | (((uint32_t)q[1] & 0xFFu) << 16) | (((uint32_t)q[3] & 0xFFu) << 24);
         const int off = 64 * (r >> 2) + 16 * (tq + qd) + 4 * (r & 3);
         *reinterpret_cast<uint32_t *>(row + off) = hi;
@@ -607,35 +611,23 @@ __device__ __forceinline__ bool consume(const Ring &r, int slab_off, const DecAu
 
 
 // ---- integer form (1..16 batch rows): mma.sync m16n8k32 / m16n8k16 on 8-bit operands ----------------------
-// D (int32, 16 x 8) = A (16 weight rows x 32 k, 8-bit) . B (32 k x 8 batch rows, 8-bit) [+ C].  AS / BS: operand is signed.
-template <bool AS, bool BS>
+// D (int32, 16 x 8) = A (16 weight rows x 32 k, 8-bit) . B (32 k x 8 columns, signed 8-bit) [+ C].  AS: A is signed.
+template <bool AS>
 __device__ __forceinline__ void imma32(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, int c0, int c1, int c2, int c3) {
-    if constexpr (AS && BS)
+    if constexpr (AS)
         asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
                      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
-    else if constexpr (AS && !BS)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
-                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
-    else if constexpr (!AS && BS)
+    else
         asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
                      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
-    else
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
-                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
 }
-template <bool AS, bool BS>
+template <bool AS>
 __device__ __forceinline__ void imma16(int (&d)[4], const uint32_t (&a)[2], uint32_t b0) {
-    if constexpr (AS && BS)
+    if constexpr (AS)
         asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
                      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(b0), "r"(0));
-    else if constexpr (AS && !BS)
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.s8.u8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
-                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(b0), "r"(0));
-    else if constexpr (!AS && BS)
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
-                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(b0), "r"(0));
     else
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
                      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(b0), "r"(0));
 }
 
@@ -649,16 +641,20 @@ __device__ __forceinline__ void static_for(F &&f) {
 
 // one k-block of one slab in the integer form.  `xs` is the staged activation tile of the k-block (rows of GQ_X8_ROW
 // bytes, then the batch rows' scales at xs_off).  Per MMA the weights are 8-bit integers and the activations one of the
-// two byte planes (x = 256 hi + lo with hi signed, lo unsigned); int32 sums per plane are exact.  At the end of the
+// two byte planes (x = 256 hi + lo); int32 sums per plane are exact.  At the end of the
 // k-block:  acc += 2^-e[n] * ( d[row] * (256 sumH + sumL) - f[row] * 64 * sum_run A''[row][run] * Sx[run][n] ).
-template <int TYPE, int MT>
+// ST (1..4 batch rows): the two planes sit side by side on the MMA's eight columns, the high bytes of row n in column n and the low
+// bytes in column n + 4, so that one MMA and one set of scale multiplications serve both; the factor 256 and the sum of the two
+// columns come at the end.
+template <int TYPE, int MT, bool ST>
 __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t *xs, int xs_off, const DecAux8 &aux, int lane, float (&acc)[MT][4]) {
     using D = Dec8<TYPE>;
     constexpr bool AS = D::A_SIGNED;
     D dec;
     dec.load(slab, lane, aux);
     const int g = lane >> 2, t = lane & 3;
-    const uint8_t *xb = xs + g * GQ_X8_ROW + 16 * t;     // unit (i, t) of batch row g; + 8 nt rows, + 256 for the low plane
+    // unit (i, t) of batch row g; + 8 nt rows, + 256 for the low plane
+    const uint8_t *xb = ST ? xs + (g & 3) * GQ_X8_ROW + 256 * (g >> 2) + 16 * t : xs + g * GQ_X8_ROW + 16 * t;
     int aH[MT][4], aL[MT][4], bH[MT][4], bL[MT][4];
     float bf[MT][4];
 #pragma unroll
@@ -671,7 +667,7 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
 #pragma unroll
         for (int nt = 0; nt < MT; ++nt) {
             xh[nt] = ld16(xb + nt * 8 * GQ_X8_ROW + 64 * I);
-            xl[nt] = ld16(xb + nt * 8 * GQ_X8_ROW + 64 * I + 256);
+            if constexpr (!ST) xl[nt] = ld16(xb + nt * 8 * GQ_X8_ROW + 64 * I + 256);
         }
         if constexpr (D::SCHEME == GQ_S16) {
             static_for<0, 4>([&](auto r_) {
@@ -683,10 +679,12 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
 #pragma unroll
                 for (int nt = 0; nt < MT; ++nt) {
                     int th[4], tl[4];
-                    imma16<AS, true>(th, a, w4(xh[nt], RR));
-                    imma16<AS, false>(tl, a, w4(xl[nt], RR));
+                    imma16<AS>(th, a, w4(xh[nt], RR));
                     aH[nt][0] += s0 * th[0]; aH[nt][1] += s0 * th[1]; aH[nt][2] += s1 * th[2]; aH[nt][3] += s1 * th[3];
-                    aL[nt][0] += s0 * tl[0]; aL[nt][1] += s0 * tl[1]; aL[nt][2] += s1 * tl[2]; aL[nt][3] += s1 * tl[3];
+                    if constexpr (!ST) {
+                        imma16<AS>(tl, a, w4(xl[nt], RR));
+                        aL[nt][0] += s0 * tl[0]; aL[nt][1] += s0 * tl[1]; aL[nt][2] += s1 * tl[2]; aL[nt][3] += s1 * tl[3];
+                    }
                 }
             });
         } else {
@@ -701,23 +699,28 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
 #pragma unroll
                 for (int nt = 0; nt < MT; ++nt) {
                     const uint32_t bh0 = V ? xh[nt].z : xh[nt].x, bh1 = V ? xh[nt].w : xh[nt].y;
-                    const uint32_t bl0 = V ? xl[nt].z : xl[nt].x, bl1 = V ? xl[nt].w : xl[nt].y;
+                    const uint32_t bl0 = ST ? 0u : V ? xl[nt].z : xl[nt].x, bl1 = ST ? 0u : V ? xl[nt].w : xl[nt].y;
                     if constexpr (D::SCHEME == GQ_FOLD) {
                         // two accumulator chains per plane (even / odd k-steps): half the dependent MMAs in a row
                         if constexpr (V == 0) {
-                            imma32<AS, true>(aH[nt], a, bh0, bh1, aH[nt][0], aH[nt][1], aH[nt][2], aH[nt][3]);
-                            imma32<AS, false>(aL[nt], a, bl0, bl1, aL[nt][0], aL[nt][1], aL[nt][2], aL[nt][3]);
+                            imma32<AS>(aH[nt], a, bh0, bh1, aH[nt][0], aH[nt][1], aH[nt][2], aH[nt][3]);
+                            if constexpr (!ST) imma32<AS>(aL[nt], a, bl0, bl1, aL[nt][0], aL[nt][1], aL[nt][2], aL[nt][3]);
                         } else {
-                            imma32<AS, true>(bH[nt], a, bh0, bh1, bH[nt][0], bH[nt][1], bH[nt][2], bH[nt][3]);
-                            imma32<AS, false>(bL[nt], a, bl0, bl1, bL[nt][0], bL[nt][1], bL[nt][2], bL[nt][3]);
+                            imma32<AS>(bH[nt], a, bh0, bh1, bH[nt][0], bH[nt][1], bH[nt][2], bH[nt][3]);
+                            if constexpr (!ST) imma32<AS>(bL[nt], a, bl0, bl1, bL[nt][0], bL[nt][1], bL[nt][2], bL[nt][3]);
                         }
                     } else {
                         int th[4], tl[4];
-                        imma32<AS, true>(th, a, bh0, bh1, 0, 0, 0, 0);
-                        imma32<AS, false>(tl, a, bl0, bl1, 0, 0, 0, 0);
+                        imma32<AS>(th, a, bh0, bh1, 0, 0, 0, 0);
+                        if constexpr (!ST) imma32<AS>(tl, a, bl0, bl1, 0, 0, 0, 0);
                         if constexpr (D::SCHEME == GQ_S32) {
                             aH[nt][0] += s0 * th[0]; aH[nt][1] += s0 * th[1]; aH[nt][2] += s1 * th[2]; aH[nt][3] += s1 * th[3];
-                            aL[nt][0] += s0 * tl[0]; aL[nt][1] += s0 * tl[1]; aL[nt][2] += s1 * tl[2]; aL[nt][3] += s1 * tl[3];
+                            if constexpr (!ST) { aL[nt][0] += s0 * tl[0]; aL[nt][1] += s0 * tl[1]; aL[nt][2] += s1 * tl[2]; aL[nt][3] += s1 * tl[3]; }
+                        } else if constexpr (ST) {
+                            bf[nt][0] = fmaf(f0, (float)th[0], bf[nt][0]);
+                            bf[nt][1] = fmaf(f0, (float)th[1], bf[nt][1]);
+                            bf[nt][2] = fmaf(f1, (float)th[2], bf[nt][2]);
+                            bf[nt][3] = fmaf(f1, (float)th[3], bf[nt][3]);
                         } else {
                             bf[nt][0] = fmaf(f0, (float)(th[0] * 256 + tl[0]), bf[nt][0]);
                             bf[nt][1] = fmaf(f0, (float)(th[1] * 256 + tl[1]), bf[nt][1]);
@@ -738,35 +741,41 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
         fc[0] *= -64.0f; fc[1] *= -64.0f;
     }
     const float z[4] = {0.f, 0.f, 0.f, 0.f};
+    const float plane = t < 2 ? 256.0f : 1.0f;          // ST: lanes t < 2 hold columns 0 .. 3
 #pragma unroll
     for (int nt = 0; nt < MT; ++nt) {
         float tot[4];
         if constexpr (D::SCHEME == GQ_F32) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) tot[j] = bf[nt][j];
+            for (int j = 0; j < 4; ++j) tot[j] = ST ? plane * bf[nt][j] : bf[nt][j];
         } else {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if constexpr (D::SCHEME == GQ_FOLD) {
                     // the even and the odd k-steps together: below 2^24 (128 weights of at most 180, and 4 * 45, times 255), exact as float
                     const int h = (aH[nt][j] << D::ODD_SHIFT) + bH[nt][j], l = (aL[nt][j] << D::ODD_SHIFT) + bL[nt][j];
-                    tot[j] = (j < 2 ? d0 : d1) * (fmaf((float)h, 256.0f, (float)l) * (1.0f / (1 << D::ODD_SHIFT)));
+                    tot[j] = (j < 2 ? d0 : d1) * ((ST ? plane * (float)h : fmaf((float)h, 256.0f, (float)l)) * (1.0f / (1 << D::ODD_SHIFT)));
                 } else {
-                    tot[j] = (j < 2 ? d0 : d1) * fmaf((float)aH[nt][j], 256.0f, (float)aL[nt][j]);
+                    tot[j] = (j < 2 ? d0 : d1) * (ST ? plane * (float)aH[nt][j] : fmaf((float)aH[nt][j], 256.0f, (float)aL[nt][j]));
                 }
             }
         }
         if constexpr (D::NCORR > 0) {
-            const uint8_t *sb = xs + (nt * 8 + g) * GQ_X8_ROW + GQ_X8_SUMS + 8 * t;
-            const uint2 bh = *reinterpret_cast<const uint2 *>(sb);
-            const uint2 bl = *reinterpret_cast<const uint2 *>(sb + 32);
             float mm[4];
-            mma16816_z(mm, ac, bh.x, bh.y, z);
-            mma16816(mm, ac, bl.x, bl.y);
+            if constexpr (ST) {
+                const uint2 b = *reinterpret_cast<const uint2 *>(xs + (g & 3) * GQ_X8_ROW + GQ_X8_SUMS + 32 * (g >> 2) + 8 * t);
+                mma16816_z(mm, ac, b.x, b.y, z);
+            } else {
+                const uint8_t *sb = xs + (nt * 8 + g) * GQ_X8_ROW + GQ_X8_SUMS + 8 * t;
+                const uint2 bh = *reinterpret_cast<const uint2 *>(sb);
+                const uint2 bl = *reinterpret_cast<const uint2 *>(sb + 32);
+                mma16816_z(mm, ac, bh.x, bh.y, z);
+                mma16816(mm, ac, bl.x, bl.y);
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j) tot[j] = fmaf(fc[j >> 1], mm[j], tot[j]);
         }
-        const float2 sx = *reinterpret_cast<const float2 *>(xs + xs_off + (nt * 8 + 2 * t) * 4);
+        const float2 sx = *reinterpret_cast<const float2 *>(xs + xs_off + (ST ? (2 * t) & 3 : nt * 8 + 2 * t) * 4);
         acc[nt][0] = fmaf(sx.x, tot[0], acc[nt][0]);
         acc[nt][1] = fmaf(sx.y, tot[1], acc[nt][1]);
         acc[nt][2] = fmaf(sx.x, tot[2], acc[nt][2]);
@@ -775,13 +784,13 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
 }
 
 
-template <int TYPE, int MT>
+template <int TYPE, int MT, bool ST>
 __device__ __forceinline__ bool consume8(const Ring &r, int xs_off, int slab_off, const DecAux8 &aux, int lane, float (&acc)[MT][4], uint32_t &ar_prev) {
     if (!ring_read_counter(r, lane, ar_prev)) return false;
     for (int i = 0, s = 0, round = 0; i < r.nk; ++i) {
         if (!mbar_wait(r.full + s, round & 1)) return false;
         const uint8_t *st = r.smem + (size_t)s * r.stage_bytes;
-        slab_kblock8<TYPE, MT>(st + slab_off, st + r.wmax, xs_off, aux, lane, acc);
+        slab_kblock8<TYPE, MT, ST>(st + slab_off, st + r.wmax, xs_off, aux, lane, acc);
         __syncwarp();
         if (lane == 0) mbar_arrive(r.empty + s);
         if (++s == r.stages) { s = 0; ++round; }
@@ -883,10 +892,11 @@ __device__ __noinline__ void fused_allreduce_block(const GemvParams &p, const ui
 // FORM 0: fp16 form (activations as fp16, weights decoded to fp16 pairs, m16n8k16 f16 MMAs), used for 17..64 batch rows.
 // FORM 1: integer form (activations as two byte planes, weights decoded to 8-bit quads, m16n8k32 / m16n8k16 integer
 // MMAs), used for 1..16 batch rows: about half the instructions per weight.
+// FORM 2: the integer form with both planes in one MMA, used for 1..4 batch rows.
 // ONLY: 0 compiles the decoders of all eleven types (the branch is per CTA); a GGML type id compiles that type alone,
 // for launches whose shards all share it (a smaller kernel; most launches of a real model are such).
 template <int MT, int FORM>
-__host__ __device__ constexpr int gq_stage_xbytes() { return FORM ? 8 * MT * GQ_X8_ROW + 32 * MT : 8 * MT * GQ_XROW_BYTES; }
+__host__ __device__ constexpr int gq_stage_xbytes() { return FORM == 2 ? 4 * GQ_X8_ROW + 16 : FORM ? 8 * MT * GQ_X8_ROW + 32 * MT : 8 * MT * GQ_XROW_BYTES; }
 
 template <int MT, int MINB, int FORM, int ONLY>
 __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_grouped_kernel(const __grid_constant__ GemvParams p) {
@@ -1031,9 +1041,9 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
         aux.grid = reinterpret_cast<const uint32_t *>(grid_s);
         aux.iq4 = iq4;
         const int xs_off = M * GQ_X8_ROW;
-#define GQ_CONSUME(T) case T: ok = consume8<T, MT>(ring, xs_off, slab_off, aux, lane, acc, ar_prev); break;
+#define GQ_CONSUME(T) case T: ok = consume8<T, MT, FORM == 2>(ring, xs_off, slab_off, aux, lane, acc, ar_prev); break;
         if constexpr (ONLY != 0) {
-            ok = consume8<(ONLY ? ONLY : GQ_Q4_K), MT>(ring, xs_off, slab_off, aux, lane, acc, ar_prev);
+            ok = consume8<(ONLY ? ONLY : GQ_Q4_K), MT, FORM == 2>(ring, xs_off, slab_off, aux, lane, acc, ar_prev);
         } else {
             switch (type) {
                 GQ_CONSUME(GQ_Q4_0) GQ_CONSUME(GQ_Q5_0) GQ_CONSUME(GQ_Q8_0) GQ_CONSUME(GQ_Q2_K) GQ_CONSUME(GQ_Q3_K) GQ_CONSUME(GQ_Q4_K)
@@ -1053,6 +1063,10 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
                 GQ_CONSUME(GQ_IQ2_XXS) GQ_CONSUME(GQ_IQ2_XS) GQ_CONSUME(GQ_IQ2_S) GQ_CONSUME(GQ_IQ1_M)
         }
 #undef GQ_CONSUME
+    }
+    if constexpr (FORM == 2) {      // columns n and n + 4: lanes t and t + 2
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[0][j] += __shfl_xor_sync(0xffffffffu, acc[0][j], 2);
     }
     if (!ok && lane == 0) report_status(p.status, GQ_DEV_TIMEOUT);   // the result is then incomplete; the status word says so
 
@@ -1462,14 +1476,14 @@ static int launch_gemv(const GemvParams &p, int64_t n_desc, cudaStream_t stream)
     return GQ_OK;
 }
 
-// integer form, M <= 8: one instantiation per type for runs of a single type, the all-types one otherwise
+// integer form, M <= 8 (FORM 1) and M <= 4 (FORM 2): one instantiation per type for runs of a single type, the all-types one otherwise
+template <int FORM>
 static int launch_gemv8_m8(const GemvParams &p, int64_t n_desc, cudaStream_t st, int only) {
     switch (only) {
-#define GQ_ONE(T) case T: return launch_gemv<1, 4, 1, T>(p, n_desc, st);
-        GQ_ONE(GQ_Q4_0) GQ_ONE(GQ_Q5_0) GQ_ONE(GQ_Q8_0) GQ_ONE(GQ_Q2_K) GQ_ONE(GQ_Q3_K) GQ_ONE(GQ_Q4_K)
-        GQ_ONE(GQ_Q5_K) GQ_ONE(GQ_Q6_K) GQ_ONE(GQ_IQ4_NL) GQ_ONE(GQ_IQ3_S) GQ_ONE(GQ_IQ4_XS) GQ_ONE(GQ_IQ3_XXS) GQ_ONE(GQ_IQ2_XXS) GQ_ONE(GQ_IQ2_XS) GQ_ONE(GQ_IQ2_S) GQ_ONE(GQ_IQ1_M)
+#define GQ_ONE(T) case T: return launch_gemv<1, 4, FORM, T>(p, n_desc, st);
+        GQ_EACH_TYPE(GQ_ONE)
 #undef GQ_ONE
-        default: return launch_gemv<1, 4, 1, 0>(p, n_desc, st);
+        default: return launch_gemv<1, 4, FORM, 0>(p, n_desc, st);
     }
 }
 
@@ -1552,7 +1566,7 @@ static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ld
     {
         // ring depth: four stages when four CTAs of them still fit an SM's shared memory, else three (swept on the
         // 64-layer stack: deeper rings with fewer resident CTAs were slower overall)
-        const int xb = !form ? 8 * mt * GQ_XROW_BYTES : mt == 1 ? gq_stage_xbytes<1, 1>() : mt == 2 ? gq_stage_xbytes<2, 1>() : gq_stage_xbytes<4, 1>();
+        const int xb = !form ? 8 * mt * GQ_XROW_BYTES : mt == 1 ? (M <= 4 ? gq_stage_xbytes<1, 2>() : gq_stage_xbytes<1, 1>()) : mt == 2 ? gq_stage_xbytes<2, 1>() : gq_stage_xbytes<4, 1>();
         const int stage_bytes = p.wbytes_max + xb;
         // (an SM has 228 KB of shared memory and the system keeps 1 KB of it per resident CTA)
         const int fixed = 64 + 8 * GQ_CONSUMER_WARPS + p.cb_bytes + 1024, red1 = GQ_CONSUMER_WARPS * mt * 512;
@@ -1569,7 +1583,7 @@ static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ld
     int rc = GQ_OK;
     if (phases & 2) {
         switch (mt) {
-            case 1: rc = launch_gemv8_m8(p, n_desc, st, (run_info >> 17) & 31); break;
+            case 1: rc = M <= 4 ? launch_gemv8_m8<2>(p, n_desc, st, (run_info >> 17) & 31) : launch_gemv8_m8<1>(p, n_desc, st, (run_info >> 17) & 31); break;
             case 2: rc = launch_gemv<2, 3, 1, 0>(p, n_desc, st); break;
             case 4: rc = form ? launch_gemv<4, 2, 1, 0>(p, n_desc, st) : launch_gemv<4, 2, 0, 0>(p, n_desc, st); break;
             default: rc = launch_gemv<8, 0, 0, 0>(p, n_desc, st); break;
