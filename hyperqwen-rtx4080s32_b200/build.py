@@ -17,7 +17,7 @@ EXT = os.path.join(_HERE, "_gq_torch.so")
 SOURCES = ["gq_b200.cu"]
 EXT_SOURCE = os.path.join(CSRC, "gq_torch.cpp")
 HEADERS = sorted(f for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))) + [os.path.join("..", "..", "include", "gq_b200.h")]
-NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "--expt-relaxed-constexpr", "-diag-suppress", "177", "-split-compile=0",
+NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "--expt-relaxed-constexpr", "-diag-suppress", "177",
               "-shared", "-Xcompiler", "-fPIC"]
 
 
