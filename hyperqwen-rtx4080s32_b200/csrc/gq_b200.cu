@@ -1562,11 +1562,11 @@ static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ld
     } else {
         p.ar = ArFused{};
     }
-    const int mt = M <= 8 ? 1 : M <= 16 ? 2 : M <= 32 ? 4 : 8;
+    const int mt = M <= 8 ? 1 : M <= 16 ? 2 : M <= 24 ? 3 : M <= 32 ? 4 : 8;
     {
         // ring depth: four stages when four CTAs of them still fit an SM's shared memory, else three (swept on the
         // 64-layer stack: deeper rings with fewer resident CTAs were slower overall)
-        const int xb = !form ? 8 * mt * GQ_XROW_BYTES : mt == 1 ? (M <= 4 ? gq_stage_xbytes<1, 2>() : gq_stage_xbytes<1, 1>()) : mt == 2 ? gq_stage_xbytes<2, 1>() : gq_stage_xbytes<4, 1>();
+        const int xb = !form ? 8 * mt * GQ_XROW_BYTES : mt == 1 ? (M <= 4 ? gq_stage_xbytes<1, 2>() : gq_stage_xbytes<1, 1>()) : gq_stage_xbytes<2, 1>();
         const int stage_bytes = p.wbytes_max + xb;
         // (an SM has 228 KB of shared memory and the system keeps 1 KB of it per resident CTA)
         const int fixed = 64 + 8 * GQ_CONSUMER_WARPS + p.cb_bytes + 1024, red1 = GQ_CONSUMER_WARPS * mt * 512;
@@ -1585,7 +1585,8 @@ static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ld
         switch (mt) {
             case 1: rc = M <= 4 ? launch_gemv8_m8<2>(p, n_desc, st, (run_info >> 17) & 31) : launch_gemv8_m8<1>(p, n_desc, st, (run_info >> 17) & 31); break;
             case 2: rc = launch_gemv<2, 3, 1, 0>(p, n_desc, st); break;
-            case 4: rc = form ? launch_gemv<4, 2, 1, 0>(p, n_desc, st) : launch_gemv<4, 2, 0, 0>(p, n_desc, st); break;
+            case 3: rc = launch_gemv<3, 2, 0, 0>(p, n_desc, st); break;
+            case 4: rc = launch_gemv<4, 2, 0, 0>(p, n_desc, st); break;
             default: rc = launch_gemv<8, 0, 0, 0>(p, n_desc, st); break;
         }
     }

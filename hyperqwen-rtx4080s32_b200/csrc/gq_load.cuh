@@ -68,17 +68,31 @@ template <int TYPE, typename Row>
 __device__ __forceinline__ void permute_slabs(const uint8_t *img, int pitch, int n_kb, uint8_t *dst, int64_t dst_stride, Row row) {
     constexpr int B = gq_type_bytes(TYPE);
     for (int w = threadIdx.x; w < 4 * B; w += GQ_LOAD_THREADS) {
-        const uint8_t *s[4];
+        int s[4];
 #pragma unroll
         for (int z = 0; z < 4; ++z) {
             int r, byte;
             gq_slab_src(TYPE, 4 * w + z, &r, &byte);
-            s[z] = img + r * pitch + (int)(reinterpret_cast<uintptr_t>(row(r)) & 15) + byte;
+            s[z] = r * pitch + (int)(reinterpret_cast<uintptr_t>(row(r)) & 15) + byte;
         }
+        // most words are four neighbouring bytes in another order; at an even address two halfword loads fetch them
+        const int lo = min(min(s[0], s[1]), min(s[2], s[3])), hi = max(max(s[0], s[1]), max(s[2], s[3]));
+        if (hi - lo == 3 && !(lo & 1)) {
+            uint32_t sel = 0;
+#pragma unroll
+            for (int z = 0; z < 4; ++z) sel |= (uint32_t)(s[z] - lo + ((s[z] - lo) & 2)) << (4 * z);      // 0 1 | 4 5: bytes of the two halfwords
+            const uint8_t *a = img + lo;
 #pragma unroll 4
-        for (int kb = 0; kb < n_kb; ++kb) {
-            const uint32_t v = (uint32_t)s[0][kb * B] | (uint32_t)s[1][kb * B] << 8 | (uint32_t)s[2][kb * B] << 16 | (uint32_t)s[3][kb * B] << 24;
-            *reinterpret_cast<uint32_t *>(dst + kb * dst_stride + 4 * w) = v;
+            for (int kb = 0; kb < n_kb; ++kb)
+                *reinterpret_cast<uint32_t *>(dst + kb * dst_stride + 4 * w) =
+                    prmt(*reinterpret_cast<const uint16_t *>(a + kb * B), *reinterpret_cast<const uint16_t *>(a + kb * B + 2), sel);
+        } else {
+#pragma unroll 4
+            for (int kb = 0; kb < n_kb; ++kb) {
+                const uint8_t *b = img + kb * B;
+                *reinterpret_cast<uint32_t *>(dst + kb * dst_stride + 4 * w) =
+                    (uint32_t)b[s[0]] | (uint32_t)b[s[1]] << 8 | (uint32_t)b[s[2]] << 16 | (uint32_t)b[s[3]] << 24;
+            }
         }
     }
 }

@@ -20,7 +20,7 @@ def _layer(parts, k):
     return lin.finalize()
 
 
-@pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 32, 33, 64, 65, 300])
+@pytest.mark.parametrize("m", [1, 4, 5, 8, 9, 16, 17, 24, 25, 32, 33, 64, 65, 300])
 def test_native_path_equals_the_custom_op(m):
     k, parts = 1024, [(192, F.Q4_K), (70, F.IQ3_S), (64, F.Q6_K)]
     lin = _layer(parts, k)
