@@ -149,6 +149,25 @@ class Run {
     int device_, info_ = 0, one_ = 0;
 };
 
+// The load-time calls, on arguments that ops.py has checked: device and stream of the tensor, then the C ABI.
+void *stream_of(const at::Tensor &t) { return c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)t.get_device()).stream(); }
+
+void repack(const at::Tensor &raw, int64_t n_out, int64_t type, int64_t nb, const at::Tensor &out) {
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)raw.get_device());
+    check(gq_repack((int)type, raw.data_ptr(), n_out, nb * 256, raw.stride(0), out.data_ptr(), stream_of(raw)), "gq_repack");
+}
+at::Tensor dequantize(const at::Tensor &tiles, int64_t n_out, int64_t k, int64_t type, bool bf16) {
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)tiles.get_device());
+    at::Tensor out = at::detail::empty_cuda({n_out, k}, bf16 ? at::kBFloat16 : at::kFloat, tiles.device(), c10::nullopt);
+    check(gq_dequant((int)type, tiles.data_ptr(), n_out, k, out.data_ptr(), bf16 ? 1 : 0, k, stream_of(tiles)), "gq_dequant");
+    return out;
+}
+void build_descs(const std::vector<int32_t> &types, const std::vector<int64_t> &n_outs, int64_t k, const std::vector<int32_t> &splits, const at::Tensor &out) {
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)out.get_device());
+    check(gq_build_descs_device((int)types.size(), types.data(), n_outs.data(), k, (int)splits.size(), splits.data(), (int32_t *)out.data_ptr(),
+                                stream_of(out)), "gq_build_descs_device");
+}
+
 // rows `ids` of a raw table -> weights; None: not the plain case
 PyObject *dequantize_rows(py::handle rawh, int64_t type, py::handle idsh, bool bf16) {
     if (!THPVariable_CheckExact(rawh.ptr()) || !THPVariable_CheckExact(idsh.ptr()) || c10::impl::dispatch_mode_enabled()) Py_RETURN_NONE;
@@ -173,6 +192,9 @@ PyObject *dequantize_rows(py::handle rawh, int64_t type, py::handle idsh, bool b
 
 PYBIND11_MODULE(_gq_torch, m) {
     m.def("set_error_type", [](py::object e) { g_error = e.release().ptr(); });
+    m.def("repack", &repack);
+    m.def("dequantize", &dequantize);
+    m.def("build_descs", &build_descs);
     m.def("dequantize_rows", [](py::handle raw, int64_t type, py::handle ids, bool bf16) {
         return py::reinterpret_steal<py::object>(dequantize_rows(raw, type, ids, bf16));
     });

@@ -91,9 +91,7 @@ def build_descs_on(device, wtypes: Sequence[int], n_outs: Sequence[int], k: int,
         return [torch.from_numpy(build_descs(wtypes, n_outs, k, s)).to(device) for s in splits]
     tiles = sum(-(-int(n) // 64) for n in n_outs)
     buf = torch.empty((tiles * sum(splits), DESC_WORDS), dtype=torch.int32, device=device)
-    with torch.cuda.device(device):
-        check(lib().gq_build_descs_device(len(wtypes), _i32_array(wtypes), _i64_array(n_outs), int(k), len(splits), _i32_array(splits),
-                                          buf.data_ptr(), _stream_ptr(buf)), "gq_build_descs_device")
+    native().build_descs([int(t) for t in wtypes], [int(n) for n in n_outs], int(k), [int(s) for s in splits], buf)
     return list(buf.split([tiles * s for s in splits]))
 
 
@@ -153,8 +151,7 @@ def repack_tiles(raw: torch.Tensor, n_out: int, wtype: int, out: torch.Tensor | 
         out = torch.empty((n_tiles, nb, 64 * bb), dtype=torch.uint8, device=raw.device)
     else:
         out = out.view(n_tiles, nb, 64 * bb)
-    with torch.cuda.device(raw.device):
-        check(lib().gq_repack(int(wtype), raw.data_ptr(), n_out, nb * 256, raw.stride(0), out.data_ptr(), _stream_ptr(raw)), "gq_repack")
+    native().repack(raw, int(n_out), int(wtype), nb, out)
     return out
 
 
@@ -176,11 +173,7 @@ def dequantize_tiles(tiles: torch.Tensor, n_out: int, k: int, wtype: int, dtype=
     _need_cuda(tiles, "tiles")
     if dtype not in (torch.float32, torch.bfloat16):
         raise GqError("dequantize_tiles produces float32 or bfloat16")
-    out = torch.empty((n_out, k), dtype=dtype, device=tiles.device)
-    with torch.cuda.device(tiles.device):
-        check(lib().gq_dequant(int(wtype), tiles.data_ptr(), n_out, k, out.data_ptr(), 0 if dtype == torch.float32 else 1, k,
-                               _stream_ptr(tiles)), "gq_dequant")
-    return out
+    return native().dequantize(tiles, int(n_out), int(k), int(wtype), dtype == torch.bfloat16)
 
 
 def repack_shards(raws: Sequence[torch.Tensor], wtypes: Sequence[int]) -> list[torch.Tensor]:
