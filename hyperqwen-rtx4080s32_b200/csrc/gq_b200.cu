@@ -476,6 +476,7 @@ struct GemvParams {
     int cb_bytes;                    // shared-memory bytes of the codebook-table region (0: the run has no codebook type)
     int cluster;         // 1: the `split` CTAs of a tile form a thread-block cluster and reduce through shared memory
     int cluster_push;    // 1: the others store their accumulators into slots of the split-0 CTA's shared memory (one cluster barrier)
+    const __nv_bfloat16 *x;  // FORM 2, one row: the activations themselves, converted by the producer warp (null: xt is prepared)
     const uint8_t *pf_ptr;   // weights the caller will multiply next (or null): prefetched into L2 while this launch computes
     int64_t pf_bytes;
     ArFused ar;
@@ -972,6 +973,40 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
     const bool push = p.cluster && p.cluster_push;
     if (push) cluster_arrive_relaxed();
 
+    if (FORM == 2 && warp == GQ_CONSUMER_WARPS && p.x) {
+        // ---- producer of a small launch for one row: the whole warp.  It copies the weight tiles like the one below, and
+        // converts the activations of each k-block straight into the stage (what prep_x8_kernel would have left in the workspace),
+        // one k-block requested ahead.  Every CTA of a k-range repeats that, 0.7 us per k-block; for it the preparation kernel falls
+        // away: 2 us of host time (1024 x 5120 Q4_K, called one by one: 8.2 -> 6.4 us) and a kernel boundary on the GPU ----
+        const uint8_t *src = p.packed + off + (int64_t)kb0 * tile_bytes;
+        const __nv_bfloat16 *xr = p.x + (int64_t)kb0 * GQ_QK + 8 * lane;
+        const int pre = nk < stages ? nk : stages;
+        if (lane == 0)
+            for (int i = 0; i < pre; ++i) bulk_g2s(smem + (size_t)i * stage_bytes, src + (int64_t)i * tile_bytes, (uint32_t)tile_bytes, full + i);
+        pdl_wait();
+        float nxt[8];
+        load8(xr, nxt);
+        for (int i = 0, s = 0, round = 0; i < nk; ++i) {
+            if (i >= pre) {
+                if (!mbar_wait_parked(empty + s, (round - 1) & 1)) { if (lane == 0) report_status(p.status, GQ_DEV_TIMEOUT); break; }
+                if (lane == 0) bulk_g2s(smem + (size_t)s * stage_bytes, src + (int64_t)i * tile_bytes, (uint32_t)tile_bytes, full + s);
+            }
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = nxt[j];
+            if (i + 1 < nk) load8(xr + (i + 1) * GQ_QK, nxt);
+            prep8_store(v, 0, 0, 1, smem + (size_t)s * stage_bytes + wmax, lane);
+            __syncwarp();
+            if (lane == 0) mbar_expect_tx(full + s, (uint32_t)tile_bytes);      // arrives: the rows are there, the tile is counted
+            if (i == nk - 3 || (i == 0 && nk < 3)) pdl_trigger();
+            if (++s == stages) { s = 0; ++round; }
+        }
+        if (!p.cluster) return;
+        if (push) { cluster_wait(); return; }
+        cluster_sync_all();
+        cluster_sync_all();
+        return;
+    }
     if (warp == GQ_CONSUMER_WARPS) {
         // ---- producer: one thread; per k-block one bulk copy of the weight tile and one of the activation tile.
         // The weights do not depend on the kernel in front of this one, so the first stages' weight copies go out
@@ -1516,7 +1551,11 @@ static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ld
     cudaStream_t st = (cudaStream_t)stream;
 
     const int form = M <= GQ_GEMV8_MAX_ROWS ? 1 : 0;
-    if (phases & 1) {
+    // Whether the grouped kernel converts the activations itself: one row, nothing folded in front, and at most four k-blocks to a
+    // CTA, up to where the conversions, one after the other, take no longer than the boundary they save (graphs of 24 layers, Q4_K:
+    // 5120 x 5120, 3.3 k-blocks, 6.8 -> 6.5 us; 7168 x 5120, 5 k-blocks, 7.4 -> 8.3; a second row adds 2 us)
+    const bool direct = (phases & 8) && M == 1 && !ar && !(pre && pre->kind) && (K / GQ_QK + split - 1) / split <= 4;
+    if ((phases & 1) && !direct) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1553,6 +1592,7 @@ static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ld
     // partials and the separate sum
     p.cluster = (split > 1 && split <= 8 && n_desc % split == 0) ? 1 : 0;
     p.cluster_push = 0;
+    p.x = direct ? (const __nv_bfloat16 *)x_dev : nullptr;
     p.pf_ptr = (next_packed_dev && next_bytes > 0 && !((uintptr_t)next_packed_dev & 15)) ? (const uint8_t *)next_packed_dev : nullptr;
     p.pf_bytes = next_bytes;
     if (ar) {

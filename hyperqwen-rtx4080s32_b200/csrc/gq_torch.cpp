@@ -135,8 +135,9 @@ class Run {
                                           (const int32_t *)d.data_ptr(), d.size(0), split, info_, y.data_ptr(), n_total_, n_total_, ws.get(), need, stream),
                       "gq_gemv_grouped_pre");
             else
-                check(gq_gemv_grouped(x.data_ptr(), m, K_, ldx, packed_.data_ptr(), (const int32_t *)d.data_ptr(), d.size(0), split, info_, y.data_ptr(),
-                                      n_total_, n_total_, ws.get(), need, stream), "gq_gemv_grouped");
+                // 15: nobody reads this workspace's status word, so a small launch may do without the preparation kernel
+                check(gq_gemv_grouped_phases(x.data_ptr(), m, K_, ldx, packed_.data_ptr(), (const int32_t *)d.data_ptr(), d.size(0), split, info_,
+                                             y.data_ptr(), n_total_, n_total_, ws.get(), need, stream, 15), "gq_gemv_grouped");
         }
         return THPVariable_Wrap(std::move(y));
     }

@@ -134,6 +134,8 @@ int gq_gemv_grouped(const void *x_dev, int64_t M, int64_t K, int64_t ldx, const 
  * bit 1 = the grouped kernel, bit 2 = the split-K partial sum.  gq_gemv_grouped is phases = 7.  A caller
  * that multiplies the same x by several runs prepares once and passes phases = 6 for the others, with the
  * same workspace (its activation area depends only on M and K); a benchmark times bit 1 alone.
+ * Bit 3 permits the library to leave the preparation out and convert the activations inside the grouped kernel, which it does
+ * for small launches of one row; the workspace's status word is then not written (gq_device_status is).
  * Reference: interface.py:164,174 quantises once per layer call for the same reason. */
 int gq_gemv_grouped_phases(const void *x_dev, int64_t M, int64_t K, int64_t ldx, const void *packed_dev, const int32_t *desc_dev,
                            int64_t n_desc, int split, int run_info, void *y_dev, int64_t ldy, int64_t n_total,

@@ -79,3 +79,27 @@ def test_descriptor_tables_written_on_the_device(parts):
     for k, splits in [(256, [1]), (5120, [1, 3, 20])]:
         for s, d in zip(splits, ops.build_descs_on("cuda", types, n_outs, k, splits)):
             assert torch.equal(d.cpu(), torch.from_numpy(ops.build_descs(types, n_outs, k, s)))
+
+
+@pytest.mark.parametrize("t", [F.Q4_K, F.Q6_K, F.Q2_K, F.IQ3_S, F.Q8_0])
+@pytest.mark.parametrize("n_out,k", [(64, 256), (70, 768), (1024, 5120), (130, 17408)])
+def test_small_launches_that_convert_their_activations(t, n_out, k):
+    """One row (two beside it) of a layer without the preparation kernel (the native path) against the prepared call, bit for
+    bit: fewer k-blocks than stages, splits of up to four, more than four, rows of odd stride, a block of zeros, an infinity."""
+    lin = GGUFLinear(k, [n_out])
+    lin.load_shard(synth.random_blocks(n_out, k, t, seed=n_out, device="cuda"), t)
+    lin.finalize()
+    packed, descs, splits, _, nb, bb = lin.gguf_groups["__all__"]
+    for m, bad in ((1, False), (1, True), (2, False)):
+        s = ops.grouped_split_for(-(-n_out // 64), nb, m=m, block_bytes=bb, sms=ops.sm_count(packed.device))
+        x = synth.activations(m, k, device="cuda")
+        x[0, :256] = 0
+        if bad:
+            x[0, 300 % k] = float("inf")
+        wide = torch.zeros((m, k + 3), dtype=torch.bfloat16, device="cuda")
+        wide[:, 2:2 + k] = x
+        want = ops.grouped_gemm(x, packed, descs[splits.index(s)], s, [t], n_out)
+        for _ in range(2):
+            assert torch.equal(lin(x).nan_to_num(7.0), want.nan_to_num(7.0))
+            assert torch.equal(lin(wide[:, 2:2 + k]).nan_to_num(7.0), want.nan_to_num(7.0))
+    assert ops.device_status() == 0
