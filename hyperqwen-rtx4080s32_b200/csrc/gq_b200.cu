@@ -886,15 +886,15 @@ __device__ __noinline__ void fused_allreduce_block(const GemvParams &p, const ui
 // registers, which it turns into more loads and MMAs in flight per warp: measured 14 % faster than the 72-register
 // build when a CTA walks ten or more k-blocks, a little slower on launches of many short CTAs, 2 % faster on the
 // mixed stack.  (Compiling both and choosing per call was slower than either alone: alternating between two large
-// kernels costs more in instruction-cache misses at every launch than the better fit gains.)  The 17..32-row form
-// is about 10 % faster with room for two CTAs (168 registers) than with the compiler's own 144; the 16- and 64-row
-// forms were best left alone.
+// kernels costs more in instruction-cache misses at every launch than the better fit gains.)  The 17..24- and 25..32-row
+// forms are about 10 % faster with room for two CTAs (168 registers) than with the compiler's own 144; the 16-row
+// form was best left alone.
 //
-// FORM 0: fp16 form (activations as fp16, weights decoded to fp16 pairs, m16n8k16 f16 MMAs), used for 17..64 batch rows.
+// FORM 0: fp16 form (activations as fp16, weights decoded to fp16 pairs, m16n8k16 f16 MMAs), used from 17 batch rows.
 // FORM 1: integer form (activations as two byte planes, weights decoded to 8-bit quads, m16n8k32 / m16n8k16 integer
 // MMAs), used for 1..16 batch rows: about half the instructions per weight.
 // FORM 2: the integer form with both planes in one MMA, used for 1..4 batch rows.
-// ONLY: 0 compiles the decoders of all eleven types (the branch is per CTA); a GGML type id compiles that type alone,
+// ONLY: 0 compiles the decoders of all types (the branch is per CTA); a GGML type id compiles that type alone,
 // for launches whose shards all share it (a smaller kernel; most launches of a real model are such).
 template <int MT, int FORM>
 __host__ __device__ constexpr int gq_stage_xbytes() { return FORM == 2 ? 4 * GQ_X8_ROW + 16 : FORM ? 8 * MT * GQ_X8_ROW + 32 * MT : 8 * MT * GQ_XROW_BYTES; }
