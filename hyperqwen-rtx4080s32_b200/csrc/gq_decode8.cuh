@@ -520,9 +520,10 @@ struct Dec8<GQ_IQ3_S> {
     template <int R, int H>
     GQ_HD uint32_t quad() const {
         constexpr int ib = R >> 1, u = R & 1;
-        const uint32_t idxb = (uint32_t)ubyte<(R & 3)>(w4(q[H], R >> 2));
+        // index byte and, above it, the qh byte in one prmt (one shift serves four runs): 17,408 x 5,120 at 1 / 8 rows 17.6 / 18.7 ->
+        // 15.6 / 17.0 us against a shift and a merge per run; IQ2_S likewise 20.5 / 22.3 -> 19.2 / 21.4
         const uint32_t hw = (ib < 4) ? qh[H].x : qh[H].y;
-        const uint32_t idx = or_and(idxb, shl_c<8 - (8 * (ib & 3) + 4 * u)>(hw), 0x100u);
+        const uint32_t idx = prmt(w4(q[H], R >> 2), hw >> (4 * u), (R & 3) | ((4 | (ib & 3)) << 4)) & 0x1FFu;
         const uint32_t e = grid[idx];
         return negate_odd_bytes(e, sign_bytes((uint32_t)ubyte<(R & 3)>(w4(sg[H], R >> 2)), smul));     // magnitudes 1, 3 .. 15
     }
@@ -736,9 +737,8 @@ struct Dec8<GQ_IQ2_S> {
     template <int R, int H>
     GQ_HD uint32_t quad() const {
         constexpr int ib = R >> 1, u = R & 1;
-        const uint32_t idxb = (uint32_t)ubyte<(R & 3)>(q[H][R >> 2]);
         const uint32_t hw = (ib < 4) ? qh[H].x : qh[H].y;
-        const uint32_t idx = or_and(idxb, shl_c<8 - (8 * (ib & 3) + 4 * u)>(hw), 0x300u);
+        const uint32_t idx = prmt(q[H][R >> 2], hw >> (4 * u), (R & 3) | ((4 | (ib & 3)) << 4)) & 0x3FFu;
         const uint32_t e = *reinterpret_cast<const uint32_t *>(grid + 8 * idx);
         // signs by arithmetic: 2-3 % faster here than negate_bytes, the other way round than in the types above
         const uint32_t nib = (uint32_t)ubyte<(R & 3)>(sg[H][R >> 2]);
