@@ -138,7 +138,8 @@ __host__ __device__ inline int64_t align256(int64_t v) { return (v + 255) & ~(in
 
 // The same row in the integer form used for 1..16 batch rows: per k-block and batch row the activations as 16-bit
 // fixed point (x * 2^e, e chosen per row and k-block so that the largest magnitude lands in [2^14, 2^15)), split into
-// two signed bytes, x = 256 hi + lo: a plane of high bytes (256 B) and one of low bytes (256 B), then the sixteen 16-weight run sums
+// two signed bytes, x = 256 hi - lo (with the minus sign they hold -32895 .. 32640, both signs of 255 * 2^7, the largest 8-bit
+// significand at that scale; 256 hi + lo ends at 32639): a plane of high bytes (256 B) and one of low bytes (256 B), then the sixteen 16-weight run sums
 // (times 2^-6) as fp16 hi parts (32 B) and lo parts (32 B).  Inside a plane the bytes are ordered for the lane that
 // reads them: 16-byte unit 4*i + t holds, for runs 4i..4i+3, the quad 4t..4t+3 with bytes in the order (0,2,1,3).
 // 576 = 64 mod 128, so the two rows a quarter-warp reads with one 16-byte load each sit in different banks.
@@ -320,10 +321,8 @@ __device__ __forceinline__ void prep8_store(const float (&v)[8], int kb, int m, 
     bad = __any_sync(0xffffffffu, bad);
     // scale = 2^(14 - e) with 2^e <= amax < 2^(e+1); a zero block keeps scale 1; a block holding a NaN or an infinity
     // gets a NaN scale, so that every output of that batch row is NaN as it would be in floating point
-    // (255 * 2^7, the largest 8-bit significand at that scale, is one more than two signed bytes hold: such a block takes half
-    // the scale, and what it holds exactly begins at 2^-6 of its largest value instead of 2^-7)
     int e = 14;
-    if (amax > 0.0f) { e = (int)(((__float_as_uint(amax) + 0x00010000u) >> 23) & 0xFF) - 127; if (e < -100) e = -100; }
+    if (amax > 0.0f) { e = (int)((__float_as_uint(amax) >> 23) & 0xFF) - 127; if (e < -100) e = -100; }
     const float scale = __uint_as_float((uint32_t)(127 + 14 - e) << 23);
     const float inv = bad ? __uint_as_float(0x7fc00000u) : __uint_as_float((uint32_t)(127 - 14 + e) << 23);
     int xi[8], sum = 0;
@@ -337,9 +336,9 @@ __device__ __forceinline__ void prep8_store(const float (&v)[8], int kb, int m, 
         const int *q = xi + 4 * qd;
         uint32_t h4[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) h4[j] = (uint32_t)((q[j] + 128) >> 8) & 0xFFu;
+        for (int j = 0; j < 4; ++j) h4[j] = (uint32_t)((q[j] + 127) >> 8) & 0xFFu;
         const uint32_t hi = h4[0] | (h4[2] << 8) | (h4[1] << 16) | (h4[3] << 24);
-        const uint32_t lo = ((uint32_t)q[0] & 0xFFu) | (((uint32_t)q[2] & 0xFFu) << 8) | (((uint32_t)q[1] & 0xFFu) << 16) | (((uint32_t)q[3] & 0xFFu) << 24);
+        const uint32_t lo = ((uint32_t)-q[0] & 0xFFu) | (((uint32_t)-q[2] & 0xFFu) << 8) | (((uint32_t)-q[1] & 0xFFu) << 16) | (((uint32_t)-q[3] & 0xFFu) << 24);
         const int off = 64 * (r >> 2) + 16 * (tq + qd) + 4 * (r & 3);
         *reinterpret_cast<uint32_t *>(row + off) = hi;
         *reinterpret_cast<uint32_t *>(row + 256 + off) = lo;
@@ -642,10 +641,10 @@ __device__ __forceinline__ void static_for(F &&f) {
 
 // one k-block of one slab in the integer form.  `xs` is the staged activation tile of the k-block (rows of GQ_X8_ROW
 // bytes, then the batch rows' scales at xs_off).  Per MMA the weights are 8-bit integers and the activations one of the
-// two byte planes (x = 256 hi + lo); int32 sums per plane are exact.  At the end of the
-// k-block:  acc += 2^-e[n] * ( d[row] * (256 sumH + sumL) - f[row] * 64 * sum_run A''[row][run] * Sx[run][n] ).
+// two byte planes (x = 256 hi - lo); int32 sums per plane are exact.  At the end of the
+// k-block:  acc += 2^-e[n] * ( d[row] * (256 sumH - sumL) - f[row] * 64 * sum_run A''[row][run] * Sx[run][n] ).
 // ST (1..4 batch rows): the two planes sit side by side on the MMA's eight columns, the high bytes of row n in column n and the low
-// bytes in column n + 4, so that one MMA and one set of scale multiplications serve both; the factor 256 and the sum of the two
+// bytes in column n + 4, so that one MMA and one set of scale multiplications serve both; the factors 256 and -1 and the sum of the two
 // columns come at the end.
 template <int TYPE, int MT, bool ST>
 __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t *xs, int xs_off, const DecAux8 &aux, int lane, float (&acc)[MT][4]) {
@@ -723,10 +722,10 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
                             bf[nt][2] = fmaf(f1, (float)th[2], bf[nt][2]);
                             bf[nt][3] = fmaf(f1, (float)th[3], bf[nt][3]);
                         } else {
-                            bf[nt][0] = fmaf(f0, (float)(th[0] * 256 + tl[0]), bf[nt][0]);
-                            bf[nt][1] = fmaf(f0, (float)(th[1] * 256 + tl[1]), bf[nt][1]);
-                            bf[nt][2] = fmaf(f1, (float)(th[2] * 256 + tl[2]), bf[nt][2]);
-                            bf[nt][3] = fmaf(f1, (float)(th[3] * 256 + tl[3]), bf[nt][3]);
+                            bf[nt][0] = fmaf(f0, (float)(th[0] * 256 - tl[0]), bf[nt][0]);
+                            bf[nt][1] = fmaf(f0, (float)(th[1] * 256 - tl[1]), bf[nt][1]);
+                            bf[nt][2] = fmaf(f1, (float)(th[2] * 256 - tl[2]), bf[nt][2]);
+                            bf[nt][3] = fmaf(f1, (float)(th[3] * 256 - tl[3]), bf[nt][3]);
                         }
                     }
                 }
@@ -742,7 +741,7 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
         fc[0] *= -64.0f; fc[1] *= -64.0f;
     }
     const float z[4] = {0.f, 0.f, 0.f, 0.f};
-    const float plane = t < 2 ? 256.0f : 1.0f;          // ST: lanes t < 2 hold columns 0 .. 3
+    const float plane = t < 2 ? 256.0f : -1.0f;          // ST: lanes t < 2 hold columns 0 .. 3
 #pragma unroll
     for (int nt = 0; nt < MT; ++nt) {
         float tot[4];
@@ -755,9 +754,9 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
                 if constexpr (D::SCHEME == GQ_FOLD) {
                     // the even and the odd k-steps together: below 2^24 (128 weights of at most 180, and 4 * 45, times 255), exact as float
                     const int h = (aH[nt][j] << D::ODD_SHIFT) + bH[nt][j], l = (aL[nt][j] << D::ODD_SHIFT) + bL[nt][j];
-                    tot[j] = (j < 2 ? d0 : d1) * ((ST ? plane * (float)h : fmaf((float)h, 256.0f, (float)l)) * (1.0f / (1 << D::ODD_SHIFT)));
+                    tot[j] = (j < 2 ? d0 : d1) * ((ST ? plane * (float)h : fmaf((float)h, 256.0f, -(float)l)) * (1.0f / (1 << D::ODD_SHIFT)));
                 } else {
-                    tot[j] = (j < 2 ? d0 : d1) * (ST ? plane * (float)aH[nt][j] : fmaf((float)aH[nt][j], 256.0f, (float)aL[nt][j]));
+                    tot[j] = (j < 2 ? d0 : d1) * (ST ? plane * (float)aH[nt][j] : fmaf((float)aH[nt][j], 256.0f, -(float)aL[nt][j]));
                 }
             }
         }

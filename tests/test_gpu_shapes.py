@@ -11,6 +11,7 @@ import torch
 from hyperqwen_rtx4080s32_b200 import _lib, formats as F
 from hyperqwen_rtx4080s32_b200 import ops, synth
 from hyperqwen_rtx4080s32_b200 import stack as S
+from hyperqwen_rtx4080s32_b200.linear import GGUFLinear
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -205,6 +206,30 @@ def test_arithmetic_error_beyond_the_output_rounding(t):
         p999, worst = ARITH_BOUNDS[form]
         assert np.percentile(extra, 99.9) <= p999 and extra.max() <= worst, \
             f"{F.TYPE_NAMES[t]} M={m} ({form} form): 99.9th percentile {np.percentile(extra, 99.9):.2e}, max {extra.max():.2e}"
+
+
+@pytest.mark.parametrize("m", [1, 2, 4, 5, 8, 9, 16])
+def test_a_block_whose_largest_significand_is_255_keeps_its_small_values(m):
+    """The integer form holds every activation within 2^-7 of its block's largest magnitude exactly, also where that magnitude
+    is 255 * 2^n of both signs, the edge of what two signed bytes hold.  All products and sums here are bf16 values, so the
+    outputs are exact: 129 * 2^-14 beside 255 * 2^-7 lost its last bit (0.8 % of it) at half the scale."""
+    k, n_out = 512, 64
+    big, small = 255 / 128, 129 / 128 / 128
+    blocks = np.zeros((n_out, k // 32, 34), dtype=np.uint8)
+    blocks[:, :, :2] = np.frombuffer(np.float16(1.0).tobytes(), dtype=np.uint8)
+    q = np.zeros((n_out, k), dtype=np.int8)
+    for row, picks in enumerate([{100: 1}, {3: 1}, {7: 1}, {3: 1, 7: 1}, {3: -1}, {356: 1}, {259: 1}, {100: -2, 3: 1, 7: 1}]):
+        for i, v in picks.items():
+            q[row, i] = v
+    blocks[:, :, 2:] = q.view(np.uint8).reshape(n_out, k // 32, 32)
+    lin = GGUFLinear(k, [n_out])
+    lin.load_shard(torch.from_numpy(blocks.reshape(n_out, -1)).to(dev()), F.Q8_0)
+    lin.finalize()
+    x = torch.zeros((m, k), dtype=torch.float64)
+    for i, v in ((3, big), (7, -big), (100, small), (259, -16 * big), (356, 16 * small)):
+        x[:, i] = v * torch.exp2(torch.arange(m) - 4.0)
+    want = x @ torch.from_numpy(q.astype(np.float64)).T
+    assert torch.equal(lin(x.to(dev(), torch.bfloat16)).double().cpu(), want)
 
 
 @pytest.mark.parametrize("t", [F.Q4_K, F.Q6_K, F.Q2_K, F.Q8_0, F.IQ3_S])
