@@ -1125,7 +1125,18 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
         }
         if (lane == 0) mbar_expect_tx(parts + warp, (uint32_t)((p.split - 1) * MT * 512));
         __syncwarp();
-        if (!mbar_wait(parts + warp, 0)) { ok = false; if (lane == 0) report_status(p.status, GQ_DEV_TIMEOUT); }
+        if (!__all_sync(0xffffffffu, mbar_wait(parts + warp, 0))) {
+            // A part is late.  Its CTA may still be inside a bounded wait of its own and store here afterwards, so this CTA must not
+            // leave before it: the barrier completes when every other thread of the cluster has left (or failed and come here too);
+            // what they stored then has a bounded time to land.
+            cluster_sync_all();
+            bool landed = false;
+            for (int i = 0; i < 100 && !landed; ++i) {
+                __nanosleep(10000);
+                landed = __all_sync(0xffffffffu, mbar_try_wait(parts + warp, 0));
+            }
+            if (!landed) { ok = false; if (lane == 0) report_status(p.status, GQ_DEV_TIMEOUT); }
+        }
         for (int s = 1; s < p.split; ++s) {
 #pragma unroll
             for (int nt = 0; nt < MT; ++nt) {

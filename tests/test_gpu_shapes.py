@@ -176,6 +176,26 @@ def test_a_wait_on_a_silent_peer_runs_out_and_the_context_stays_usable():
     assert ops.device_status() == 0
 
 
+@pytest.mark.parametrize("m", [1, 8])
+def test_a_split_part_that_never_comes_ends_with_a_status(m):
+    """Split-K inside a cluster when a part stays away: a descriptor table in which two CTAs of a cluster of three take
+    themselves for the receiving one.  Their waits run out after the kernel's own limit (4 s), they leave only after the
+    third CTA has, status 1 is read, and the context stays usable.  (Nothing is out of bounds: every CTA stays in its tile.)"""
+    k, n_out, t = 5120, 128, F.Q4_K
+    raw = synth.random_blocks(n_out, k, t, seed=5, device=dev())
+    packed = ops.repack_tiles(raw, n_out, t).reshape(-1)
+    table = ops.build_descs([t], [n_out], k, 3)
+    good = torch.from_numpy(table.copy()).to(dev())
+    table[1::3, 6] = 0
+    x = synth.activations(m, k, device=dev())
+    want = ops.grouped_gemm(x, packed, good, 3, [t], n_out)
+    assert ops.device_status() == 0
+    ops.grouped_gemm(x, packed, torch.from_numpy(table).to(dev()), 3, [t], n_out)
+    assert ops.device_status() == 1
+    assert torch.equal(ops.grouped_gemm(x, packed, good, 3, [t], n_out), want)
+    assert ops.device_status() == 0
+
+
 # what the arithmetic of each form may add to the final bf16 rounding, as a fraction of the 2-norm of the products
 # w[n,k] * x[m,k] of an output (99.9th percentile, maximum).  Integer form: activations are 16-bit fixed point per
 # 256-block, everything else is exact integer arithmetic — 2^-16; the reference pins its kernel to the same 2e-5
