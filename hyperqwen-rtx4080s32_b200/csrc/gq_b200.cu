@@ -1257,6 +1257,16 @@ static int allow_smem(int bytes) {
     if (dev < 64) done_mask.fetch_or(1ull << dev);
     return GQ_OK;
 }
+// The matrix kernels are launched programmatically, one behind the other, and read tables and weights before they wait for the
+// kernel in front: what a load kernel has written is formally visible to them only if something on the stream has waited for that
+// kernel.  This launch is that something: an ordinary one, so it starts after the load kernel has completed, and whatever is
+// launched behind it starts later still.
+__global__ void publish_kernel() {}
+static int publish(cudaStream_t st) {
+    publish_kernel<<<1, 32, 0, st>>>();
+    GQ_LAUNCHED();
+    return GQ_OK;
+}
 #define GQ_EACH_TYPE(X)                                                                                                     \
     X(GQ_Q4_0) X(GQ_Q5_0) X(GQ_Q8_0) X(GQ_Q2_K) X(GQ_Q3_K) X(GQ_Q4_K) X(GQ_Q5_K) X(GQ_Q6_K) X(GQ_IQ4_NL) X(GQ_IQ3_S) X(GQ_IQ4_XS) \
     X(GQ_IQ3_XXS) X(GQ_IQ2_XXS) X(GQ_IQ2_XS) X(GQ_IQ2_S) X(GQ_IQ1_M)
@@ -1285,7 +1295,7 @@ extern "C" int gq_repack(int type, const void *raw_dev, int64_t n_out, int64_t K
 #undef GQ_ONE
     }
     GQ_LAUNCHED();
-    return GQ_OK;
+    return publish((cudaStream_t)stream);
 }
 
 extern "C" int gq_unrepack(int type, const void *tiles_dev, int64_t n_out, int64_t K, void *raw_dev, int64_t raw_row_stride, void *stream) {
@@ -1455,6 +1465,7 @@ extern "C" int64_t gq_build_descs_device(int n_shards, const int32_t *types, con
     sh.n = n_shards; sp.n = n_splits;
     build_descs_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, (cudaStream_t)stream>>>(sh, sp, (int)(K / GQ_QK), (int)tiles, (int)rows, desc_dev);
     GQ_LAUNCHED();
+    if (int rc = publish((cudaStream_t)stream)) return rc;
     return rows;
 }
 

@@ -238,7 +238,7 @@ class GGUFLinearMethod:
         layer.gguf_groups = {}
         for run in runs:
             packed, views, descs, splits, nb, block_bytes = ops.prepare_grouped_layer(
-                [tiles[sid] for sid in run], [layer.gguf_tiles_rows[sid] for sid in run], [layer.gguf_tiles_types[sid] for sid in run])
+                [tiles[sid] for sid in run], [layer.gguf_tiles_rows[sid] for sid in run], [layer.gguf_tiles_types[sid] for sid in run], wait=False)
             tiles.update(zip(run, views))
             layer.gguf_groups[run[0]] = (packed, descs, splits, run, nb, block_bytes)
         # the native call path of a layer that is one run (every layer whose shards are all tiled)
@@ -246,6 +246,9 @@ class GGUFLinearMethod:
         if len(runs) == 1 and len(runs[0]) == len(order):
             layer.gguf_native = ops.NativeRun(layer.gguf_groups[order[0]], [layer.gguf_tiles_rows[sid] for sid in order],
                                               [layer.gguf_tiles_types[sid] for sid in order])
+        # the layer may be called from any stream next: what was queued here is done first
+        for device in {group[0].device for group in layer.gguf_groups.values()}:
+            torch.cuda.current_stream(device).synchronize()
 
     def check_status(self, device=None) -> None:
         """Raise if any kernel of the path has reported a bounded wait that ran out on the device since the last

@@ -84,14 +84,18 @@ def build_descs(wtypes: Sequence[int], n_outs: Sequence[int], k: int, split: int
     return out
 
 
-def build_descs_on(device, wtypes: Sequence[int], n_outs: Sequence[int], k: int, splits: Sequence[int]) -> list[torch.Tensor]:
-    """The descriptor tables of several splits on a device, written there by a kernel (no copy, no synchronisation)."""
+def build_descs_on(device, wtypes: Sequence[int], n_outs: Sequence[int], k: int, splits: Sequence[int], wait: bool = True) -> list[torch.Tensor]:
+    """The descriptor tables of several splits on a device.  They hold addresses, so the caller's stream has finished with them
+    (and with all that was queued before, such as the repack of the weights they describe) when this returns: a layer may be
+    called from any stream and thread once it is loaded.  wait=False leaves that wait to the caller."""
     device = torch.device(device)
     if device.type != "cuda" or len(wtypes) > MAX_DEVICE_SHARDS or len(splits) > MAX_DEVICE_SPLITS:
         return [torch.from_numpy(build_descs(wtypes, n_outs, k, s)).to(device) for s in splits]
     tiles = sum(-(-int(n) // 64) for n in n_outs)
     buf = torch.empty((tiles * sum(splits), DESC_WORDS), dtype=torch.int32, device=device)
     native().build_descs([int(t) for t in wtypes], [int(n) for n in n_outs], int(k), [int(s) for s in splits], buf)
+    if wait:
+        torch.cuda.current_stream(buf.device).synchronize()
     return list(buf.split([tiles * s for s in splits]))
 
 
@@ -237,11 +241,12 @@ def pack_tiles(shards: Sequence[tuple[torch.Tensor, int, int]]):
     return packed, meta
 
 
-def prepare_grouped_layer(tiles_list: Sequence[torch.Tensor], n_outs: Sequence[int], wtypes: Sequence[int], ms=range(1, GEMV_MAX_ROWS + 1)):
+def prepare_grouped_layer(tiles_list: Sequence[torch.Tensor], n_outs: Sequence[int], wtypes: Sequence[int], ms=range(1, GEMV_MAX_ROWS + 1), *,
+                          wait: bool = True):
     """The loader's step for a run of shards (reference: prepare_grouped_layer,
     gguf-plugin/gluon/tiles_grouped.py:253-267): (packed buffer, the shards' tiles as views into it, the
     descriptor tables of every split a batch of 1..64 rows can choose plus split 1, those splits, nb, the
-    run's average bytes per 256 weights)."""
+    run's average bytes per 256 weights).  `wait` as in build_descs_on."""
     packed, meta = pack_tiles(list(zip(tiles_list, n_outs, wtypes)))
     views, off = [], 0
     for t in tiles_list:
@@ -252,7 +257,7 @@ def prepare_grouped_layer(tiles_list: Sequence[torch.Tensor], n_outs: Sequence[i
     block_bytes = int(round(sum(int(n) * F.BYTES_PER_256[int(w)] for n, w in zip(n_outs, wtypes)) / max(1, n_total)))
     sms = sm_count(packed.device)
     splits = sorted({grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sms) for m in {_ROW_CLASS[m] for m in ms}} | {1})
-    descs = build_descs_on(packed.device, wtypes, n_outs, nb * 256, splits)
+    descs = build_descs_on(packed.device, wtypes, n_outs, nb * 256, splits, wait)
     return packed, views, descs, splits, nb, block_bytes
 
 

@@ -55,7 +55,8 @@ int gq_slab_map(int type, int32_t *map);
 
 /* Raw GGUF rows -> packed tiles.  raw_dev: uint8 [n_out, (K/256)*bytes_per_256], row stride
  * raw_row_stride bytes (>= the row's bytes; any alignment).  out_dev: gq_packed_bytes bytes, 16-byte
- * aligned.  Rows past n_out in the last tile are written as zeros.
+ * aligned.  Rows past n_out in the last tile are written as zeros.  A call that multiplies the tiles may follow on the
+ * stream at once.
  * Reference: repack_tiles (gguf-plugin/gluon/tiles.py:128-130) called from _create_tiles
  * (gguf-plugin/patches/gguf-tiles-all-types.patch:73-131). */
 int gq_repack(int type, const void *raw_dev, int64_t n_out, int64_t K, int64_t raw_row_stride, void *out_dev, void *stream);
@@ -87,8 +88,8 @@ int64_t gq_desc_rows(int n_shards, const int64_t *n_outs, int split);
 int64_t gq_build_descs(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split, int32_t *desc_host);
 
 /* The tables of several splits written on the device, back to back (desc_dev has room for the gq_desc_rows of all of them,
- * 16-byte aligned), by one kernel on `stream`, so that loading a layer copies and waits for nothing.  Returns the number of
- * rows.  Up to GQ_MAX_DEVICE_SHARDS shards and GQ_MAX_DEVICE_SPLITS splits, GQ_ERR_LIMIT beyond. */
+ * 16-byte aligned), by one kernel on `stream`, without a copy.  A call that uses them may follow on the stream at once; the host
+ * does not wait, so another stream needs an event.  Returns the number of rows.  Up to GQ_MAX_DEVICE_SHARDS shards and GQ_MAX_DEVICE_SPLITS splits, GQ_ERR_LIMIT beyond. */
 #define GQ_MAX_DEVICE_SHARDS 8
 #define GQ_MAX_DEVICE_SPLITS 8
 int64_t gq_build_descs_device(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int n_splits, const int32_t *splits,
@@ -123,7 +124,10 @@ int64_t gq_workspace_bytes(int64_t M, int64_t K, int64_t n_total, int split);
  *   workspace_dev  at least gq_workspace_bytes(M, K, n_total, split) bytes, 256-byte aligned
  * Launches: activation preparation and the grouped kernel; splits up to 8 are reduced inside the kernel
  * (one thread-block cluster per tile, fixed summation order), larger ones by a third launch that sums fp32
- * partials from the workspace.  M == 0 is a no-op.  Reference: gluon_mul_mat_tiles_grouped for M <= 32 and the bm-64 wide form
+ * partials from the workspace.  M == 0 is a no-op.  The grouped kernel reads packed_dev and desc_dev ahead of its wait for the
+ * kernel in front (programmatic dependent launch): after a kernel other than those of the load calls above that writes either, let
+ * some other operation of the stream, or an event, come between.  The calls below behave alike.
+ * Reference: gluon_mul_mat_tiles_grouped for M <= 32 and the bm-64 wide form
  * (gguf-plugin/gluon/interface.py:141-188), quantize_activations_256, grouped_gemm, sum_partials
  * (gguf-plugin/gluon/tiles_grouped.py:110-162,1204-1275). */
 int gq_gemv_grouped(const void *x_dev, int64_t M, int64_t K, int64_t ldx, const void *packed_dev, const int32_t *desc_dev,

@@ -81,6 +81,48 @@ def test_descriptor_tables_written_on_the_device(parts):
             assert torch.equal(d.cpu(), torch.from_numpy(ops.build_descs(types, n_outs, k, s)))
 
 
+def test_a_loaded_run_is_complete_when_the_load_returns():
+    """A table holds addresses and any stream may call the layer next: the load's stream has nothing left to do."""
+    tiles = ops.repack_tiles(synth.random_blocks(64, 512, F.Q4_K, seed=1, device="cuda"), 64, F.Q4_K)
+    torch.cuda._sleep(200_000_000)
+    assert not torch.cuda.current_stream().query()
+    ops.prepare_grouped_layer([tiles], [64], [F.Q4_K])
+    assert torch.cuda.current_stream().query()
+    torch.cuda._sleep(200_000_000)
+    _layer([(64, F.Q4_K), (64, F.Q6_K), (64, F.IQ3_S)], 512)
+    assert torch.cuda.current_stream().query()
+
+
+@pytest.mark.parametrize("writer", ["gq_build_descs_device", "gq_repack"])
+def test_load_kernels_are_ordered_in_front_of_programmatic_launches(writer):
+    """The matrix kernels read tables and weights before they wait for the kernel in front of them, so no programmatic
+    launch may follow directly on a kernel that writes either.  Captured, not run: the edges of the graph tell."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    k, n, t = 512, 64, F.Q4_K
+    raw = synth.random_blocks(n, k, t, seed=2, device="cuda")
+    tiles = ops.repack_tiles(raw, n, t)
+    desc = ops.build_descs_on("cuda", [t], [n], k, [1])[0]
+    x, y = synth.activations(8, k, device="cuda"), torch.empty((8, n), dtype=torch.bfloat16, device="cuda")
+    ws = torch.empty(_lib.lib().gq_workspace_bytes(8, k, n, 1), dtype=torch.uint8, device="cuda")
+    ops.grouped_gemm(x, tiles, desc, 1, [t], n, out=y, workspace=ws)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        if writer == "gq_repack":
+            _lib.native().repack(raw, n, t, k // 256, tiles)
+        else:
+            _lib.native().build_descs([t], [n], k, [1], desc)
+        ops.grouped_gemm(x, tiles, desc, 1, [t], n, out=y, workspace=ws)
+    raw_graph = rt.cudaGraph_t(init_value=graph.raw_cuda_graph())
+    count = rt.cudaGraphGetEdges_v2(raw_graph)[-1]
+    err, src, dst, data, count = rt.cudaGraphGetEdges_v2(raw_graph, count)
+    assert int(err) == 0 and count >= 2
+    src, dst = [int(s) for s in src], [int(d) for d in dst]
+    programmatic = [e.type == rt.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic for e in data]
+    first = [not p for s, p in zip(src, programmatic) if s not in dst]
+    assert any(programmatic) and first and all(first)
+
+
 @pytest.mark.parametrize("t", [F.Q4_K, F.Q6_K, F.Q2_K, F.IQ3_S, F.Q8_0])
 @pytest.mark.parametrize("n_out,k", [(64, 256), (70, 768), (1024, 5120), (130, 17408)])
 def test_small_launches_that_convert_their_activations(t, n_out, k):
