@@ -40,13 +40,20 @@ const char *error_text(int rc) {
 }
 PyObject *g_error = PyExc_RuntimeError;      // GqError of _lib.py, kept for the life of the process
 
-void check(int64_t rc, const char *what) {
+void raise_if(int64_t rc, const char *what) {
     if (rc >= 0) return;
     std::string msg = std::string(what) + " failed (" + std::to_string(rc) + "): " + error_text((int)rc);
     if (rc == GQ_ERR_CUDA) msg += std::string(": ") + gq_last_cuda_error();
     PyErr_SetString(g_error, msg.c_str());
     throw py::error_already_set();
 }
+
+// what a call of the C ABI returned, kept until the GIL is held again
+struct Status {
+    int64_t rc = 0;
+    const char *what = "";
+    void check() const { raise_if(rc, what); }
+};
 
 inline bool plain_cuda(const at::Tensor &t, int device) {
     return t.is_cuda() && t.layout() == at::kStrided && t.get_device() == device && !t.requires_grad();
@@ -59,7 +66,7 @@ class Run {
         : packed_(std::move(packed)), descs_(std::move(descs)), splits_(std::move(splits)), K_(nb * 256), decode_rows_(decode_rows),
           pre_rows_(pre_rows), device_(packed_.get_device()) {
         std::vector<int32_t> t32(types.begin(), types.end());
-        check(info_ = gq_run_info((int)t32.size(), t32.data()), "gq_run_info");
+        raise_if(info_ = gq_run_info((int)t32.size(), t32.data()), "gq_run_info");
         for (int64_t n : n_outs) n_total_ += n;
         one_ = index_of(1);
         for (int64_t s : split_of_rows) by_rows_.push_back(index_of(s));
@@ -87,7 +94,7 @@ class Run {
 
     PyObject *call(py::handle xh, int pre, const at::Tensor *weight, const at::Tensor *residual, const at::Tensor *residual_out, float eps) {
         if (!THPVariable_CheckExact(xh.ptr()) || c10::impl::dispatch_mode_enabled()) return none();
-        const at::Tensor &x = THPVariable_Unpack(xh.ptr());
+        const at::Tensor x = THPVariable_Unpack(xh.ptr());      // a reference of its own: the GIL is released below
         const int64_t width = pre == 1 ? 2 * K_ : K_, nd = x.dim();
         if (nd < 1 || !plain_cuda(x, device_) || x.scalar_type() != at::kBFloat16 || x.size(-1) != width || x.stride(-1) != 1) return none();
         int64_t m = 1, ldx = width;
@@ -109,37 +116,49 @@ class Run {
         }
         const bool wide = m > decode_rows_;
         if (wide && ((ldx & 7) || (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15))) return none();
+        at::Tensor y;
+        Status status;
+        {
+            // the allocator and a full launch queue can keep the caller waiting: other Python threads go on meanwhile
+            py::gil_scoped_release unlocked;
+            status = launch(x, m, ldx, pre, weight, residual, residual_out, eps, y);
+        }
+        status.check();
+        return THPVariable_Wrap(std::move(y));
+    }
+
+    // the call itself, without the GIL: output and scratch, then the C ABI
+    Status launch(const at::Tensor &x, int64_t m, int64_t ldx, int pre, const at::Tensor *weight, const at::Tensor *residual,
+                  const at::Tensor *residual_out, float eps, at::Tensor &y) const {
+        const bool wide = m > decode_rows_;
         c10::cuda::CUDAGuard guard((c10::DeviceIndex)device_);
         void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device_).stream();
         at::DimVector sizes(x.sizes().begin(), x.sizes().end());
         sizes.back() = n_total_;
-        at::Tensor y = at::detail::empty_cuda(sizes, at::kBFloat16, x.device(), c10::nullopt);
+        y = at::detail::empty_cuda(sizes, at::kBFloat16, x.device(), c10::nullopt);
         auto *alloc = c10::cuda::CUDACachingAllocator::get();
         if (wide) {
             const int64_t n_desc = descs_[one_].size(0), need = gq_prefill_workspace_bytes(m, K_, n_total_, n_desc);
-            check(need, "gq_prefill_workspace_bytes");
+            if (need < 0) return {need, "gq_prefill_workspace_bytes"};
             c10::DataPtr ws = alloc->allocate((size_t)need + 1024);
             const uintptr_t base = (reinterpret_cast<uintptr_t>(ws.get()) + 1023) & ~(uintptr_t)1023;
-            check(gq_gemm_prefill(x.data_ptr(), m, K_, ldx, packed_.data_ptr(), (const int32_t *)descs_[one_].data_ptr(), n_desc, info_, y.data_ptr(),
-                                  n_total_, n_total_, (void *)base, need, stream), "gq_gemm_prefill");
-        } else {
-            const int i = by_rows_[m];
-            const int split = (int)splits_[i];
-            const at::Tensor &d = descs_[i];
-            const int64_t need = gq_workspace_bytes(m, K_, n_total_, split);
-            check(need, "gq_workspace_bytes");
-            c10::DataPtr ws = alloc->allocate((size_t)need);
-            if (pre)
-                check(gq_gemv_grouped_pre(x.data_ptr(), m, K_, ldx, pre, weight ? weight->data_ptr() : nullptr, residual ? residual->data_ptr() : nullptr,
-                                          residual_out ? residual_out->data_ptr() : nullptr, residual ? residual->stride(0) : 0, eps, packed_.data_ptr(),
-                                          (const int32_t *)d.data_ptr(), d.size(0), split, info_, y.data_ptr(), n_total_, n_total_, ws.get(), need, stream),
-                      "gq_gemv_grouped_pre");
-            else
-                // 15: nobody reads this workspace's status word, so a small launch may do without the preparation kernel
-                check(gq_gemv_grouped_phases(x.data_ptr(), m, K_, ldx, packed_.data_ptr(), (const int32_t *)d.data_ptr(), d.size(0), split, info_,
-                                             y.data_ptr(), n_total_, n_total_, ws.get(), need, stream, 15), "gq_gemv_grouped");
+            return {gq_gemm_prefill(x.data_ptr(), m, K_, ldx, packed_.data_ptr(), (const int32_t *)descs_[one_].data_ptr(), n_desc, info_, y.data_ptr(),
+                                    n_total_, n_total_, (void *)base, need, stream), "gq_gemm_prefill"};
         }
-        return THPVariable_Wrap(std::move(y));
+        const int i = by_rows_[m];
+        const int split = (int)splits_[i];
+        const at::Tensor &d = descs_[i];
+        const int64_t need = gq_workspace_bytes(m, K_, n_total_, split);
+        if (need < 0) return {need, "gq_workspace_bytes"};
+        c10::DataPtr ws = alloc->allocate((size_t)need);
+        if (pre)
+            return {gq_gemv_grouped_pre(x.data_ptr(), m, K_, ldx, pre, weight ? weight->data_ptr() : nullptr, residual ? residual->data_ptr() : nullptr,
+                                        residual_out ? residual_out->data_ptr() : nullptr, residual ? residual->stride(0) : 0, eps, packed_.data_ptr(),
+                                        (const int32_t *)d.data_ptr(), d.size(0), split, info_, y.data_ptr(), n_total_, n_total_, ws.get(), need, stream),
+                    "gq_gemv_grouped_pre"};
+        // 15: nobody reads this workspace's status word, so a small launch may do without the preparation kernel
+        return {gq_gemv_grouped_phases(x.data_ptr(), m, K_, ldx, packed_.data_ptr(), (const int32_t *)d.data_ptr(), d.size(0), split, info_,
+                                       y.data_ptr(), n_total_, n_total_, ws.get(), need, stream, 15), "gq_gemv_grouped"};
     }
 
     at::Tensor packed_;
@@ -154,38 +173,58 @@ class Run {
 void *stream_of(const at::Tensor &t) { return c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)t.get_device()).stream(); }
 
 void repack(const at::Tensor &raw, int64_t n_out, int64_t type, int64_t nb, const at::Tensor &out) {
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)raw.get_device());
-    check(gq_repack((int)type, raw.data_ptr(), n_out, nb * 256, raw.stride(0), out.data_ptr(), stream_of(raw)), "gq_repack");
+    Status status;
+    {
+        py::gil_scoped_release unlocked;
+        c10::cuda::CUDAGuard guard((c10::DeviceIndex)raw.get_device());
+        status = {gq_repack((int)type, raw.data_ptr(), n_out, nb * 256, raw.stride(0), out.data_ptr(), stream_of(raw)), "gq_repack"};
+    }
+    status.check();
 }
 at::Tensor dequantize(const at::Tensor &tiles, int64_t n_out, int64_t k, int64_t type, bool bf16) {
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)tiles.get_device());
-    at::Tensor out = at::detail::empty_cuda({n_out, k}, bf16 ? at::kBFloat16 : at::kFloat, tiles.device(), c10::nullopt);
-    check(gq_dequant((int)type, tiles.data_ptr(), n_out, k, out.data_ptr(), bf16 ? 1 : 0, k, stream_of(tiles)), "gq_dequant");
+    Status status;
+    at::Tensor out;
+    {
+        py::gil_scoped_release unlocked;
+        c10::cuda::CUDAGuard guard((c10::DeviceIndex)tiles.get_device());
+        out = at::detail::empty_cuda({n_out, k}, bf16 ? at::kBFloat16 : at::kFloat, tiles.device(), c10::nullopt);
+        status = {gq_dequant((int)type, tiles.data_ptr(), n_out, k, out.data_ptr(), bf16 ? 1 : 0, k, stream_of(tiles)), "gq_dequant"};
+    }
+    status.check();
     return out;
 }
 void build_descs(const std::vector<int32_t> &types, const std::vector<int64_t> &n_outs, int64_t k, const std::vector<int32_t> &splits, const at::Tensor &out) {
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)out.get_device());
-    check(gq_build_descs_device((int)types.size(), types.data(), n_outs.data(), k, (int)splits.size(), splits.data(), (int32_t *)out.data_ptr(),
-                                stream_of(out)), "gq_build_descs_device");
+    Status status;
+    {
+        py::gil_scoped_release unlocked;
+        c10::cuda::CUDAGuard guard((c10::DeviceIndex)out.get_device());
+        status = {gq_build_descs_device((int)types.size(), types.data(), n_outs.data(), k, (int)splits.size(), splits.data(), (int32_t *)out.data_ptr(),
+                                        stream_of(out)), "gq_build_descs_device"};
+    }
+    status.check();
 }
 
 // rows `ids` of a raw table -> weights; None: not the plain case
 PyObject *dequantize_rows(py::handle rawh, int64_t type, py::handle idsh, bool bf16) {
     if (!THPVariable_CheckExact(rawh.ptr()) || !THPVariable_CheckExact(idsh.ptr()) || c10::impl::dispatch_mode_enabled()) Py_RETURN_NONE;
-    const at::Tensor &raw = THPVariable_Unpack(rawh.ptr()), &ids = THPVariable_Unpack(idsh.ptr());
+    const at::Tensor raw = THPVariable_Unpack(rawh.ptr()), ids = THPVariable_Unpack(idsh.ptr());
     const int B = gq_bytes_per_256((int)type);
     if (!raw.is_cuda() || raw.scalar_type() != at::kByte || raw.dim() != 2 || raw.stride(1) != 1 || raw.size(0) == 0 || B == 0 || raw.size(1) == 0 ||
         raw.size(1) % B || !ids.is_cuda() || ids.get_device() != raw.get_device() || !ids.is_contiguous() || ids.numel() == 0 ||
         (ids.scalar_type() != at::kLong && ids.scalar_type() != at::kInt)) Py_RETURN_NONE;
-    const int device = raw.get_device();
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
-    void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
     const int64_t K = raw.size(1) / B * 256;
     at::DimVector sizes(ids.sizes().begin(), ids.sizes().end());
     sizes.push_back(K);
-    at::Tensor out = at::detail::empty_cuda(sizes, bf16 ? at::kBFloat16 : at::kFloat, raw.device(), c10::nullopt);
-    check(gq_dequant_rows((int)type, raw.data_ptr(), raw.size(0), K, raw.stride(0), ids.data_ptr(), ids.scalar_type() == at::kLong ? 8 : 4, ids.numel(),
-                          out.data_ptr(), bf16 ? 1 : 0, K, stream), "gq_dequant_rows");
+    at::Tensor out;
+    Status status;
+    {
+        py::gil_scoped_release unlocked;
+        c10::cuda::CUDAGuard guard((c10::DeviceIndex)raw.get_device());
+        out = at::detail::empty_cuda(sizes, bf16 ? at::kBFloat16 : at::kFloat, raw.device(), c10::nullopt);
+        status = {gq_dequant_rows((int)type, raw.data_ptr(), raw.size(0), K, raw.stride(0), ids.data_ptr(), ids.scalar_type() == at::kLong ? 8 : 4,
+                                  ids.numel(), out.data_ptr(), bf16 ? 1 : 0, K, stream_of(raw)), "gq_dequant_rows"};
+    }
+    status.check();
     return THPVariable_Wrap(std::move(out));
 }
 

@@ -1,6 +1,8 @@
 """The native call path of GGUFLinearMethod.apply against the custom op, which runs the same kernels: the same bits for
 every row count at the edges of the dispatch and every input layout, and the general path where the native one steps aside."""
 import copy
+import threading
+import time
 
 import pytest
 import torch
@@ -79,6 +81,33 @@ def test_descriptor_tables_written_on_the_device(parts):
     for k, splits in [(256, [1]), (5120, [1, 3, 20])]:
         for s, d in zip(splits, ops.build_descs_on("cuda", types, n_outs, k, splits)):
             assert torch.equal(d.cpu(), torch.from_numpy(ops.build_descs(types, n_outs, k, s)))
+
+
+def test_other_threads_run_while_a_call_waits_for_the_launch_queue():
+    """A full launch queue holds the caller back, not the interpreter."""
+    lin = _layer([(64, F.Q4_K), (64, F.Q6_K), (64, F.IQ3_S)], 512)
+    x = synth.activations(8, 512, device="cuda")
+    lin(x)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(2_000_000_000)                     # about a second
+    took = []
+
+    def calls():
+        t0 = time.monotonic()
+        for _ in range(4000):
+            lin(x)
+        took.append(time.monotonic() - t0)
+
+    worker = threading.Thread(target=calls)
+    gap, last = 0.0, time.monotonic()
+    worker.start()
+    while worker.is_alive():
+        time.sleep(1e-3)
+        now = time.monotonic()
+        gap, last = max(gap, now - last), now
+    worker.join()
+    torch.cuda.synchronize()
+    assert took[0] > 0.5 and gap < 0.3, (took, gap)
 
 
 def test_a_loaded_run_is_complete_when_the_load_returns():
