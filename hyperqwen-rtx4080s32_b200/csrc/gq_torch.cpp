@@ -7,11 +7,12 @@
 // row count — and does the call's host work here: output and scratch from torch's caching allocator on the current
 // stream, then the C ABI of include/gq_b200.h.
 //
-// forward() answers None for whatever is not the plain case (dtype, layout, device, autograd, torch dispatch modes, a
-// call of zero rows); the caller then takes the general path, which also states the errors.
+// forward() answers None for whatever is not the plain case (dtype, layout, device, autograd, torch modes, tracing, function
+// transforms, a call of zero rows); the caller then takes the general path, which also states the errors.
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
-#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -55,9 +56,20 @@ struct Status {
     void check() const { raise_if(rc, what); }
 };
 
-inline bool plain_cuda(const at::Tensor &t, int device) {
-    return t.is_cuda() && t.layout() == at::kStrided && t.get_device() == device && !t.requires_grad();
+// Whether nothing stands between a torch call and its kernel on this thread: no dispatch or function mode, no tracer, no
+// function transform (vmap, jvp).  Each of them shows in the thread's own dispatch keys or as a function mode.
+inline bool plain_thread() {
+    const uint64_t keys = c10::impl::tls_local_dispatch_key_set().included_.raw_repr();
+    return !(keys & ~c10::default_included_set.raw_repr()) && !at::impl::torch_function_mode_enabled();
 }
+// Whether a tensor is what its memory says: a dense CUDA tensor with no key beside the usual ones (negative view, zero tensor,
+// a transform's or a mode's wrapper)
+inline bool plain_tensor(const at::Tensor &t) {
+    constexpr c10::DispatchKeySet usual({c10::DispatchKey::CUDA, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::ADInplaceOrView,
+                                         c10::DispatchKey::AutocastCUDA});
+    return t.is_cuda() && !(t.key_set().raw_repr() & ~usual.raw_repr()) && !t.has_names();
+}
+inline bool plain_cuda(const at::Tensor &t, int device) { return plain_tensor(t) && t.get_device() == device && !t.requires_grad(); }
 
 class Run {
   public:
@@ -93,7 +105,7 @@ class Run {
     static PyObject *none() { Py_RETURN_NONE; }
 
     PyObject *call(py::handle xh, int pre, const at::Tensor *weight, const at::Tensor *residual, const at::Tensor *residual_out, float eps) {
-        if (!THPVariable_CheckExact(xh.ptr()) || c10::impl::dispatch_mode_enabled()) return none();
+        if (!THPVariable_CheckExact(xh.ptr()) || !plain_thread()) return none();
         const at::Tensor x = THPVariable_Unpack(xh.ptr());      // a reference of its own: the GIL is released below
         const int64_t width = pre == 1 ? 2 * K_ : K_, nd = x.dim();
         if (nd < 1 || !plain_cuda(x, device_) || x.scalar_type() != at::kBFloat16 || x.size(-1) != width || x.stride(-1) != 1) return none();
@@ -206,11 +218,11 @@ void build_descs(const std::vector<int32_t> &types, const std::vector<int64_t> &
 
 // rows `ids` of a raw table -> weights; None: not the plain case
 PyObject *dequantize_rows(py::handle rawh, int64_t type, py::handle idsh, bool bf16) {
-    if (!THPVariable_CheckExact(rawh.ptr()) || !THPVariable_CheckExact(idsh.ptr()) || c10::impl::dispatch_mode_enabled()) Py_RETURN_NONE;
+    if (!THPVariable_CheckExact(rawh.ptr()) || !THPVariable_CheckExact(idsh.ptr()) || !plain_thread()) Py_RETURN_NONE;
     const at::Tensor raw = THPVariable_Unpack(rawh.ptr()), ids = THPVariable_Unpack(idsh.ptr());
     const int B = gq_bytes_per_256((int)type);
-    if (!raw.is_cuda() || raw.scalar_type() != at::kByte || raw.dim() != 2 || raw.stride(1) != 1 || raw.size(0) == 0 || B == 0 || raw.size(1) == 0 ||
-        raw.size(1) % B || !ids.is_cuda() || ids.get_device() != raw.get_device() || !ids.is_contiguous() || ids.numel() == 0 ||
+    if (!plain_tensor(raw) || !plain_tensor(ids) || raw.scalar_type() != at::kByte || raw.dim() != 2 || raw.stride(1) != 1 || raw.size(0) == 0 || B == 0 || raw.size(1) == 0 ||
+        raw.size(1) % B || ids.get_device() != raw.get_device() || !ids.is_contiguous() || ids.numel() == 0 ||
         (ids.scalar_type() != at::kLong && ids.scalar_type() != at::kInt)) Py_RETURN_NONE;
     const int64_t K = raw.size(1) / B * 256;
     at::DimVector sizes(ids.sizes().begin(), ids.sizes().end());

@@ -83,6 +83,37 @@ def test_descriptor_tables_written_on_the_device(parts):
             assert torch.equal(d.cpu(), torch.from_numpy(ops.build_descs(types, n_outs, k, s)))
 
 
+@pytest.mark.parametrize("how", ["vmap", "negative view", "trace", "function mode", "zero tensor"])
+def test_native_path_stands_aside_for_what_is_not_a_plain_tensor_call(how):
+    """Transforms, tracing, modes and tensors whose memory is not their value go through the custom op, as without the
+    native path."""
+    k, m = 512, 4
+    lin = _layer([(64, F.Q4_K), (64, F.Q6_K), (64, F.IQ3_S)], k)
+    x, x2 = synth.activations(m, k, device="cuda"), synth.activations(2 * m, k, device="cuda").reshape(2, m, k)
+    if how == "vmap":
+        with pytest.raises(RuntimeError, match="Batching rule"):      # the custom op has none
+            torch.func.vmap(lin)(x2)
+    elif how == "negative view":
+        assert torch.equal(lin(torch._neg_view(x)), lin(-x))
+    elif how == "trace":
+        traced = torch.jit.trace(lin, x, check_trace=False)
+        assert torch.equal(traced(x2[0]), lin(x2[0]))
+    elif how == "function mode":
+        class Seen(torch.overrides.TorchFunctionMode):
+            names = []
+
+            def __torch_function__(self, func, types, args=(), kwargs=None):
+                self.names.append(str(func))
+                return func(*args, **(kwargs or {}))
+
+        want = lin(x)
+        with Seen():
+            assert torch.equal(lin(x), want)
+        assert any("fused_mul_mat_gguf_tiles_grouped" in n for n in Seen.names)
+    else:
+        assert not lin(torch._efficientzerotensor((m, k), dtype=torch.bfloat16, device="cuda")).any()
+
+
 def test_other_threads_run_while_a_call_waits_for_the_launch_queue():
     """A full launch queue holds the caller back, not the interpreter."""
     lin = _layer([(64, F.Q4_K), (64, F.Q6_K), (64, F.IQ3_S)], 512)
