@@ -252,7 +252,8 @@ constexpr int dequant_rows_smem() {
 // ---- embedding lookup: rows `ids` of a raw table -> row-major weights --------------------------------------------
 // One CTA takes sixteen ids and up to eight k-blocks: the raw bytes are gathered into shared memory, permuted into slabs
 // there, and each warp decodes one k-block.  One launch and one pass over memory; gathering, repacking and dequantising as
-// three kernels cost 80 us for 2048 IQ2_S rows of 5120 (24 MB), this one 10.6.  An id outside the table is reported, its row is not read.
+// three kernels cost 80 us for 2048 IQ2_S rows of 5120 (24 MB), this one 10.6.  An id outside the table is reported, its row is not read,
+// its output is NaN.
 template <int TYPE, bool BF16>
 __global__ void __launch_bounds__(GQ_LOAD_THREADS) dequant_rows_kernel(const uint8_t *__restrict__ raw, int64_t n_rows, int nb, int64_t row_stride,
                                                                        const void *__restrict__ ids, int ids64, int64_t n_ids, void *__restrict__ out,
@@ -288,6 +289,13 @@ __global__ void __launch_bounds__(GQ_LOAD_THREADS) dequant_rows_kernel(const uin
     const bool vec = !((reinterpret_cast<uintptr_t>(out) & 15) | ((ld * (BF16 ? 2 : 4)) & 15));
     uint8_t *o = reinterpret_cast<uint8_t *>(out) + (i0 * ld + (int64_t)(kb0 + warp) * 256) * (BF16 ? 2 : 4);
     dequant_slab<TYPE, BF16>(slabs + warp * 16 * B, aux, lane, dyn + warp * GQ_DEQ_STAGE, o, ld, rows, vec);
+    __syncwarp();
+    for (int r = 0; r < rows; ++r)
+        if (s_id[r] < 0)
+            for (int c = lane; c < 256; c += 32) {
+                if constexpr (BF16) reinterpret_cast<uint16_t *>(o)[r * ld + c] = 0x7fc0u;
+                else reinterpret_cast<uint32_t *>(o)[r * ld + c] = 0x7fc00000u;
+            }
 }
 
 }  // namespace gq

@@ -255,7 +255,7 @@ class GGUFLinearMethod:
         check (the result of that call was incomplete).  Synchronises; meant for the engine to call between steps."""
         code = ops.device_status(device, clear=True)
         if code:
-            raise RuntimeError(f"gq_b200: a kernel reported device status {code} (1: a bounded wait ran out, 2: bad shape) since the last check")
+            raise RuntimeError(f"gq_b200: a kernel reported device status {code} (1: a bounded wait ran out; 2: bad shape, a tile's type that contradicts the call, or an id outside an embedding table) since the last check")
 
     # ---- a6 ----
     def apply(self, layer: torch.nn.Module, x: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:

@@ -154,7 +154,11 @@ def load_gguf(path: str, device="cuda", strict: bool = True) -> LoadedModel:
 def embedding_lookup(raw: torch.Tensor, wtype: int, ids: torch.Tensor, dtype=torch.bfloat16) -> torch.Tensor:
     """Rows `ids` of a quantized embedding table raw uint8 [vocab, row_bytes] (kept raw, as the plugin keeps it:
     gguf-tiles-all-types.patch:80-89) dequantised to [*ids.shape, K]: one launch gathers the rows' bytes and decodes
-    them with the decoders that serve the weights — bit-identical to gguf.quants.dequantize of those rows."""
+    them with the decoders that serve the weights — bit-identical to gguf.quants.dequantize of those rows.
+
+    An id outside the table: in host memory it raises IndexError.  On the device nothing can be raised without waiting for it; its
+    row is not read, its output is NaN, and ops.device_status (GGUFLinearMethod.check_status, which an engine calls between steps)
+    reports 2."""
     from . import ops
 
     if int(wtype) not in F.SUPPORTED_TYPES:

@@ -192,8 +192,9 @@ def repack_shards(raws: Sequence[torch.Tensor], wtypes: Sequence[int]) -> list[t
 
 
 def dequantize_rows(raw: torch.Tensor, wtype: int, ids: torch.Tensor, dtype=torch.float32) -> torch.Tensor:
-    """Rows `ids` (int32 or int64, any shape) of a raw uint8 table [rows, row_bytes] -> [*ids.shape, K], in one launch; the
-    values are those of dequantize_tiles.  An id outside the table is reported through device_status."""
+    """Rows `ids` (int32 or int64, any shape and layout) of a raw uint8 table [rows, row_bytes] -> [*ids.shape, K], in one launch;
+    the values are those of dequantize_tiles.  An id outside the table raises IndexError where ids are in host memory; on the
+    device its row is not read, its output is NaN and device_status reports 2."""
     out = native().dequantize_rows(raw, int(wtype), ids, dtype is torch.bfloat16) if dtype in (torch.float32, torch.bfloat16) else None
     if out is not None:
         return out
@@ -203,12 +204,26 @@ def dequantize_rows(raw: torch.Tensor, wtype: int, ids: torch.Tensor, dtype=torc
     bb = F.BYTES_PER_256[int(wtype)]
     if raw.dtype != torch.uint8 or raw.dim() != 2 or raw.shape[1] % bb:
         raise GqError(f"raw must be uint8 [rows, whole {bb}-byte k-blocks], got {raw.dtype} {tuple(raw.shape)}")
-    k = raw.shape[1] // bb * F.QK
-    rows = raw.index_select(0, ids.reshape(-1).to(raw.device))       # layouts and index types the kernel does not read
-    n = int(rows.shape[0])
+    if ids.dtype not in (torch.int32, torch.int64):
+        raise GqError(f"ids must be int32 or int64, got {ids.dtype}")
+    n_rows, k = raw.shape[0], raw.shape[1] // bb * F.QK
+    out = torch.empty((*ids.shape, k), dtype=dtype, device=raw.device)
+    n = ids.numel()
     if n == 0:
-        return torch.empty((*ids.shape, k), dtype=dtype, device=raw.device)
-    return dequantize_tiles(repack_tiles(rows, n, int(wtype)), n, k, int(wtype), dtype=dtype).reshape(*ids.shape, k)
+        return out
+    if n_rows == 0 or (not ids.is_cuda and (int(ids.min()) < 0 or int(ids.max()) >= n_rows)):
+        raise IndexError(f"ids reach outside the table's {n_rows} rows")
+    flat = ids.reshape(-1).to(raw.device)
+    if raw.stride(1) != 1:
+        # a table whose rows the kernel does not read in place: the rows asked for, ids outside the table kept outside
+        inside = (flat >= 0) & (flat < n_rows)
+        raw = raw.index_select(0, flat.clamp(0, n_rows - 1))
+        flat = torch.where(inside, torch.arange(n, device=raw.device), -1)
+    flat = flat.contiguous()
+    with torch.cuda.device(raw.device):
+        check(lib().gq_dequant_rows(int(wtype), raw.data_ptr(), raw.shape[0], k, raw.stride(0), flat.data_ptr(), flat.element_size(), n, out.data_ptr(),
+                                    0 if dtype == torch.float32 else 1, k, _stream_ptr(raw)), "gq_dequant_rows")
+    return out
 
 
 def _adjacent(tiles: Sequence[torch.Tensor]) -> bool:

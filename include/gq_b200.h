@@ -73,7 +73,7 @@ int gq_dequant(int type, const void *tiles_dev, int64_t n_out, int64_t K, void *
 
 /* Rows of a raw (not packed) table -> dequantised weights [n_ids, K], row stride ld elements: the quantized embedding lookup.
  * raw_dev uint8 [n_rows, raw_row_stride], ids_dev int32 or int64 (ids_bytes 4 or 8); out_dtype as gq_dequant.  An id outside
- * [0, n_rows) is not read: its output row is unspecified and the device's status word (gq_device_status) becomes 2.
+ * [0, n_rows) is not read: its output row is NaN and the device's status word (gq_device_status) becomes 2.
  * Reference: the plugin keeps the embedding raw and gathers its rows (gguf-plugin/patches/gguf-tiles-all-types.patch:80-89). */
 int gq_dequant_rows(int type, const void *raw_dev, int64_t n_rows, int64_t K, int64_t raw_row_stride, const void *ids_dev, int ids_bytes,
                     int64_t n_ids, void *out_dev, int out_dtype, int64_t ld, void *stream);
@@ -263,7 +263,8 @@ int gq_gemm_prefill(const void *x_dev, int64_t M, int64_t K, int64_t ldx, const 
 int gq_read_status(const void *workspace_dev, int64_t workspace_bytes, void *stream);
 
 /* The largest device status code any kernel of this library has reported on the current device since the word was
- * last cleared (synchronises the stream; clear != 0 resets it after reading): 0, or a positive GQ_DEV_* code.  Every
+ * last cleared (synchronises the stream; clear != 0 resets it after reading): 0, or a positive GQ_DEV_* code (those above; 2 also
+ * for an id outside the table given to gq_dequant_rows).  Every
  * kernel that sets a workspace's status word sets this one too, so a caller that frees its workspace after each call,
  * or uses the entry point without a workspace argument, still sees a timeout.  Meant to be called between steps.
  * Reference: none (the reference's kernels have no waits that can run out). */

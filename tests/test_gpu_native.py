@@ -75,6 +75,35 @@ def test_load_and_lookup_kernels_at_the_edges(t):
     assert torch.equal(got[[0, 3]].cpu(), want[[0, n - 1]])
 
 
+@pytest.mark.parametrize("t", [F.Q6_K, F.IQ2_S])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_lookup_answers_alike_for_every_layout(t, dt):
+    """Ids and tables in every layout: the same rows, and an id outside the table gives NaN and status 2 on the device and an
+    IndexError from host memory."""
+    n, k = 40, 2304
+    raw = synth.random_blocks(n, k, t, seed=77, device="cuda")
+    want = torch.from_numpy(oracle.dequantize(raw.cpu().numpy(), t)).to(dt)
+    good = torch.tensor([[3, 39, 0], [7, 3, 20]], device="cuda")
+    bad = torch.tensor([[3, 40, 0], [7, -1, 20]], device="cuda")
+    wide = torch.zeros((n, 2 * raw.shape[1]), dtype=torch.uint8, device="cuda")
+    wide[:, ::2] = raw
+    spread = torch.stack([good, bad], -1)
+    for table in (raw, wide[:, ::2], torch.cat([raw, raw], 1)[:, raw.shape[1]:]):
+        for ids in (good, good.int(), good.t().contiguous().t(), spread[..., 0], good.cpu()):
+            assert torch.equal(ops.dequantize_rows(table, t, ids, dt).cpu(), want[good.cpu()])
+        assert ops.device_status() == 0
+        for ids in (bad, bad.int(), bad.t().contiguous().t(), spread[..., 1]):
+            got = ops.dequantize_rows(table, t, ids, dt).cpu()
+            assert bool(got[0, 1].isnan().all()) and bool(got[1, 1].isnan().all())
+            assert torch.equal(got[:, [0, 2]], want[bad.cpu()[:, [0, 2]]])
+            assert ops.device_status() == 2
+        with pytest.raises(IndexError):
+            ops.dequantize_rows(table, t, bad.cpu(), dt)
+        assert ops.dequantize_rows(table, t, good[:0], dt).shape == (0, 3, k)
+    with pytest.raises(RuntimeError):
+        ops.dequantize_rows(raw, t, good.float(), dt)
+
+
 @pytest.mark.parametrize("parts", [[(1, F.Q4_K)], [(130, F.Q4_K), (64, F.Q8_0), (70, F.IQ1_M)], [(64 * i, F.Q6_K) for i in range(1, 9)]])
 def test_descriptor_tables_written_on_the_device(parts):
     n_outs, types = [n for n, _ in parts], [t for _, t in parts]
