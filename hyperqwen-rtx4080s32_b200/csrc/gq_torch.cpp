@@ -221,7 +221,7 @@ PyObject *dequantize_rows(py::handle rawh, int64_t type, py::handle idsh, bool b
     if (!THPVariable_CheckExact(rawh.ptr()) || !THPVariable_CheckExact(idsh.ptr()) || !plain_thread()) Py_RETURN_NONE;
     const at::Tensor raw = THPVariable_Unpack(rawh.ptr()), ids = THPVariable_Unpack(idsh.ptr());
     const int B = gq_bytes_per_256((int)type);
-    if (!plain_tensor(raw) || !plain_tensor(ids) || raw.scalar_type() != at::kByte || raw.dim() != 2 || raw.stride(1) != 1 || raw.size(0) == 0 || B == 0 || raw.size(1) == 0 ||
+    if (!plain_tensor(raw) || !plain_tensor(ids) || raw.scalar_type() != at::kByte || raw.dim() != 2 || raw.stride(1) != 1 || raw.stride(0) < raw.size(1) || raw.size(0) == 0 || B == 0 || raw.size(1) == 0 ||
         raw.size(1) % B || ids.get_device() != raw.get_device() || !ids.is_contiguous() || ids.numel() == 0 ||
         (ids.scalar_type() != at::kLong && ids.scalar_type() != at::kInt)) Py_RETURN_NONE;
     const int64_t K = raw.size(1) / B * 256;

@@ -214,7 +214,7 @@ def dequantize_rows(raw: torch.Tensor, wtype: int, ids: torch.Tensor, dtype=torc
     if n_rows == 0 or (not ids.is_cuda and (int(ids.min()) < 0 or int(ids.max()) >= n_rows)):
         raise IndexError(f"ids reach outside the table's {n_rows} rows")
     flat = ids.reshape(-1).to(raw.device)
-    if raw.stride(1) != 1:
+    if raw.stride(1) != 1 or raw.stride(0) < raw.shape[1]:
         # a table whose rows the kernel does not read in place: the rows asked for, ids outside the table kept outside
         inside = (flat >= 0) & (flat < n_rows)
         raw = raw.index_select(0, flat.clamp(0, n_rows - 1))

@@ -102,6 +102,9 @@ def test_lookup_answers_alike_for_every_layout(t, dt):
         assert ops.dequantize_rows(table, t, good[:0], dt).shape == (0, 3, k)
     with pytest.raises(RuntimeError):
         ops.dequantize_rows(raw, t, good.float(), dt)
+    one = raw[5:6].expand(n, -1)        # a table of one repeated row: row stride 0
+    assert torch.equal(ops.dequantize_rows(one, t, good, dt).cpu(), want[5].expand(2, 3, -1))
+    assert ops.device_status() == 0
 
 
 @pytest.mark.parametrize("parts", [[(1, F.Q4_K)], [(130, F.Q4_K), (64, F.Q8_0), (70, F.IQ1_M)], [(64 * i, F.Q6_K) for i in range(1, 9)]])
