@@ -238,7 +238,8 @@ class GGUFLinearMethod:
         layer.gguf_groups = {}
         for run in runs:
             packed, views, descs, splits, nb, block_bytes = ops.prepare_grouped_layer(
-                [tiles[sid] for sid in run], [layer.gguf_tiles_rows[sid] for sid in run], [layer.gguf_tiles_types[sid] for sid in run], wait=False)
+                [tiles[sid] for sid in run], [layer.gguf_tiles_rows[sid] for sid in run], [layer.gguf_tiles_types[sid] for sid in run],
+                wait=False, in_place=True)
             tiles.update(zip(run, views))
             layer.gguf_groups[run[0]] = (packed, descs, splits, run, nb, block_bytes)
         # the native call path of a layer that is one run (every layer whose shards are all tiled)

@@ -237,8 +237,9 @@ def _adjacent(tiles: Sequence[torch.Tensor]) -> bool:
     return True
 
 
-def pack_tiles(shards: Sequence[tuple[torch.Tensor, int, int]]):
-    """[(tiles, n_out, type)] -> (packed uint8 buffer, meta): the shards' tiles back to back in one buffer."""
+def pack_tiles(shards: Sequence[tuple[torch.Tensor, int, int]], in_place: bool = False):
+    """[(tiles, n_out, type)] -> (packed uint8 buffer, meta): the shards' tiles back to back in one buffer.  Several shards are
+    copied, so the caller's tiles stay its own; in_place gives them up, and those that lie back to back already become the buffer."""
     nb = None
     for t, n_out, wt in shards:
         if t.shape[0] != -(-n_out // 64) or (nb is not None and t.shape[1] != nb):
@@ -247,7 +248,7 @@ def pack_tiles(shards: Sequence[tuple[torch.Tensor, int, int]]):
     tiles = [t for t, _, _ in shards]
     if len(shards) == 1:
         packed = tiles[0].reshape(-1)
-    elif _adjacent(tiles):
+    elif in_place and _adjacent(tiles):
         packed = tiles[0].as_strided((sum(t.numel() for t in tiles),), (1,))
     else:
         packed = torch.cat([t.reshape(-1) for t in tiles])
@@ -257,12 +258,12 @@ def pack_tiles(shards: Sequence[tuple[torch.Tensor, int, int]]):
 
 
 def prepare_grouped_layer(tiles_list: Sequence[torch.Tensor], n_outs: Sequence[int], wtypes: Sequence[int], ms=range(1, GEMV_MAX_ROWS + 1), *,
-                          wait: bool = True):
+                          wait: bool = True, in_place: bool = False):
     """The loader's step for a run of shards (reference: prepare_grouped_layer,
     gguf-plugin/gluon/tiles_grouped.py:253-267): (packed buffer, the shards' tiles as views into it, the
     descriptor tables of every split a batch of 1..64 rows can choose plus split 1, those splits, nb, the
-    run's average bytes per 256 weights).  `wait` as in build_descs_on."""
-    packed, meta = pack_tiles(list(zip(tiles_list, n_outs, wtypes)))
+    run's average bytes per 256 weights).  `wait` as in build_descs_on, `in_place` as in pack_tiles."""
+    packed, meta = pack_tiles(list(zip(tiles_list, n_outs, wtypes)), in_place)
     views, off = [], 0
     for t in tiles_list:
         views.append(packed[off:off + t.numel()].view(t.shape))

@@ -119,6 +119,25 @@ def test_build_descs_rejects_bad_arguments(gq_lib):
     assert gq_lib.gq_workspace_bytes(8, 768, 64, 2) > gq_lib.gq_workspace_bytes(8, 768, 64, 1) > 0
 
 
+def test_pack_tiles_copies_unless_the_caller_gives_its_tiles_up():
+    """Tiles that happen to lie back to back in the caller's memory, at an odd address here, are copied into a buffer of the
+    run's own; in_place hands them over."""
+    import torch
+
+    from hyperqwen_rtx4080s32_b200 import ops
+
+    size = 64 * F.BYTES_PER_256[F.Q4_K]
+    staging = torch.arange(1 + 3 * size, dtype=torch.int64).to(torch.uint8)
+    a, b = staging[1:1 + size].view(1, 1, size), staging[1 + size:].view(2, 1, size)
+    shards = [(a, 64, F.Q4_K), (b, 128, F.Q4_K)]
+    packed, _ = ops.pack_tiles(shards)
+    assert packed.untyped_storage().data_ptr() != staging.untyped_storage().data_ptr() and packed.data_ptr() % 16 == 0
+    assert torch.equal(packed, staging[1:])
+    assert ops.pack_tiles(shards, in_place=True)[0].data_ptr() == a.data_ptr()
+    got = ops.prepare_grouped_layer([a, b], [64, 128], [F.Q4_K, F.Q4_K])[0]
+    assert got.untyped_storage().data_ptr() != staging.untyped_storage().data_ptr()
+
+
 def test_repack_reference_in_numpy_round_trips():
     """The slab map applied in numpy: repack is a permutation plus zero rows, and inverts exactly, for
     n_out not a multiple of the tile (48, 70, 130) and nb in {1, 3, 4} (the reference's shapes)."""
