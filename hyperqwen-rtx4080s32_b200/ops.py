@@ -115,6 +115,11 @@ ROW_CLASSES = (8, 16, 32, 64)    # the row counts that end a form of the grouped
 _ROW_CLASS = [next(c for c in ROW_CLASSES if m <= c) for m in range(GEMV_MAX_ROWS + 1)]
 
 
+def _row_class(m: int) -> int:
+    """The class of any row count: those beyond the grouped kernel's own limit are answered as its largest."""
+    return _ROW_CLASS[max(0, min(int(m), GEMV_MAX_ROWS))]
+
+
 _RUN_INFO: dict[tuple[int, ...], int] = {}      # bounded by the combinations of types a model's merged layers have
 
 
@@ -272,7 +277,7 @@ def prepare_grouped_layer(tiles_list: Sequence[torch.Tensor], n_outs: Sequence[i
     n_tiles = sum(-(-int(n) // 64) for n in n_outs)
     block_bytes = int(round(sum(int(n) * F.BYTES_PER_256[int(w)] for n, w in zip(n_outs, wtypes)) / max(1, n_total)))
     sms = sm_count(packed.device)
-    splits = sorted({grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sms) for m in {_ROW_CLASS[m] for m in ms}} | {1})
+    splits = sorted({grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sms) for m in {_row_class(m) for m in ms}} | {1})
     descs = build_descs_on(packed.device, wtypes, n_outs, nb * 256, splits, wait)
     return packed, views, descs, splits, nb, block_bytes
 

@@ -93,6 +93,20 @@ def test_split_policy_on_the_decoder_shapes(gq_lib):
     assert got == {"q": 6, "qkv": 4, "gate": 2, "gate_up": 1, "down": 6, "kv": 6}
 
 
+def test_a_run_is_prepared_for_any_row_counts():
+    """The tables of exactly the splits that these row counts choose, and split 1; a count above the grouped kernel's limit is
+    answered like the largest it takes."""
+    import torch
+
+    from hyperqwen_rtx4080s32_b200 import ops
+
+    tiles = torch.zeros((80, 20, 64 * F.BYTES_PER_256[F.Q4_K]), dtype=torch.uint8)
+    for ms in ([1], [9, 16], [64], [100, 512], range(1, 130)):
+        _, _, descs, splits, nb, bb = ops.prepare_grouped_layer([tiles], [5120], [F.Q4_K], ms)
+        assert splits == sorted({ops.grouped_split_for(80, nb, m=m, block_bytes=bb) for m in ms} | {1})
+        assert [len(d) for d in descs] == [80 * s for s in splits]
+
+
 def test_fused_allreduce_buffer_size_and_argument_checks(gq_lib):
     b2 = gq_lib.gq_fused_allreduce_buffer_bytes(2, 64, 5120)
     b8 = gq_lib.gq_fused_allreduce_buffer_bytes(8, 64, 5120)
