@@ -16,6 +16,7 @@ LIB = os.path.join(_HERE, "libgq_b200.so")
 EXT = os.path.join(_HERE, "_gq_torch.so")
 SOURCES = ["gq_b200.cu"]
 EXT_SOURCE = os.path.join(CSRC, "gq_torch.cpp")
+EXT_STAMP = os.path.join(CSRC, "_generated", "gq_torch.stamp")     # what the extension was compiled against
 HEADERS = sorted(f for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))) + [os.path.join("..", "..", "include", "gq_b200.h")]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "--expt-relaxed-constexpr", "-diag-suppress", "177",
               "-shared", "-Xcompiler", "-fPIC"]
@@ -36,9 +37,28 @@ def build(force: bool = False, verbose: bool = False) -> str:
     deps = srcs + [os.path.join(CSRC, h) for h in HEADERS] + [table_h]
     if force or not os.path.exists(LIB) or os.path.getmtime(LIB) < _newest(deps):
         _build_lib(srcs, verbose)
-    if force or not os.path.exists(EXT) or os.path.getmtime(EXT) < _newest([EXT_SOURCE, os.path.join(CSRC, HEADERS[-1])]):
+    if force or not _ext_current():
         _build_ext()
     return LIB
+
+
+def _ext_tag() -> str:
+    """The binary interfaces the extension is compiled against: torch's C++ classes and this Python's."""
+    import sysconfig
+
+    import torch
+
+    return f"torch {torch.__version__} cxx11abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)} python {sysconfig.get_config_var('SOABI')}"
+
+
+def _ext_current() -> bool:
+    if not os.path.exists(EXT) or os.path.getmtime(EXT) < _newest([EXT_SOURCE, os.path.join(CSRC, HEADERS[-1])]):
+        return False
+    try:
+        with open(EXT_STAMP) as f:
+            return f.read() == _ext_tag()
+    except OSError:
+        return False
 
 
 def _build_lib(srcs, verbose: bool) -> None:
@@ -61,6 +81,8 @@ def _build_ext() -> None:
     cmd += [EXT_SOURCE, "-o", EXT, "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10",
             "-L" + _HERE, "-lgq_b200", "-Wl,-rpath,$ORIGIN"]
     subprocess.check_call(cmd, cwd=CSRC)
+    with open(EXT_STAMP, "w") as f:
+        f.write(_ext_tag())
 
 
 if __name__ == "__main__":

@@ -30,6 +30,21 @@ def test_linear_method_matches_vllm_linear_method_base():
     assert isinstance(cfg.get_quant_method(torch.nn.Linear(4, 4)), GGUFLinearMethod)
 
 
+def test_the_extension_is_rebuilt_for_another_torch_or_python(tmp_path, monkeypatch):
+    from hyperqwen_rtx4080s32_b200 import build
+
+    ext, stamp = tmp_path / "_gq_torch.so", tmp_path / "stamp"
+    monkeypatch.setattr(build, "EXT", str(ext))
+    monkeypatch.setattr(build, "EXT_STAMP", str(stamp))
+    assert not build._ext_current()
+    ext.touch()
+    assert not build._ext_current()                     # built, but against what?
+    stamp.write_text(build._ext_tag())
+    assert build._ext_current()
+    monkeypatch.setattr(torch, "__version__", "1.0.0")
+    assert not build._ext_current()
+
+
 def test_token_embedding_stays_raw_and_lm_head_is_tiled_by_class_name():
     """gguf-tiles-all-types.patch:80-89: isinstance(VocabParallelEmbedding) and not isinstance(ParallelLMHead)."""
     class VocabParallelEmbedding(torch.nn.Module):
