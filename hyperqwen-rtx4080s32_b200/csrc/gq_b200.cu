@@ -7,7 +7,6 @@
 #include <atomic>
 #include <mutex>
 #include <unordered_map>
-#include <vector>
 #include "../../include/gq_b200.h"
 #include "gq_decode.cuh"
 #include "gq_decode8.cuh"
@@ -1389,38 +1388,44 @@ __host__ __device__ inline void desc_row(const DescShard &s, int64_t nb, int spl
     r[6] = part;
     r[7] = 0;
 }
-// the shards of a run back to back, checked against what a row's 32-bit fields can hold; returns the number of rows
-static int64_t desc_shards(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split, DescShard *out) {
-    if (n_shards <= 0 || !types || !n_outs) return GQ_ERR_ARG;
-    if (K <= 0 || K % GQ_QK) return GQ_ERR_SHAPE;
-    const int64_t nb = K / GQ_QK;
-    if (split < 1 || split > nb) return GQ_ERR_ARG;
+// The shards of a run back to back, one after the other, checked against what a row's 32-bit fields can hold.
+struct DescWalk {
     int64_t base16 = 0, col0 = 0, rows = 0;
-    for (int i = 0; i < n_shards; ++i) {
-        const int B = gq_type_bytes(types[i]);
+    int next(int type, int64_t n_out, int64_t nb, int split, DescShard *out) {
+        const int B = gq_type_bytes(type);
         if (!B) return GQ_ERR_TYPE;
-        if (n_outs[i] < 0) return GQ_ERR_SHAPE;
-        const int64_t n_tiles = (n_outs[i] + 63) / 64;
+        if (n_out < 0) return GQ_ERR_SHAPE;
+        const int64_t n_tiles = (n_out + 63) / 64;
         // the largest values are those of the shard's last tile; an empty shard writes none
         if (n_tiles && (base16 + (n_tiles - 1) * nb * 4 * B > 0x7fffffff || col0 + (n_tiles - 1) * 64 > 0x7fffffff)) return GQ_ERR_LIMIT;
-        if (n_tiles) out[i] = {types[i], (int)n_tiles, (int)n_outs[i], (int)col0, (int)base16};
-        else out[i] = {types[i], 0, 0, 0, 0};
+        if (n_tiles) *out = {type, (int)n_tiles, (int)n_out, (int)col0, (int)base16};
+        else *out = {type, 0, 0, 0, 0};
         base16 += n_tiles * nb * 4 * B;
-        col0 += n_outs[i];
+        col0 += n_out;
         rows += n_tiles * split;
+        return GQ_OK;
     }
-    return rows;
+};
+static int desc_args(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split) {
+    if (n_shards <= 0 || !types || !n_outs) return GQ_ERR_ARG;
+    if (K <= 0 || K % GQ_QK) return GQ_ERR_SHAPE;
+    return split < 1 || split > K / GQ_QK ? GQ_ERR_ARG : GQ_OK;
 }
 
 extern "C" int64_t gq_build_descs(int n_shards, const int32_t *types, const int64_t *n_outs, int64_t K, int split, int32_t *desc_host) {
-    if (n_shards <= 0 || !desc_host) return GQ_ERR_ARG;
-    std::vector<DescShard> sh((size_t)n_shards);
-    const int64_t rows = desc_shards(n_shards, types, n_outs, K, split, sh.data());
-    if (rows < 0) return rows;
-    for (const DescShard &s : sh)
+    if (!desc_host) return GQ_ERR_ARG;
+    if (int rc = desc_args(n_shards, types, n_outs, K, split)) return rc;
+    DescShard s;
+    DescWalk check;         // nothing is written for a run that is refused
+    for (int i = 0; i < n_shards; ++i)
+        if (int rc = check.next(types[i], n_outs[i], K / GQ_QK, split, &s)) return rc;
+    DescWalk walk;
+    for (int i = 0; i < n_shards; ++i) {
+        walk.next(types[i], n_outs[i], K / GQ_QK, split, &s);
         for (int t = 0; t < s.n_tiles; ++t)
             for (int p = 0; p < split; ++p, desc_host += GQ_DESC_WORDS) desc_row(s, K / GQ_QK, split, t, p, desc_host);
-    return rows;
+    }
+    return walk.rows;
 }
 
 struct DescShards {
@@ -1452,8 +1457,11 @@ extern "C" int64_t gq_build_descs_device(int n_shards, const int32_t *types, con
     if (!desc_dev || ((uintptr_t)desc_dev & 15) || n_splits <= 0 || !splits) return GQ_ERR_ARG;
     DescShards sh;
     DescSplits sp;
-    const int64_t tiles = desc_shards(n_shards, types, n_outs, K, 1, sh.s);
-    if (tiles < 0) return tiles;
+    if (int rc = desc_args(n_shards, types, n_outs, K, 1)) return rc;
+    DescWalk walk;
+    for (int i = 0; i < n_shards; ++i)
+        if (int rc = walk.next(types[i], n_outs[i], K / GQ_QK, 1, sh.s + i)) return rc;
+    const int64_t tiles = walk.rows;
     int64_t rows = 0;
     for (int i = 0; i < n_splits; ++i) {
         if (splits[i] < 1 || splits[i] > K / GQ_QK) return GQ_ERR_ARG;

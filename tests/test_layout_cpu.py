@@ -129,6 +129,7 @@ def test_build_descs_rejects_bad_arguments(gq_lib):
     assert gq_lib.gq_build_descs(1, (ctypes.c_int32 * 1)(99), n, 768, 1, buf) == -1
     assert gq_lib.gq_build_descs(1, (ctypes.c_int32 * 1)(12), n, 700, 1, buf) == -2
     assert gq_lib.gq_build_descs(1, (ctypes.c_int32 * 1)(12), n, 768, 4, buf) == -3     # split > nb
+    assert gq_lib.gq_build_descs(2 ** 31 - 1, None, None, 768, 1, buf) == -3        # refused, whatever room that many shards would take
     assert gq_lib.gq_workspace_bytes(8, 700, 64, 1) == -2
     assert gq_lib.gq_workspace_bytes(8, 768, 64, 2) > gq_lib.gq_workspace_bytes(8, 768, 64, 1) > 0
 
