@@ -2015,10 +2015,15 @@ static int launch_prefill(PrefillParams &p, const PrefillPlan &pl, int maxb, cud
     attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
-    cfg.gridDim = dim3((unsigned)(pl.split * SETS), (unsigned)(prefill_ctas(p.n_desc, pl) / SETS), (unsigned)pl.tiles); cfg.blockDim = dim3(32 * (8 * SETS + 3));
-    cfg.dynamicSmemBytes = (size_t)total; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = na;
-    GQ_CUDA(cudaLaunchKernelEx(&cfg, gemm_prefill_kernel<SETS, WIDE>, p));
-    GQ_LAUNCHED();
+    cfg.blockDim = dim3(32 * (8 * SETS + 3)); cfg.dynamicSmemBytes = (size_t)total; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = na;
+    // a grid has room for 65,535 units (8.4 or 16.8 million output columns): a run of more takes several launches
+    const int64_t n_desc = p.n_desc, step = (int64_t)65535 * 2 * SETS;
+    for (int64_t d = 0; d < n_desc; d += step, p.desc += step * GQ_DESC_WORDS) {
+        p.n_desc = (int)(n_desc - d < step ? n_desc - d : step);
+        cfg.gridDim = dim3((unsigned)(pl.split * SETS), (unsigned)(prefill_ctas(p.n_desc, pl) / SETS), (unsigned)pl.tiles);
+        GQ_CUDA(cudaLaunchKernelEx(&cfg, gemm_prefill_kernel<SETS, WIDE>, p));
+        GQ_LAUNCHED();
+    }
     return GQ_OK;
 }
 
@@ -2037,7 +2042,6 @@ extern "C" int gq_gemm_prefill(const void *x_dev, int64_t M, int64_t K, int64_t 
     int *status; float *ex; uint8_t *xp;
     const int64_t need = pf_ws_layout(K, pl, workspace_dev, &status, &ex, &xp);
     if (workspace_bytes < need) return GQ_ERR_WORKSPACE;
-    if (prefill_ctas(n_desc, pl) / pl.sets > 65535) return GQ_ERR_LIMIT;
     if (int rc = ensure_tables()) return rc;
     PrefillParams p = {};
     p.packed = (const uint8_t *)packed_dev; p.desc = desc_dev; p.n_desc = (int)n_desc; p.xp = xp; p.ex = ex;

@@ -12,6 +12,20 @@ pytestmark = pytest.mark.gpu
 TOL = 6e-3      # bf16 output rounding (2^-8 of the value) plus the fp16 rounding of the weights
 
 
+def test_a_run_of_more_columns_than_a_grid_has_units():
+    """131,080 tiles, 65,540 pairs of them: more than one launch takes.  Every row of the table names the same tile."""
+    k, n, m, t = 256, 131080, 33, F.Q4_K
+    raw = synth.random_blocks(64, k, t, seed=8)
+    tiles = ops.repack_tiles(raw.cuda(), 64, t)
+    table = np.repeat(ops.build_descs([t], [64], k, 1), n, axis=0)
+    table[:, 2] = 64 * np.arange(n)
+    x = synth.activations(m, k, device="cuda")
+    y = ops.prefill_gemm(x, tiles.reshape(-1), torch.from_numpy(table).cuda(), 64 * n, wtypes=[t]).view(m, n, 64)
+    assert oracle.rel_err(y[:, 0].float().cpu().numpy(), oracle.matmul_f64(x.float().cpu().numpy(), raw.numpy(), t)) < TOL
+    assert bool((y == y[:, :1]).all())
+    assert ops.device_status() == 0
+
+
 @pytest.mark.parametrize("m", [33, 48, 49, 127, 128, 129, 144, 255, 256, 257, 513, 520])
 @pytest.mark.parametrize("parts,k", [([(64, F.Q4_K), (64, F.Q8_0), (70, F.IQ3_S)], 512), ([(129, F.IQ1_M), (33, F.Q2_K)], 2048), ([(200, F.Q6_K)], 4352)])
 def test_tiles_splits_and_ragged_outputs(m, parts, k):
