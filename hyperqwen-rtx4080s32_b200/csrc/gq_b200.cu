@@ -1982,6 +1982,14 @@ static int64_t pf_ws_layout(int64_t K, const PrefillPlan &pl, void *base, int **
     return off;
 }
 
+extern "C" int gq_prefill_plan(int64_t M, int64_t K, int64_t n_desc, int sm_count, int32_t *plan) {
+    if (M <= 0 || K <= 0 || K % GQ_QK || n_desc <= 0) return GQ_ERR_SHAPE;
+    if (!plan) return GQ_ERR_ARG;
+    const PrefillPlan p = prefill_plan(n_desc, M, K / GQ_QK, sm_count);
+    plan[0] = p.N; plan[1] = p.tiles; plan[2] = p.split; plan[3] = p.sets; plan[4] = p.wide;
+    return GQ_OK;
+}
+
 extern "C" int64_t gq_prefill_workspace_bytes(int64_t M, int64_t K, int64_t n_total, int64_t n_desc) {
     if (M < 0 || K <= 0 || K % GQ_QK || n_total < 0 || n_desc < 0) return GQ_ERR_SHAPE;
     if (M == 0) return 256;

@@ -120,6 +120,13 @@ def _row_class(m: int) -> int:
     return _ROW_CLASS[max(0, min(int(m), GEMV_MAX_ROWS))]
 
 
+def prefill_plan(m: int, k: int, n_tiles: int, sms: int | None = None) -> dict[str, int]:
+    """How the large-batch path cuts a call of m rows (gq_prefill_plan)."""
+    out = np.zeros(5, dtype=np.int32)
+    check(lib().gq_prefill_plan(int(m), int(k), int(n_tiles), int(sms or sm_count()), out.ctypes.data_as(ctypes.c_void_p)), "gq_prefill_plan")
+    return dict(zip(("rows", "tiles", "split", "sets", "wide"), out.tolist()))
+
+
 _RUN_INFO: dict[tuple[int, ...], int] = {}      # bounded by the combinations of types a model's merged layers have
 
 

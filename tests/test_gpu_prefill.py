@@ -1,5 +1,6 @@
-"""The tcgen05 path where its cuts end: batch tiles of 16-row steps up to 128 (two CTAs per SM) and 256, several balanced
-tiles, K split over a cluster, runs with an odd number of tiles and outputs whose rows are not four-byte aligned."""
+"""The tcgen05 path where its cuts end, in each of its shapes (named by the plan that the library states): batch tiles in
+16-row steps up to 128 (two CTAs per SM), up to 256 and up to 384 (CTA pairs), several balanced tiles, K split over a cluster,
+last pairs with one, two or three of their four tiles, and outputs whose rows are not four-byte aligned."""
 import numpy as np
 import pytest
 import torch
@@ -42,4 +43,38 @@ def test_tiles_splits_and_ragged_outputs(m, parts, k):
         wide = torch.full((m, n + 6 + pad), float("nan"), dtype=torch.bfloat16, device="cuda")
         ops.prefill_gemm(x, packed, d1, n, out=wide[:, 3:3 + n], wtypes=types)
         assert torch.equal(wide[:, 3:3 + n], y) and bool(torch.isnan(wide[:, :3]).all()) and bool(torch.isnan(wide[:, 3 + n:]).all())
+    assert ops.device_status() == 0
+
+
+# (tiles of 64 rows, k-blocks, batch rows) -> (batch rows of a tile, batch tiles, parts of K, sets, wide) on 148 SMs
+PLANS = [((33, 16, 257), (288, 1, 4, 2, 1)), ((34, 16, 300), (320, 1, 4, 2, 1)), ((35, 16, 300), (320, 1, 4, 2, 1)), ((37, 16, 257), (288, 1, 4, 2, 1)),
+         ((45, 16, 384), (384, 1, 4, 2, 1)), ((74, 16, 383), (384, 1, 3, 2, 1)), ((97, 17, 350), (352, 1, 2, 2, 1)), ((33, 16, 520), (288, 2, 3, 2, 1)),
+         ((149, 4, 300), (320, 1, 1, 2, 1)), ((147, 5, 641), (352, 2, 1, 2, 1)),
+         ((35, 16, 256), (256, 1, 4, 2, 0)), ((33, 16, 385), (208, 2, 3, 2, 0)), ((75, 9, 385), (208, 2, 1, 2, 0)),
+         ((35, 16, 128), (128, 1, 4, 1, 0)), ((35, 34, 40), (48, 1, 7, 1, 0)), ((149, 5, 100), (112, 1, 1, 1, 0))]
+
+
+@pytest.mark.parametrize("size,plan", PLANS)
+def test_every_shape_with_ragged_pairs_and_mixed_types(size, plan):
+    """A run of four types, three with a codebook table beside the rings, whose tiles share CTAs and pairs: the plan is the
+    one named, and the outputs agree with the oracle in a sample of columns from every tile."""
+    tiles, nb, m = size
+    if ops.sm_count() == 148:
+        assert tuple(ops.prefill_plan(m, 256 * nb, tiles).values()) == plan
+    k, types = 256 * nb, [F.Q8_0, F.IQ1_M, F.IQ3_S, F.IQ2_S]
+    n_outs = [64 * 5, 64 * 7 - 3, 64 * 9 - 61, 64 * (tiles - 21) - 1]
+    raws = [synth.random_blocks(n, k, t, seed=500 + tiles + i, device="cuda") for i, (n, t) in enumerate(zip(n_outs, types))]
+    packed, _, descs, splits, _, _ = ops.prepare_grouped_layer([ops.repack_tiles(r, n, t) for r, n, t in zip(raws, n_outs, types)], n_outs, types)
+    d1, n = descs[splits.index(1)], sum(n_outs)
+    x = synth.activations(m, k, device="cuda")
+    y = ops.prefill_gemm(x, packed, d1, n, wtypes=types)
+    xf, at = x.float().cpu().numpy(), 0
+    for raw, rows, t in zip(raws, n_outs, types):
+        pick = np.unique(np.concatenate([np.arange(0, rows, 61), np.arange(63, rows, 64), [rows - 1]]))
+        ref = oracle.matmul_f64(xf, raw[torch.from_numpy(pick).cuda()].cpu().numpy(), t)
+        assert oracle.rel_err(y[:, torch.from_numpy(at + pick).cuda()].float().cpu().numpy(), ref) < TOL, F.TYPE_NAMES[t]
+        at += rows
+    wide = torch.full((m, n + 7), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.prefill_gemm(x, packed, d1, n, out=wide[:, 3:3 + n], wtypes=types)
+    assert torch.equal(wide[:, 3:3 + n], y) and bool(torch.isnan(wide[:, :3]).all()) and bool(torch.isnan(wide[:, 3 + n:]).all())
     assert ops.device_status() == 0
