@@ -249,7 +249,7 @@ class GGUFLinearMethod:
                                               [layer.gguf_tiles_types[sid] for sid in order])
         # the layer may be called from any stream next: what was queued here is done first
         for device in {group[0].device for group in layer.gguf_groups.values()}:
-            torch.cuda.current_stream(device).synchronize()
+            ops.finish_stream(device)
 
     def check_status(self, device=None) -> None:
         """Raise if any kernel of the path has reported a bounded wait that ran out on the device since the last

@@ -183,6 +183,11 @@ def test_a_loaded_run_is_complete_when_the_load_returns():
     torch.cuda._sleep(200_000_000)
     _layer([(64, F.Q4_K), (64, F.Q6_K), (64, F.IQ3_S)], 512)
     assert torch.cuda.current_stream().query()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):       # part of a graph: complete when the graph is
+        _, _, descs, splits, _, _ = ops.prepare_grouped_layer([tiles], [64], [F.Q4_K])
+    graph.replay()
+    assert torch.equal(descs[0].cpu(), torch.from_numpy(ops.build_descs([F.Q4_K], [64], 512, splits[0])))
 
 
 @pytest.mark.parametrize("writer", ["gq_build_descs_device", "gq_repack"])
