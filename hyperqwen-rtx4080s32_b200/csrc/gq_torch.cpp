@@ -14,6 +14,7 @@
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <pybind11/pybind11.h>
@@ -205,6 +206,13 @@ at::Tensor dequantize(const at::Tensor &tiles, int64_t n_out, int64_t k, int64_t
     status.check();
     return out;
 }
+// waits for the caller's stream on the tensor's device; one that is being captured has nothing to wait for
+void finish(const at::Tensor &t) {
+    py::gil_scoped_release unlocked;
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)t.get_device());
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)
+        c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)t.get_device()).synchronize();
+}
 void build_descs(const std::vector<int32_t> &types, const std::vector<int64_t> &n_outs, int64_t k, const std::vector<int32_t> &splits, const at::Tensor &out) {
     Status status;
     {
@@ -247,6 +255,7 @@ PYBIND11_MODULE(_gq_torch, m) {
     m.def("repack", &repack);
     m.def("dequantize", &dequantize);
     m.def("build_descs", &build_descs);
+    m.def("finish", &finish);
     m.def("dequantize_rows", [](py::handle raw, int64_t type, py::handle ids, bool bf16) {
         return py::reinterpret_steal<py::object>(dequantize_rows(raw, type, ids, bf16));
     });

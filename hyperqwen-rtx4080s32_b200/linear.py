@@ -248,8 +248,8 @@ class GGUFLinearMethod:
             layer.gguf_native = ops.NativeRun(layer.gguf_groups[order[0]], [layer.gguf_tiles_rows[sid] for sid in order],
                                               [layer.gguf_tiles_types[sid] for sid in order])
         # the layer may be called from any stream next: what was queued here is done first
-        for device in {group[0].device for group in layer.gguf_groups.values()}:
-            ops.finish_stream(device)
+        for packed in {group[0].device: group[0] for group in layer.gguf_groups.values()}.values():
+            ops.native().finish(packed)
 
     def check_status(self, device=None) -> None:
         """Raise if any kernel of the path has reported a bounded wait that ran out on the device since the last

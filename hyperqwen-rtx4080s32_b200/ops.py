@@ -84,13 +84,6 @@ def build_descs(wtypes: Sequence[int], n_outs: Sequence[int], k: int, split: int
     return out
 
 
-def finish_stream(device) -> None:
-    """Wait for the caller's stream on `device`; a stream that is being captured has nothing to wait for."""
-    with torch.cuda.device(device):
-        if not torch.cuda.is_current_stream_capturing():
-            torch.cuda.current_stream().synchronize()
-
-
 def build_descs_on(device, wtypes: Sequence[int], n_outs: Sequence[int], k: int, splits: Sequence[int], wait: bool = True) -> list[torch.Tensor]:
     """The descriptor tables of several splits on a device.  They hold addresses, so the caller's stream has finished with them
     (and with all that was queued before, such as the repack of the weights they describe) when this returns: a layer may be
@@ -102,7 +95,7 @@ def build_descs_on(device, wtypes: Sequence[int], n_outs: Sequence[int], k: int,
     buf = torch.empty((tiles * sum(splits), DESC_WORDS), dtype=torch.int32, device=device)
     native().build_descs([int(t) for t in wtypes], [int(n) for n in n_outs], int(k), [int(s) for s in splits], buf)
     if wait:
-        finish_stream(buf.device)
+        native().finish(buf)
     return list(buf.split([tiles * s for s in splits]))
 
 
