@@ -240,7 +240,7 @@ def test_rejects_bad_arguments_on_the_host(gq_lib):
     with pytest.raises(GqError):
         ops.repack_tiles(raw.cpu(), n_out, t)
     x = torch.zeros((1, k), dtype=torch.bfloat16, device=dev())
-    ws = torch.empty(256, dtype=torch.uint8, device=dev())
+    ws = torch.zeros(256, dtype=torch.uint8, device=dev())
     with pytest.raises(GqError, match="workspace"):
         ops.grouped_gemm(x, tiles.reshape(-1), d, 1, [t], n_out, workspace=ws)
     assert gq_lib.gq_read_status(ws.data_ptr(), 256, 0) >= 0
