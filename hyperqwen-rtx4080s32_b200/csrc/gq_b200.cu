@@ -1167,7 +1167,7 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
     }
     if (p.ar.world > 0 && (p.split == 1 || p.cluster)) {
         // tensor parallel, row-parallel layer: this rank's partial output does not go to y but, as bf16, through
-        // the warp's scratch to every rank; y receives the sum over ranks (fused_allreduce_tile)
+        // the warp's scratch to every rank; y receives the sum over ranks (fused_allreduce_block)
         __nv_bfloat16 *blk = reinterpret_cast<__nv_bfloat16 *>(reinterpret_cast<uint8_t *>(red) + warp * MT * 512);
 #pragma unroll
         for (int nt = 0; nt < MT; ++nt)
@@ -1751,7 +1751,7 @@ extern "C" int gq_gemv_grouped_static(const void *x_dev, int64_t M, int64_t K, i
 
 // ---- the same call fused with the all-reduce of a row-parallel layer ---------------------------------------
 // Every rank multiplies its K shard; the kernel's epilogue exchanges the bf16 partial outputs through peer memory
-// and leaves the sum over ranks in y on every rank (fused_allreduce_tile).  Same arithmetic as the grouped call
+// and leaves the sum over ranks in y on every rank (fused_allreduce_block).  Same arithmetic as the grouped call
 // followed by gq_allreduce_push, without the second launch and its latency.
 static int64_t fused_ar_units(int64_t max_n_total) { return (max_n_total / 64 + 64) * GQ_CONSUMER_WARPS; }
 static int64_t fused_ar_header(int64_t max_n_total) { return (4 * fused_ar_units(max_n_total) + 4095) & ~(int64_t)4095; }

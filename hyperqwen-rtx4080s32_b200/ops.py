@@ -23,7 +23,7 @@ from ._lib import DESC_WORDS, MAX_GEMV_ROWS, GqError, check, lib, native
 TILE_TYPES = F.SUPPORTED_TYPES   # every supported type is held tile-major (the reference: GLUON_TILE_TYPES)
 GEMV_MAX_ROWS = MAX_GEMV_ROWS    # the grouped kernel's own limit (the C ABI accepts up to 64 rows)
 MAX_DEVICE_SHARDS = MAX_DEVICE_SPLITS = 8     # GQ_MAX_DEVICE_SHARDS, GQ_MAX_DEVICE_SPLITS
-DECODE_MAX_ROWS = 32             # row-count dispatch threshold: above it the tcgen05 kernel takes over
+DECODE_MAX_ROWS = 32             # above it the tcgen05 kernel takes over; see mul_mat_tiles_grouped for why the line lies there
 
 def _stream_ptr(t: torch.Tensor) -> int:
     return torch.cuda.current_stream(t.device).cuda_stream
@@ -487,17 +487,20 @@ def mul_mat_tiles_grouped(x: torch.Tensor, packed: torch.Tensor, descs: list[tor
     """A layer's run of shards in one call: x bf16 [M, K] -> [M, sum(n_outs)] (reference:
     gluon_mul_mat_tiles_grouped, gguf-plugin/gluon/interface.py:141-188).  The row-count dispatch lives
     here, inside the op: up to 32 rows one grouped launch at the split of the table for that row count; above, the
-    tcgen05 dequant-GEMM (weights dequantised into shared memory once per 64, 128 or 256 batch rows)."""
+    tcgen05 dequant-GEMM (weights dequantised into tensor memory once per tile of up to 128, 256 or 384 batch rows)."""
     m = int(x.shape[0])
     n_total = sum(int(n) for n in n_outs)
     out = torch.empty((m, n_total), dtype=x.dtype, device=x.device)
     if m == 0:
         return out
     n_tiles = sum(-(-int(n) // 64) for n in n_outs)
-    # up to 32 rows the grouped kernel streams the weights once per 8 (integer form, to 16 rows) or 32 (fp16 form) rows;
-    # from 33 rows the tcgen05 kernel (64-row variant, two CTAs per SM, split-K on narrow layers) dequantises each weight
-    # once for all rows and is faster on every layer of the stack (gate_up at 64 rows: 79 us against 116 us for two
-    # 32-row launches of the grouped kernel; down: 58 against 84)
+    # up to 32 rows the grouped kernel streams the weights once for the batch; from 33 rows that would be twice, and the tcgen05
+    # kernel dequantises each weight once for all rows.  Whole calls in microseconds, grouped / tcgen05, at 16, 24 and 32 rows:
+    # 2 x 17408 x 5120 Q4_K 35.1 / 40.6, 46.3 / 41.3, 57.1 / 41.5; IQ3_S 43.3 / 55.5, 63.3 / 56.5, 70.9 / 56.6; 5120 x 17408 Q4_K
+    # 22.8 / 28.1, 29.2 / 29.3, 35.2 / 29.3; 5120 x 4352 IQ3_S 11.8 / 16.9, 15.1 / 17.2, 16.4 / 17.2.  Between 17 and 32 rows the
+    # tcgen05 kernel is thus the faster one on the wide layers.  The line stays at 32 for the precision: the grouped kernel
+    # multiplies exact weights, the other rounds them to fp16 (error beyond the output's rounding 4e-7 against 9e-5 of the
+    # result's norm)
     if m <= DECODE_MAX_ROWS:
         s = grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sm_count(x.device))
         if s not in desc_splits:
