@@ -193,7 +193,7 @@ def dequantize_tiles(tiles: torch.Tensor, n_out: int, k: int, wtype: int, dtype=
 
 
 def repack_shards(raws: Sequence[torch.Tensor], wtypes: Sequence[int]) -> list[torch.Tensor]:
-    """repack_tiles of each shard, the shards' tiles back to back in one buffer: pack_tiles then has nothing to copy."""
+    """repack_tiles of each shard, the shards' tiles back to back in one buffer: pack_tiles(in_place=True) then has nothing to copy."""
     for raw in raws:
         _need_cuda(raw, "raw")
     if len(raws) == 1 or any(r.device != raws[0].device for r in raws):
