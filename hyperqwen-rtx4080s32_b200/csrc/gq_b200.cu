@@ -10,6 +10,7 @@
 #include "../../include/gq_b200.h"
 #include "gq_decode.cuh"
 #include "gq_decode8.cuh"
+#include "gq_scale16.cuh"
 #include <type_traits>
 #include "_generated/gq_tables.h"
 
@@ -114,167 +115,62 @@ static std::atomic<unsigned long long> g_peer_wait_ns{GQ_WAIT_LIMIT_NS};
 #include "gq_load.cuh"
 #include "gq_prefill.cuh"
 
-// ---------------------------------------------------------------------------------------------------
-// activation preparation: bf16 row -> fp16 row scaled by a power of two (so any bf16 magnitude fits fp16
-// exactly), the row's inverse scale, and per 16-weight run the fp32 sum split into fp16 hi + lo (the B operand
-// of the minimum-term MMA).  One CTA per batch row.  Plays the role of the reference's quantize_activations_256
-// (gguf-plugin/gluon/tiles_grouped.py:110-139) without quantising: activations keep all their bf16 bits.
-// ---------------------------------------------------------------------------------------------------
 struct Workspace {
     int *status;
-    float *ex;        // [M]
-    uint8_t *xt;      // [nb][M][GQ_XROW_BYTES]: per k-block, per batch row: 256 fp16 | pad | 16 run sums hi | 16 lo
+    uint8_t *xt;      // [nb] tiles of the prepared activations of one k-block (gq_x_tile_bytes)
     float *partials;  // [S][M][n_total]
 };
 
-// one batch row of one k-block in the staged activation tile: 256 fp16 activations (512 B), 32 B of padding
-// (row stride 608 B = 96 mod 128, so the rows an MMA reads together sit in distinct banks), then the sixteen
-// 16-weight run sums as fp16 hi parts (32 B) and lo parts (32 B)
-#define GQ_XROW_BYTES 608
-#define GQ_XROW_SX 544
-
 __host__ __device__ inline int64_t align256(int64_t v) { return (v + 255) & ~(int64_t)255; }
 
-// The same row in the integer form used for 1..16 batch rows: per k-block and batch row the activations as 16-bit
+// One batch row of one k-block of the staged activation tile, in the form that the kernel multiplies: 512 bytes of activations, then the
+// sixteen 16-weight run sums as fp16 hi and lo parts (64 bytes).  576 = 64 mod 128, so the two rows a quarter-warp reads with one 16-byte
+// load each sit in different banks.  After the rows of a k-block come their scales (fp32, one per batch row, padded to a multiple of 16
+// bytes): what the products have to be multiplied by.
+//
+// fp16 form (above GQ_GEMV8_MAX_ROWS rows): x * 2^e as fp16, e chosen per row and k-block so that the largest magnitude lands in
+// [512, 1024).  16-byte unit 4*P + t holds, of run pair (2P, 2P + 1), the quads 4t..4t+3: one load serves two MMAs.  The sums: unit t
+// holds the hi parts of runs 4t..4t+3, then their lo parts.
+//
+// Integer form (up to GQ_GEMV8_MAX_ROWS rows): the activations as 16-bit
 // fixed point (x * 2^e, e chosen per row and k-block so that the largest magnitude lands in [2^14, 2^15)), split into
 // two signed bytes, x = 256 hi - lo (with the minus sign they hold -32895 .. 32640, both signs of 255 * 2^7, the largest 8-bit
 // significand at that scale; 256 hi + lo ends at 32639): a plane of high bytes (256 B) and one of low bytes (256 B), then the sixteen 16-weight run sums
 // (times 2^-6) as fp16 hi parts (32 B) and lo parts (32 B).  Inside a plane the bytes are ordered for the lane that
 // reads them: 16-byte unit 4*i + t holds, for runs 4i..4i+3, the quad 4t..4t+3 with bytes in the order (0,2,1,3).
-// 576 = 64 mod 128, so the two rows a quarter-warp reads with one 16-byte load each sit in different banks.
-// After the rows of a k-block come their scales 2^-e (fp32, one per batch row, padded to a multiple of 16 bytes).
 #define GQ_PRE_NONE 0
 #define GQ_PRE_SILU_MUL 1
 #define GQ_PRE_ADD_RMSNORM 2
-#define GQ_X8_ROW 576
-#define GQ_X8_SUMS 512
+#define GQ_X_ROW 576
+#define GQ_X_SUMS 512
 #ifndef GQ_GEMV8_MAX_ROWS
 #define GQ_GEMV8_MAX_ROWS 16      // up to here the integer form runs; above it the fp16 form
 #endif
 
-__host__ __device__ inline int gq_x8_tile_bytes(int M) { return M * GQ_X8_ROW + ((4 * M + 15) & ~15); }
+__host__ __device__ inline int gq_x_tile_bytes(int M) { return M * GQ_X_ROW + ((4 * M + 15) & ~15); }
+
+// prepared activations of one k-block: batches above GQ_WIDE_ROWS are multiplied that many rows at a time, each part with tiles of its own
+#define GQ_WIDE_ROWS 32
+static int64_t gq_x_bytes(int64_t M) { return M <= GQ_WIDE_ROWS ? gq_x_tile_bytes((int)M) : gq_x_tile_bytes(GQ_WIDE_ROWS) + gq_x_bytes(M - GQ_WIDE_ROWS); }
 
 static int64_t ws_layout(int64_t M, int64_t K, int64_t n_total, int split, void *base, Workspace *ws) {
     int64_t off = 256;
-    const int64_t o_ex = off; off = align256(off + M * 4);
-    const int64_t xt_bytes = M <= GQ_GEMV8_MAX_ROWS ? (K / GQ_QK) * gq_x8_tile_bytes((int)M) : (K / GQ_QK) * M * GQ_XROW_BYTES;
-    const int64_t o_xt = off; off = align256(off + xt_bytes);
+    const int64_t o_xt = off; off = align256(off + (K / GQ_QK) * gq_x_bytes(M));
     const int64_t o_p = off; if (split > 1) off = align256(off + (int64_t)split * M * n_total * 4);
     if (ws && base) {
         uint8_t *b = (uint8_t *)base;
-        ws->status = (int *)b; ws->ex = (float *)(b + o_ex); ws->xt = b + o_xt; ws->partials = (float *)(b + o_p);
+        ws->status = (int *)b; ws->xt = b + o_xt; ws->partials = (float *)(b + o_p);
     }
     return off;
 }
 
-#define GQ_PREP_THREADS 512
-#define GQ_PREP_VECS 5      // 16-byte loads a thread keeps in registers: rows up to 512 * 5 * 8 = 20480 activations are read once
-
-// eight activations (half a 16-weight run) -> fp16 at `scale`, stored into the staged tile; the run's fp32 sum is
-// completed with the neighbouring lane, which holds the other half
-__device__ __forceinline__ void prep_store8(const uint4 &v, int64_t vec, float scale, int M, int m, uint8_t *__restrict__ xt) {
-    const __nv_bfloat162 *b = reinterpret_cast<const __nv_bfloat162 *>(&v);
-    uint4 o;
-    __half2 *oh = reinterpret_cast<__half2 *>(&o);
-    float sum = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float2 f = __bfloat1622float2(b[j]);
-        oh[j] = __floats2half2_rn(f.x * scale, f.y * scale);
-        sum += __low2float(oh[j]) + __high2float(oh[j]);
-    }
-    const int64_t k = vec * 8;                       // first activation of this vector
-    const int kb = (int)(k >> 8), rr = (int)((k >> 4) & 15);
-    uint8_t *row = xt + ((int64_t)kb * M + m) * GQ_XROW_BYTES;
-    *reinterpret_cast<uint4 *>(row + (k & 255) * 2) = o;
-    // the two halves of a run sit in lanes 2i and 2i+1: the same order of additions as one pass over the run
-    const float other = __shfl_xor_sync(0xffffffffu, sum, 1);
-    if (!(vec & 1)) {
-        const float tot = sum + other;
-        const __half hi = __float2half_rn(tot);
-        const __half lo = __float2half_rn(tot - __half2float(hi));
-        __half *so = reinterpret_cast<__half *>(row + GQ_XROW_SX);
-        so[rr] = hi;
-        so[16 + rr] = lo;
-    }
-}
-
-__global__ void __launch_bounds__(GQ_PREP_THREADS) prep_x_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int K, int M,
-                                                                 float *__restrict__ ex, uint8_t *__restrict__ xt, int *status) {
-    __shared__ float red[GQ_PREP_THREADS / 32];
-    __shared__ float s_scale;
-    const int m = blockIdx.x;
-    pdl_trigger();    // the grouped kernel behind this one may start fetching weights
-    pdl_wait();       // whatever ran before (possibly still reading this workspace) has finished
-    if (m == 0 && threadIdx.x == 0) *status = 0;
-    const __nv_bfloat16 *xr = x + (int64_t)m * ldx;
-    const int nvec = K >> 3;
-    const bool vec_ok = ((reinterpret_cast<uintptr_t>(xr) & 15) == 0);      // 16-byte loads need an aligned row
-    uint4 v[GQ_PREP_VECS];
-    float amax = 0.0f;
-    if (vec_ok) {
-#pragma unroll
-        for (int i = 0; i < GQ_PREP_VECS; ++i) {
-            const int idx = threadIdx.x + i * GQ_PREP_THREADS;
-            v[i] = idx < nvec ? __ldg(reinterpret_cast<const uint4 *>(xr) + idx) : make_uint4(0u, 0u, 0u, 0u);
-        }
-#pragma unroll
-        for (int i = 0; i < GQ_PREP_VECS; ++i) amax = fmaxf(amax, amax8(v[i]));
-        for (int idx = threadIdx.x + GQ_PREP_VECS * GQ_PREP_THREADS; idx < nvec; idx += GQ_PREP_THREADS)
-            amax = fmaxf(amax, amax8(__ldg(reinterpret_cast<const uint4 *>(xr) + idx)));
-    } else {
-        for (int idx = threadIdx.x; idx < nvec; idx += GQ_PREP_THREADS) {
-            uint4 t;
-            uint32_t *tw = reinterpret_cast<uint32_t *>(&t);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) tw[j] = *reinterpret_cast<const uint32_t *>(xr + 8 * idx + 2 * j);
-            amax = fmaxf(amax, amax8(t));
-        }
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float a = red[0];
-        for (int i = 1; i < GQ_PREP_THREADS / 32; ++i) a = fmaxf(a, red[i]);
-        // scale = 2^(9 - e), amax * scale in [512, 1024); identity for a zero, tiny or non-finite row
-        int e = 9;
-        if (a > 0.0f && a < 3.0e38f) { e = (int)((__float_as_uint(a) >> 23) & 0xFF) - 127; if (e < -100) e = -100; }
-        s_scale = __uint_as_float((uint32_t)(127 + 9 - e) << 23);
-        ex[m] = __uint_as_float((uint32_t)(127 - 9 + e) << 23);
-    }
-    __syncthreads();
-    const float scale = s_scale;
-    // nvec is a multiple of 32 (K of 256), so whole warps run every iteration and the lane-pair exchange is safe
-    if (vec_ok) {
-#pragma unroll
-        for (int i = 0; i < GQ_PREP_VECS; ++i) {
-            const int idx = threadIdx.x + i * GQ_PREP_THREADS;
-            if (idx < nvec) prep_store8(v[i], idx, scale, M, m, xt);
-        }
-        for (int idx = threadIdx.x + GQ_PREP_VECS * GQ_PREP_THREADS; idx < nvec; idx += GQ_PREP_THREADS)
-            prep_store8(__ldg(reinterpret_cast<const uint4 *>(xr) + idx), idx, scale, M, m, xt);
-    } else {
-        for (int idx = threadIdx.x; idx < nvec; idx += GQ_PREP_THREADS) {
-            uint4 t;
-            uint32_t *tw = reinterpret_cast<uint32_t *>(&t);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) tw[j] = *reinterpret_cast<const uint32_t *>(xr + 8 * idx + 2 * j);
-            prep_store8(t, idx, scale, M, m, xt);
-        }
-    }
-}
-
-
 // ---------------------------------------------------------------------------------------------------
-// activation preparation, integer form (1..16 batch rows): one warp per (batch row, k-block).  The 256 activations
-// become 16-bit fixed point at a power-of-two scale of their own (exact for every value within 2^-7 of the block's
-// largest magnitude, rounded to 2^-16 of it below), stored as the two byte planes, the run sums and the scale
-// described at GQ_X8_ROW.  Plays the role of the reference's quantize_activations_256
+// activation preparation: one warp per (batch row, k-block).  The 256 activations become 16-bit fixed point (integer form: exact for every
+// value within 2^-7 of the block's largest magnitude, rounded to 2^-16 of it below) or fp16 (fp16 form: exact within 2^-26 of it) at a
+// power-of-two scale of their own, stored with the run sums and the scale as described at GQ_X_ROW.  Plays the role of the reference's quantize_activations_256
 // (gguf-plugin/gluon/tiles_grouped.py:110-139), which keeps 8 bits per activation; this keeps 16.
 // ---------------------------------------------------------------------------------------------------
-#define GQ_PREP8_WARPS 8
+#define GQ_PREP_WARPS 8
 
 // The op in front of a linear layer, folded into its activation preparation: what vLLM runs as a kernel of its own
 // between two linears reads its input here, on the way into the fixed-point planes, instead of writing a bf16 tensor
@@ -327,7 +223,7 @@ __device__ __forceinline__ void prep8_store(const float (&v)[8], int kb, int m, 
     int xi[8], sum = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) { xi[j] = bad ? 0 : __float2int_rn(v[j] * scale); sum += xi[j]; }
-    uint8_t *row = xt + (int64_t)kb * gq_x8_tile_bytes(M) + (int64_t)m * GQ_X8_ROW;
+    uint8_t *row = xt + (int64_t)kb * gq_x_tile_bytes(M) + (int64_t)m * GQ_X_ROW;
     // this lane holds quads 2*(lane & 1) and 2*(lane & 1) + 1 of run lane >> 1
     const int r = lane >> 1, tq = 2 * (lane & 1);
 #pragma unroll
@@ -347,22 +243,61 @@ __device__ __forceinline__ void prep8_store(const float (&v)[8], int kb, int m, 
         const float f = (float)sum * 0.015625f;          // exact: |sum| < 2^20
         const __half hi = __float2half_rn(f);
         const __half lo = __float2half_rn(f - __half2float(hi));
-        __half *so = reinterpret_cast<__half *>(row + GQ_X8_SUMS);
+        __half *so = reinterpret_cast<__half *>(row + GQ_X_SUMS);
         so[r] = hi;
         so[16 + r] = lo;
     }
-    if (lane == 0) *reinterpret_cast<float *>(xt + (int64_t)kb * gq_x8_tile_bytes(M) + (int64_t)M * GQ_X8_ROW + 4 * m) = inv;
+    if (lane == 0) *reinterpret_cast<float *>(xt + (int64_t)kb * gq_x_tile_bytes(M) + (int64_t)M * GQ_X_ROW + 4 * m) = inv;
 }
 
+// the same into the fp16 form
+__device__ __forceinline__ void prep16_store(const float (&v)[8], int kb, int m, int M, uint8_t *__restrict__ xt, int lane) {
+    float amax = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
+#pragma unroll
+    for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    // scale = 2^(9 - e) with 2^e <= amax < 2^(e+1); a zero block and one holding an infinity keep scale 1: its infinities and NaNs (which
+    // fmaxf passes over) reach the products as such
+    int e = 9;
+    if (amax > 0.0f && amax < 3.0e38f) { e = (int)((__float_as_uint(amax) >> 23) & 0xFF) - 127; if (e < -100) e = -100; }
+    const float scale = __uint_as_float((uint32_t)(127 + 9 - e) << 23);
+    uint32_t o[4];
+    float sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const __half2 h = __floats2half2_rn(v[2 * j] * scale, v[2 * j + 1] * scale);
+        o[j] = h2_as_u32(h);
+        sum += __low2float(h) + __high2float(h);
+    }
+    uint8_t *row = xt + (int64_t)kb * gq_x_tile_bytes(M) + (int64_t)m * GQ_X_ROW;
+    const int r = lane >> 1, tq = 2 * (lane & 1);            // this lane holds quads tq and tq + 1 of run r
+    uint8_t *dst = row + 64 * (r >> 1) + 16 * tq + 8 * (r & 1);
+    *reinterpret_cast<uint2 *>(dst) = make_uint2(o[0], o[1]);
+    *reinterpret_cast<uint2 *>(dst + 16) = make_uint2(o[2], o[3]);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    if (!(lane & 1)) {
+        const __half hi = __float2half_rn(sum);
+        __half *so = reinterpret_cast<__half *>(row + GQ_X_SUMS + 16 * (r >> 2) + 2 * (r & 3));
+        so[0] = hi;
+        so[4] = __float2half_rn(sum - __half2float(hi));
+    }
+    if (lane == 0) *reinterpret_cast<float *>(xt + (int64_t)kb * gq_x_tile_bytes(M) + (int64_t)M * GQ_X_ROW + 4 * m) = __uint_as_float((uint32_t)(127 - 9 + e) << 23);
+}
+template <int FORM>
+__device__ __forceinline__ void prep_store(const float (&v)[8], int kb, int m, int M, uint8_t *__restrict__ xt, int lane) {
+    if constexpr (FORM) prep8_store(v, kb, m, M, xt, lane);
+    else prep16_store(v, kb, m, M, xt, lane);
+}
 
-template <int PRE>
-__global__ void __launch_bounds__(32 * GQ_PREP8_WARPS) prep_x8_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int M, uint8_t *__restrict__ xt,
+template <int PRE, int FORM>
+__global__ void __launch_bounds__(32 * GQ_PREP_WARPS) prep_x_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int M, uint8_t *__restrict__ xt,
                                                                       int *status, const PreOp pre) {
     const int lane = threadIdx.x & 31, kb = blockIdx.x;
-    const int m = blockIdx.y * GQ_PREP8_WARPS + (threadIdx.x >> 5);
+    const int m = blockIdx.y * GQ_PREP_WARPS + (threadIdx.x >> 5);
     pdl_trigger();    // the grouped kernel behind this one may start fetching weights
     pdl_wait();       // whatever ran before (possibly still reading this workspace) has finished
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status = 0;
+    if (status && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status = 0;
     if (m >= M) return;
     const __nv_bfloat16 *xr = x + (int64_t)m * ldx + (int64_t)kb * GQ_QK + 8 * lane;
     float v[8];
@@ -373,23 +308,24 @@ __global__ void __launch_bounds__(32 * GQ_PREP8_WARPS) prep_x8_kernel(const __nv
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = bf16_round(bf16_round(v[j] / (1.0f + expf(-v[j]))) * u[j]);
     }
-    prep8_store(v, kb, m, M, xt, lane);
+    prep_store<FORM>(v, kb, m, M, xt, lane);
 }
 
 // RMSNorm (with the residual add) in front of the layer: grid (batch rows, k-blocks / 8).  Every CTA sums the squares of
 // its whole row (a few KB from L2), then each warp converts one k-block.
-__global__ void __launch_bounds__(32 * GQ_PREP8_WARPS) prep_x8_norm_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int M, uint8_t *__restrict__ xt,
+template <int FORM>
+__global__ void __launch_bounds__(32 * GQ_PREP_WARPS) prep_x_norm_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int M, uint8_t *__restrict__ xt,
                                                                            int *status, const PreOp pre) {
-    __shared__ float red[GQ_PREP8_WARPS];
+    __shared__ float red[GQ_PREP_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, m = blockIdx.x;
     pdl_trigger();
     pdl_wait();
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status = 0;
+    if (status && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status = 0;
     const __nv_bfloat16 *row = x + (int64_t)m * ldx;
     const __nv_bfloat16 *res = pre.residual ? pre.residual + (int64_t)m * pre.ld_res : nullptr;
     float ss = 0.0f;
 #pragma unroll 4
-    for (int c = threadIdx.x; c < pre.K / 8; c += 32 * GQ_PREP8_WARPS) {
+    for (int c = threadIdx.x; c < pre.K / 8; c += 32 * GQ_PREP_WARPS) {
         float a[8];
         load8(row + 8 * c, a);
         if (res) {
@@ -407,9 +343,9 @@ __global__ void __launch_bounds__(32 * GQ_PREP8_WARPS) prep_x8_norm_kernel(const
     __syncthreads();
     ss = 0.0f;
 #pragma unroll
-    for (int i = 0; i < GQ_PREP8_WARPS; ++i) ss += red[i];
+    for (int i = 0; i < GQ_PREP_WARPS; ++i) ss += red[i];
     const float rs = rsqrtf(ss / (float)pre.K + pre.eps);
-    const int kb = blockIdx.y * GQ_PREP8_WARPS + warp;
+    const int kb = blockIdx.y * GQ_PREP_WARPS + warp;
     if (kb < pre.K / GQ_QK) {
         const int64_t col = (int64_t)kb * GQ_QK + 8 * lane;
         float v[8], w[8];
@@ -434,12 +370,12 @@ __global__ void __launch_bounds__(32 * GQ_PREP8_WARPS) prep_x8_norm_kernel(const
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = bf16_round(bf16_round(v[j] * rs) * w[j]);
-        prep8_store(v, kb, m, M, xt, lane);
+        prep_store<FORM>(v, kb, m, M, xt, lane);
     }
 }
 
 // ---------------------------------------------------------------------------------------------------
-// grouped small-batch kernel.  One CTA per descriptor row (64 output columns of one shard x a k-range):
+// grouped small-batch kernel, integer form.  One CTA per descriptor row (64 output columns of one shard x a k-range):
 // a producer warp streams the tile's k-blocks (one bulk copy each) plus the matching activation rows through
 // an mbarrier ring; four consumer warps each own a 16-row slab, dequantise it in registers and run m16n8k16
 // MMAs with the weights on the M side and the batch rows on the N side (8 batch rows per MMA, MT MMAs deep).
@@ -464,7 +400,6 @@ struct GemvParams {
     const uint8_t *packed;
     const int32_t *desc;
     const uint8_t *xt;
-    const float *ex;
     __nv_bfloat16 *y;
     float *partials;
     int *status;
@@ -477,95 +412,21 @@ struct GemvParams {
     const __nv_bfloat16 *x;  // FORM 2, one row: the activations themselves, converted by the producer warp (null: xt is prepared)
     const uint8_t *pf_ptr;   // weights the caller will multiply next (or null): prefetched into L2 while this launch computes
     int64_t pf_bytes;
+    // fp16 form
+    int n_tiles;             // 64-row tiles of the run
+    int part_rows;           // batch rows of a split's image in `partials`
+    int cb_stride;           // distance of the two tiles' codebook tables (0: a run of one type, one table)
+    int ar_at;               // shared-memory offset of the fused all-reduce's scratch
     ArFused ar;
 };
 
-template <int TYPE, int MT, int P>
-struct PairStep {
-    __device__ __forceinline__ static void run(const Dec<TYPE> &dec, const uint8_t *xs, int g, int t, float (&blk)[MT][4], const float (&z)[4]) {
-        uint32_t a[2][4];
-        dec.template pair<P>(a);
-        const uint8_t *xb = xs + g * GQ_XROW_BYTES + 8 * t + 64 * P;   // run 2P at halves 32P + 4t
-        if constexpr (Dec<TYPE>::GROUP == 32) {
-            float s0, s1;
-            dec.template scale<P>(s0, s1);
-#pragma unroll
-            for (int nt = 0; nt < MT; ++nt) {
-                float tmp[4];
-                const uint2 b0 = *reinterpret_cast<const uint2 *>(xb + nt * 8 * GQ_XROW_BYTES);
-                const uint2 b1 = *reinterpret_cast<const uint2 *>(xb + nt * 8 * GQ_XROW_BYTES + 32);
-                mma16816_z(tmp, a[0], b0.x, b0.y, z);
-                mma16816(tmp, a[1], b1.x, b1.y);
-                blk[nt][0] = fmaf(s0, tmp[0], blk[nt][0]);
-                blk[nt][1] = fmaf(s0, tmp[1], blk[nt][1]);
-                blk[nt][2] = fmaf(s1, tmp[2], blk[nt][2]);
-                blk[nt][3] = fmaf(s1, tmp[3], blk[nt][3]);
-            }
-        } else {
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                float s0, s1;
-                if (u == 0) dec.template scale<2 * P>(s0, s1); else dec.template scale<2 * P + 1>(s0, s1);
-#pragma unroll
-                for (int nt = 0; nt < MT; ++nt) {
-                    float tmp[4];
-                    const uint2 b = *reinterpret_cast<const uint2 *>(xb + nt * 8 * GQ_XROW_BYTES + 32 * u);
-                    mma16816_z(tmp, a[u], b.x, b.y, z);
-                    blk[nt][0] = fmaf(s0, tmp[0], blk[nt][0]);
-                    blk[nt][1] = fmaf(s0, tmp[1], blk[nt][1]);
-                    blk[nt][2] = fmaf(s1, tmp[2], blk[nt][2]);
-                    blk[nt][3] = fmaf(s1, tmp[3], blk[nt][3]);
-                }
-            }
-        }
-        if constexpr (P < 7) PairStep<TYPE, MT, P + 1>::run(dec, xs, g, t, blk, z);
-    }
-};
-
-// one k-block of one slab: acc += d * sum_groups(scale * (W_int . x)) - sum_sets f * (A'' . run sums)
-template <int TYPE, int MT>
-__device__ __forceinline__ void slab_kblock(const uint8_t *slab, const uint8_t *xs, const DecAux &aux, int lane, float (&acc)[MT][4],
-                                            const float (&z)[4]) {
-    Dec<TYPE> dec;
-    dec.load(slab, lane, aux);
-    const int g = lane >> 2, t = lane & 3;
-    float blk[MT][4];
-#pragma unroll
-    for (int nt = 0; nt < MT; ++nt) blk[nt][0] = blk[nt][1] = blk[nt][2] = blk[nt][3] = 0.f;
-    PairStep<TYPE, MT, 0>::run(dec, xs, g, t, blk, z);
-    float d0, d1;
-    dec.kscale(d0, d1);
-#pragma unroll
-    for (int nt = 0; nt < MT; ++nt) {
-        acc[nt][0] = fmaf(d0, blk[nt][0], acc[nt][0]);
-        acc[nt][1] = fmaf(d0, blk[nt][1], acc[nt][1]);
-        acc[nt][2] = fmaf(d1, blk[nt][2], acc[nt][2]);
-        acc[nt][3] = fmaf(d1, blk[nt][3], acc[nt][3]);
-    }
-    constexpr int NC = Dec<TYPE>::NCORR;
-    if constexpr (NC > 0) {
-        uint32_t ac[NC][4];
-        float fc[NC][2];
-        dec.corr(ac, fc);
-#pragma unroll
-        for (int nt = 0; nt < MT; ++nt) {
-            const uint8_t *sb = xs + (nt * 8 + g) * GQ_XROW_BYTES + GQ_XROW_SX + 8 * t;
-            const uint2 bh = *reinterpret_cast<const uint2 *>(sb);
-            const uint2 bl = *reinterpret_cast<const uint2 *>(sb + 32);
-#pragma unroll
-            for (int j = 0; j < NC; ++j) {
-                float mm[4];
-                mma16816_z(mm, ac[j], bh.x, bh.y, z);
-                mma16816(mm, ac[j], bl.x, bl.y);
-                acc[nt][0] = fmaf(-fc[j][0], mm[0], acc[nt][0]);
-                acc[nt][1] = fmaf(-fc[j][0], mm[1], acc[nt][1]);
-                acc[nt][2] = fmaf(-fc[j][1], mm[2], acc[nt][2]);
-                acc[nt][3] = fmaf(-fc[j][1], mm[3], acc[nt][3]);
-            }
-        }
+template <int I, int N, typename F>
+__device__ __forceinline__ void static_for(F &&f) {
+    if constexpr (I < N) {
+        f(std::integral_constant<int, I>{});
+        static_for<I + 1, N>(f);
     }
 }
-
 
 // The stage ring of one CTA: per stage the weight tile of one k-block and the matching activation tile, filled by two
 // bulk copies that complete on the stage's "full" mbarrier; the four consumer warps hand a stage back through its
@@ -591,24 +452,6 @@ __device__ __forceinline__ bool ring_read_counter(const Ring &r, int lane, uint3
     return true;
 }
 
-// the consumer loop of one warp for a CTA whose shard is of TYPE: waits for each stage, processes its slab,
-// releases the stage.  Returns false if a bounded wait ran out.
-template <int TYPE, int MT>
-__device__ __forceinline__ bool consume(const Ring &r, int slab_off, const DecAux &aux, int lane, float (&acc)[MT][4], uint32_t &ar_prev) {
-    float z[4] = {0.f, 0.f, 0.f, 0.f};
-    if (!ring_read_counter(r, lane, ar_prev)) return false;
-    for (int i = 0, s = 0, round = 0; i < r.nk; ++i) {
-        if (!mbar_wait(r.full + s, round & 1)) return false;
-        const uint8_t *st = r.smem + (size_t)s * r.stage_bytes;
-        slab_kblock<TYPE, MT>(st + slab_off, st + r.wmax, aux, lane, acc, z);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(r.empty + s);
-        if (++s == r.stages) { s = 0; ++round; }
-    }
-    return true;
-}
-
-
 // ---- integer form (1..16 batch rows): mma.sync m16n8k32 / m16n8k16 on 8-bit operands ----------------------
 // D (int32, 16 x 8) = A (16 weight rows x 32 k, 8-bit) . B (32 k x 8 columns, signed 8-bit) [+ C].  AS: A is signed.
 template <bool AS>
@@ -630,15 +473,7 @@ __device__ __forceinline__ void imma16(int (&d)[4], const uint32_t (&a)[2], uint
                      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(b0), "r"(0));
 }
 
-template <int I, int N, typename F>
-__device__ __forceinline__ void static_for(F &&f) {
-    if constexpr (I < N) {
-        f(std::integral_constant<int, I>{});
-        static_for<I + 1, N>(f);
-    }
-}
-
-// one k-block of one slab in the integer form.  `xs` is the staged activation tile of the k-block (rows of GQ_X8_ROW
+// one k-block of one slab in the integer form.  `xs` is the staged activation tile of the k-block (rows of GQ_X_ROW
 // bytes, then the batch rows' scales at xs_off).  Per MMA the weights are 8-bit integers and the activations one of the
 // two byte planes (x = 256 hi - lo); int32 sums per plane are exact.  At the end of the
 // k-block:  acc += 2^-e[n] * ( d[row] * (256 sumH - sumL) - f[row] * 64 * sum_run A''[row][run] * Sx[run][n] ).
@@ -653,7 +488,7 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
     dec.load(slab, lane, aux);
     const int g = lane >> 2, t = lane & 3;
     // unit (i, t) of batch row g; + 8 nt rows, + 256 for the low plane
-    const uint8_t *xb = ST ? xs + (g & 3) * GQ_X8_ROW + 256 * (g >> 2) + 16 * t : xs + g * GQ_X8_ROW + 16 * t;
+    const uint8_t *xb = ST ? xs + (g & 3) * GQ_X_ROW + 256 * (g >> 2) + 16 * t : xs + g * GQ_X_ROW + 16 * t;
     int aH[MT][4], aL[MT][4], bH[MT][4], bL[MT][4];
     float bf[MT][4];
 #pragma unroll
@@ -665,8 +500,8 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
         uint4 xh[MT], xl[MT];
 #pragma unroll
         for (int nt = 0; nt < MT; ++nt) {
-            xh[nt] = ld16(xb + nt * 8 * GQ_X8_ROW + 64 * I);
-            if constexpr (!ST) xl[nt] = ld16(xb + nt * 8 * GQ_X8_ROW + 64 * I + 256);
+            xh[nt] = ld16(xb + nt * 8 * GQ_X_ROW + 64 * I);
+            if constexpr (!ST) xl[nt] = ld16(xb + nt * 8 * GQ_X_ROW + 64 * I + 256);
         }
         if constexpr (D::SCHEME == GQ_S16) {
             static_for<0, 4>([&](auto r_) {
@@ -762,10 +597,10 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
         if constexpr (D::NCORR > 0) {
             float mm[4];
             if constexpr (ST) {
-                const uint2 b = *reinterpret_cast<const uint2 *>(xs + (g & 3) * GQ_X8_ROW + GQ_X8_SUMS + 32 * (g >> 2) + 8 * t);
+                const uint2 b = *reinterpret_cast<const uint2 *>(xs + (g & 3) * GQ_X_ROW + GQ_X_SUMS + 32 * (g >> 2) + 8 * t);
                 mma16816_z(mm, ac, b.x, b.y, z);
             } else {
-                const uint8_t *sb = xs + (nt * 8 + g) * GQ_X8_ROW + GQ_X8_SUMS + 8 * t;
+                const uint8_t *sb = xs + (nt * 8 + g) * GQ_X_ROW + GQ_X_SUMS + 8 * t;
                 const uint2 bh = *reinterpret_cast<const uint2 *>(sb);
                 const uint2 bl = *reinterpret_cast<const uint2 *>(sb + 32);
                 mma16816_z(mm, ac, bh.x, bh.y, z);
@@ -783,6 +618,8 @@ __device__ __forceinline__ void slab_kblock8(const uint8_t *slab, const uint8_t 
 }
 
 
+// the consumer loop of one warp for a CTA whose shard is of TYPE: waits for each stage, processes its slab,
+// releases the stage.  Returns false if a bounded wait ran out.
 template <int TYPE, int MT, bool ST>
 __device__ __forceinline__ bool consume8(const Ring &r, int xs_off, int slab_off, const DecAux8 &aux, int lane, float (&acc)[MT][4], uint32_t &ar_prev) {
     if (!ring_read_counter(r, lane, ar_prev)) return false;
@@ -880,22 +717,23 @@ __device__ __noinline__ void fused_allreduce_block(const GemvParams &p, const ui
     }
 }
 
+// The integer form of the grouped kernel (1..GQ_GEMV8_MAX_ROWS rows; above: gemv_wide_kernel).
 // MINB = CTAs per SM the compiler must leave room for (0: its own choice).  For the M <= 8 form 4 gives it 96
 // registers, which it turns into more loads and MMAs in flight per warp: measured 14 % faster than the 72-register
 // build when a CTA walks ten or more k-blocks, a little slower on launches of many short CTAs, 2 % faster on the
 // mixed stack.  (Compiling both and choosing per call was slower than either alone: alternating between two large
-// kernels costs more in instruction-cache misses at every launch than the better fit gains.)  The 17..24- and 25..32-row
-// forms are about 10 % faster with room for two CTAs (168 registers) than with the compiler's own 144; the 16-row
-// form was best left alone.
+// kernels costs more in instruction-cache misses at every launch than the better fit gains.)
 //
-// FORM 0: fp16 form (activations as fp16, weights decoded to fp16 pairs, m16n8k16 f16 MMAs), used from 17 batch rows.
-// FORM 1: integer form (activations as two byte planes, weights decoded to 8-bit quads, m16n8k32 / m16n8k16 integer
-// MMAs), used for 1..16 batch rows: about half the instructions per weight.
+// FORM 1: activations as two byte planes, weights decoded to 8-bit quads, m16n8k32 / m16n8k16 integer MMAs: about half the
+// instructions per weight of the fp16 form.  (At 9..16 rows the fp16 form is faster where a run is scaled per 16 weights, slower elsewhere:
+// 2 x 17,408 x 5,120 at 16 rows, integer / fp16, IQ3_S + Q2_K 41.9 / 37.3 us, Q3_K + IQ3_S 39.8 / 41.7, IQ4_XS 41 / 47; 7,168 x 5,120
+// 13.3 / 15.6.)
 // FORM 2: the integer form with both planes in one MMA, used for 1..4 batch rows.
 // ONLY: 0 compiles the decoders of all types (the branch is per CTA); a GGML type id compiles that type alone,
 // for launches whose shards all share it (a smaller kernel; most launches of a real model are such).
+// FORM 0 stands for the fp16 form's stage here.
 template <int MT, int FORM>
-__host__ __device__ constexpr int gq_stage_xbytes() { return FORM == 2 ? 4 * GQ_X8_ROW + 16 : FORM ? 8 * MT * GQ_X8_ROW + 32 * MT : 8 * MT * GQ_XROW_BYTES; }
+__host__ __device__ constexpr int gq_stage_xbytes() { return FORM == 2 ? 4 * GQ_X_ROW + 16 : 8 * MT * GQ_X_ROW + 32 * MT; }
 
 template <int MT, int MINB, int FORM, int ONLY>
 __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_grouped_kernel(const __grid_constant__ GemvParams p) {
@@ -907,7 +745,7 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)stages * stage_bytes);
     uint64_t *empty = full + stages;
     uint64_t *parts = empty + stages;          // push-form split-K: per consumer warp, the other splits' sums have landed
-    uint2 *grid_s = reinterpret_cast<uint2 *>(parts + GQ_CONSUMER_WARPS);
+    uint32_t *grid_s = reinterpret_cast<uint32_t *>(parts + GQ_CONSUMER_WARPS);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int32_t *d = p.desc + (int64_t)blockIdx.x * GQ_DESC_WORDS;
@@ -921,7 +759,7 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
     // a tile whose type contradicts the call's run_info (not the single type it named, or a codebook type it did not
     // announce, which has no table space): report and leave (every CTA of a cluster works on the same tile, so a cluster
     // leaves as one)
-    if ((ONLY != 0 && d[1] != ONLY) || (gq_cb_kind(type) >= 0 && gq_cb_bytes(gq_cb_kind(type), FORM) > p.cb_bytes)) {
+    if ((ONLY != 0 && d[1] != ONLY) || (gq_cb_kind(type) >= 0 && gq_cb_bytes(gq_cb_kind(type)) > p.cb_bytes)) {
         if (threadIdx.x == 0) { pdl_wait(); report_status(p.status, GQ_DEV_BAD_SHAPE); }      // after the preparation kernel has cleared the word
         return;
     }
@@ -941,14 +779,12 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
     // the codebook table of this CTA's type, at the start of the table region: filled by the consumer warps while the
     // producer's first copies are already on their way, closed by a barrier among the consumers only
     if (p.cb_bytes && warp < GQ_CONSUMER_WARPS) {
-        uint32_t *g32 = reinterpret_cast<uint32_t *>(grid_s);
+        uint32_t *g32 = grid_s;
         if ((ONLY == 0 || ONLY == GQ_IQ3_S) && type == GQ_IQ3_S) {
-            if constexpr (FORM) { for (int i = threadIdx.x; i < 512; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq3s_grid[i]); }
-            else { for (int i = threadIdx.x; i < 512; i += 32 * GQ_CONSUMER_WARPS) grid_s[i] = iq3s_grid_entry(c_iq3s_grid[i]); }
+            for (int i = threadIdx.x; i < 512; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq3s_grid[i]);
         }
         if ((ONLY == 0 || ONLY == GQ_IQ3_XXS) && type == GQ_IQ3_XXS) {
-            if constexpr (FORM) { for (int i = threadIdx.x; i < 256; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq3xxs_grid[i]); }
-            else { for (int i = threadIdx.x; i < 256; i += 32 * GQ_CONSUMER_WARPS) grid_s[i] = iq3s_grid_entry(c_iq3xxs_grid[i]); }
+            for (int i = threadIdx.x; i < 256; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq3xxs_grid[i]);
         }
         if ((ONLY == 0 || ONLY == GQ_IQ2_XXS) && type == GQ_IQ2_XXS) {
             for (int i = threadIdx.x; i < 512; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq2xxs_grid[i]);
@@ -973,7 +809,7 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
 
     if (FORM == 2 && warp == GQ_CONSUMER_WARPS && p.x) {
         // ---- producer of a small launch for one row: the whole warp.  It copies the weight tiles like the one below, and
-        // converts the activations of each k-block straight into the stage (what prep_x8_kernel would have left in the workspace),
+        // converts the activations of each k-block straight into the stage (what prep_x_kernel would have left in the workspace),
         // one k-block requested ahead.  Every CTA of a k-range repeats that, 0.7 us per k-block; for it the preparation kernel falls
         // away: 2 us of host time (1024 x 5120 Q4_K, called one by one: 8.2 -> 6.4 us) and a kernel boundary on the GPU ----
         const uint8_t *src = p.packed + off + (int64_t)kb0 * tile_bytes;
@@ -1012,7 +848,7 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
         // kernel behind this one is allowed to start launching when this CTA has two k-blocks left. ----
         if (lane == 0) {
             const uint8_t *src = p.packed + off + (int64_t)kb0 * tile_bytes;
-            const uint32_t abytes = FORM ? (uint32_t)gq_x8_tile_bytes(M) : (uint32_t)M * GQ_XROW_BYTES;
+            const uint32_t abytes = (uint32_t)gq_x_tile_bytes(M);
             const uint8_t *xsrc = p.xt + (int64_t)kb0 * abytes;
             const int pre = nk < stages ? nk : stages;
             for (int i = 0; i < pre; ++i) {
@@ -1057,7 +893,7 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
     bool ok = true;
     uint32_t ar_prev = 0;
     const int slab_off = warp * 16 * B;
-    // the IQ4 codebook in four registers: signed bytes for the integer form, + 128 for the fp16 form
+    // the IQ4 codebook in four registers, as signed bytes
     Iq4Table iq4;
     {
         uint32_t tb[4];
@@ -1065,38 +901,25 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
         for (int j = 0; j < 4; ++j) {
             tb[j] = 0;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) tb[j] |= (uint32_t)(uint8_t)(c_iq4_kvalues[4 * j + i] + (FORM ? 0 : 128)) << (8 * i);
+            for (int i = 0; i < 4; ++i) tb[j] |= (uint32_t)(uint8_t)c_iq4_kvalues[4 * j + i] << (8 * i);
         }
         iq4 = {tb[0], tb[1], tb[2], tb[3]};
     }
-    if constexpr (FORM) {
-        DecAux8 aux;
-        aux.grid = reinterpret_cast<const uint32_t *>(grid_s);
-        aux.iq4 = iq4;
-        const int xs_off = M * GQ_X8_ROW;
+    const int xs_off = M * GQ_X_ROW;
+    DecAux8 aux;
+    aux.grid = grid_s;
+    aux.iq4 = iq4;
 #define GQ_CONSUME(T) case T: ok = consume8<T, MT, FORM == 2>(ring, xs_off, slab_off, aux, lane, acc, ar_prev); break;
-        if constexpr (ONLY != 0) {
-            ok = consume8<(ONLY ? ONLY : GQ_Q4_K), MT, FORM == 2>(ring, xs_off, slab_off, aux, lane, acc, ar_prev);
-        } else {
-            switch (type) {
-                GQ_CONSUME(GQ_Q4_0) GQ_CONSUME(GQ_Q5_0) GQ_CONSUME(GQ_Q8_0) GQ_CONSUME(GQ_Q2_K) GQ_CONSUME(GQ_Q3_K) GQ_CONSUME(GQ_Q4_K)
-                GQ_CONSUME(GQ_Q5_K) GQ_CONSUME(GQ_Q6_K) GQ_CONSUME(GQ_IQ4_NL) GQ_CONSUME(GQ_IQ3_S) GQ_CONSUME(GQ_IQ4_XS) GQ_CONSUME(GQ_IQ3_XXS)
-                GQ_CONSUME(GQ_IQ2_XXS) GQ_CONSUME(GQ_IQ2_XS) GQ_CONSUME(GQ_IQ2_S) GQ_CONSUME(GQ_IQ1_M)
-            }
-        }
-#undef GQ_CONSUME
+    if constexpr (ONLY != 0) {
+        ok = consume8<(ONLY ? ONLY : GQ_Q4_K), MT, FORM == 2>(ring, xs_off, slab_off, aux, lane, acc, ar_prev);
     } else {
-        DecAux aux;
-        aux.grid = grid_s;
-        aux.iq4 = iq4;
-#define GQ_CONSUME(T) case T: ok = consume<T, MT>(ring, slab_off, aux, lane, acc, ar_prev); break;
         switch (type) {
             GQ_CONSUME(GQ_Q4_0) GQ_CONSUME(GQ_Q5_0) GQ_CONSUME(GQ_Q8_0) GQ_CONSUME(GQ_Q2_K) GQ_CONSUME(GQ_Q3_K) GQ_CONSUME(GQ_Q4_K)
             GQ_CONSUME(GQ_Q5_K) GQ_CONSUME(GQ_Q6_K) GQ_CONSUME(GQ_IQ4_NL) GQ_CONSUME(GQ_IQ3_S) GQ_CONSUME(GQ_IQ4_XS) GQ_CONSUME(GQ_IQ3_XXS)
-                GQ_CONSUME(GQ_IQ2_XXS) GQ_CONSUME(GQ_IQ2_XS) GQ_CONSUME(GQ_IQ2_S) GQ_CONSUME(GQ_IQ1_M)
+            GQ_CONSUME(GQ_IQ2_XXS) GQ_CONSUME(GQ_IQ2_XS) GQ_CONSUME(GQ_IQ2_S) GQ_CONSUME(GQ_IQ1_M)
         }
-#undef GQ_CONSUME
     }
+#undef GQ_CONSUME
     if constexpr (FORM == 2) {      // columns n and n + 4: lanes t and t + 2
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[0][j] += __shfl_xor_sync(0xffffffffu, acc[0][j], 2);
@@ -1175,7 +998,7 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
             for (int j = 0; j < 4; ++j) {
                 const int rl = g + 8 * (j >> 1), n = nt * 8 + 2 * t + (j & 1);
                 const bool valid = ok && warp * 16 + rl < nvalid && n < p.M;
-                blk[n * 16 + rl] = __float2bfloat16_rn(valid ? (FORM ? acc[nt][j] : acc[nt][j] * p.ex[n]) : 0.0f);
+                blk[n * 16 + rl] = __float2bfloat16_rn(valid ? acc[nt][j] : 0.0f);
             }
         __syncwarp();
         const int ncols = nvalid - warp * 16 < 16 ? nvalid - warp * 16 : 16;
@@ -1193,12 +1016,13 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
             const int r = warp * 16 + g + 8 * (j >> 1);      // row inside the 64-row tile
             const int n = nt * 8 + 2 * t + (j & 1);          // batch row
             if (ok && r < nvalid && n < p.M) {
-                const float v = FORM ? acc[nt][j] : acc[nt][j] * p.ex[n];    // the integer form scales per k-block
-                if (p.split == 1 || p.cluster) p.y[(int64_t)n * p.ldy + col0 + r] = __float2bfloat16_rn(v);
-                else p.partials[((int64_t)split_idx * p.M + n) * p.n_total + col0 + r] = v;
+                if (p.split == 1 || p.cluster) p.y[(int64_t)n * p.ldy + col0 + r] = __float2bfloat16_rn(acc[nt][j]);
+                else p.partials[((int64_t)split_idx * p.M + n) * p.n_total + col0 + r] = acc[nt][j];
             }
         }
 }
+
+#include "gq_wide.cuh"
 
 // Y = sum over splits of the fp32 partials, rounded once to bf16 (reference: sum_partials,
 // gguf-plugin/gluon/tiles_grouped.py:142-162)
@@ -1483,19 +1307,21 @@ extern "C" int gq_split_for(int64_t n_tiles, int64_t nb, int64_t M, int avg_byte
     if (sm_count <= 0) sm_count = 148;
     // from sweeps on B200 (Q4_K / Q2_K / IQ3_S / IQ4_XS; 80- to 544-tile layers at K 5120 and 17408): the
     // largest split that (a) leaves a CTA at least three k-blocks, (b) stays inside one thread-block cluster (8), and
-    // (c) keeps the launch in one wave of the CTAs that the kernel for M rows has resident on an SM (four to 8 rows, three to 16,
-    // two above) — counting that clusters cannot use every slot: a launch of clusters of S fills at most about 1 - 0.03 (S - 1)
-    // of them before a second wave starts.  (With four for every M, 80 tiles at K 5120 ran as 480 CTAs: Q4_K 14.2 us at 16 rows
-    // and 23.8 at 27, with the splits of this rule, 4 and 3, 10.4 and 16.7.)
-    const int64_t per_sm = M <= 8 ? 4 : M <= 16 ? 3 : 2, slots = per_sm * sm_count;
-    int64_t s_max = nb / 3;
+    // (c) keeps the launch in one wave of the CTAs that the kernel for M rows has resident on an SM (four to 8 rows, three to 16;
+    // above, two of two tiles each) — counting that clusters cannot use every slot: a launch of clusters of S fills at most about
+    // 1 - 0.03 (S - 1) of them before a second wave starts.  (With four for every M, 80 tiles at K 5120 ran as 480 CTAs: Q4_K 14.2 us
+    // at 16 rows, with the split of this rule, 4, 10.4.  Above 16 rows, 27: 80 tiles as 6 / 7 parts 15.7 / 22.0 us, 112 tiles as
+    // 4 / 5 parts 20.0 / 29.2, 136 tiles as 3 / 4 parts 27.0 / 22.9, where clusters of 4 still fit at 0.92 of the slots.)
+    const bool wide = M > GQ_GEMV8_MAX_ROWS;
+    const int64_t per_sm = M <= 8 ? 4 : wide ? 2 : 3, slots = per_sm * sm_count, units = wide ? (n_tiles + 1) / 2 : n_tiles;
+    int64_t s_max = (wide ? nb + 1 : nb) / 3;       // 5120 x 4352, seventeen k-blocks, at 27 rows: 5 / 6 parts 15.4 / 13.0 us
     if (s_max > 8) s_max = 8;
     int64_t s = 1;
     for (int64_t c = 2; c <= s_max; ++c)
-        if (c * n_tiles * 100 <= slots * (100 - 3 * (c - 1))) s = c;
+        if (c * units * 100 <= slots * (wide && c == 4 ? 92 : 100 - 3 * (c - 1))) s = c;
     // 9 .. 16 rows, one CTA short of what an SM holds: two parts in a wave and a quarter are 13 - 20 % faster (272 tiles: Q4_K
     // 25.8 -> 22.4 us, IQ3_S 34.6 -> 28.0)
-    if (per_sm == 3 && s == 1 && s_max >= 2 && n_tiles * 3 < slots * 2) s = 2;
+    if (per_sm == 3 && s == 1 && s_max >= 2 && units * 3 < slots * 2) s = 2;
     if (s > nb) s = nb;
     return (int)s;
 }
@@ -1564,6 +1390,78 @@ extern "C" int gq_run_info(int n_shards, const int32_t *types) {
     return maxb | ((cb ? 1 : 0) << 16) | (single << 17) | (cb << 22);
 }
 
+// the activation preparation of `rows` batch rows (form 1: integer, 0: fp16)
+static int launch_prep(const __nv_bfloat16 *x, int64_t rows, int64_t K, int64_t ldx, uint8_t *xt, int *status, int form, const PreOp *pre, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.dynamicSmemBytes = 0; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 1;
+    cfg.gridDim = dim3((unsigned)(K / GQ_QK), (unsigned)((rows + GQ_PREP_WARPS - 1) / GQ_PREP_WARPS)); cfg.blockDim = dim3(32 * GQ_PREP_WARPS);
+    const PreOp po = pre ? *pre : PreOp{};
+    if (po.kind == GQ_PRE_ADD_RMSNORM) {
+        cfg.gridDim = dim3((unsigned)rows, (unsigned)((K / GQ_QK + GQ_PREP_WARPS - 1) / GQ_PREP_WARPS));
+        GQ_CUDA(cudaLaunchKernelEx(&cfg, form ? prep_x_norm_kernel<1> : prep_x_norm_kernel<0>, x, ldx, (int)rows, xt, status, po));
+    } else {
+        auto *kern = po.kind == GQ_PRE_SILU_MUL ? (form ? prep_x_kernel<GQ_PRE_SILU_MUL, 1> : prep_x_kernel<GQ_PRE_SILU_MUL, 0>)
+                                                : (form ? prep_x_kernel<GQ_PRE_NONE, 1> : prep_x_kernel<GQ_PRE_NONE, 0>);
+        GQ_CUDA(cudaLaunchKernelEx(&cfg, kern, x, ldx, (int)rows, xt, status, po));
+    }
+    GQ_LAUNCHED();
+    return GQ_OK;
+}
+
+// an SM has 228 KB of shared memory, of which the system keeps 1 KB per resident CTA
+static int resident_ctas(int smem, int cap) { const int n = (228 * 1024) / (smem + 1024); return n < cap ? n : cap; }
+
+// integer form: up to GQ_GEMV8_MAX_ROWS rows
+static int launch_gemv8(GemvParams &p, int run_info, int64_t n_desc, cudaStream_t st) {
+    // CTAs an SM holds by their registers, and the deepest ring of three or four stages that leaves room for them (swept on the 64-layer
+    // stack: deeper rings with fewer resident CTAs were slower)
+    const int mt = p.M <= 8 ? 1 : 2, cap = mt == 1 ? 4 : 3;
+    const int stage_bytes = p.wbytes_max + (p.M <= 4 ? gq_stage_xbytes<1, 2>() : 8 * mt * GQ_X_ROW + 32 * mt), red1 = GQ_CONSUMER_WARPS * mt * 512;
+    const auto resident = [&](int stages, int red) { return resident_ctas(stages * stage_bytes + 64 + 8 * GQ_CONSUMER_WARPS + p.cb_bytes + red, cap); };
+    // split-K in a cluster: the push form of the reduction needs a scratch slot per other split in every CTA; it is used when that
+    // costs no resident CTA at three stages
+    p.cluster_push = p.cluster && resident(3, red1 * (p.split - 1)) >= resident(3, red1) ? 1 : 0;
+    p.stages = resident(4, p.cluster_push ? red1 * (p.split - 1) : red1) >= cap ? 4 : 3;
+    if (mt == 2) return launch_gemv<2, 3, 1, 0>(p, n_desc, st);
+    return p.M <= 4 ? launch_gemv8_m8<2>(p, n_desc, st, (run_info >> 17) & 31) : launch_gemv8_m8<1>(p, n_desc, st, (run_info >> 17) & 31);
+}
+
+// fp16 form: up to GQ_WIDE_ROWS rows
+template <int MT>
+static int launch_wide_mt(GemvParams &p, int run_info, cudaStream_t st) {
+    // the deepest ring of two to four stages that costs no resident CTA
+    p.cb_stride = (run_info >> 17) & 31 ? 0 : p.cb_bytes;
+    const int stage_bytes = 2 * p.wbytes_max + gq_stage_xbytes<MT, 0>(), tables = p.cb_bytes + p.cb_stride, scratch = p.ar.world ? GQ_WIDE_WARPS * MT * 512 : 0;
+    const auto bytes = [&](int stages) { return stages * (stage_bytes + 16) + tables + scratch; };
+    p.stages = 2;
+    while (p.stages < 4 && resident_ctas(bytes(p.stages + 1), 2) >= resident_ctas(bytes(2), 2)) ++p.stages;
+    p.ar_at = p.stages * (stage_bytes + 16) + tables;
+    if (bytes(p.stages) > 232448) return GQ_ERR_LIMIT;
+    if (int rc = allow_smem<gemv_wide_kernel<MT>>(232448)) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (p.cluster) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = (unsigned)p.split; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1;
+        ++na;
+    }
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+    cfg.gridDim = dim3((unsigned)((p.n_tiles + 1) / 2 * p.split)); cfg.blockDim = dim3(32 * (GQ_WIDE_WARPS + 1)); cfg.dynamicSmemBytes = bytes(p.stages);
+    cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = na;
+    GQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_wide_kernel<MT>, p));
+    GQ_LAUNCHED();
+    return GQ_OK;
+}
+static int launch_wide(GemvParams &p, int run_info, cudaStream_t st) {
+    return p.M <= 16 ? launch_wide_mt<2>(p, run_info, st) : p.M <= 24 ? launch_wide_mt<3>(p, run_info, st) : launch_wide_mt<4>(p, run_info, st);
+}
+
 static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ldx, const void *packed_dev, const int32_t *desc_dev,
                              int64_t n_desc, int split, int run_info, void *y_dev, int64_t ldy, int64_t n_total, void *workspace_dev,
                              int64_t workspace_bytes, void *stream, int phases, const void *next_packed_dev, int64_t next_bytes,
@@ -1579,88 +1477,47 @@ static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ld
     if (int rc = ensure_tables()) return rc;
     cudaStream_t st = (cudaStream_t)stream;
 
-    const int form = M <= GQ_GEMV8_MAX_ROWS ? 1 : 0;
+    if (pre && pre->kind && M > GQ_WIDE_ROWS) return GQ_ERR_SHAPE;
+    const int maxb = run_info & 0xFFFF;
+    if ((phases & 6) && (maxb < 56 || maxb > 272 || (maxb & 1))) return GQ_ERR_ARG;
+    // split-K up to 8 reduces inside a thread-block cluster (portable cluster size); larger splits keep the fp32
+    // partials and the separate sum
+    const int cluster = (split > 1 && split <= 8 && n_desc % split == 0) ? 1 : 0;
+    if (ar && (phases & 6)) {
+        if (split > 1 && !cluster) return GQ_ERR_ARG;        // the exchange needs the whole tile sum in one CTA
+        if (n_desc / split * GQ_CONSUMER_WARPS > ar->units) return GQ_ERR_LIMIT;
+    }
+    const bool wide = M > GQ_GEMV8_MAX_ROWS;
+    if (wide && n_desc % split) return GQ_ERR_ARG;            // a CTA of the fp16 form takes two tiles' rows of one part
     // Whether the grouped kernel converts the activations itself: one row, nothing folded in front, and at most four k-blocks to a
     // CTA, up to where the conversions, one after the other, take no longer than the boundary they save (graphs of 24 layers, Q4_K:
     // 5120 x 5120, 3.3 k-blocks, 6.8 -> 6.5 us; 7168 x 5120, 5 k-blocks, 7.4 -> 8.3; a second row adds 2 us)
     const bool direct = (phases & 8) && M == 1 && !ar && !(pre && pre->kind) && (K / GQ_QK + split - 1) / split <= 4;
-    if ((phases & 1) && !direct) {
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.dynamicSmemBytes = 0; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 1;
-        if (form) {
-            cfg.gridDim = dim3((unsigned)(K / GQ_QK), (unsigned)((M + GQ_PREP8_WARPS - 1) / GQ_PREP8_WARPS)); cfg.blockDim = dim3(32 * GQ_PREP8_WARPS);
-            const PreOp po = pre ? *pre : PreOp{};
-            if (po.kind == GQ_PRE_ADD_RMSNORM) {
-                cfg.gridDim = dim3((unsigned)M, (unsigned)((K / GQ_QK + GQ_PREP8_WARPS - 1) / GQ_PREP8_WARPS));
-                GQ_CUDA(cudaLaunchKernelEx(&cfg, prep_x8_norm_kernel, (const __nv_bfloat16 *)x_dev, ldx, (int)M, ws.xt, ws.status, po));
-            } else {
-                auto *kern = po.kind == GQ_PRE_SILU_MUL ? prep_x8_kernel<GQ_PRE_SILU_MUL> : prep_x8_kernel<GQ_PRE_NONE>;
-                GQ_CUDA(cudaLaunchKernelEx(&cfg, kern, (const __nv_bfloat16 *)x_dev, ldx, (int)M, ws.xt, ws.status, po));
-            }
-        } else {
-            if (pre && pre->kind) return GQ_ERR_SHAPE;      // the folded ops exist in the integer form's preparation only
-            cfg.gridDim = dim3((unsigned)M); cfg.blockDim = dim3(GQ_PREP_THREADS);
-            GQ_CUDA(cudaLaunchKernelEx(&cfg, prep_x_kernel, (const __nv_bfloat16 *)x_dev, ldx, (int)K, (int)M, ws.ex, ws.xt, ws.status));
-        }
-        GQ_LAUNCHED();
-    }
-    if (!(phases & 6)) return GQ_OK;
 
     GemvParams p;
-    p.packed = (const uint8_t *)packed_dev; p.desc = desc_dev; p.xt = ws.xt; p.ex = ws.ex;
-    p.y = (__nv_bfloat16 *)y_dev; p.partials = ws.partials; p.status = ws.status;
-    p.M = (int)M; p.K = (int)K; p.nb = (int)(K / GQ_QK); p.split = split; p.ldy = ldy; p.n_total = n_total;
-    const int maxb = run_info & 0xFFFF;
-    if (maxb < 56 || maxb > 272 || (maxb & 1)) return GQ_ERR_ARG;
+    p.packed = (const uint8_t *)packed_dev; p.desc = desc_dev; p.status = ws.status;
+    p.K = (int)K; p.nb = (int)(K / GQ_QK); p.split = split; p.ldy = ldy; p.n_total = n_total;
     p.wbytes_max = 64 * maxb;   // every stage can hold a tile of any shard of the run
-    p.cb_bytes = gq_cb_region_max((run_info >> 22) & 63, form);
-    // split-K up to 8 reduces inside a thread-block cluster (portable cluster size); larger splits keep the fp32
-    // partials and the separate sum
-    p.cluster = (split > 1 && split <= 8 && n_desc % split == 0) ? 1 : 0;
-    p.cluster_push = 0;
+    p.cb_bytes = gq_cb_region_max((run_info >> 22) & 63);
+    p.cluster = cluster; p.cluster_push = 0;
     p.x = direct ? (const __nv_bfloat16 *)x_dev : nullptr;
-    p.pf_ptr = (next_packed_dev && next_bytes > 0 && !((uintptr_t)next_packed_dev & 15)) ? (const uint8_t *)next_packed_dev : nullptr;
-    p.pf_bytes = next_bytes;
-    if (ar) {
-        if (split > 1 && !p.cluster) return GQ_ERR_ARG;        // the exchange needs the whole tile sum in one CTA
-        if (n_desc / split * GQ_CONSUMER_WARPS > ar->units) return GQ_ERR_LIMIT;
-        p.ar = *ar;
-    } else {
-        p.ar = ArFused{};
+    p.n_tiles = (int)(n_desc / split); p.part_rows = (int)M;
+    p.ar = ar ? *ar : ArFused{};
+    // the batch rows at a time that the kernel takes: all of them, except for the fp16 form of more than GQ_WIDE_ROWS
+    for (int64_t r0 = 0; r0 < M; r0 += GQ_WIDE_ROWS) {
+        const int64_t rows = M - r0 < GQ_WIDE_ROWS ? M - r0 : GQ_WIDE_ROWS;
+        const __nv_bfloat16 *x = (const __nv_bfloat16 *)x_dev + r0 * ldx;
+        p.M = (int)rows;
+        p.xt = ws.xt + (r0 ? p.nb * gq_x_bytes(r0) : 0);
+        p.y = (__nv_bfloat16 *)y_dev + r0 * ldy; p.partials = ws.partials + r0 * n_total;
+        if ((phases & 1) && !direct)
+            if (int rc = launch_prep(x, rows, K, ldx, const_cast<uint8_t *>(p.xt), r0 ? nullptr : ws.status, wide ? 0 : 1, pre, st)) return rc;
+        if (!(phases & 2)) continue;
+        p.pf_ptr = (r0 + rows == M && next_packed_dev && next_bytes > 0 && !((uintptr_t)next_packed_dev & 15)) ? (const uint8_t *)next_packed_dev : nullptr;
+        p.pf_bytes = next_bytes;
+        if (int rc = wide ? launch_wide(p, run_info, st) : launch_gemv8(p, run_info, n_desc, st)) return rc;
     }
-    const int mt = M <= 8 ? 1 : M <= 16 ? 2 : M <= 24 ? 3 : M <= 32 ? 4 : 8;
-    {
-        // ring depth: four stages when four CTAs of them still fit an SM's shared memory, else three (swept on the
-        // 64-layer stack: deeper rings with fewer resident CTAs were slower overall)
-        const int xb = !form ? 8 * mt * GQ_XROW_BYTES : mt == 1 ? (M <= 4 ? gq_stage_xbytes<1, 2>() : gq_stage_xbytes<1, 1>()) : gq_stage_xbytes<2, 1>();
-        const int stage_bytes = p.wbytes_max + xb;
-        // (an SM has 228 KB of shared memory and the system keeps 1 KB of it per resident CTA)
-        const int fixed = 64 + 8 * GQ_CONSUMER_WARPS + p.cb_bytes + 1024, red1 = GQ_CONSUMER_WARPS * mt * 512;
-        // split-K in a cluster: the push form of the reduction needs a scratch slot per other split in every CTA; it
-        // is used when that costs no resident CTA (the ring then has three stages; its depth does not matter)
-        if (p.cluster) {
-            const int pull = (228 * 1024) / (3 * stage_bytes + fixed + red1), push = (228 * 1024) / (3 * stage_bytes + fixed + red1 * (split - 1));
-            const int cap = mt == 1 ? 4 : 8;     // resident CTAs the register budget allows anyway
-            p.cluster_push = (push > cap ? cap : push) >= (pull > cap ? cap : pull) ? 1 : 0;
-        }
-        const int red = p.cluster_push ? red1 * (split - 1) : red1;
-        p.stages = (4 * (4 * stage_bytes + fixed + red) <= 228 * 1024) ? 4 : 3;
-    }
-    int rc = GQ_OK;
-    if (phases & 2) {
-        switch (mt) {
-            case 1: rc = M <= 4 ? launch_gemv8_m8<2>(p, n_desc, st, (run_info >> 17) & 31) : launch_gemv8_m8<1>(p, n_desc, st, (run_info >> 17) & 31); break;
-            case 2: rc = launch_gemv<2, 3, 1, 0>(p, n_desc, st); break;
-            case 3: rc = launch_gemv<3, 2, 0, 0>(p, n_desc, st); break;
-            case 4: rc = launch_gemv<4, 2, 0, 0>(p, n_desc, st); break;
-            default: rc = launch_gemv<8, 0, 0, 0>(p, n_desc, st); break;
-        }
-    }
-    if (rc) return rc;
-    if (split > 1 && !p.cluster && (phases & 4)) {
+    if (split > 1 && !cluster && (phases & 4)) {
         const int64_t n = M * n_total;
         sum_partials_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ws.partials, split, M, n_total, (__nv_bfloat16 *)y_dev, ldy);
         GQ_LAUNCHED();

@@ -54,6 +54,31 @@ GQ_HD inline float s8f(uint32_t word, int byte) { return (float)(int)(int8_t)((w
 #define GQ_SIGN01 0x40008000u
 #define GQ_SIGN23 0x10002000u
 
+// The same as byte masks: the product carries bit i (0..3) of a sign nibble to the top bit of byte (0,2,1,3)[i], and prmt's replicating
+// selectors turn the top bits into byte masks; bits 4 and 5 above a nibble may be set, their products hit none of the four places.  For
+// a nibble that sits four bits up the multiplier is shifted down by four, so lanes need no shift of their own (`sign_mul`).
+#define GQ_SIGN8_MUL ((1u << 7) | (1u << 22) | (1u << 13) | (1u << 28))
+GQ_HD inline uint32_t sign_mul(int shn) { return GQ_SIGN8_MUL >> shn; }
+GQ_HD inline uint32_t sign_bytes(uint32_t nib, uint32_t mul) { return prmt(nib * mul, 0u, 0xBA98u); }
+// the odd bytes of e negated where m is set, in one instruction: -e = ~e + 1, and ~e is even (also of bytes 128 + odd: 128 - odd)
+GQ_HD inline uint32_t negate_odd_bytes(uint32_t e, uint32_t m) { return lop3<(0xF0 ^ 0xCC) | 0xAA>(e, m, 0x01010101u); }
+// byte K of w, zero-extended to 32 bits (one prmt)
+template <int K>
+GQ_HD inline int ubyte(uint32_t w) { return (int)prmt(w, 0u, 0x4440u | K); }
+
+// The lane's four signs from a stored 7-bit index (whose eighth sign is the parity of the seven): even lanes of a quad take the lower
+// nibble, odd ones the upper, whose fourth bit is the parity.  `nib` leaves it in place (four bits up for odd lanes).
+struct SignIndex {
+    uint32_t keep, par;
+    int shn;
+    GQ_HD void init(int t) {
+        shn = 4 * (t & 1);
+        keep = (t & 1) ? 0x70u : 0x0fu;
+        par = (t & 1) ? 128u : 0u;
+    }
+    GQ_HD uint32_t nib(uint32_t f) const { return popc32(f) * par + (f & keep); }
+};
+
 // the IQ4 codebook as unsigned bytes (value + 128) in four registers, filled by the kernel from the
 // generated table
 struct Iq4Table { uint32_t t0, t1, t2, t3; };
@@ -75,8 +100,8 @@ GQ_HD inline void iq4_word(uint32_t w, const Iq4Table &T, uint32_t (&lo)[2], uin
 GQ_HD inline uint32_t bytes_h2(uint32_t w, uint32_t sel) { return prmt(w, GQ_MAGICB, sel); }
 
 struct DecAux {
-    const uint2 *grid;        // shared memory: the codebook of the type being decoded — IQ3_S (512) / IQ3_XXS (256) entries
-                              // {fp16(m0,m1), fp16(m2,m3)}; IQ2_*: 8 magnitude bytes per entry, each word in quad byte order
+    const uint32_t *grid;     // shared memory: the codebook of the type being decoded, magnitudes as bytes, each word in quad byte order
+                              // (0,2,1,3) — IQ3_S (512, + 128 each) / IQ3_XXS (256) entries of one word, IQ2_* and IQ1_M of two
     Iq4Table iq4;
 };
 
@@ -643,26 +668,29 @@ struct Dec<GQ_Q3_K> {
 };
 
 
-// ---- IQ3_S ----------------------------------------------------------------------------------------
+// ---- IQ3_S: the grid in shared memory holds 128 + magnitude (odd, 1 .. 15), so that one lop3 leaves 128 +- it; fragments are
+// 1152 + weight ---------------------------------------------------------------------------------------
 template <>
 struct Dec<GQ_IQ3_S> {
     static constexpr int GROUP = 32;
     static constexpr int NCORR = 0;
     uint4 q[2];      // 16 grid-index bytes per row (byte r = run r)
-    uint4 sg[2];     // 16 sign bytes per row, pre-shifted so that the lane's nibble is the low one
+    uint4 sg[2];     // 16 sign nibbles per row (byte r: the lane's four signs of run r, four bits up for odd t)
+    uint32_t smul;
     uint2 qh[2];     // the eight qh bytes per row, pre-shifted by t
     uint32_t sce[2], sco[2], dd[2];   // scale nibbles of even / odd sub-blocks, one per byte
-    const uint2 *grid;
+    const uint32_t *grid;
     GQ_HD void load(const uint8_t *slab, int lane, const DecAux &aux) {
         grid = aux.grid;
         const int t = lane & 3;
+        const uint32_t keep = 0x0f0f0f0fu << (4 * (t & 1));
+        smul = sign_mul(4 * (t & 1));
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int row = (lane >> 2) + 8 * h;
             q[h] = ld16(slab + 512 * h + 16 * lane);
             uint4 s = ld16(slab + 1024 + 32 * row + 16 * (t >> 1));
-            const int sh = 4 * (t & 1);
-            s.x >>= sh; s.y >>= sh; s.z >>= sh; s.w >>= sh;
+            s.x &= keep; s.y &= keep; s.z &= keep; s.w &= keep;
             sg[h] = s;
             uint2 hq = ld8(slab + 1536 + 8 * row);
             hq.x >>= t; hq.y >>= t;
@@ -676,13 +704,12 @@ struct Dec<GQ_IQ3_S> {
     template <int R>
     GQ_HD void run(int h, uint32_t &a01, uint32_t &a23) const {
         constexpr int ib = R >> 1, u = R & 1;
-        const uint32_t idxb = (w4(q[h], R >> 2) >> (8 * (R & 3))) & 0xFFu;
+        // index byte and, above it, the qh byte in one prmt (one shift serves four runs)
         const uint32_t hw = (ib < 4) ? qh[h].x : qh[h].y;
-        const uint32_t idx = or_and(idxb, shl_c<8 - (8 * (ib & 3) + 4 * u)>(hw), 0x100u);
-        const uint2 e = grid[idx];
-        const uint32_t nib = (w4(sg[h], R >> 2) >> (8 * (R & 3))) & 0xFFu;
-        a01 = xor_and(e.x, nib * GQ_SIGN01, 0x80008000u);
-        a23 = xor_and(e.y, nib * GQ_SIGN23, 0x80008000u);
+        const uint32_t idx = prmt(w4(q[h], R >> 2), hw >> (4 * u), (R & 3) | ((4 | (ib & 3)) << 4)) & 0x1FFu;
+        const uint32_t e = negate_odd_bytes(grid[idx], sign_bytes((uint32_t)ubyte<(R & 3)>(w4(sg[h], R >> 2)), smul));
+        a01 = prmt(e, GQ_MAGICB, 0x5250u);
+        a23 = prmt(e, GQ_MAGICB, 0x5351u);
     }
     template <int P>
     GQ_HD void pair(uint32_t (&a)[2][4]) const {
@@ -701,9 +728,18 @@ struct Dec<GQ_IQ3_S> {
     }
     GQ_HD void kscale(float &d0, float &d1) const { d0 = f16bits(dd[0]); d1 = f16bits(dd[1]); }
     static constexpr bool HAS_MIN = false;
-    template <int R> static constexpr float offs() { return 0.0f; }
+    template <int R> static constexpr float offs() { return 1152.0f; }
 };
 
+// What a type with magnitudes and separate signs delivers per run and row half: the magnitudes as fp16 pairs of 1024 + m, and words whose
+// bits 15 and 31 are the signs of the pair (other bits are anything).  signed_pair: the exact signed value.
+struct MagSign {
+    uint32_t m01, m23, s01, s23;
+};
+GQ_HD inline MagSign mag_sign(uint32_t e, uint32_t nib, int shn) {
+    return {prmt(e, GQ_MAGICB, 0x5250u), prmt(e, GQ_MAGICB, 0x5351u), nib * (GQ_SIGN01 >> shn), nib * (GQ_SIGN23 >> shn)};
+}
+GQ_HD inline uint32_t signed_pair(uint32_t m, uint32_t s) { return xor_and(hsub2(m, h2k(1024)), s, 0x80008000u); }
 
 // ---- IQ3_XXS: d | 64 grid-index bytes | eight words of four 7-bit sign indices and a 4-bit scale ----------------
 // weight = d (2 s + 1) / 4 x magnitude x sign; the eighth sign of a group of eight is the parity of the stored seven
@@ -715,13 +751,14 @@ struct Dec<GQ_IQ3_XXS> {
     uint4 q[2];          // 16 grid-index bytes per row (byte r = run r)
     uint32_t sw[2][8];   // the sign-and-scale word of each sub-block
     uint32_t dd[2];
-    int sh0, shn;        // 7 (t >> 1): the lane's sign index inside a half sub-block; 4 (t & 1): its nibble of the mask
-    const uint2 *grid;
+    int sh;              // 7 (t >> 1): the lane's sign index of the first run of a sub-block; the second run's is 14 bits up
+    SignIndex sx;
+    const uint32_t *grid;
     GQ_HD void load(const uint8_t *slab, int lane, const DecAux &aux) {
         grid = aux.grid;
         const int t = lane & 3;
-        sh0 = 7 * (t >> 1);
-        shn = 4 * (t & 1);
+        sh = 7 * (t >> 1);
+        sx.init(t);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int row = (lane >> 2) + 8 * h;
@@ -733,14 +770,14 @@ struct Dec<GQ_IQ3_XXS> {
         }
     }
     template <int R>
+    GQ_HD MagSign mags(int h) const {
+        const uint32_t e = grid[(uint32_t)ubyte<(R & 3)>(w4(q[h], R >> 2))];
+        return mag_sign(e, sx.nib((sw[h][R >> 1] >> ((R & 1) ? sh + 14 : sh)) & 0x7Fu), sx.shn);
+    }
+    template <int R>
     GQ_HD void run(int h, uint32_t &a01, uint32_t &a23) const {
-        const uint32_t idx = (w4(q[h], R >> 2) >> (8 * (R & 3))) & 0xFFu;
-        const uint2 e = grid[idx];
-        const uint32_t f = (sw[h][R >> 1] >> (14 * (R & 1) + sh0)) & 0x7Fu;
-        const uint32_t mask = f | (popc32(f) << 7);          // bit 7: the parity (higher bits fall outside the nibble)
-        const uint32_t nib = (mask >> shn) & 0xFu;
-        a01 = xor_and(e.x, nib * GQ_SIGN01, 0x80008000u);
-        a23 = xor_and(e.y, nib * GQ_SIGN23, 0x80008000u);
+        const MagSign v = mags<R>(h);
+        a01 = signed_pair(v.m01, v.s01); a23 = signed_pair(v.m23, v.s23);
     }
     template <int P>
     GQ_HD void pair(uint32_t (&a)[2][4]) const {
@@ -765,11 +802,6 @@ struct Dec<GQ_IQ3_XXS> {
 // magnitude x sign (gguf-plugin/gluon/iq2.py:6-23).  The shared-memory grid is the integer form's (bytes in quad order
 // (0,2,1,3) per word); the bytes become fp16 through the 1024 + byte pattern. ----
 GQ_HD inline uint32_t pick_alt_bytes16(uint32_t a, uint32_t b, int tp) { return prmt(a, b, 0x6420u + 0x1111u * (uint32_t)tp); }
-// the lane's word e of a grid entry and its four sign bits -> the fp16 pairs (w0, w1), (w2, w3)
-GQ_HD inline void iq2_pairs(uint32_t e, uint32_t nib, uint32_t &a01, uint32_t &a23) {
-    a01 = xor_and(hsub2(prmt(e, GQ_MAGICB, 0x5250u), h2k(1024)), nib * GQ_SIGN01, 0x80008000u);
-    a23 = xor_and(hsub2(prmt(e, GQ_MAGICB, 0x5351u), h2k(1024)), nib * GQ_SIGN23, 0x80008000u);
-}
 GQ_HD inline float odd_scale_f32(uint32_t s) { return u32_as_f32(0x4B000001u + 2u * s) - 8388608.0f; }    // 2 s + 1
 
 template <>
@@ -779,13 +811,14 @@ struct Dec<GQ_IQ2_XXS> {
     uint32_t q[2][4];    // grid-index byte of run r in byte r & 3 of word r >> 2
     uint32_t sw[2][8];
     uint32_t dd[2];
-    int sh0, shn;
+    int sh;
+    SignIndex sx;
     const uint8_t *grid;
     GQ_HD void load(const uint8_t *slab, int lane, const DecAux &aux) {
         const int t = lane & 3, tp = t >> 1;
         grid = reinterpret_cast<const uint8_t *>(aux.grid) + 4 * (t & 1);
-        sh0 = 7 * tp;
-        shn = 4 * (t & 1);
+        sh = 7 * tp;
+        sx.init(t);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int row = (lane >> 2) + 8 * h;
@@ -799,12 +832,14 @@ struct Dec<GQ_IQ2_XXS> {
         }
     }
     template <int R>
+    GQ_HD MagSign mags(int h) const {
+        const uint32_t e = *reinterpret_cast<const uint32_t *>(grid + 8 * (uint32_t)ubyte<(R & 3)>(q[h][R >> 2]));
+        return mag_sign(e, sx.nib((sw[h][R >> 1] >> ((R & 1) ? sh + 14 : sh)) & 0x7Fu), sx.shn);
+    }
+    template <int R>
     GQ_HD void run(int h, uint32_t &a01, uint32_t &a23) const {
-        const uint32_t idx = (q[h][R >> 2] >> (8 * (R & 3))) & 0xFFu;
-        const uint32_t e = *reinterpret_cast<const uint32_t *>(grid + 8 * idx);
-        const uint32_t f = (sw[h][R >> 1] >> (14 * (R & 1) + sh0)) & 0x7Fu;
-        const uint32_t mask = f | (popc32(f) << 7);
-        iq2_pairs(e, (mask >> shn) & 0xFu, a01, a23);
+        const MagSign v = mags<R>(h);
+        a01 = signed_pair(v.m01, v.s01); a23 = signed_pair(v.m23, v.s23);
     }
     template <int P>
     GQ_HD void pair(uint32_t (&a)[2][4]) const {
@@ -828,12 +863,12 @@ struct Dec<GQ_IQ2_XS> {
     uint32_t v[2][8];    // the halfword (9-bit grid index, 7-bit sign index) of run r in half r & 1 of word r >> 1
     uint2 sc[2];         // scales[8] of the row: byte ib = nibbles of runs 2 ib, 2 ib + 1
     uint32_t dd[2];
-    int shn;
+    SignIndex sx;
     const uint8_t *grid;
     GQ_HD void load(const uint8_t *slab, int lane, const DecAux &aux) {
         const int t = lane & 3, tp = t >> 1;
         grid = reinterpret_cast<const uint8_t *>(aux.grid) + 4 * (t & 1);
-        shn = 4 * (t & 1);
+        sx.init(t);
         const uint32_t sel = 0x5410u + 0x2222u * (uint32_t)tp;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -849,12 +884,16 @@ struct Dec<GQ_IQ2_XS> {
         }
     }
     template <int R>
+    GQ_HD MagSign mags(int h) const {
+        const uint32_t w = v[h][R >> 1];
+        const uint32_t goff = (R & 1) ? (w >> 13) & 0xFF8u : (w << 3) & 0xFF8u;
+        const uint32_t e = *reinterpret_cast<const uint32_t *>(grid + goff);
+        return mag_sign(e, sx.nib((R & 1) ? w >> 25 : (w >> 9) & 0x7Fu), sx.shn);
+    }
+    template <int R>
     GQ_HD void run(int h, uint32_t &a01, uint32_t &a23) const {
-        const uint32_t hw = (v[h][R >> 1] >> (16 * (R & 1))) & 0xFFFFu;
-        const uint32_t e = *reinterpret_cast<const uint32_t *>(grid + 8 * (hw & 511u));
-        const uint32_t f = hw >> 9;
-        const uint32_t mask = f | (popc32(f) << 7);
-        iq2_pairs(e, (mask >> shn) & 0xFu, a01, a23);
+        const MagSign v = mags<R>(h);
+        a01 = signed_pair(v.m01, v.s01); a23 = signed_pair(v.m23, v.s23);
     }
     template <int P>
     GQ_HD void pair(uint32_t (&a)[2][4]) const {
@@ -903,13 +942,17 @@ struct Dec<GQ_IQ2_S> {
         }
     }
     template <int R>
-    GQ_HD void run(int h, uint32_t &a01, uint32_t &a23) const {
+    GQ_HD MagSign mags(int h) const {
         constexpr int ib = R >> 1, u = R & 1;
-        const uint32_t idxb = (q[h][R >> 2] >> (8 * (R & 3))) & 0xFFu;
         const uint32_t hw = (ib < 4) ? qh[h].x : qh[h].y;
-        const uint32_t idx = or_and(idxb, shl_c<8 - (8 * (ib & 3) + 4 * u)>(hw), 0x300u);
+        const uint32_t idx = prmt(q[h][R >> 2], hw >> (4 * u), (R & 3) | ((4 | (ib & 3)) << 4)) & 0x3FFu;
         const uint32_t e = *reinterpret_cast<const uint32_t *>(grid + 8 * idx);
-        iq2_pairs(e, (sg[h][R >> 2] >> (8 * (R & 3))) & 0xFu, a01, a23);
+        return mag_sign(e, (uint32_t)ubyte<(R & 3)>(sg[h][R >> 2]), 0);
+    }
+    template <int R>
+    GQ_HD void run(int h, uint32_t &a01, uint32_t &a23) const {
+        const MagSign v = mags<R>(h);
+        a01 = signed_pair(v.m01, v.s01); a23 = signed_pair(v.m23, v.s23);
     }
     template <int P>
     GQ_HD void pair(uint32_t (&a)[2][4]) const {
@@ -985,12 +1028,7 @@ struct Dec<GQ_IQ1_M> {
     template <int R> static constexpr float offs() { return 0.0f; }
 };
 
-// one entry of the IQ3_S / IQ3_XXS shared-memory grid: the four magnitude bytes of a grid word as two fp16 pairs
-GQ_HD inline uint2 iq3s_grid_entry(uint32_t w) {
-    uint2 e;
-    e.x = h2_as_u32(__floats2half2_rn((float)(w & 0xFF), (float)((w >> 8) & 0xFF)));
-    e.y = h2_as_u32(__floats2half2_rn((float)((w >> 16) & 0xFF), (float)(w >> 24)));
-    return e;
-}
+// one entry of the IQ3_S shared-memory grid: the four magnitude bytes + 128, in quad byte order
+GQ_HD inline uint32_t iq3s_grid_entry(uint32_t w) { return prmt(w, 0u, 0x3120u) | 0x80808080u; }
 
 }  // namespace gq

@@ -36,9 +36,7 @@ GQ_HD inline uint32_t nib0(uint32_t w) { return w & 0x0f0f0f0fu; }
 GQ_HD inline uint32_t nib1(uint32_t w) { return (w >> 4) & 0x0f0f0f0fu; }
 template <int HI>
 GQ_HD inline uint32_t nibx(uint32_t w) { return HI ? nib1(w) : nib0(w); }
-// byte K of w, zero- or sign-extended to 32 bits (one prmt)
-template <int K>
-GQ_HD inline int ubyte(uint32_t w) { return (int)prmt(w, 0u, 0x4440u | K); }
+// byte K of w, sign-extended to 32 bits (one prmt)
 template <int K>
 GQ_HD inline int sbyte(uint32_t w) { return (int)prmt(w, 0u, ((8u | K) * 0x1110u) | K); }
 // four unsigned bytes (each below 128) + 96, then the top bit flipped: the bytes of (value - 32) as int8
@@ -470,19 +468,12 @@ struct Dec8<GQ_Q3_K> {
 #define GQ_IQ3S8_SMEM_BYTES 2048
 // one entry of the int8 IQ3_S shared-memory grid: the four magnitude bytes in quad byte order (0,2,1,3)
 GQ_HD inline uint32_t iq3s_grid_entry8(uint32_t w) { return prmt(w, 0u, 0x3120u); }
-// Signs.  The product carries bit i (0..3) of a sign nibble to the top bit of byte (0,2,1,3)[i], and prmt's replicating selectors
-// turn the top bits into byte masks; bits 4 and 5 above a nibble may be set, their products hit none of the four places.  For a nibble
-// that sits four bits up the multiplier is shifted down by four, so lanes need no shift of their own (`sign_mul`).
-#define GQ_SIGN8_MUL ((1u << 7) | (1u << 22) | (1u << 13) | (1u << 28))
-GQ_HD inline uint32_t sign_mul(int shn) { return GQ_SIGN8_MUL >> shn; }
-GQ_HD inline uint32_t sign_bytes(uint32_t nib, uint32_t mul) { return prmt(nib * mul, 0u, 0xBA98u); }
+// Signs as byte masks (sign_bytes).
 // Measured at 17,408 x 5,120, 1 / 8 rows (against a spread of the four bits to 0 / 1 bytes, a multiply by 255, an exclusive or and an
 // add): IQ3_S 18.2 / 19.4 -> 17.7 / 18.7 us, IQ3_XXS 20.8 / 21.7 -> 19.4 / 20.5, IQ2_XXS 19.5 / 20.9 -> 18.3 / 19.7, IQ2_XS
 // 20.6 / 23.1 -> 19.9 / 22.1; the types are bound by their issue slots.
 // the bytes of e (each 1..127) negated where m is set: the subtraction's borrows make every byte -e
 GQ_HD inline uint32_t negate_bytes(uint32_t e, uint32_t m) { return lop3<((0xF0 & ~0xAA) | (0xCC & 0xAA)) & 0xFF>(e, 0x01010100u - e, m); }
-// the same for odd bytes, in one instruction: -e = ~e + 1, and ~e is even
-GQ_HD inline uint32_t negate_odd_bytes(uint32_t e, uint32_t m) { return lop3<(0xF0 ^ 0xCC) | 0xAA>(e, m, 0x01010101u); }
 
 // ---- IQ3_S ----------------------------------------------------------------------------------------
 template <>
@@ -543,15 +534,10 @@ struct Dec8<GQ_IQ3_S> {
 // Shared memory: the 256 grid words.  The lane's four sign bits come from the stored 7-bit index by arithmetic (the index
 // with its parity as bit 7, then the lane's nibble): a 128-entry table of them in shared memory was measured 12-14 %
 // slower — with the grid lookups the type is bound by shared-memory gathers, not by the integer pipe.
-// `f`: the lane's sign index, 7 bits; odd lanes take its upper nibble, whose fourth bit is the parity.
-struct SignIndex {
-    uint32_t keep, par, mul;
-    GQ_HD void init(int t) {
-        keep = (t & 1) ? 0x70u : 0x0fu;
-        par = (t & 1) ? 128u : 0u;
-        mul = sign_mul(4 * (t & 1));
-    }
-    GQ_HD uint32_t bytes(uint32_t f) const { return sign_bytes(popc32(f) * par + (f & keep), mul); }
+struct SignIndex8 : SignIndex {
+    uint32_t mul;
+    GQ_HD void init(int t) { SignIndex::init(t); mul = sign_mul(shn); }
+    GQ_HD uint32_t bytes(uint32_t f) const { return sign_bytes(nib(f), mul); }
 };
 
 template <>
@@ -563,7 +549,7 @@ struct Dec8<GQ_IQ3_XXS> {
     uint32_t sw[2][8];   // the sign-and-scale word of each sub-block
     uint32_t dd[2];
     int sh;              // 7 (t >> 1): the lane's sign index of the first run of a sub-block; the second run's is 14 bits up
-    SignIndex sx;
+    SignIndex8 sx;
     const uint32_t *grid;
     GQ_HD void load(const uint8_t *slab, int lane, const DecAux8 &aux) {
         grid = aux.grid;
@@ -616,7 +602,7 @@ struct Dec8<GQ_IQ2_XXS> {
     uint32_t sw[2][8];   // the sign-and-scale word of each sub-block
     uint32_t dd[2];
     int sh;
-    SignIndex sx;
+    SignIndex8 sx;
     const uint8_t *grid;            // offset by the lane's half of an entry
     GQ_HD void load(const uint8_t *slab, int lane, const DecAux8 &aux) {
         const int t = lane & 3, tp = t >> 1;
@@ -667,7 +653,7 @@ struct Dec8<GQ_IQ2_XS> {
     static constexpr int NCORR = 0;
     uint32_t v[2][8];    // the halfword (9-bit grid index, 7-bit sign index) of run r in half r & 1 of word r >> 1
     uint32_t sce[2][2], sco[2][2], dd[2];
-    SignIndex sx;
+    SignIndex8 sx;
     const uint8_t *grid;
     GQ_HD void load(const uint8_t *slab, int lane, const DecAux8 &aux) {
         const int t = lane & 3, tp = t >> 1;

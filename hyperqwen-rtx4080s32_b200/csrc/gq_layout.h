@@ -70,7 +70,7 @@ GQ_HD constexpr int gq_type_chunks(int type) {
 }
 
 // Codebook types keep a table of grid entries in shared memory while a kernel decodes them.  Kind index of a type
-// (-1: not a codebook type), and the table's bytes in the integer form (form 1: magnitudes as bytes) and in the fp16 form (form 0).
+// (-1: not a codebook type), and the table's bytes (magnitudes as bytes, one or two words per entry).
 GQ_HD constexpr int gq_cb_kind(int type) {
     switch (type) {
         case GQ_IQ3_S: return 0;
@@ -83,10 +83,10 @@ GQ_HD constexpr int gq_cb_kind(int type) {
     }
 }
 #define GQ_CB_KINDS 6
-GQ_HD constexpr int gq_cb_bytes(int kind, int form) {
+GQ_HD constexpr int gq_cb_bytes(int kind) {
     switch (kind) {
-        case 0: return form ? 2048 : 4096;     // IQ3_S: 512 entries of 4 bytes / of two fp16 pairs
-        case 1: return form ? 1024 : 2048;     // IQ3_XXS: 256 entries of 4 bytes / of two fp16 pairs
+        case 0: return 2048;                   // IQ3_S: 512 entries of 4 bytes
+        case 1: return 1024;                   // IQ3_XXS: 256 entries of 4 bytes
         case 2: return 2048;                   // IQ2_XXS: 256 entries of 8 bytes
         case 3: return 4096;                   // IQ2_XS: 512 entries of 8 bytes
         case 4: return 8192;                   // IQ2_S: 1024 entries of 8 bytes
@@ -95,17 +95,17 @@ GQ_HD constexpr int gq_cb_bytes(int kind, int form) {
     }
 }
 // a kernel whose CTAs decode one type each keeps the CTA's table at the start of a region sized for the largest
-GQ_HD inline int gq_cb_region_max(int mask, int form) {
+GQ_HD inline int gq_cb_region_max(int mask) {
     int m = 0;
     for (int k = 0; k < GQ_CB_KINDS; ++k)
-        if (((mask >> k) & 1) && gq_cb_bytes(k, form) > m) m = gq_cb_bytes(k, form);
+        if (((mask >> k) & 1) && gq_cb_bytes(k) > m) m = gq_cb_bytes(k);
     return m;
 }
-// a kernel whose CTAs may decode two types keeps the tables of all types of the run side by side (fp16 form)
+// a kernel whose CTAs may decode two types keeps the tables of all types of the run side by side
 GQ_HD inline int gq_cb_offset(int mask, int kind) {
     int o = 0;
     for (int k = 0; k < kind; ++k)
-        if ((mask >> k) & 1) o += gq_cb_bytes(k, 0);
+        if ((mask >> k) & 1) o += gq_cb_bytes(k);
     return o;
 }
 GQ_HD inline int gq_cb_region_sum(int mask) { return gq_cb_offset(mask, GQ_CB_KINDS); }

@@ -15,13 +15,12 @@ namespace gq {
 #define GQ_LOAD_THREADS 256
 #define GQ_LOAD_WARPS (GQ_LOAD_THREADS / 32)
 
-// the codebook table of TYPE in the fp16 form of its decoder (gq_cb_bytes(kind, 0) bytes of shared memory)
+// the codebook table of TYPE for the fp16 decoders of gq_decode.cuh (gq_cb_bytes(kind) bytes of shared memory)
 __device__ __forceinline__ void fill_codebook(int type, uint8_t *dst, int tid, int nthreads) {
     uint32_t *t32 = reinterpret_cast<uint32_t *>(dst);
-    uint2 *t64 = reinterpret_cast<uint2 *>(dst);
     switch (type) {
-        case GQ_IQ3_S: for (int i = tid; i < 512; i += nthreads) t64[i] = iq3s_grid_entry(c_iq3s_grid[i]); break;
-        case GQ_IQ3_XXS: for (int i = tid; i < 256; i += nthreads) t64[i] = iq3s_grid_entry(c_iq3xxs_grid[i]); break;
+        case GQ_IQ3_S: for (int i = tid; i < 512; i += nthreads) t32[i] = iq3s_grid_entry(c_iq3s_grid[i]); break;
+        case GQ_IQ3_XXS: for (int i = tid; i < 256; i += nthreads) t32[i] = prmt(c_iq3xxs_grid[i], 0u, 0x3120u); break;
         case GQ_IQ2_XXS: for (int i = tid; i < 512; i += nthreads) t32[i] = prmt(c_iq2xxs_grid[i], 0u, 0x3120u); break;
         case GQ_IQ2_XS: for (int i = tid; i < 1024; i += nthreads) t32[i] = prmt(c_iq2xs_grid[i], 0u, 0x3120u); break;
         case GQ_IQ2_S: for (int i = tid; i < 2048; i += nthreads) t32[i] = prmt(c_iq2s_grid[i], 0u, 0x3120u); break;
@@ -220,7 +219,7 @@ __device__ __forceinline__ void dequant_slab(const uint8_t *slab, const DecAux &
 template <int TYPE, bool BF16>
 __global__ void __launch_bounds__(GQ_LOAD_THREADS) dequant_kernel(const uint8_t *__restrict__ tiles, int64_t n_out, int nb, int kc, void *__restrict__ out,
                                                                   int64_t ld) {
-    constexpr int B = gq_type_bytes(TYPE), CB = gq_cb_kind(TYPE) >= 0 ? gq_cb_bytes(gq_cb_kind(TYPE), 0) : 0;
+    constexpr int B = gq_type_bytes(TYPE), CB = gq_cb_kind(TYPE) >= 0 ? gq_cb_bytes(gq_cb_kind(TYPE)) : 0;
     extern __shared__ __align__(16) uint8_t sm[];       // [codebook][the warps' output staging]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, slab = blockIdx.x;
     if constexpr (CB > 0) {
@@ -228,7 +227,7 @@ __global__ void __launch_bounds__(GQ_LOAD_THREADS) dequant_kernel(const uint8_t 
         __syncthreads();
     }
     DecAux aux;
-    aux.grid = reinterpret_cast<const uint2 *>(sm);
+    aux.grid = reinterpret_cast<const uint32_t *>(sm);
     aux.iq4 = iq4_table_biased();
     const int64_t row0 = (int64_t)slab * 16;
     const int rows = n_out - row0 < 16 ? (n_out - row0 > 0 ? (int)(n_out - row0) : 0) : 16;
@@ -243,11 +242,11 @@ __global__ void __launch_bounds__(GQ_LOAD_THREADS) dequant_kernel(const uint8_t 
 }
 
 template <int TYPE, bool BF16>
-constexpr int dequant_smem() { return (gq_cb_kind(TYPE) >= 0 ? gq_cb_bytes(gq_cb_kind(TYPE), 0) : 0) + (BF16 ? GQ_LOAD_WARPS * GQ_DEQ_STAGE : 0); }
+constexpr int dequant_smem() { return (gq_cb_kind(TYPE) >= 0 ? gq_cb_bytes(gq_cb_kind(TYPE)) : 0) + (BF16 ? GQ_LOAD_WARPS * GQ_DEQ_STAGE : 0); }
 template <int TYPE>
 constexpr int dequant_rows_smem() {
     const int img = 16 * stage_pitch(GQ_LOAD_WARPS * gq_type_bytes(TYPE)), st = GQ_LOAD_WARPS * GQ_DEQ_STAGE;
-    return (img > st ? img : st) + GQ_LOAD_WARPS * 16 * gq_type_bytes(TYPE) + (gq_cb_kind(TYPE) >= 0 ? gq_cb_bytes(gq_cb_kind(TYPE), 0) : 0);
+    return (img > st ? img : st) + GQ_LOAD_WARPS * 16 * gq_type_bytes(TYPE) + (gq_cb_kind(TYPE) >= 0 ? gq_cb_bytes(gq_cb_kind(TYPE)) : 0);
 }
 // ---- embedding lookup: rows `ids` of a raw table -> row-major weights --------------------------------------------
 // One CTA takes sixteen ids and up to eight k-blocks: the raw bytes are gathered into shared memory, permuted into slabs
@@ -284,7 +283,7 @@ __global__ void __launch_bounds__(GQ_LOAD_THREADS) dequant_rows_kernel(const uin
     __syncthreads();
     if (warp >= n_kb) return;
     DecAux aux;
-    aux.grid = reinterpret_cast<const uint2 *>(cb);
+    aux.grid = reinterpret_cast<const uint32_t *>(cb);
     aux.iq4 = iq4_table_biased();
     const bool vec = !((reinterpret_cast<uintptr_t>(out) & 15) | ((ld * (BF16 ? 2 : 4)) & 15));
     uint8_t *o = reinterpret_cast<uint8_t *>(out) + (i0 * ld + (int64_t)(kb0 + warp) * 256) * (BF16 ? 2 : 4);

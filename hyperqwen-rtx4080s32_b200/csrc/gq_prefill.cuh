@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
         if (slab < 4 ? has0 : has1) {
             DecAux aux;
             const int cb = slab < 4 ? cb0 : cb1;
-            aux.grid = reinterpret_cast<const uint2 *>(tables + (cb ? 16 * (cb - 2) : 0));
+            aux.grid = reinterpret_cast<const uint32_t *>(tables + (cb ? 16 * (cb - 2) : 0));
             aux.iq4 = iq4_table_biased();
             PfRings r;
             r.wring = wring; r.wstage_bytes = p.wstage_bytes; r.wstages = p.wstages;

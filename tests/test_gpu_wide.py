@@ -1,0 +1,61 @@
+"""The grouped kernel's fp16 form (17 to 32 rows a launch, two tiles to a CTA) where its shapes end: one to four column tiles, an odd number
+of tiles, halves of different types, a ragged last tile, fewer k-blocks than ring stages, every way a split is reduced, two launches above
+32 rows."""
+import numpy as np
+import pytest
+import torch
+
+from hyperqwen_rtx4080s32_b200 import formats as F
+from hyperqwen_rtx4080s32_b200 import ops, synth
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _beyond_rounding(y, exact, norm):
+    """What an output is off by beyond half a bf16 ulp of the exact value, over the 2-norm of its products."""
+    ulp = 2.0 ** (np.floor(np.log2(np.maximum(np.abs(exact), 1e-30))) - 7)
+    return float(np.max((np.abs(y - exact) - 0.5 * ulp) / norm))
+
+
+@pytest.mark.parametrize("t", sorted(F.SUPPORTED_TYPES))
+@pytest.mark.parametrize("m, k, splits", [(17, 256, [1]), (24, 1280, [1, 2, 5]), (25, 2048, [3, 8]), (32, 2560, [4, 9]), (33, 512, [1, 2]), (64, 768, [3])])
+def test_every_type_beside_another(t, m, k, splits):
+    """A run of five tiles, three of type t (the last one of 6 rows) and two of another: the tiles that share a CTA differ in type, and
+    the last CTA has one.  Weights and activations enter exactly, so beyond the output rounding there are the fp32 sums: at most
+    K / 256 + 17 roundings of 2^-23 (the tensor core truncates) of partial sums of a few norms, below 2^-15 of the norm here."""
+    other = F.IQ2_S if t != F.IQ2_S else F.Q8_0
+    types, n_outs = [t, other], [134, 100]
+    raws = [synth.random_blocks(n, k, w, seed=11 * w + n) for n, w in zip(n_outs, types)]
+    packed = torch.cat([ops.repack_tiles(r.cuda(), n, w).reshape(-1) for r, n, w in zip(raws, n_outs, types)])
+    x = synth.activations(m, k, device="cuda")
+    xd = x.double().cpu().numpy()
+    w = np.concatenate([oracle.dequantize(r.numpy(), wt) for r, wt in zip(raws, types)]).astype(np.float64)
+    exact, norm = xd @ w.T, np.sqrt((xd ** 2) @ (w ** 2).T)
+    first = None
+    for s in splits:
+        d = torch.from_numpy(ops.build_descs(types, n_outs, k, s)).cuda()
+        y = ops.grouped_gemm(x, packed, d, s, types, sum(n_outs))
+        assert _beyond_rounding(y.double().cpu().numpy(), exact, norm) < 2.0 ** -15, (F.TYPE_NAMES[t], m, k, s)
+        assert torch.equal(y, ops.grouped_gemm(x, packed, d, s, types, sum(n_outs)))          # a fixed order of the additions
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("m", [17, 40])
+def test_scales_zeros_and_non_finite_rows(m):
+    """Per-block activation scales: rows of very different magnitude, a block of zeros, and a row with an infinity, which must not reach
+    the other rows."""
+    n, k, t = 192, 1024, F.Q5_K
+    raw = synth.random_blocks(n, k, t, seed=3)
+    packed = ops.repack_tiles(raw.cuda(), n, t).reshape(-1)
+    d = torch.from_numpy(ops.build_descs([t], [n], k, 2)).cuda()
+    x = synth.activations(m, k, device="cuda")
+    x[1] *= 2.0 ** 60
+    x[2] *= 2.0 ** -60
+    x[3, 256:512] = 0
+    x[4, :256] *= 2.0 ** 20
+    x[m - 1, 700] = float("inf")
+    y = ops.grouped_gemm(x, packed, d, 2, [t], n).double().cpu().numpy()
+    assert not np.isfinite(y[m - 1]).any()
+    xd, w = x.double().cpu().numpy()[:m - 1], oracle.dequantize(raw.numpy(), t).astype(np.float64)
+    assert _beyond_rounding(y[:m - 1], xd @ w.T, np.sqrt((xd ** 2) @ (w ** 2).T)) < 2.0 ** -15
