@@ -1865,7 +1865,7 @@ static int launch_prefill(PrefillParams &p, const PrefillPlan &pl, int maxb, cud
     p.wstages = (left - p.bstages * bbytes) / p.wstage_bytes;
     if (p.wstages > GQ_PF_MAX_STAGES) p.wstages = GQ_PF_MAX_STAGES;
     p.wstages -= p.wstages % SETS;        // each set walks stages of its own
-    if (p.wstages < 1) return GQ_ERR_LIMIT;
+    if (p.wstages < 1 || p.bstages < (SETS == 1 ? GQ_PF_SL1 : GQ_PF_SL2)) return GQ_ERR_LIMIT;
     left -= p.wstages * p.wstage_bytes + p.bstages * bbytes;
     while (p.bstages < GQ_PF_SLOTS * (WIDE ? 1 : SETS) && left >= bbytes) { ++p.bstages; left -= bbytes; }
     if (int rc = allow_smem<gemm_prefill_kernel<SETS, WIDE>>(total)) return rc;
@@ -1920,10 +1920,17 @@ extern "C" int gq_gemm_prefill(const void *x_dev, int64_t M, int64_t K, int64_t 
     cudaStream_t st = (cudaStream_t)stream;
     {
         cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.gridDim = dim3((unsigned)(pl.tiles * pl.N)); cfg.blockDim = dim3(GQ_PF_PREP_THREADS); cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 1;
+        int64_t parts = (K / 8 + GQ_PF_PREP_THREADS * GQ_PF_PREP_VECS - 1) / (GQ_PF_PREP_THREADS * GQ_PF_PREP_VECS);
+        const int64_t fill = (int64_t)device_sms() * 10 / (pl.tiles * pl.N);       // beyond what the GPU holds of these CTAs there is no latency left to hide
+        if (parts > fill) parts = fill > 1 ? fill : 1;
+        if (parts > 8) parts = 8;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = (unsigned)parts; attr[1].val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned)(pl.tiles * pl.N), (unsigned)parts); cfg.blockDim = dim3(GQ_PF_PREP_THREADS); cfg.stream = st; cfg.attrs = attr;
+        cfg.numAttrs = parts > 1 ? 2 : 1;
         GQ_CUDA(cudaLaunchKernelEx(&cfg, prep_x_prefill_kernel, (const __nv_bfloat16 *)x_dev, ldx, (int)K, (int)M, pl.N, pl.sets == 1 ? 0 : pl.wide ? pl.N / 2 : pl.N, ex, xp, status));
         GQ_LAUNCHED();
     }

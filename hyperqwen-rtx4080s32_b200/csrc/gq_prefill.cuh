@@ -37,6 +37,12 @@
 namespace gq {
 
 #define GQ_PF_SLOTS 4                        // A slots of a ring: the four 64-wide k-slices of a k-block
+// k-slices that share a barrier (a dequantiser's wait, store and announcement; the MMA issuer's wait and commit).  Up to 128 batch rows the
+// MMAs of a slice are short beside its decoding and the hand-over counts: two a barrier, 34,816 x 5,120 at 64 rows, one / two / four, Q4_K
+// 41.3 / 38.0 / 44.6 us, IQ3_S 59.0 / 55.4 / 56.5, Q2_K 43.9 / 39.9 / 45.4.  Above, the MMAs have to follow the slices closely: Q4_K at 517
+// rows, one / two, 153 / 173 us.
+#define GQ_PF_SL1 2
+#define GQ_PF_SL2 1
 #define GQ_PF_MAX_STAGES 6                   // upper bound of the weight ring
 
 struct PrefillParams {
@@ -175,12 +181,12 @@ struct PfRings {
 // the dequantiser loop of one warp for a tile of TYPE: k-blocks set, set + SETS, ... of this CTA's nkb; k-block kb fills the
 // A ring kb % RINGS once the MMAs of k-block kb - RINGS have read it.  Barriers are waited on phase by phase: wfull because the
 // weight ring has a multiple of SETS stages, afree because it belongs to a set's k-blocks, not to the ring.
-template <int TYPE, int SETS, int RINGS>
+template <int TYPE, int SETS, int RINGS, int SL>
 __device__ __forceinline__ bool pf_dequant(const PfRings &r, int slab_off, int set, int nkb, uint32_t ta, const DecAux &aux, int lane) {
     int ws = set % r.wstages, wround = set / r.wstages;
     for (int kb = set; kb < nkb; kb += SETS) {
         const int prev = kb - RINGS;
-        uint64_t *afree = r.afree + GQ_PF_SLOTS * ((kb + SETS - RINGS) % SETS);
+        uint64_t *afree = r.afree + GQ_PF_SLOTS / SL * ((kb + SETS - RINGS) % SETS);
         if (!mbar_wait(r.wfull + ws, wround & 1)) return false;
         Dec<TYPE> dec;
         dec.load(r.wring + (size_t)ws * r.wstage_bytes + slab_off, lane, aux);
@@ -192,14 +198,18 @@ __device__ __forceinline__ bool pf_dequant(const PfRings &r, int slab_off, int s
             constexpr int J = decltype(j_)::value;
             uint32_t o[16];
             pf_slice<TYPE, J>(dec, o);
-            if (prev >= 0 && !mbar_wait(afree + J, (prev / SETS) & 1)) return false;
-            __syncwarp();
-            tc_fence_after();
+            if constexpr (J % SL == 0) {
+                if (prev >= 0 && !mbar_wait(afree + J / SL, (prev / SETS) & 1)) return false;
+                __syncwarp();
+                tc_fence_after();
+            }
             tmem_st_16x256b_x4(ta + 32 * J, o);
-            tmem_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(r.afull + 8 * J);
+            if constexpr (J % SL == SL - 1) {
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(r.afull + 8 * (J / SL));
+            }
             return true;
         };
         if (!slice(std::integral_constant<int, 0>{}) || !slice(std::integral_constant<int, 1>{}) || !slice(std::integral_constant<int, 2>{}) ||
@@ -232,13 +242,14 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
     // layout: [activation ring][weight ring][codebook tables of the run's types]; the reduction of a split reuses the rings
     __shared__ __align__(8) uint64_t bars[2 * GQ_PF_MAX_STAGES + 2 * GQ_PF_SLOTS * SETS + 1];
     __shared__ uint32_t tmem_slot;
+    __shared__ int s_out[2][2];          // first output column and columns of the two tiles: the epilogue does not wait for global memory
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int N = p.N, bbytes = N * 128 / SETS;          // a CTA of a pair holds half of the batch rows of a slice
     uint8_t *wring = smem + p.bstages * bbytes;
     uint8_t *tables = wring + p.wstages * p.wstage_bytes;
-    constexpr int RINGS = WIDE ? 1 : SETS, CG = SETS;
+    constexpr int RINGS = WIDE ? 1 : SETS, CG = SETS, SL = SETS == 1 ? GQ_PF_SL1 : GQ_PF_SL2, GROUPS = GQ_PF_SLOTS / SL;
     uint64_t *wfull = bars, *wfree = bars + GQ_PF_MAX_STAGES;
-    uint64_t *afull = bars + 2 * GQ_PF_MAX_STAGES, *afree = afull + GQ_PF_SLOTS * RINGS, *done = afree + GQ_PF_SLOTS * SETS;
+    uint64_t *afull = bars + 2 * GQ_PF_MAX_STAGES, *afree = afull + GROUPS * RINGS, *done = afree + GROUPS * SETS;
     constexpr uint32_t TMEM_COLS = 256u * SETS, D_COLS = TMEM_COLS - 32u * GQ_PF_SLOTS * RINGS;      // the A slots follow the accumulator
     constexpr int DEQ = 8 * SETS;
 
@@ -287,8 +298,8 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
         const int in_pair = p.n_desc - 2 * unit * CG;
         const uint32_t pair_slabs = (uint32_t)(in_pair < 2 * CG ? in_pair : 2 * CG) * 4;
         for (int s = 0; s < p.wstages; ++s) { mbar_init(wfull + s, 1); mbar_init(wfree + s, slabs ? slabs : 1); }
-        for (int s = 0; s < GQ_PF_SLOTS * RINGS; ++s) mbar_init(afull + s, half ? 1 : pair_slabs + CG);
-        for (int s = 0; s < GQ_PF_SLOTS * SETS; ++s) mbar_init(afree + s, 1);
+        for (int s = 0; s < GROUPS * RINGS; ++s) mbar_init(afull + s, half ? SL : pair_slabs + SL + CG - 1);
+        for (int s = 0; s < GROUPS * SETS; ++s) mbar_init(afree + s, 1);
         mbar_init(done, 1);
         fence_barrier_init();
         fence_proxy_async();
@@ -296,6 +307,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
         if (has0)
             for (int kb = 0; kb < SETS && kb < nkb; ++kb) load_weights(kb, kb);
     }
+    if (threadIdx.x < 4) s_out[threadIdx.x >> 1][threadIdx.x & 1] = (threadIdx.x >> 1 ? d1 : d0)[2 + (threadIdx.x & 1)];
     __syncwarp();
     if (warp == DEQ + 2) tmem_alloc<CG>(&tmem_slot, TMEM_COLS);
     // the codebook tables of the two tiles' types, each at its place among the tables of the run's types
@@ -329,8 +341,8 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
             const uint8_t *src = p.xp + (((int64_t)mt * p.nb + kb0) * 4 * CG + half) * bbytes;
             for (int i = 0, st = 0; i < 4 * nkb; ++i) {
                 const int o = i - p.bstages;
-                if (o >= 0 && !mbar_wait_parked(afree + ((o >> 2) % SETS) * GQ_PF_SLOTS + (o & 3), ((o >> 2) / SETS) & 1)) { ok = false; break; }
-                uint64_t *full = afull + ((i >> 2) % RINGS) * GQ_PF_SLOTS + (i & 3);
+                if (o >= 0 && !mbar_wait_parked(afree + ((o >> 2) % SETS) * GROUPS + (o & 3) / SL, ((o >> 2) / SETS) & 1)) { ok = false; break; }
+                uint64_t *full = afull + ((i >> 2) % RINGS) * GROUPS + (i & 3) / SL;
                 mbar_expect_tx(full, (uint32_t)bbytes);
                 bulk_g2s(smem + (size_t)st * bbytes, src + (int64_t)i * CG * bbytes, (uint32_t)bbytes, full);
                 if (++st == p.bstages) st = 0;
@@ -341,9 +353,9 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
     } else if (warp == DEQ + 2 && half) {
         // ---- relay of the pair's second CTA: its activation rows are there -> the issuing CTA's barrier ----
         for (int kb = 0; kb < nkb && ok; ++kb) {
-            const int slot0 = GQ_PF_SLOTS * (kb % RINGS);
+            const int slot0 = GROUPS * (kb % RINGS);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < GROUPS; ++j) {
                 if (!mbar_wait(afull + slot0 + j, (uint32_t)(kb / RINGS) & 1u)) { ok = false; break; }
                 if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(afull + slot0 + j), leader));
             }
@@ -361,12 +373,14 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
         for (int kb = 0; kb < nkb && ok; ++kb) {
             const int ring = kb % RINGS;
             const uint32_t parity = (uint32_t)(kb / RINGS) & 1u;
-            uint64_t *full = afull + GQ_PF_SLOTS * ring, *free = afree + GQ_PF_SLOTS * (kb % SETS);
+            uint64_t *full = afull + GROUPS * ring, *free = afree + GROUPS * (kb % SETS);
             const uint32_t ta = tmem + D_COLS + 32u * GQ_PF_SLOTS * ring;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                if (!mbar_wait(full + j, parity)) { ok = false; break; }
-                tc_fence_after();
+                if (j % SL == 0) {
+                    if (!mbar_wait(full + j / SL, parity)) { ok = false; break; }
+                    tc_fence_after();
+                }
                 if (elect_one()) {
                     const uint64_t bd = bdesc0 + boff;
 #pragma unroll
@@ -376,7 +390,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
                         if constexpr (WIDE) umma_ts_f16<CG>(tmem + nmma, ta + 32 * j + 8 * kk, bd + 8 / CG * nmma + 2 * kk, idesc, acc);      // 128 bytes a row
                     }
                     // the slot and the activation stage may be overwritten once these MMAs have read them
-                    umma_commit<CG>(j == 3 && kb + 1 == nkb ? done : free + j, ctas);
+                    if (j % SL == SL - 1) umma_commit<CG>(j == 3 && kb + 1 == nkb ? done : free + j / SL, ctas);
                 }
                 boff += bstep;
                 if (boff == bwrap) boff = 0;
@@ -395,10 +409,10 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
             PfRings r;
             r.wring = wring; r.wstage_bytes = p.wstage_bytes; r.wstages = p.wstages;
             r.wfull = wfull; r.wfree = wfree; r.afree = afree;
-            r.afull = map_to_rank(smem_u32(afull + GQ_PF_SLOTS * ring), CG > 1 ? leader : cluster_ctarank());
+            r.afull = map_to_rank(smem_u32(afull + GROUPS * ring), CG > 1 ? leader : cluster_ctarank());
             const int slab_off = (slab < 4 ? 0 : wb0) + (slab & 3) * 32 * p.half_bytes[type & 31];
             const uint32_t ta = tmem + D_COLS + 32u * GQ_PF_SLOTS * ring + ((uint32_t)(16 * slab) << 16);
-#define GQ_PF(T) case T: ok = pf_dequant<T, SETS, RINGS>(r, slab_off, set, nkb, ta, aux, lane); break;
+#define GQ_PF(T) case T: ok = pf_dequant<T, SETS, RINGS, SL>(r, slab_off, set, nkb, ta, aux, lane); break;
             switch (type) {
                 GQ_PF(GQ_Q4_0) GQ_PF(GQ_Q5_0) GQ_PF(GQ_Q8_0) GQ_PF(GQ_Q2_K) GQ_PF(GQ_Q3_K) GQ_PF(GQ_Q4_K)
                 GQ_PF(GQ_Q5_K) GQ_PF(GQ_Q6_K) GQ_PF(GQ_IQ4_NL) GQ_PF(GQ_IQ3_S) GQ_PF(GQ_IQ4_XS) GQ_PF(GQ_IQ3_XXS)
@@ -416,11 +430,10 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
 
     // ---- epilogue: warps 0 .. DEQ-1; lane l of partition q is row 32 q + l of the pair of tiles ----
     const int q = warp & 3, e = warp >> 2, feat = 32 * q + lane;
-    const int32_t *dt = (feat < 64) ? d0 : d1;
-    const int rt = feat & 63;
-    const bool tile_ok = feat < 64 ? has0 : has1, row_ok = tile_ok && rt < dt[3];
-    const int64_t col = (int64_t)dt[2] + rt;
-    const bool pair_ok = tile_ok && (rt | 1) < dt[3] && !(p.ldy & 1) && !((reinterpret_cast<uintptr_t>(p.y) + 2 * (uintptr_t)(col - (lane & 1))) & 3);
+    const int rt = feat & 63, n_cols = s_out[feat >> 6][1];
+    const bool tile_ok = feat < 64 ? has0 : has1, row_ok = tile_ok && rt < n_cols;
+    const int64_t col = (int64_t)s_out[feat >> 6][0] + rt;
+    const bool pair_ok = tile_ok && (rt | 1) < n_cols && !(p.ldy & 1) && !((reinterpret_cast<uintptr_t>(p.y) + 2 * (uintptr_t)(col - (lane & 1))) & 3);
     const uint32_t td = tmem + ((uint32_t)(32 * q) << 16);
     if (p.split == 1) {
         if (warp < DEQ && ok) {
@@ -429,9 +442,9 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
                 uint32_t a[8];
                 tmem_ld_32x32b_x8(td + c, a);
                 const float4 e0 = *reinterpret_cast<const float4 *>(s_ex + c), e1 = *reinterpret_cast<const float4 *>(s_ex + c + 4);
-                tmem_wait_ld();
                 const float es[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
                 float v[8];
+                tmem_wait_ld();
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(a[j]) * es[j];
                 pf_store8(p, v, mt * N + c, col, row_ok, pair_ok, lane);
@@ -445,15 +458,16 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
         cluster_sync_all();                 // every CTA of the cluster has finished with its rings
         if (warp < DEQ) {
             const uint32_t mine = smem_u32(buf) + (uint32_t)(part * (ch >> 2) * 128 + feat) * 16;
+            uint32_t a[8];
+            if (8 * e < N) tmem_ld_32x32b_x8(td + 8 * e, a);
 #pragma unroll 1
             for (int c = 8 * e; c < N; c += 8 * (DEQ / 4)) {
                 const int r = c / ch;
-                uint32_t a[8];
-                tmem_ld_32x32b_x8(td + c, a);
-                tmem_wait_ld();
                 const uint32_t dst = map_to_rank(mine, (uint32_t)(r * CG + half)) + (uint32_t)((c - r * ch) >> 2) * 2048;
+                tmem_wait_ld();
                 st_cluster_f4(dst, __uint_as_float(a[0]), __uint_as_float(a[1]), __uint_as_float(a[2]), __uint_as_float(a[3]));
                 st_cluster_f4(dst + 2048, __uint_as_float(a[4]), __uint_as_float(a[5]), __uint_as_float(a[6]), __uint_as_float(a[7]));
+                if (c + 8 * (DEQ / 4) < N) tmem_ld_32x32b_x8(td + c + 8 * (DEQ / 4), a);
             }
             __syncwarp();
         }
@@ -507,26 +521,31 @@ __device__ __forceinline__ float amax8(const uint4 &v) {
 // activation preparation for the prefill path: bf16 row -> fp16 scaled by an exact power of two, stored in the
 // MMA's shared-memory layout (tiles of N rows x 64 k, K-major, 16-byte chunks XOR-swizzled by row % 8) so the
 // kernel's producer moves a whole k-slice with one bulk copy.  For CTA pairs a slice holds the rows of the first CTA, then
-// those of the second: of every `nmma` rows that an MMA takes, the first half is the first CTA's.  One CTA per row of the padded batch; the row is read once and
-// kept in registers between the maximum and the conversion (the first 128 * 5 * 8 = 5120 activations).  128 threads of few
+// those of the second: of every `nmma` rows that an MMA takes, the first half is the first CTA's.  The row is read once and kept in
+// registers between the maximum and the conversion: 5120 activations to a CTA of 128 threads, longer rows over a cluster of up to eight
+// CTAs, which exchange their maxima (what eight do not hold is read twice).  128 threads of few
 // registers, so that these CTAs fit beside those of a matrix kernel: they are in place when the kernel in front ends, and the
 // matrix kernel behind them gets its SMs, fetches weights and decodes while they run (with 512 threads a CTA kept it off its SM).
+// Bound by the latency of its loads and, beyond a few hundred rows, by how many of these CTAs an SM holds: rows of 17,408 in one CTA each
+// took 6 us at 64 rows and 17 at 517, a sixth of the layer.
 #define GQ_PF_PREP_THREADS 128
 #define GQ_PF_PREP_VECS 5
-__global__ void __launch_bounds__(GQ_PF_PREP_THREADS, 10) prep_x_prefill_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int K, int M, int N, int nmma,
+__global__ void __launch_bounds__(GQ_PF_PREP_THREADS, 9) prep_x_prefill_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int K, int M, int N, int nmma,
                                                                             float *__restrict__ ex, uint8_t *__restrict__ xp, int *status) {
-    __shared__ float red[GQ_PF_PREP_THREADS / 32];
-    const int m = blockIdx.x, n = m % N, nvec = K >> 3, hn = nmma >> 1;
+    __shared__ float red[GQ_PF_PREP_THREADS / 32], peers[8];
+    const int part = blockIdx.y, parts = gridDim.y, m = blockIdx.x, n = m % N, nvec = K >> 3, hn = nmma >> 1;
     const int r = nmma ? (n % nmma) / hn * (N >> 1) + n / nmma * hn + n % hn : n;
     uint8_t *dst = xp + (int64_t)(m / N) * (K / 64) * (N * 128) + r * 128;
     const int phase = r & 7;
+    if (parts > 1) cluster_arrive_relaxed();      // collected before the first store into another CTA: by then it runs
     pdl_trigger();    // the kernel behind this one may start fetching weights
     pdl_wait();       // whatever ran before (possibly still reading this workspace) has finished
-    if (m == 0 && threadIdx.x == 0) *status = 0;
+    if (m == 0 && part == 0 && threadIdx.x == 0) *status = 0;
+    const int first = part * GQ_PF_PREP_THREADS + threadIdx.x, step = parts * GQ_PF_PREP_THREADS;       // the thread's chunks of the row
     const auto put = [&](int c, const uint4 &o) { *reinterpret_cast<uint4 *>(dst + (int64_t)(c >> 3) * (N * 128) + (((c & 7) ^ phase) << 4)) = o; };
     if (m >= M) {
         // rows past the batch inside the last tile: zeros (their outputs are never stored)
-        for (int c = threadIdx.x; c < nvec; c += GQ_PF_PREP_THREADS) put(c, make_uint4(0, 0, 0, 0));
+        for (int c = first; c < nvec; c += step) put(c, make_uint4(0, 0, 0, 0));
         return;
     }
     const uint4 *xr = reinterpret_cast<const uint4 *>(x + (int64_t)m * ldx);
@@ -534,12 +553,12 @@ __global__ void __launch_bounds__(GQ_PF_PREP_THREADS, 10) prep_x_prefill_kernel(
     float amax = 0.0f;
 #pragma unroll
     for (int i = 0; i < GQ_PF_PREP_VECS; ++i) {
-        const int c = threadIdx.x + i * GQ_PF_PREP_THREADS;
+        const int c = first + i * step;
         v[i] = c < nvec ? __ldg(xr + c) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int i = 0; i < GQ_PF_PREP_VECS; ++i) amax = fmaxf(amax, amax8(v[i]));
-    for (int c = threadIdx.x + GQ_PF_PREP_VECS * GQ_PF_PREP_THREADS; c < nvec; c += GQ_PF_PREP_THREADS) amax = fmaxf(amax, amax8(__ldg(xr + c)));
+    for (int c = first + GQ_PF_PREP_VECS * step; c < nvec; c += step) amax = fmaxf(amax, amax8(__ldg(xr + c)));
 #pragma unroll
     for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
@@ -547,11 +566,17 @@ __global__ void __launch_bounds__(GQ_PF_PREP_THREADS, 10) prep_x_prefill_kernel(
     float a = red[0];
 #pragma unroll
     for (int i = 1; i < GQ_PF_PREP_THREADS / 32; ++i) a = fmaxf(a, red[i]);
+    if (parts > 1) {      // the cluster is the row: every CTA puts its maximum into all of them
+        cluster_wait();
+        if ((int)threadIdx.x < parts) st_cluster_f32(map_to_rank(smem_u32(peers + part), threadIdx.x), a);
+        cluster_sync_all();
+        for (int i = 0; i < parts; ++i) a = fmaxf(a, peers[i]);
+    }
     // scale = 2^(9 - e), amax * scale in [512, 1024); identity for a zero, tiny or non-finite row
     int e = 9;
     if (a > 0.0f && a < 3.0e38f) { e = (int)((__float_as_uint(a) >> 23) & 0xFF) - 127; if (e < -100) e = -100; }
     const float scale = __uint_as_float((uint32_t)(127 + 9 - e) << 23);
-    if (threadIdx.x == 0) ex[m] = __uint_as_float((uint32_t)(127 - 9 + e) << 23);
+    if (part == 0 && threadIdx.x == 0) ex[m] = __uint_as_float((uint32_t)(127 - 9 + e) << 23);
     const auto convert = [&](int c, const uint4 &w) {
         const __nv_bfloat162 *b = reinterpret_cast<const __nv_bfloat162 *>(&w);
         uint4 o;
@@ -562,10 +587,10 @@ __global__ void __launch_bounds__(GQ_PF_PREP_THREADS, 10) prep_x_prefill_kernel(
     };
 #pragma unroll
     for (int i = 0; i < GQ_PF_PREP_VECS; ++i) {
-        const int c = threadIdx.x + i * GQ_PF_PREP_THREADS;
+        const int c = first + i * step;
         if (c < nvec) convert(c, v[i]);
     }
-    for (int c = threadIdx.x + GQ_PF_PREP_VECS * GQ_PF_PREP_THREADS; c < nvec; c += GQ_PF_PREP_THREADS) convert(c, __ldg(xr + c));
+    for (int c = first + GQ_PF_PREP_VECS * step; c < nvec; c += step) convert(c, __ldg(xr + c));
 }
 
 }  // namespace gq
