@@ -496,8 +496,8 @@ def mul_mat_tiles_grouped(x: torch.Tensor, packed: torch.Tensor, descs: list[tor
     n_tiles = sum(-(-int(n) // 64) for n in n_outs)
     # up to 32 rows the grouped kernel streams the weights once for the batch; from 33 rows that would be twice, and the tcgen05
     # kernel dequantises each weight once for all rows.  Whole calls in microseconds, grouped / tcgen05, at 16, 24 and 32 rows:
-    # 2 x 17408 x 5120 Q4_K 35.1 / 40.6, 46.3 / 41.3, 57.1 / 41.5; IQ3_S 43.3 / 55.5, 63.3 / 56.5, 70.9 / 56.6; 5120 x 17408 Q4_K
-    # 22.8 / 28.1, 29.2 / 29.3, 35.2 / 29.3; 5120 x 4352 IQ3_S 11.8 / 16.9, 15.1 / 17.2, 16.4 / 17.2.  Between 17 and 32 rows the
+    # 2 x 17408 x 5120 Q4_K 33.8 / 37.7, 39.7 / 37.7, 46.4 / 37.7; IQ3_S 42.8 / 52.9, 50.2 / 52.9, 57.0 / 52.9 (the tcgen05 kernel's time,
+    # measured at 64 rows, hardly depends on them).  Between 24 and 32 rows the
     # tcgen05 kernel is thus the faster one on the wide layers.  The line stays at 32 for the precision: the grouped kernel
     # multiplies exact weights, the other rounds them to fp16 (error beyond the output's rounding 4e-7 against 9e-5 of the
     # result's norm)
