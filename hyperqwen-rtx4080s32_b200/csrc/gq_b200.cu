@@ -149,13 +149,9 @@ __host__ __device__ inline int64_t align256(int64_t v) { return (v + 255) & ~(in
 
 __host__ __device__ inline int gq_x_tile_bytes(int M) { return M * GQ_X_ROW + ((4 * M + 15) & ~15); }
 
-// prepared activations of one k-block: batches above GQ_WIDE_ROWS are multiplied that many rows at a time, each part with tiles of its own
-#define GQ_WIDE_ROWS 32
-static int64_t gq_x_bytes(int64_t M) { return M <= GQ_WIDE_ROWS ? gq_x_tile_bytes((int)M) : gq_x_tile_bytes(GQ_WIDE_ROWS) + gq_x_bytes(M - GQ_WIDE_ROWS); }
-
 static int64_t ws_layout(int64_t M, int64_t K, int64_t n_total, int split, void *base, Workspace *ws) {
     int64_t off = 256;
-    const int64_t o_xt = off; off = align256(off + (K / GQ_QK) * gq_x_bytes(M));
+    const int64_t o_xt = off; off = align256(off + (K / GQ_QK) * gq_x_tile_bytes((int)M));
     const int64_t o_p = off; if (split > 1) off = align256(off + (int64_t)split * M * n_total * 4);
     if (ws && base) {
         uint8_t *b = (uint8_t *)base;
@@ -375,7 +371,7 @@ __global__ void __launch_bounds__(32 * GQ_PREP_WARPS) prep_x_norm_kernel(const _
 }
 
 // ---------------------------------------------------------------------------------------------------
-// grouped small-batch kernel, integer form.  One CTA per descriptor row (64 output columns of one shard x a k-range):
+// grouped small-batch kernel.  One CTA per descriptor row (64 output columns of one shard x a k-range):
 // a producer warp streams the tile's k-blocks (one bulk copy each) plus the matching activation rows through
 // an mbarrier ring; four consumer warps each own a 16-row slab, dequantise it in registers and run m16n8k16
 // MMAs with the weights on the M side and the batch rows on the N side (8 batch rows per MMA, MT MMAs deep).
@@ -412,11 +408,6 @@ struct GemvParams {
     const __nv_bfloat16 *x;  // FORM 2, one row: the activations themselves, converted by the producer warp (null: xt is prepared)
     const uint8_t *pf_ptr;   // weights the caller will multiply next (or null): prefetched into L2 while this launch computes
     int64_t pf_bytes;
-    // fp16 form
-    int n_tiles;             // 64-row tiles of the run
-    int part_rows;           // batch rows of a split's image in `partials`
-    int cb_stride;           // distance of the two tiles' codebook tables (0: a run of one type, one table)
-    int ar_at;               // shared-memory offset of the fused all-reduce's scratch
     ArFused ar;
 };
 
@@ -717,28 +708,33 @@ __device__ __noinline__ void fused_allreduce_block(const GemvParams &p, const ui
     }
 }
 
-// The integer form of the grouped kernel (1..GQ_GEMV8_MAX_ROWS rows; above: gemv_wide_kernel).
+#include "gq_fp16.cuh"
+
 // MINB = CTAs per SM the compiler must leave room for (0: its own choice).  For the M <= 8 form 4 gives it 96
 // registers, which it turns into more loads and MMAs in flight per warp: measured 14 % faster than the 72-register
 // build when a CTA walks ten or more k-blocks, a little slower on launches of many short CTAs, 2 % faster on the
 // mixed stack.  (Compiling both and choosing per call was slower than either alone: alternating between two large
-// kernels costs more in instruction-cache misses at every launch than the better fit gains.)
+// kernels costs more in instruction-cache misses at every launch than the better fit gains.)  The fp16 form has room for two CTAs (168
+// registers); three were slower up to two waves.
 //
 // FORM 1: activations as two byte planes, weights decoded to 8-bit quads, m16n8k32 / m16n8k16 integer MMAs: about half the
 // instructions per weight of the fp16 form.  (At 9..16 rows the fp16 form is faster where a run is scaled per 16 weights, slower elsewhere:
 // 2 x 17,408 x 5,120 at 16 rows, integer / fp16, IQ3_S + Q2_K 41.9 / 37.3 us, Q3_K + IQ3_S 39.8 / 41.7, IQ4_XS 41 / 47; 7,168 x 5,120
 // 13.3 / 15.6.)
 // FORM 2: the integer form with both planes in one MMA, used for 1..4 batch rows.
+// FORM 0: activations as fp16, weights as exact fp16 integers (gq_fp16.cuh), used above GQ_GEMV8_MAX_ROWS rows.
 // ONLY: 0 compiles the decoders of all types (the branch is per CTA); a GGML type id compiles that type alone,
 // for launches whose shards all share it (a smaller kernel; most launches of a real model are such).
-// FORM 0 stands for the fp16 form's stage here.
 template <int MT, int FORM>
 __host__ __device__ constexpr int gq_stage_xbytes() { return FORM == 2 ? 4 * GQ_X_ROW + 16 : 8 * MT * GQ_X_ROW + 32 * MT; }
+
+template <int MT>
+__host__ __device__ constexpr bool gq_red_in_ring() { return MT == 8; }
 
 template <int MT, int MINB, int FORM, int ONLY>
 __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_grouped_kernel(const __grid_constant__ GemvParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    // layout: [stages x (weights wbytes_max | activation tile)] [full barriers] [empty barriers] [IQ3_S grid] [reduction scratch]
+    // layout: [stages x (weights wbytes_max | activation tile)] [full barriers] [empty barriers] [codebook table] [reduction scratch]
     const int stages = p.stages, wmax = p.wbytes_max, M = p.M;
     constexpr int xbytes = gq_stage_xbytes<MT, FORM>();
     const int stage_bytes = wmax + xbytes;
@@ -756,10 +752,10 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
     const int tile_bytes = 64 * B;
     const int nk = kb1 - kb0;
 
-    // a tile whose type contradicts the call's run_info (not the single type it named, or a codebook type it did not
-    // announce, which has no table space): report and leave (every CTA of a cluster works on the same tile, so a cluster
-    // leaves as one)
-    if ((ONLY != 0 && d[1] != ONLY) || (gq_cb_kind(type) >= 0 && gq_cb_bytes(gq_cb_kind(type)) > p.cb_bytes)) {
+    // a tile whose type contradicts the call's run_info (not the single type that this kernel is for; fp16 form: no type at all, or one of
+    // wider tiles than a stage holds; a codebook type without table space): report and leave (every CTA of a cluster works on the same
+    // tile, so a cluster leaves as one)
+    if ((ONLY != 0 && d[1] != ONLY) || (FORM == 0 && (B == 0 || tile_bytes > wmax)) || (gq_cb_kind(type) >= 0 && gq_cb_bytes(gq_cb_kind(type)) > p.cb_bytes)) {
         if (threadIdx.x == 0) { pdl_wait(); report_status(p.status, GQ_DEV_BAD_SHAPE); }      // after the preparation kernel has cleared the word
         return;
     }
@@ -780,23 +776,27 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
     // producer's first copies are already on their way, closed by a barrier among the consumers only
     if (p.cb_bytes && warp < GQ_CONSUMER_WARPS) {
         uint32_t *g32 = grid_s;
-        if ((ONLY == 0 || ONLY == GQ_IQ3_S) && type == GQ_IQ3_S) {
-            for (int i = threadIdx.x; i < 512; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq3s_grid[i]);
-        }
-        if ((ONLY == 0 || ONLY == GQ_IQ3_XXS) && type == GQ_IQ3_XXS) {
-            for (int i = threadIdx.x; i < 256; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq3xxs_grid[i]);
-        }
-        if ((ONLY == 0 || ONLY == GQ_IQ2_XXS) && type == GQ_IQ2_XXS) {
-            for (int i = threadIdx.x; i < 512; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq2xxs_grid[i]);
-        }
-        if ((ONLY == 0 || ONLY == GQ_IQ2_XS) && type == GQ_IQ2_XS) {
-            for (int i = threadIdx.x; i < 1024; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq2xs_grid[i]);
-        }
-        if ((ONLY == 0 || ONLY == GQ_IQ2_S) && type == GQ_IQ2_S) {
-            for (int i = threadIdx.x; i < 2048; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq2s_grid[i]);
-        }
-        if ((ONLY == 0 || ONLY == GQ_IQ1_M) && type == GQ_IQ1_M) {
-            for (int i = threadIdx.x; i < 4096; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq1_grid[i]);
+        if constexpr (FORM == 0) {
+            fill_codebook(type, reinterpret_cast<uint8_t *>(grid_s), threadIdx.x, 32 * GQ_CONSUMER_WARPS);
+        } else {
+            if ((ONLY == 0 || ONLY == GQ_IQ3_S) && type == GQ_IQ3_S) {
+                for (int i = threadIdx.x; i < 512; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq3s_grid[i]);
+            }
+            if ((ONLY == 0 || ONLY == GQ_IQ3_XXS) && type == GQ_IQ3_XXS) {
+                for (int i = threadIdx.x; i < 256; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq3xxs_grid[i]);
+            }
+            if ((ONLY == 0 || ONLY == GQ_IQ2_XXS) && type == GQ_IQ2_XXS) {
+                for (int i = threadIdx.x; i < 512; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq2xxs_grid[i]);
+            }
+            if ((ONLY == 0 || ONLY == GQ_IQ2_XS) && type == GQ_IQ2_XS) {
+                for (int i = threadIdx.x; i < 1024; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq2xs_grid[i]);
+            }
+            if ((ONLY == 0 || ONLY == GQ_IQ2_S) && type == GQ_IQ2_S) {
+                for (int i = threadIdx.x; i < 2048; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq2s_grid[i]);
+            }
+            if ((ONLY == 0 || ONLY == GQ_IQ1_M) && type == GQ_IQ1_M) {
+                for (int i = threadIdx.x; i < 4096; i += 32 * GQ_CONSUMER_WARPS) g32[i] = iq3s_grid_entry8(c_iq1_grid[i]);
+            }
         }
         asm volatile("bar.sync 1, %0;" ::"n"(32 * GQ_CONSUMER_WARPS) : "memory");
     }
@@ -893,9 +893,24 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
     bool ok = true;
     uint32_t ar_prev = 0;
     const int slab_off = warp * 16 * B;
-    // the IQ4 codebook in four registers, as signed bytes
-    Iq4Table iq4;
-    {
+    const int xs_off = M * GQ_X_ROW;
+#define GQ_EACH_CONSUME \
+        switch (type) { \
+            GQ_CONSUME(GQ_Q4_0) GQ_CONSUME(GQ_Q5_0) GQ_CONSUME(GQ_Q8_0) GQ_CONSUME(GQ_Q2_K) GQ_CONSUME(GQ_Q3_K) GQ_CONSUME(GQ_Q4_K) \
+            GQ_CONSUME(GQ_Q5_K) GQ_CONSUME(GQ_Q6_K) GQ_CONSUME(GQ_IQ4_NL) GQ_CONSUME(GQ_IQ3_S) GQ_CONSUME(GQ_IQ4_XS) GQ_CONSUME(GQ_IQ3_XXS) \
+            GQ_CONSUME(GQ_IQ2_XXS) GQ_CONSUME(GQ_IQ2_XS) GQ_CONSUME(GQ_IQ2_S) GQ_CONSUME(GQ_IQ1_M) \
+        }
+    if constexpr (FORM == 0) {
+        DecAux aux;
+        aux.grid = grid_s;
+        aux.iq4 = iq4_table_biased();
+#define GQ_CONSUME(T) case T: ok = consume<T, MT>(ring, xs_off, slab_off, aux, lane, acc, ar_prev); break;
+        GQ_EACH_CONSUME
+#undef GQ_CONSUME
+    } else {
+        DecAux8 aux;
+        aux.grid = grid_s;
+        // the IQ4 codebook in four registers, as signed bytes
         uint32_t tb[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -903,23 +918,13 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
 #pragma unroll
             for (int i = 0; i < 4; ++i) tb[j] |= (uint32_t)(uint8_t)c_iq4_kvalues[4 * j + i] << (8 * i);
         }
-        iq4 = {tb[0], tb[1], tb[2], tb[3]};
-    }
-    const int xs_off = M * GQ_X_ROW;
-    DecAux8 aux;
-    aux.grid = grid_s;
-    aux.iq4 = iq4;
+        aux.iq4 = {tb[0], tb[1], tb[2], tb[3]};
 #define GQ_CONSUME(T) case T: ok = consume8<T, MT, FORM == 2>(ring, xs_off, slab_off, aux, lane, acc, ar_prev); break;
-    if constexpr (ONLY != 0) {
-        ok = consume8<(ONLY ? ONLY : GQ_Q4_K), MT, FORM == 2>(ring, xs_off, slab_off, aux, lane, acc, ar_prev);
-    } else {
-        switch (type) {
-            GQ_CONSUME(GQ_Q4_0) GQ_CONSUME(GQ_Q5_0) GQ_CONSUME(GQ_Q8_0) GQ_CONSUME(GQ_Q2_K) GQ_CONSUME(GQ_Q3_K) GQ_CONSUME(GQ_Q4_K)
-            GQ_CONSUME(GQ_Q5_K) GQ_CONSUME(GQ_Q6_K) GQ_CONSUME(GQ_IQ4_NL) GQ_CONSUME(GQ_IQ3_S) GQ_CONSUME(GQ_IQ4_XS) GQ_CONSUME(GQ_IQ3_XXS)
-            GQ_CONSUME(GQ_IQ2_XXS) GQ_CONSUME(GQ_IQ2_XS) GQ_CONSUME(GQ_IQ2_S) GQ_CONSUME(GQ_IQ1_M)
-        }
-    }
+        if constexpr (ONLY != 0) ok = consume8<(ONLY ? ONLY : GQ_Q4_K), MT, FORM == 2>(ring, xs_off, slab_off, aux, lane, acc, ar_prev);
+        else { GQ_EACH_CONSUME }
 #undef GQ_CONSUME
+    }
+#undef GQ_EACH_CONSUME
     if constexpr (FORM == 2) {      // columns n and n + 4: lanes t and t + 2
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[0][j] += __shfl_xor_sync(0xffffffffu, acc[0][j], 2);
@@ -928,8 +933,10 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
 
     // ---- epilogue: rows of the MMA are output columns, columns of the MMA are batch rows ----
     const int g = lane >> 2, t = lane & 3;
-    // scratch of its own behind the ring (a slower warp may still read the ring): GQ_CONSUMER_WARPS x MT x 512 bytes
-    float4 *red = reinterpret_cast<float4 *>(reinterpret_cast<uint8_t *>(grid_s) + p.cb_bytes);
+    // scratch of its own behind the ring (a slower warp may still read the ring): GQ_CONSUMER_WARPS x MT x 512 bytes.  Of eight column tiles
+    // it would cost a resident CTA, and takes the ring's place once all four warps are through.
+    float4 *red = reinterpret_cast<float4 *>(gq_red_in_ring<MT>() ? smem : reinterpret_cast<uint8_t *>(grid_s) + p.cb_bytes);
+    if constexpr (gq_red_in_ring<MT>()) asm volatile("bar.sync 1, %0;" ::"n"(32 * GQ_CONSUMER_WARPS) : "memory");
     if (push) {
         cluster_wait();         // the rendezvous entered at the start: every CTA of the cluster is running
         // split-K inside a cluster, push form: the warps of splits 1.. store their accumulators into their slot of the split-0
@@ -1021,8 +1028,6 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
             }
         }
 }
-
-#include "gq_wide.cuh"
 
 // Y = sum over splits of the fp32 partials, rounded once to bf16 (reference: sum_partials,
 // gguf-plugin/gluon/tiles_grouped.py:142-162)
@@ -1307,21 +1312,19 @@ extern "C" int gq_split_for(int64_t n_tiles, int64_t nb, int64_t M, int avg_byte
     if (sm_count <= 0) sm_count = 148;
     // from sweeps on B200 (Q4_K / Q2_K / IQ3_S / IQ4_XS; 80- to 544-tile layers at K 5120 and 17408): the
     // largest split that (a) leaves a CTA at least three k-blocks, (b) stays inside one thread-block cluster (8), and
-    // (c) keeps the launch in one wave of the CTAs that the kernel for M rows has resident on an SM (four to 8 rows, three to 16;
-    // above, two of two tiles each) — counting that clusters cannot use every slot: a launch of clusters of S fills at most about
-    // 1 - 0.03 (S - 1) of them before a second wave starts.  (With four for every M, 80 tiles at K 5120 ran as 480 CTAs: Q4_K 14.2 us
-    // at 16 rows, with the split of this rule, 4, 10.4.  Above 16 rows, 27: 80 tiles as 6 / 7 parts 15.7 / 22.0 us, 112 tiles as
-    // 4 / 5 parts 20.0 / 29.2, 136 tiles as 3 / 4 parts 27.0 / 22.9, where clusters of 4 still fit at 0.92 of the slots.)
-    const bool wide = M > GQ_GEMV8_MAX_ROWS;
-    const int64_t per_sm = M <= 8 ? 4 : wide ? 2 : 3, slots = per_sm * sm_count, units = wide ? (n_tiles + 1) / 2 : n_tiles;
-    int64_t s_max = (wide ? nb + 1 : nb) / 3;       // 5120 x 4352, seventeen k-blocks, at 27 rows: 5 / 6 parts 15.4 / 13.0 us
+    // (c) keeps the launch in one wave of the CTAs that the kernel for M rows has resident on an SM (four to 8 rows, three to 16,
+    // two above) — counting that clusters cannot use every slot: a launch of clusters of S fills at most about 1 - 0.03 (S - 1)
+    // of them before a second wave starts.  (With four for every M, 80 tiles at K 5120 ran as 480 CTAs: Q4_K 14.2 us at 16 rows,
+    // with the split of this rule, 4, 10.4.)
+    const int64_t per_sm = M <= 8 ? 4 : M <= 16 ? 3 : 2, slots = per_sm * sm_count;
+    int64_t s_max = nb / 3;
     if (s_max > 8) s_max = 8;
     int64_t s = 1;
     for (int64_t c = 2; c <= s_max; ++c)
-        if (c * units * 100 <= slots * (wide && c == 4 ? 92 : 100 - 3 * (c - 1))) s = c;
+        if (c * n_tiles * 100 <= slots * (100 - 3 * (c - 1))) s = c;
     // 9 .. 16 rows, one CTA short of what an SM holds: two parts in a wave and a quarter are 13 - 20 % faster (272 tiles: Q4_K
     // 25.8 -> 22.4 us, IQ3_S 34.6 -> 28.0)
-    if (per_sm == 3 && s == 1 && s_max >= 2 && units * 3 < slots * 2) s = 2;
+    if (per_sm == 3 && s == 1 && s_max >= 2 && n_tiles * 3 < slots * 2) s = 2;
     if (s > nb) s = nb;
     return (int)s;
 }
@@ -1336,7 +1339,7 @@ static int launch_gemv(const GemvParams &p, int64_t n_desc, cudaStream_t stream)
     constexpr int xbytes = gq_stage_xbytes<MT, FORM>();
     const int stage_bytes = p.wbytes_max + xbytes;
     const size_t smem = (size_t)p.stages * stage_bytes + (size_t)p.stages * 16 + 8 * GQ_CONSUMER_WARPS + (size_t)p.cb_bytes +
-                        (size_t)GQ_CONSUMER_WARPS * MT * 512 * (p.cluster_push ? p.split - 1 : 1);
+                        (gq_red_in_ring<MT>() ? 0 : (size_t)GQ_CONSUMER_WARPS * MT * 512 * (p.cluster_push ? p.split - 1 : 1));
     if (smem > 232448) return GQ_ERR_LIMIT;
     // opt in once per device to the largest dynamic shared memory a CTA can have
     static std::atomic<unsigned long long> done_mask{0};
@@ -1414,52 +1417,35 @@ static int launch_prep(const __nv_bfloat16 *x, int64_t rows, int64_t K, int64_t 
 // an SM has 228 KB of shared memory, of which the system keeps 1 KB per resident CTA
 static int resident_ctas(int smem, int cap) { const int n = (228 * 1024) / (smem + 1024); return n < cap ? n : cap; }
 
-// integer form: up to GQ_GEMV8_MAX_ROWS rows
-static int launch_gemv8(GemvParams &p, int run_info, int64_t n_desc, cudaStream_t st) {
-    // CTAs an SM holds by their registers, and the deepest ring of three or four stages that leaves room for them (swept on the 64-layer
-    // stack: deeper rings with fewer resident CTAs were slower)
-    const int mt = p.M <= 8 ? 1 : 2, cap = mt == 1 ? 4 : 3;
-    const int stage_bytes = p.wbytes_max + (p.M <= 4 ? gq_stage_xbytes<1, 2>() : 8 * mt * GQ_X_ROW + 32 * mt), red1 = GQ_CONSUMER_WARPS * mt * 512;
-    const auto resident = [&](int stages, int red) { return resident_ctas(stages * stage_bytes + 64 + 8 * GQ_CONSUMER_WARPS + p.cb_bytes + red, cap); };
+// One tile to a CTA.  CTAs that an SM holds by their registers: four to 8 rows, three to 16, two above.  Rings: integer form, the deepest of
+// three or four stages that leaves room for those CTAs (swept on the 64-layer stack: deeper rings with fewer resident CTAs were slower);
+// fp16 form, whose activation tiles are larger, of two to four; where its launch fits one CTA per SM it takes four, beside which few types
+// leave room for a second CTA (two shared an SM while others stood idle: 640 x 17,408 at 27 rows, Q4_K 14.6 -> 10.5 us, IQ4_XS 17.4 -> 12.3).
+// The fp16 form with two tiles and eight consumer warps to a CTA (96 registers) was 4 - 9 % faster on 34,816 x 5,120 of Q2_K, Q4_K or Q8_0
+// and slower elsewhere: 5,120 x 5,120 at 17 rows Q4_K 10.5 -> 13.9, Q5_0 12.2 -> 16.4, 1,024 x 5,120 at 27 rows Q8_0 8.0 -> 13.4.
+static int launch_grouped(GemvParams &p, int run_info, int64_t n_desc, cudaStream_t st) {
+    const bool fp16 = p.M > GQ_GEMV8_MAX_ROWS;
+    const int mt = p.M <= 8 ? 1 : p.M <= 16 ? 2 : p.M <= 24 ? 3 : p.M <= 32 ? 4 : 8, low = fp16 ? 2 : 3;
+    const bool alone = fp16 && n_desc * 100 <= (int64_t)device_sms() * (100 - 3 * (p.split - 1));         // as gq_split_for counts the places for clusters
+    const int cap = alone ? 1 : mt == 1 ? 4 : mt == 2 ? 3 : 2;
+    const int stage_bytes = p.wbytes_max + (p.M <= 4 ? gq_stage_xbytes<1, 2>() : 8 * mt * GQ_X_ROW + 32 * mt), red1 = mt == 8 ? 0 : GQ_CONSUMER_WARPS * mt * 512;
+    const auto resident = [&](int stages, int red, int most) { return resident_ctas(stages * stage_bytes + 64 + 8 * GQ_CONSUMER_WARPS + p.cb_bytes + red, most); };
     // split-K in a cluster: the push form of the reduction needs a scratch slot per other split in every CTA; it is used when that
-    // costs no resident CTA at three stages
-    p.cluster_push = p.cluster && resident(3, red1 * (p.split - 1)) >= resident(3, red1) ? 1 : 0;
-    p.stages = resident(4, p.cluster_push ? red1 * (p.split - 1) : red1) >= cap ? 4 : 3;
-    if (mt == 2) return launch_gemv<2, 3, 1, 0>(p, n_desc, st);
-    return p.M <= 4 ? launch_gemv8_m8<2>(p, n_desc, st, (run_info >> 17) & 31) : launch_gemv8_m8<1>(p, n_desc, st, (run_info >> 17) & 31);
-}
-
-// fp16 form: up to GQ_WIDE_ROWS rows
-template <int MT>
-static int launch_wide_mt(GemvParams &p, int run_info, cudaStream_t st) {
-    // the deepest ring of two to four stages that costs no resident CTA
-    p.cb_stride = (run_info >> 17) & 31 ? 0 : p.cb_bytes;
-    const int stage_bytes = 2 * p.wbytes_max + gq_stage_xbytes<MT, 0>(), tables = p.cb_bytes + p.cb_stride, scratch = p.ar.world ? GQ_WIDE_WARPS * MT * 512 : 0;
-    const auto bytes = [&](int stages) { return stages * (stage_bytes + 16) + tables + scratch; };
-    p.stages = 2;
-    while (p.stages < 4 && resident_ctas(bytes(p.stages + 1), 2) >= resident_ctas(bytes(2), 2)) ++p.stages;
-    p.ar_at = p.stages * (stage_bytes + 16) + tables;
-    if (bytes(p.stages) > 232448) return GQ_ERR_LIMIT;
-    if (int rc = allow_smem<gemv_wide_kernel<MT>>(232448)) return rc;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[2];
-    int na = 0;
-    if (p.cluster) {
-        attr[na].id = cudaLaunchAttributeClusterDimension;
-        attr[na].val.clusterDim.x = (unsigned)p.split; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1;
-        ++na;
+    // costs no resident CTA at the shallowest ring
+    p.cluster_push = p.cluster && red1 && resident(low, red1 * (p.split - 1), cap) >= resident(low, red1, cap) ? 1 : 0;
+    const int red = p.cluster_push ? red1 * (p.split - 1) : red1;
+    if (fp16) {
+        for (p.stages = 2; p.stages < 4 && resident(p.stages + 1, red, cap) >= resident(2, red, cap);) ++p.stages;
+    } else {
+        p.stages = resident(4, red, cap) >= cap ? 4 : 3;
     }
-    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[na].val.programmaticStreamSerializationAllowed = 1;
-    ++na;
-    cfg.gridDim = dim3((unsigned)((p.n_tiles + 1) / 2 * p.split)); cfg.blockDim = dim3(32 * (GQ_WIDE_WARPS + 1)); cfg.dynamicSmemBytes = bytes(p.stages);
-    cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = na;
-    GQ_CUDA(cudaLaunchKernelEx(&cfg, gemv_wide_kernel<MT>, p));
-    GQ_LAUNCHED();
-    return GQ_OK;
-}
-static int launch_wide(GemvParams &p, int run_info, cudaStream_t st) {
-    return p.M <= 16 ? launch_wide_mt<2>(p, run_info, st) : p.M <= 24 ? launch_wide_mt<3>(p, run_info, st) : launch_wide_mt<4>(p, run_info, st);
+    switch (mt) {
+        case 1: return p.M <= 4 ? launch_gemv8_m8<2>(p, n_desc, st, (run_info >> 17) & 31) : launch_gemv8_m8<1>(p, n_desc, st, (run_info >> 17) & 31);
+        case 2: return launch_gemv<2, 3, 1, 0>(p, n_desc, st);
+        case 3: return launch_gemv<3, 2, 0, 0>(p, n_desc, st);
+        case 4: return launch_gemv<4, 2, 0, 0>(p, n_desc, st);
+        default: return launch_gemv<8, 2, 0, 0>(p, n_desc, st);
+    }
 }
 
 static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ldx, const void *packed_dev, const int32_t *desc_dev,
@@ -1477,7 +1463,7 @@ static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ld
     if (int rc = ensure_tables()) return rc;
     cudaStream_t st = (cudaStream_t)stream;
 
-    if (pre && pre->kind && M > GQ_WIDE_ROWS) return GQ_ERR_SHAPE;
+    if (pre && pre->kind && M > GQ_GEMV8_MAX_ROWS) return GQ_ERR_SHAPE;       // the folded ops exist in the integer form's preparation only
     const int maxb = run_info & 0xFFFF;
     if ((phases & 6) && (maxb < 56 || maxb > 272 || (maxb & 1))) return GQ_ERR_ARG;
     // split-K up to 8 reduces inside a thread-block cluster (portable cluster size); larger splits keep the fp32
@@ -1487,35 +1473,26 @@ static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ld
         if (split > 1 && !cluster) return GQ_ERR_ARG;        // the exchange needs the whole tile sum in one CTA
         if (n_desc / split * GQ_CONSUMER_WARPS > ar->units) return GQ_ERR_LIMIT;
     }
-    const bool wide = M > GQ_GEMV8_MAX_ROWS;
-    if (wide && n_desc % split) return GQ_ERR_ARG;            // a CTA of the fp16 form takes two tiles' rows of one part
     // Whether the grouped kernel converts the activations itself: one row, nothing folded in front, and at most four k-blocks to a
     // CTA, up to where the conversions, one after the other, take no longer than the boundary they save (graphs of 24 layers, Q4_K:
     // 5120 x 5120, 3.3 k-blocks, 6.8 -> 6.5 us; 7168 x 5120, 5 k-blocks, 7.4 -> 8.3; a second row adds 2 us)
     const bool direct = (phases & 8) && M == 1 && !ar && !(pre && pre->kind) && (K / GQ_QK + split - 1) / split <= 4;
 
-    GemvParams p;
-    p.packed = (const uint8_t *)packed_dev; p.desc = desc_dev; p.status = ws.status;
-    p.K = (int)K; p.nb = (int)(K / GQ_QK); p.split = split; p.ldy = ldy; p.n_total = n_total;
-    p.wbytes_max = 64 * maxb;   // every stage can hold a tile of any shard of the run
-    p.cb_bytes = gq_cb_region_max((run_info >> 22) & 63);
-    p.cluster = cluster; p.cluster_push = 0;
-    p.x = direct ? (const __nv_bfloat16 *)x_dev : nullptr;
-    p.n_tiles = (int)(n_desc / split); p.part_rows = (int)M;
-    p.ar = ar ? *ar : ArFused{};
-    // the batch rows at a time that the kernel takes: all of them, except for the fp16 form of more than GQ_WIDE_ROWS
-    for (int64_t r0 = 0; r0 < M; r0 += GQ_WIDE_ROWS) {
-        const int64_t rows = M - r0 < GQ_WIDE_ROWS ? M - r0 : GQ_WIDE_ROWS;
-        const __nv_bfloat16 *x = (const __nv_bfloat16 *)x_dev + r0 * ldx;
-        p.M = (int)rows;
-        p.xt = ws.xt + (r0 ? p.nb * gq_x_bytes(r0) : 0);
-        p.y = (__nv_bfloat16 *)y_dev + r0 * ldy; p.partials = ws.partials + r0 * n_total;
-        if ((phases & 1) && !direct)
-            if (int rc = launch_prep(x, rows, K, ldx, const_cast<uint8_t *>(p.xt), r0 ? nullptr : ws.status, wide ? 0 : 1, pre, st)) return rc;
-        if (!(phases & 2)) continue;
-        p.pf_ptr = (r0 + rows == M && next_packed_dev && next_bytes > 0 && !((uintptr_t)next_packed_dev & 15)) ? (const uint8_t *)next_packed_dev : nullptr;
+    if ((phases & 1) && !direct)
+        if (int rc = launch_prep((const __nv_bfloat16 *)x_dev, M, K, ldx, ws.xt, ws.status, M > GQ_GEMV8_MAX_ROWS ? 0 : 1, pre, st)) return rc;
+    if (phases & 2) {
+        GemvParams p;
+        p.packed = (const uint8_t *)packed_dev; p.desc = desc_dev; p.xt = ws.xt;
+        p.y = (__nv_bfloat16 *)y_dev; p.partials = ws.partials; p.status = ws.status;
+        p.M = (int)M; p.K = (int)K; p.nb = (int)(K / GQ_QK); p.split = split; p.ldy = ldy; p.n_total = n_total;
+        p.wbytes_max = 64 * maxb;   // every stage can hold a tile of any shard of the run
+        p.cb_bytes = gq_cb_region_max((run_info >> 22) & 63);
+        p.cluster = cluster;
+        p.x = direct ? (const __nv_bfloat16 *)x_dev : nullptr;
+        p.pf_ptr = (next_packed_dev && next_bytes > 0 && !((uintptr_t)next_packed_dev & 15)) ? (const uint8_t *)next_packed_dev : nullptr;
         p.pf_bytes = next_bytes;
-        if (int rc = wide ? launch_wide(p, run_info, st) : launch_gemv8(p, run_info, n_desc, st)) return rc;
+        p.ar = ar ? *ar : ArFused{};
+        if (int rc = launch_grouped(p, run_info, n_desc, st)) return rc;
     }
     if (split > 1 && !cluster && (phases & 4)) {
         const int64_t n = M * n_total;

@@ -118,7 +118,8 @@ int64_t gq_workspace_bytes(int64_t M, int64_t K, int64_t n_total, int split);
 
 /* Y[M, n_total] = X[M, K] . W^T for a run of packed shards, 1 <= M <= GQ_MAX_GEMV_ROWS.
  *   x_dev     bf16 [M, K], row stride ldx elements
- *   packed_dev, desc_dev, n_desc, split   the run's tiles and the descriptor table built for `split`
+ *   packed_dev, desc_dev, n_desc, split   the run's tiles and the descriptor table built for `split`: each row stands for itself, except
+ *             that for a split of 2..8 and a multiple of it as n_desc every `split` rows in turn are the parts of one tile
  *   run_info  gq_run_info of the run's types
  *   y_dev     bf16, row stride ldy elements; the run writes columns [0, n_total)
  *   workspace_dev  at least gq_workspace_bytes(M, K, n_total, split) bytes, 256-byte aligned
@@ -262,8 +263,9 @@ int gq_gemm_prefill(const void *x_dev, int64_t M, int64_t K, int64_t ldx, const 
 
 /* Reads the device status word of the last call on this workspace (synchronises the stream): 0, or
  * a positive GQ_DEV_* code (1: a bounded wait ran out; 2: a shape or a tile's type contradicts the call's arguments —
- * an odd column count in the fused all-reduce, a tile that is not of the single type run_info names, a codebook type run_info
- * does not announce; the CTA concerned computed nothing). */
+ * an odd column count in the fused all-reduce, or a tile of a type that run_info leaves out and for which the call has no kernel (up to
+ * 8 rows: not the single type run_info names), no table (a codebook type) or, above 16 rows, no room (more bytes than the widest type
+ * announced); the CTA concerned computed nothing.  Any other tile is multiplied as what its table row says). */
 int gq_read_status(const void *workspace_dev, int64_t workspace_bytes, void *stream);
 
 /* The largest device status code any kernel of this library has reported on the current device since the word was

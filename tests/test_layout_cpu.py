@@ -93,6 +93,16 @@ def test_split_policy_on_the_decoder_shapes(gq_lib):
     assert got == {"q": 6, "qkv": 4, "gate": 2, "gate_up": 1, "down": 6, "kv": 6}
 
 
+@pytest.mark.parametrize("m, per_sm", [(17, 2), (27, 2), (32, 2), (48, 2), (64, 2)])
+def test_split_policy_above_16_rows_is_one_rule_for_all_sizes(gq_lib, m, per_sm):
+    """Two CTAs per SM: the largest split up to 8 whose parts all have three k-blocks and whose clusters, of which S fill 1 - 0.03 (S - 1)
+    of the places, fit one wave.  No number of tiles or k-blocks is an exception."""
+    for nb in (1, 3, 5, 6, 8, 14, 16, 17, 18, 20, 24, 68):
+        for n_tiles in range(1, 700):
+            fits = [s for s in range(2, 9) if nb // s >= 3 and 100 * s * n_tiles <= per_sm * 148 * (100 - 3 * (s - 1))]
+            assert gq_lib.gq_split_for(n_tiles, nb, m, 144, 148) == max(fits, default=1), (n_tiles, nb)
+
+
 def test_a_run_is_prepared_for_any_row_counts():
     """The tables of exactly the splits that these row counts choose, and split 1; a count above the grouped kernel's limit is
     answered like the largest it takes."""
