@@ -140,7 +140,13 @@ __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&v)[
                  : "r"(taddr)
                  : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// the registers of a load in flight pass through its wait, so that nothing reads, copies or merges them before it
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&v)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])
+                 :
+                 : "memory");
+}
 
 // ---- k-slice J (runs 4J .. 4J+3) of one slab: decode, scale -> fp16 weights as the registers of one 16x256b.x4 store --------
 template <int TYPE, int J>
@@ -444,7 +450,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
                 const float4 e0 = *reinterpret_cast<const float4 *>(s_ex + c), e1 = *reinterpret_cast<const float4 *>(s_ex + c + 4);
                 const float es[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
                 float v[8];
-                tmem_wait_ld();
+                tmem_wait_ld(a);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(a[j]) * es[j];
                 pf_store8(p, v, mt * N + c, col, row_ok, pair_ok, lane);
@@ -458,16 +464,15 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
         cluster_sync_all();                 // every CTA of the cluster has finished with its rings
         if (warp < DEQ) {
             const uint32_t mine = smem_u32(buf) + (uint32_t)(part * (ch >> 2) * 128 + feat) * 16;
-            uint32_t a[8];
-            if (8 * e < N) tmem_ld_32x32b_x8(td + 8 * e, a);
 #pragma unroll 1
             for (int c = 8 * e; c < N; c += 8 * (DEQ / 4)) {
+                uint32_t a[8];
+                tmem_ld_32x32b_x8(td + c, a);
                 const int r = c / ch;
                 const uint32_t dst = map_to_rank(mine, (uint32_t)(r * CG + half)) + (uint32_t)((c - r * ch) >> 2) * 2048;
-                tmem_wait_ld();
+                tmem_wait_ld(a);
                 st_cluster_f4(dst, __uint_as_float(a[0]), __uint_as_float(a[1]), __uint_as_float(a[2]), __uint_as_float(a[3]));
                 st_cluster_f4(dst + 2048, __uint_as_float(a[4]), __uint_as_float(a[5]), __uint_as_float(a[6]), __uint_as_float(a[7]));
-                if (c + 8 * (DEQ / 4) < N) tmem_ld_32x32b_x8(td + c + 8 * (DEQ / 4), a);
             }
             __syncwarp();
         }
