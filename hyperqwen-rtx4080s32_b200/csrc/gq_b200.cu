@@ -1830,22 +1830,9 @@ extern "C" int64_t gq_prefill_workspace_bytes(int64_t M, int64_t K, int64_t n_to
     return pf_ws_layout(K, prefill_plan(n_desc, M, K / GQ_QK, device_sms()), nullptr, nullptr, nullptr, nullptr);
 }
 
-template <int SETS, bool WIDE>
-static int launch_prefill(PrefillParams &p, const PrefillPlan &pl, int maxb, cudaStream_t st) {
-    const int total = SETS == 1 ? GQ_PF_SMEM_1 : GQ_PF_SMEM_2, tables = gq_cb_region_sum(p.cb_mask), bbytes = pl.N * 128 / SETS;
-    p.wstage_bytes = 128 * maxb;
-    // the activation ring takes four slices (one k-block), the weight ring the rest; a run whose widest type leaves no two
-    // weight stages beside them takes activation stages away, down to two
-    int left = total - 1024 - tables;
-    p.bstages = 4;
-    while (p.bstages > 2 && (left - p.bstages * bbytes) / p.wstage_bytes < 2) --p.bstages;
-    p.wstages = (left - p.bstages * bbytes) / p.wstage_bytes;
-    if (p.wstages > GQ_PF_MAX_STAGES) p.wstages = GQ_PF_MAX_STAGES;
-    p.wstages -= p.wstages % SETS;        // each set walks stages of its own
-    if (p.wstages < 1 || p.bstages < (SETS == 1 ? GQ_PF_SL1 : GQ_PF_SL2)) return GQ_ERR_LIMIT;
-    left -= p.wstages * p.wstage_bytes + p.bstages * bbytes;
-    while (p.bstages < GQ_PF_SLOTS * (WIDE ? 1 : SETS) && left >= bbytes) { ++p.bstages; left -= bbytes; }
-    if (int rc = allow_smem<gemm_prefill_kernel<SETS, WIDE>>(total)) return rc;
+template <int SETS, bool WIDE, int SL>
+static int launch_prefill_kernel(PrefillParams &p, const PrefillPlan &pl, int smem, cudaStream_t st) {
+    if (int rc = allow_smem<gemm_prefill_kernel<SETS, WIDE, SL>>(smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     int na = 0;
@@ -1857,16 +1844,37 @@ static int launch_prefill(PrefillParams &p, const PrefillPlan &pl, int maxb, cud
     attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
-    cfg.blockDim = dim3(32 * (8 * SETS + 3)); cfg.dynamicSmemBytes = (size_t)total; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = na;
+    cfg.blockDim = dim3(32 * (8 * SETS + 3)); cfg.dynamicSmemBytes = (size_t)smem; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = na;
     // a grid has room for 65,535 units (8.4 or 16.8 million output columns): a run of more takes several launches
     const int64_t n_desc = p.n_desc, step = (int64_t)65535 * 2 * SETS;
     for (int64_t d = 0; d < n_desc; d += step, p.desc += step * GQ_DESC_WORDS) {
         p.n_desc = (int)(n_desc - d < step ? n_desc - d : step);
         cfg.gridDim = dim3((unsigned)(pl.split * SETS), (unsigned)(prefill_ctas(p.n_desc, pl) / SETS), (unsigned)pl.tiles);
-        GQ_CUDA(cudaLaunchKernelEx(&cfg, gemm_prefill_kernel<SETS, WIDE>, p));
+        GQ_CUDA(cudaLaunchKernelEx(&cfg, gemm_prefill_kernel<SETS, WIDE, SL>, p));
         GQ_LAUNCHED();
     }
     return GQ_OK;
+}
+
+template <int SETS, bool WIDE>
+static int launch_prefill(PrefillParams &p, const PrefillPlan &pl, int maxb, int only, cudaStream_t st) {
+    const int total = SETS == 1 ? GQ_PF_SMEM_1 : GQ_PF_SMEM_2, tables = gq_cb_region_sum(p.cb_mask), bbytes = pl.N * 128 / SETS;
+    p.wstage_bytes = 128 * maxb;
+    // the activation ring takes four slices (one k-block), the weight ring the rest; a run whose widest type leaves no two
+    // weight stages beside them takes activation stages away, down to two
+    int left = total - 1024 - tables;
+    p.bstages = 4;
+    while (p.bstages > 2 && (left - p.bstages * bbytes) / p.wstage_bytes < 2) --p.bstages;
+    p.wstages = (left - p.bstages * bbytes) / p.wstage_bytes;
+    if (p.wstages > GQ_PF_MAX_STAGES) p.wstages = GQ_PF_MAX_STAGES;
+    p.wstages -= p.wstages % SETS;        // each set walks stages of its own
+    if (p.wstages < 1) return GQ_ERR_LIMIT;
+    left -= p.wstages * p.wstage_bytes + p.bstages * bbytes;
+    while (p.bstages < GQ_PF_SLOTS * (WIDE ? 1 : SETS) && left >= bbytes) { ++p.bstages; left -= bbytes; }
+    if constexpr (SETS == 1) {
+        if ((p.bstages == GQ_PF_SLOTS || p.cb_mask) && !(only == GQ_Q4_0 && pl.N > 64)) return launch_prefill_kernel<SETS, WIDE, 2>(p, pl, total, st);
+    }
+    return launch_prefill_kernel<SETS, WIDE, 1>(p, pl, total, st);
 }
 
 extern "C" int gq_gemm_prefill(const void *x_dev, int64_t M, int64_t K, int64_t ldx, const void *packed_dev, const int32_t *desc_dev,
@@ -1911,8 +1919,9 @@ extern "C" int gq_gemm_prefill(const void *x_dev, int64_t M, int64_t K, int64_t 
         GQ_CUDA(cudaLaunchKernelEx(&cfg, prep_x_prefill_kernel, (const __nv_bfloat16 *)x_dev, ldx, (int)K, (int)M, pl.N, pl.sets == 1 ? 0 : pl.wide ? pl.N / 2 : pl.N, ex, xp, status));
         GQ_LAUNCHED();
     }
-    if (pl.wide) return launch_prefill<2, true>(p, pl, maxb, st);
-    return pl.sets == 1 ? launch_prefill<1, false>(p, pl, maxb, st) : launch_prefill<2, false>(p, pl, maxb, st);
+    const int only = (run_info >> 17) & 31;
+    if (pl.wide) return launch_prefill<2, true>(p, pl, maxb, only, st);
+    return pl.sets == 1 ? launch_prefill<1, false>(p, pl, maxb, only, st) : launch_prefill<2, false>(p, pl, maxb, only, st);
 }
 
 extern "C" int gq_device_status(int clear, void *stream) {

@@ -37,12 +37,13 @@
 namespace gq {
 
 #define GQ_PF_SLOTS 4                        // A slots of a ring: the four 64-wide k-slices of a k-block
-// k-slices that share a barrier (a dequantiser's wait, store and announcement; the MMA issuer's wait and commit).  Up to 128 batch rows the
-// MMAs of a slice are short beside its decoding and the hand-over counts: two a barrier, 34,816 x 5,120 at 64 rows, one / two / four, Q4_K
-// 41.3 / 38.0 / 44.6 us, IQ3_S 59.0 / 55.4 / 56.5, Q2_K 43.9 / 39.9 / 45.4.  Above, the MMAs have to follow the slices closely: Q4_K at 517
-// rows, one / two, 153 / 173 us.
-#define GQ_PF_SL1 2
-#define GQ_PF_SL2 1
+// k-slices that share a barrier (a dequantiser's wait, store and announcement; the MMA issuer's wait and commit): SL.  Up to 128 batch rows
+// (SETS = 1) the MMAs of a slice are short beside its decoding and the hand-over counts: two a barrier, 34,816 x 5,120 at 64 rows, one / two /
+// four, Q4_K 41.3 / 38.0 / 44.6 us, IQ3_S 59.0 / 55.4 / 56.5, Q2_K 43.9 / 39.9 / 45.4.  Above, the MMAs have to follow the slices closely: Q4_K
+// at 517 rows, one / two, 153 / 173 us.  Two also need an activation ring of the whole k-block, or the copies of a pair wait for the MMAs of
+// the pair before (Q8_0 at 96 to 128 rows, Q6_K at 128): 34,816 x 5,120 at 128 rows, one / two, Q8_0 58.9 / 71.1 us, 1,024 x 5,120 at 112 rows
+// 13.2 / 15.3 — except in a run with a codebook type, whose decoding takes longer still (Q8_0 beside IQ2_S at 112 rows 76.3 / 68.9).  And Q4_0,
+// which has the least to decode, hands over singly beyond 64 rows: 1,024 x 5,120 at 128 rows 13.1 / 13.8 us.
 #define GQ_PF_MAX_STAGES 6                   // upper bound of the weight ring
 
 struct PrefillParams {
@@ -242,7 +243,7 @@ __device__ __forceinline__ void pf_store8(const PrefillParams &p, const float (&
     }
 }
 
-template <int SETS, bool WIDE>
+template <int SETS, bool WIDE, int SL>
 __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_prefill_kernel(const __grid_constant__ PrefillParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // layout: [activation ring][weight ring][codebook tables of the run's types]; the reduction of a split reuses the rings
@@ -253,7 +254,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
     const int N = p.N, bbytes = N * 128 / SETS;          // a CTA of a pair holds half of the batch rows of a slice
     uint8_t *wring = smem + p.bstages * bbytes;
     uint8_t *tables = wring + p.wstages * p.wstage_bytes;
-    constexpr int RINGS = WIDE ? 1 : SETS, CG = SETS, SL = SETS == 1 ? GQ_PF_SL1 : GQ_PF_SL2, GROUPS = GQ_PF_SLOTS / SL;
+    constexpr int RINGS = WIDE ? 1 : SETS, CG = SETS, GROUPS = GQ_PF_SLOTS / SL;
     uint64_t *wfull = bars, *wfree = bars + GQ_PF_MAX_STAGES;
     uint64_t *afull = bars + 2 * GQ_PF_MAX_STAGES, *afree = afull + GROUPS * RINGS, *done = afree + GROUPS * SETS;
     constexpr uint32_t TMEM_COLS = 256u * SETS, D_COLS = TMEM_COLS - 32u * GQ_PF_SLOTS * RINGS;      // the A slots follow the accumulator

@@ -78,3 +78,22 @@ def test_every_shape_with_ragged_pairs_and_mixed_types(size, plan):
     ops.prefill_gemm(x, packed, d1, n, out=wide[:, 3:3 + n], wtypes=types)
     assert torch.equal(wide[:, 3:3 + n], y) and bool(torch.isnan(wide[:, :3]).all()) and bool(torch.isnan(wide[:, 3 + n:]).all())
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("types", [[F.Q8_0], [F.Q6_K], [F.Q4_0], [F.Q4_0, F.Q2_K], [F.Q8_0, F.IQ2_S], [F.IQ1_M, F.Q8_0]])
+@pytest.mark.parametrize("m", [64, 65, 80, 96, 112, 113, 128])
+def test_slices_handed_over_singly_and_in_pairs(types, m):
+    """Up to 128 rows two k-slices share a barrier where the activation ring holds a k-block or a codebook type decodes slowly; else each has
+    its own: rings of two, three and four slices, both ways.  A row's result does not depend on the batch around it, so calls of 16 rows,
+    which cut the rings otherwise, agree to the bit."""
+    k, n_outs = 2304, [134, 100][:len(types)]
+    raws = [synth.random_blocks(n, k, t, seed=n + t) for n, t in zip(n_outs, types)]
+    packed = torch.cat([ops.repack_tiles(r.cuda(), n, t).reshape(-1) for r, n, t in zip(raws, n_outs, types)])
+    d1, n = torch.from_numpy(ops.build_descs(types, n_outs, k, 1)).cuda(), sum(n_outs)
+    x = synth.activations(m, k, device="cuda")
+    y = ops.prefill_gemm(x, packed, d1, n, wtypes=types)
+    ref = np.concatenate([oracle.matmul_f64(x.float().cpu().numpy(), r.numpy(), t) for r, t in zip(raws, types)], axis=1)
+    assert oracle.rel_err(y.float().cpu().numpy(), ref) < TOL
+    if ops.prefill_plan(m, k, 3 + len(types) * 2 - 2)["split"] == ops.prefill_plan(16, k, 3 + len(types) * 2 - 2)["split"]:
+        assert torch.equal(torch.cat([ops.prefill_gemm(x[i:i + 16], packed, d1, n, wtypes=types) for i in range(0, m, 16)]), y)
+    assert ops.device_status() == 0
