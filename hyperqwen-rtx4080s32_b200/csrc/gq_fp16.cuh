@@ -4,9 +4,13 @@
 #pragma once
 #include "gq_scale16.cuh"
 
-// pairs of runs whose MMAs follow one another in one accumulator before it is added in fp32
+// Pairs of runs whose MMAs follow one another in one accumulator before it is added in fp32: the tensor core truncates where an fp32 add rounds,
+// so a chain over the whole k-block (eight pairs) left the codebook types with two to three times the error of a form that adds up each
+// scale group's sum in fp32 (rms over the norm of the products, N(0, 1) activations: IQ2_S 1.85e-7 against 7.6e-8, by pairs 7.3e-8; IQ3_S 1.4e-7
+// against 6.3e-8, 6.7e-8).  The types with a minimum or an offset lose far more in that form (Q4_K 6.8e-6, with the fold 1.4e-7) and keep the
+// long chain.  Whole calls at 27 rows, eight pairs / one: 34,816 x 5,120 IQ3_S 56 / 60 us, IQ2_XS 64 / 65.
 template <int TYPE>
-constexpr int gq_fold_chain() { return 8; }
+constexpr int gq_fold_chain() { return gq_cb_kind(TYPE) >= 0 ? 1 : 8; }
 
 // One k-block of one slab:  acc += sx[n] * ( d[row] * sum_runs(scale * (W_int . x)) - f[row] * (A'' . run sums) ).
 // Types whose field x scale is an exact fp16 integer (gq_folds) enter the MMA with the scale multiplied in, and the MMAs of a k-block
@@ -85,10 +89,13 @@ __device__ __forceinline__ void slab_kblock(const uint8_t *slab, const uint8_t *
 #pragma unroll
     for (int nt = 0; nt < MT; ++nt) {
         const float2 sx = *reinterpret_cast<const float2 *>(xs + xs_off + (nt * 8 + 2 * t) * 4);
-        float tot[4];
+        if constexpr (C0 == NC) {           // sx is a power of two: d * sx is exact
 #pragma unroll
-        for (int j = 0; j < 4; ++j) tot[j] = d[j >> 1] * blk[nt][j];
-        if constexpr (C0 < NC) {
+            for (int j = 0; j < 4; ++j) acc[nt][j] = fmaf(d[j >> 1] * (j & 1 ? sx.y : sx.x), blk[nt][j], acc[nt][j]);
+        } else {
+            float tot[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) tot[j] = d[j >> 1] * blk[nt][j];
             const uint4 b = ld16(xs + (nt * 8 + g) * GQ_X_ROW + GQ_X_SUMS + 16 * t);
 #pragma unroll
             for (int c = C0; c < NC; ++c) {
@@ -98,9 +105,9 @@ __device__ __forceinline__ void slab_kblock(const uint8_t *slab, const uint8_t *
 #pragma unroll
                 for (int j = 0; j < 4; ++j) tot[j] = fmaf(-fc[c][j >> 1], mm[j], tot[j]);
             }
-        }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[nt][j] = fmaf(j & 1 ? sx.y : sx.x, tot[j], acc[nt][j]);
+            for (int j = 0; j < 4; ++j) acc[nt][j] = fmaf(j & 1 ? sx.y : sx.x, tot[j], acc[nt][j]);
+        }
     }
 }
 

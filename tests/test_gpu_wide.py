@@ -102,3 +102,24 @@ def test_a_table_stands_for_itself(m):
             ref = ops.grouped_gemm(xx, packed, table, split, types, n)[:, cols].double()
             assert float((y[:, cols].double() - ref).norm() / ref.norm()) < 4e-3       # bf16 of the same sums in another order
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("t", [F.IQ3_S, F.IQ3_XXS, F.IQ2_XXS, F.IQ2_XS, F.IQ2_S, F.IQ1_M])
+@pytest.mark.parametrize("m", [17, 32, 64])
+def test_fp32_sums_of_the_codebook_types(t, m):
+    """The sums of one k-block before any rounding to bf16 (a split of one k-block a part, not summed up): eight pair sums are added in fp32 and
+    scaled, eight roundings of at most 2^-24 of a value no larger than about the 2-norm of the products, evenly spread: rms 2^-24 (8 / 3)^0.5."""
+    n, k = 256, 2560
+    raw = synth.random_blocks(n, k, t, seed=t, device="cuda")
+    tiles = ops.repack_tiles(raw, n, t)
+    w = ops.dequantize_tiles(tiles, n, k, t).double()
+    x = synth.activations(m, k, device="cuda")
+    s = k // 256
+    d = torch.from_numpy(ops.build_descs([t], [n], k, s)).cuda()
+    ws = torch.zeros(ops.lib().gq_workspace_bytes(m, k, n, s), dtype=torch.uint8, device="cuda")
+    ops.grouped_gemm(x, tiles.reshape(-1), d, s, [t], n, workspace=ws, phases=3)
+    parts = ws[-(s * m * n * 4):].view(torch.float32).view(s, m, n).double()         # a multiple of 256 bytes at the end
+    xs, wk = x.double().view(m, s, 256).transpose(0, 1), w.view(n, s, 256).permute(1, 2, 0)
+    err = (parts - xs @ wk) / ((xs ** 2) @ (wk ** 2)).sqrt()
+    assert float(err.square().mean().sqrt()) < 2.0 ** -24 * (8 / 3) ** 0.5
+    assert ops.device_status() == 0
