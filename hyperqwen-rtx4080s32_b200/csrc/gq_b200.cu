@@ -1806,6 +1806,21 @@ static PrefillPlan prefill_plan(int64_t n_desc, int64_t M, int64_t nb, int sms) 
     return best;
 }
 
+// CTAs to a row of the activation preparation (prep_x_prefill_kernel; `rows` of the padded batch): as many as hold it, up to four of them per
+// SM in all, and two while the GPU holds twice the rows (nine CTAs per SM; short of the last of them unless a row fills three).  One up to
+// 8,192 activations, where a cluster costs more than the second reading of what one CTA does not keep, unless all of them get an SM of
+// their own.  Whole calls with 1 / 2 / 3 / 4 CTAs: 5,120 x 17,408 at 64 rows 32.3 / 30.2 / 29.4 / 29.0 us, at 384 71.1 / 66.5 / 66.7 / 66.9,
+// at 600 113.3 / 109.3; 2,048 x 17,408 at 384 57.8 / 55.9 / 58.4; 2,048 x 8,704 at 600 54.4 / 57.4; 5,120 x 6,144 at 160 18.9 / 20.5;
+// 2,048 x 7,680 at 64 15.5 / 13.5, at 128 17.4 / 19.5.
+static int prefill_prep_parts(int64_t K, int64_t rows, int sms) {
+    const int64_t per = GQ_PF_PREP_THREADS * GQ_PF_PREP_VECS * 8;
+    if (K < 8192 && !(K >= per + per / 2 && 2 * rows <= sms)) return 1;
+    int64_t parts = 4 * (int64_t)sms / rows;
+    if (parts < 2) parts = 2 * rows <= (int64_t)sms * (K >= 3 * per ? GQ_PF_PREP_CTAS : GQ_PF_PREP_CTAS - 1) ? 2 : 1;
+    if (parts > (K + per - 1) / per) parts = (K + per - 1) / per;
+    return (int)(parts > 8 ? 8 : parts);
+}
+
 static int64_t pf_ws_layout(int64_t K, const PrefillPlan &pl, void *base, int **status, float **ex, uint8_t **xp) {
     const int64_t rows = (int64_t)pl.tiles * pl.N;
     int64_t off = 256;
@@ -1908,10 +1923,7 @@ extern "C" int gq_gemm_prefill(const void *x_dev, int64_t M, int64_t K, int64_t 
         cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
-        int64_t parts = (K / 8 + GQ_PF_PREP_THREADS * GQ_PF_PREP_VECS - 1) / (GQ_PF_PREP_THREADS * GQ_PF_PREP_VECS);
-        const int64_t fill = (int64_t)device_sms() * 10 / (pl.tiles * pl.N);       // beyond what the GPU holds of these CTAs there is no latency left to hide
-        if (parts > fill) parts = fill > 1 ? fill : 1;
-        if (parts > 8) parts = 8;
+        const int parts = prefill_prep_parts(K, (int64_t)pl.tiles * pl.N, device_sms());
         attr[1].id = cudaLaunchAttributeClusterDimension;
         attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = (unsigned)parts; attr[1].val.clusterDim.z = 1;
         cfg.gridDim = dim3((unsigned)(pl.tiles * pl.N), (unsigned)parts); cfg.blockDim = dim3(GQ_PF_PREP_THREADS); cfg.stream = st; cfg.attrs = attr;

@@ -528,15 +528,16 @@ __device__ __forceinline__ float amax8(const uint4 &v) {
 // MMA's shared-memory layout (tiles of N rows x 64 k, K-major, 16-byte chunks XOR-swizzled by row % 8) so the
 // kernel's producer moves a whole k-slice with one bulk copy.  For CTA pairs a slice holds the rows of the first CTA, then
 // those of the second: of every `nmma` rows that an MMA takes, the first half is the first CTA's.  The row is read once and kept in
-// registers between the maximum and the conversion: 5120 activations to a CTA of 128 threads, longer rows over a cluster of up to eight
-// CTAs, which exchange their maxima (what eight do not hold is read twice).  128 threads of few
+// registers between the maximum and the conversion: 5120 activations to a CTA of 128 threads, long rows over a cluster of up to eight CTAs
+// (prefill_prep_parts), which exchange their maxima (what they do not hold is read twice).  128 threads of few
 // registers, so that these CTAs fit beside those of a matrix kernel: they are in place when the kernel in front ends, and the
 // matrix kernel behind them gets its SMs, fetches weights and decodes while they run (with 512 threads a CTA kept it off its SM).
 // Bound by the latency of its loads and, beyond a few hundred rows, by how many of these CTAs an SM holds: rows of 17,408 in one CTA each
 // took 6 us at 64 rows and 17 at 517, a sixth of the layer.
 #define GQ_PF_PREP_THREADS 128
 #define GQ_PF_PREP_VECS 5
-__global__ void __launch_bounds__(GQ_PF_PREP_THREADS, 9) prep_x_prefill_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int K, int M, int N, int nmma,
+#define GQ_PF_PREP_CTAS 9        // of them that an SM holds
+__global__ void __launch_bounds__(GQ_PF_PREP_THREADS, GQ_PF_PREP_CTAS) prep_x_prefill_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int K, int M, int N, int nmma,
                                                                             float *__restrict__ ex, uint8_t *__restrict__ xp, int *status) {
     __shared__ float red[GQ_PF_PREP_THREADS / 32], peers[8];
     const int part = blockIdx.y, parts = gridDim.y, m = blockIdx.x, n = m % N, nvec = K >> 3, hn = nmma >> 1;

@@ -1,5 +1,5 @@
 """The activation preparation of the tcgen05 path where a row is longer than one CTA keeps in registers: spread over a cluster of two to
-eight CTAs at few rows, read twice at many rows or beyond eight CTAs."""
+eight CTAs at few rows, read twice at many rows, beyond eight CTAs or below 8,192 activations."""
 import pytest
 import torch
 
@@ -13,8 +13,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("k", [5120, 5376, 10496, 17408, 41216])
 @pytest.mark.parametrize("m", [33, 100, 400, 1500])
 def test_a_rows_scale_covers_all_of_it(m, k):
-    """The largest magnitude of a row sits in its first, a middle or its last chunk; the others are 2^-6 of it, which a scale taken from
-    a part of the row would carry out of fp16's range or, unscaled, below its precision.  Also a row of zeros, rows at both ends of bf16's range and a NaN.
+    """The largest magnitude of a row sits in its first, a middle or its last chunk; the others are about 2^-12 of it (2^-6 beside
+    64), which a scale taken from a part of the row would carry out of fp16's range or, unscaled, below its precision.  Also a row of zeros, rows at both ends of bf16's range and a NaN.
     Weights are rounded to fp16 (2^-11 each), activations exact: 3e-3 of the norm is five times what K of them leave."""
     n, t = 70, F.Q4_0
     raw = synth.random_blocks(n, k, t, seed=k)
@@ -37,3 +37,9 @@ def test_a_rows_scale_covers_all_of_it(m, k):
         err = (y[rows] - exact[rows]).abs() - exact[rows].abs() * 2.0 ** -8
         assert float((err / norm[rows].clamp_min(1e-300)).max()) < 3e-3
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("m, k", [(64, 7680), (80, 7680), (33, 8192), (148, 8192), (300, 10496), (480, 8704), (592, 8704), (600, 8704), (480, 17408), (600, 17408), (672, 17408)])
+def test_where_the_ctas_of_a_row_change(m, k):
+    """Row counts on both sides of each step of the rule that picks them."""
+    test_a_rows_scale_covers_all_of_it(m, k)
