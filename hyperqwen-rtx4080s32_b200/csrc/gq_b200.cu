@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(32 * GQ_PREP_WARPS) prep_x_kernel(const __nv_b
     const int m = blockIdx.y * GQ_PREP_WARPS + (threadIdx.x >> 5);
     pdl_trigger();    // the grouped kernel behind this one may start fetching weights
     pdl_wait();       // whatever ran before (possibly still reading this workspace) has finished
-    if (status && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status = 0;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status = 0;
     if (m >= M) return;
     const __nv_bfloat16 *xr = x + (int64_t)m * ldx + (int64_t)kb * GQ_QK + 8 * lane;
     float v[8];
@@ -309,14 +309,13 @@ __global__ void __launch_bounds__(32 * GQ_PREP_WARPS) prep_x_kernel(const __nv_b
 
 // RMSNorm (with the residual add) in front of the layer: grid (batch rows, k-blocks / 8).  Every CTA sums the squares of
 // its whole row (a few KB from L2), then each warp converts one k-block.
-template <int FORM>
 __global__ void __launch_bounds__(32 * GQ_PREP_WARPS) prep_x_norm_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int M, uint8_t *__restrict__ xt,
                                                                            int *status, const PreOp pre) {
     __shared__ float red[GQ_PREP_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, m = blockIdx.x;
     pdl_trigger();
     pdl_wait();
-    if (status && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status = 0;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status = 0;
     const __nv_bfloat16 *row = x + (int64_t)m * ldx;
     const __nv_bfloat16 *res = pre.residual ? pre.residual + (int64_t)m * pre.ld_res : nullptr;
     float ss = 0.0f;
@@ -366,7 +365,7 @@ __global__ void __launch_bounds__(32 * GQ_PREP_WARPS) prep_x_norm_kernel(const _
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = bf16_round(bf16_round(v[j] * rs) * w[j]);
-        prep_store<FORM>(v, kb, m, M, xt, lane);
+        prep8_store(v, kb, m, M, xt, lane);
     }
 }
 
@@ -1393,7 +1392,8 @@ extern "C" int gq_run_info(int n_shards, const int32_t *types) {
     return maxb | ((cb ? 1 : 0) << 16) | (single << 17) | (cb << 22);
 }
 
-// the activation preparation of `rows` batch rows (form 1: integer, 0: fp16)
+// the activation preparation of `rows` batch rows (form 1: integer, 0: fp16, which has no folded op: the entry points end those at
+// GQ_GEMV8_MAX_ROWS)
 static int launch_prep(const __nv_bfloat16 *x, int64_t rows, int64_t K, int64_t ldx, uint8_t *xt, int *status, int form, const PreOp *pre, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -1404,10 +1404,9 @@ static int launch_prep(const __nv_bfloat16 *x, int64_t rows, int64_t K, int64_t 
     const PreOp po = pre ? *pre : PreOp{};
     if (po.kind == GQ_PRE_ADD_RMSNORM) {
         cfg.gridDim = dim3((unsigned)rows, (unsigned)((K / GQ_QK + GQ_PREP_WARPS - 1) / GQ_PREP_WARPS));
-        GQ_CUDA(cudaLaunchKernelEx(&cfg, form ? prep_x_norm_kernel<1> : prep_x_norm_kernel<0>, x, ldx, (int)rows, xt, status, po));
+        GQ_CUDA(cudaLaunchKernelEx(&cfg, prep_x_norm_kernel, x, ldx, (int)rows, xt, status, po));
     } else {
-        auto *kern = po.kind == GQ_PRE_SILU_MUL ? (form ? prep_x_kernel<GQ_PRE_SILU_MUL, 1> : prep_x_kernel<GQ_PRE_SILU_MUL, 0>)
-                                                : (form ? prep_x_kernel<GQ_PRE_NONE, 1> : prep_x_kernel<GQ_PRE_NONE, 0>);
+        auto *kern = po.kind == GQ_PRE_SILU_MUL ? prep_x_kernel<GQ_PRE_SILU_MUL, 1> : form ? prep_x_kernel<GQ_PRE_NONE, 1> : prep_x_kernel<GQ_PRE_NONE, 0>;
         GQ_CUDA(cudaLaunchKernelEx(&cfg, kern, x, ldx, (int)rows, xt, status, po));
     }
     GQ_LAUNCHED();
@@ -1463,7 +1462,6 @@ static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ld
     if (int rc = ensure_tables()) return rc;
     cudaStream_t st = (cudaStream_t)stream;
 
-    if (pre && pre->kind && M > GQ_GEMV8_MAX_ROWS) return GQ_ERR_SHAPE;       // the folded ops exist in the integer form's preparation only
     const int maxb = run_info & 0xFFFF;
     if ((phases & 6) && (maxb < 56 || maxb > 272 || (maxb & 1))) return GQ_ERR_ARG;
     // split-K up to 8 reduces inside a thread-block cluster (portable cluster size); larger splits keep the fp32
