@@ -216,8 +216,10 @@ __device__ __forceinline__ void dequant_slab(const uint8_t *slab, const DecAux &
 // Bound by HBM (the bf16 output is 3.6x the packed bytes of a 4.5-bit type); the previous kernel turned the slab back into
 // raw order in shared memory and decoded every weight on its own from there.  17408 x 5120 Q5_K to bf16: 50 us = 4.8 TB/s
 // (before: 406 us).
+// (CTAs per SM that the compiler leaves registers for: its own choice, except where that is four with a spill: 17,408 x 5,120 IQ2_S 49.2 us,
+// with three 46.5)
 template <int TYPE, bool BF16>
-__global__ void __launch_bounds__(GQ_LOAD_THREADS) dequant_kernel(const uint8_t *__restrict__ tiles, int64_t n_out, int nb, int kc, void *__restrict__ out,
+__global__ void __launch_bounds__(GQ_LOAD_THREADS, BF16 && TYPE == GQ_IQ2_S ? 3 : 0) dequant_kernel(const uint8_t *__restrict__ tiles, int64_t n_out, int nb, int kc, void *__restrict__ out,
                                                                   int64_t ld) {
     constexpr int B = gq_type_bytes(TYPE), CB = gq_cb_kind(TYPE) >= 0 ? gq_cb_bytes(gq_cb_kind(TYPE)) : 0;
     extern __shared__ __align__(16) uint8_t sm[];       // [codebook][the warps' output staging]
