@@ -494,13 +494,10 @@ def mul_mat_tiles_grouped(x: torch.Tensor, packed: torch.Tensor, descs: list[tor
     if m == 0:
         return out
     n_tiles = sum(-(-int(n) // 64) for n in n_outs)
-    # up to 32 rows the grouped kernel streams the weights once for the batch; from 33 rows that would be twice, and the tcgen05
-    # kernel dequantises each weight once for all rows.  Whole calls in microseconds, grouped / tcgen05, at 16, 24 and 32 rows:
-    # 2 x 17408 x 5120 Q4_K 33.8 / 37.7, 39.7 / 37.7, 46.4 / 37.7; IQ3_S 42.8 / 52.9, 50.2 / 52.9, 57.0 / 52.9 (the tcgen05 kernel's time,
-    # measured at 64 rows, hardly depends on them).  Between 24 and 32 rows the
-    # tcgen05 kernel is thus the faster one on the wide layers.  The line stays at 32 for the precision: the grouped kernel
-    # multiplies exact weights, the other rounds them to fp16 (error beyond the output's rounding 4e-7 against 9e-5 of the
-    # result's norm)
+    # The line at 32 rows is one of precision: the grouped kernel multiplies exact weights, the tcgen05 kernel rounds them to fp16 (error
+    # beyond the output's rounding 4e-7 against 9e-5 of the result's norm).  The tcgen05 kernel decodes a weight once for all rows, and from
+    # about 20 rows it is the faster one on the wide layers; whole calls in microseconds, grouped at 17 / 27 rows and tcgen05 at 64, whose time
+    # hardly depends on them: 2 x 17408 x 5120 Q4_K 41 / 49 and 38, IQ3_S 52 / 60 and 53; 5120 x 5120 Q4_K 10.4 / 12.2 and 13.7.
     if m <= DECODE_MAX_ROWS:
         s = grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sm_count(x.device))
         if s not in desc_splits:
