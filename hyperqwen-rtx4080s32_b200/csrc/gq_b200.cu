@@ -1305,27 +1305,66 @@ extern "C" int64_t gq_build_descs_device(int n_shards, const int32_t *types, con
     return rows;
 }
 
+// CTAs of the grouped kernel that an SM holds by their registers, by the batch rows of a call
+static int gemv_ctas_per_sm(int64_t M) { return M <= 8 ? 4 : M <= 16 ? 3 : 2; }
+
+// How many thread-block clusters of 1 .. 8 CTAs the GPU holds side by side with one to four CTAs to an SM (cudaOccupancyMaxActiveClusters on
+// 148 SMs: a cluster lies within one of the GPU's processing clusters, and what is left of each stays empty).
+static int64_t cluster_places(int per_sm, int split, int sms) {
+    static const short places[4][8] = {{148, 74, 45, 33, 26, 22, 15, 15}, {296, 148, 93, 71, 56, 45, 37, 33}, {444, 222, 142, 104, 82, 71, 56, 48},
+                                       {592, 296, 187, 142, 112, 93, 78, 71}};
+    return (int64_t)places[per_sm - 1][split - 1] * sms / 148;
+}
+// The fewest CTAs to an SM (at most `most`) with which `tiles` clusters of `split` find places side by side; 0: they take more than one wave.
+// The last places are not counted on: 136 clusters of three for 142 places, and 112 of five for 112, ran as two waves.
+static int ctas_per_sm_for(int64_t tiles, int split, int most, int sms) {
+    for (int r = 1; r <= most; ++r)
+        if (tiles * 100 <= cluster_places(r, split, sms) * 93) return r;
+    return 0;
+}
+
+// An SM's time for a launch is what its CTAs need together, so up to 16 rows the split is chosen with the number of CTAs to an SM, which
+// launch_grouped then holds every SM to: left to the hardware, a launch of fewer CTAs than places fills some SMs and leaves others idle, because
+// under programmatic launch the SMs that finish first take all they can hold (and a cluster of eight fits on two SMs).  The costs are in k-blocks'
+// times of a CTA alone on its SM, fitted to sweeps of all splits at 4 .. 544 tiles x 5 .. 68 k-blocks of Q4_K, IQ3_S and IQ4_XS, over which calls
+// take 0.92 (up to 8 rows) and 0.91 (to 16) of the time under the rule before (the largest split of a single wave that leaves three k-blocks to a
+// CTA, the CTAs placed by the hardware).  Microseconds, before / now: 8,704 x 5,120 IQ3_S at 8 / 12 rows 13.5 / 11.7 and 17.1 / 13.6;
+// 1,280 x 17,408 IQ4_XS at 8 rows 13.8 / 9.5; 5,120 x 5,120 Q4_K 7.5 / 7.5; 17,408 x 5,120 Q4_K at 1 row 13.3 / 13.4.
+struct SplitCost {
+    double kb[4];                      // a k-block of a CTA, by the CTAs on its SM
+    double split, part;                // a split at all, and per part
+    double work, tail, start, crowd;   // more than one wave: the whole work over all SMs, the last CTA's, its start, per part
+};
 extern "C" int gq_split_for(int64_t n_tiles, int64_t nb, int64_t M, int avg_bytes_per_256, int sm_count) {
-    (void)avg_bytes_per_256;
     if (n_tiles <= 0 || nb <= 0) return 1;
     if (sm_count <= 0) sm_count = 148;
-    // from sweeps on B200 (Q4_K / Q2_K / IQ3_S / IQ4_XS; 80- to 544-tile layers at K 5120 and 17408): the
-    // largest split that (a) leaves a CTA at least three k-blocks, (b) stays inside one thread-block cluster (8), and
-    // (c) keeps the launch in one wave of the CTAs that the kernel for M rows has resident on an SM (four to 8 rows, three to 16,
-    // two above) — counting that clusters cannot use every slot: a launch of clusters of S fills at most about 1 - 0.03 (S - 1)
-    // of them before a second wave starts.  (With four for every M, 80 tiles at K 5120 ran as 480 CTAs: Q4_K 14.2 us at 16 rows,
-    // with the split of this rule, 4, 10.4.)
-    const int64_t per_sm = M <= 8 ? 4 : M <= 16 ? 3 : 2, slots = per_sm * sm_count;
-    int64_t s_max = nb / 3;
-    if (s_max > 8) s_max = 8;
-    int64_t s = 1;
-    for (int64_t c = 2; c <= s_max; ++c)
-        if (c * n_tiles * 100 <= slots * (100 - 3 * (c - 1))) s = c;
-    // 9 .. 16 rows, one CTA short of what an SM holds: two parts in a wave and a quarter are 13 - 20 % faster (272 tiles: Q4_K
-    // 25.8 -> 22.4 us, IQ3_S 34.6 -> 28.0)
-    if (per_sm == 3 && s == 1 && s_max >= 2 && n_tiles * 3 < slots * 2) s = 2;
-    if (s > nb) s = nb;
-    return (int)s;
+    const int most = gemv_ctas_per_sm(M);
+    const int64_t slots = (int64_t)most * sm_count;
+    int s = 1;
+    if (most == 2) {
+        // the largest split up to 8 that leaves a CTA three k-blocks and the launch one wave, clusters of S filling 1 - 0.03 (S - 1) of the
+        // places (the sweeps above 16 rows left little to a finer rule: 0.97 of the time)
+        for (int S = 2; S <= 8 && S <= nb / 3; ++S)
+            if (S * n_tiles * 100 <= slots * (100 - 3 * (S - 1))) s = S;
+        return s;
+    }
+    static const SplitCost costs[2] = {{{0.80, 1.08, 1.47, 1.95}, 0.72, 0.04, 1.67, 0.96, 0.32, 0.46}, {{0.90, 1.21, 1.80, 0.0}, 0.29, 0.033, 1.94, 0.64, 0.34, 0.67}};
+    const SplitCost &c = costs[most == 4 ? 0 : 1];
+    double best = 1e300;
+    for (int S = 1; S <= 8 && S <= nb; ++S) {
+        const int r = ctas_per_sm_for(n_tiles, S, most, sm_count);
+        const double kb = 0.5 * (double)((nb + S - 1) / S) + 0.5 * (double)nb / S;      // parts differ by one k-block
+        double cost;
+        // (tiles of 13 KB and more: four CTAs to an SM have no room for the pushed reduction, and short parts do not repay the other:
+        // 5,120 x 4,352 Q6_K at 4 rows with 5 / 6 parts 7.8 / 9.2 us)
+        if (avg_bytes_per_256 >= 200 && r == 4 && nb >= 8 && S > nb / 3) continue;
+        if (r) cost = kb * c.kb[r - 1];
+        else if (S > 1 && n_tiles * S * 10 > slots * 14) continue;
+        else cost = (double)n_tiles * (double)nb / sm_count * c.kb[most - 1] / most * c.work + kb * c.tail + c.start + c.crowd * (S - 1);
+        cost += (S > 1 ? c.split : 0.0) + c.part * S;
+        if (cost < best * (1.0 - 1e-9)) { best = cost; s = S; }
+    }
+    return s;
 }
 
 extern "C" int64_t gq_workspace_bytes(int64_t M, int64_t K, int64_t n_total, int split) {
@@ -1334,12 +1373,17 @@ extern "C" int64_t gq_workspace_bytes(int64_t M, int64_t K, int64_t n_total, int
 }
 
 template <int MT, int MINB, int FORM, int ONLY>
-static int launch_gemv(const GemvParams &p, int64_t n_desc, cudaStream_t stream) {
+static int launch_gemv(const GemvParams &p, int64_t n_desc, int apart, cudaStream_t stream) {
     constexpr int xbytes = gq_stage_xbytes<MT, FORM>();
     const int stage_bytes = p.wbytes_max + xbytes;
-    const size_t smem = (size_t)p.stages * stage_bytes + (size_t)p.stages * 16 + 8 * GQ_CONSUMER_WARPS + (size_t)p.cb_bytes +
+    size_t smem = (size_t)p.stages * stage_bytes + (size_t)p.stages * 16 + 8 * GQ_CONSUMER_WARPS + (size_t)p.cb_bytes +
                         (gq_red_in_ring<MT>() ? 0 : (size_t)GQ_CONSUMER_WARPS * MT * 512 * (p.cluster_push ? p.split - 1 : 1));
     if (smem > 232448) return GQ_ERR_LIMIT;
+    // `apart` CTAs to an SM and not one more (0: as many as fit): they ask for so much shared memory
+    if (apart) {
+        const size_t least = ((size_t)(228 * 1024) / (apart + 1) - 1024 + 16) & ~(size_t)15;
+        if (smem < least) smem = least;
+    }
     // opt in once per device to the largest dynamic shared memory a CTA can have
     static std::atomic<unsigned long long> done_mask{0};
     int dev = 0;
@@ -1370,12 +1414,12 @@ static int launch_gemv(const GemvParams &p, int64_t n_desc, cudaStream_t stream)
 
 // integer form, M <= 8 (FORM 1) and M <= 4 (FORM 2): one instantiation per type for runs of a single type, the all-types one otherwise
 template <int FORM>
-static int launch_gemv8_m8(const GemvParams &p, int64_t n_desc, cudaStream_t st, int only) {
+static int launch_gemv8_m8(const GemvParams &p, int64_t n_desc, int apart, cudaStream_t st, int only) {
     switch (only) {
-#define GQ_ONE(T) case T: return launch_gemv<1, 4, FORM, T>(p, n_desc, st);
+#define GQ_ONE(T) case T: return launch_gemv<1, 4, FORM, T>(p, n_desc, apart, st);
         GQ_EACH_TYPE(GQ_ONE)
 #undef GQ_ONE
-        default: return launch_gemv<1, 4, FORM, 0>(p, n_desc, st);
+        default: return launch_gemv<1, 4, FORM, 0>(p, n_desc, apart, st);
     }
 }
 
@@ -1416,17 +1460,20 @@ static int launch_prep(const __nv_bfloat16 *x, int64_t rows, int64_t K, int64_t 
 // an SM has 228 KB of shared memory, of which the system keeps 1 KB per resident CTA
 static int resident_ctas(int smem, int cap) { const int n = (228 * 1024) / (smem + 1024); return n < cap ? n : cap; }
 
-// One tile to a CTA.  CTAs that an SM holds by their registers: four to 8 rows, three to 16, two above.  Rings: integer form, the deepest of
-// three or four stages that leaves room for those CTAs (swept on the 64-layer stack: deeper rings with fewer resident CTAs were slower);
-// fp16 form, whose activation tiles are larger, of two to four; where its launch fits one CTA per SM it takes four, beside which few types
-// leave room for a second CTA (two shared an SM while others stood idle: 640 x 17,408 at 27 rows, Q4_K 14.6 -> 10.5 us, IQ4_XS 17.4 -> 12.3).
+// One tile to a CTA.  Rings: integer form, the deepest of three or four stages that leaves room for the CTAs that an SM is to hold (swept on
+// the 64-layer stack: deeper rings with fewer resident CTAs were slower); fp16 form, whose activation tiles are larger, of two to four; where
+// its launch fits one CTA per SM it takes four, beside which few types leave room for a second CTA.
 // The fp16 form with two tiles and eight consumer warps to a CTA (96 registers) was 4 - 9 % faster on 34,816 x 5,120 of Q2_K, Q4_K or Q8_0
 // and slower elsewhere: 5,120 x 5,120 at 17 rows Q4_K 10.5 -> 13.9, Q5_0 12.2 -> 16.4, 1,024 x 5,120 at 27 rows Q8_0 8.0 -> 13.4.
 static int launch_grouped(GemvParams &p, int run_info, int64_t n_desc, cudaStream_t st) {
     const bool fp16 = p.M > GQ_GEMV8_MAX_ROWS;
     const int mt = p.M <= 8 ? 1 : p.M <= 16 ? 2 : p.M <= 24 ? 3 : p.M <= 32 ? 4 : 8, low = fp16 ? 2 : 3;
-    const bool alone = fp16 && n_desc * 100 <= (int64_t)device_sms() * (100 - 3 * (p.split - 1));         // as gq_split_for counts the places for clusters
-    const int cap = alone ? 1 : mt == 1 ? 4 : mt == 2 ? 3 : 2;
+    // as many CTAs to an SM as the launch needs and no more (gq_split_for); a launch of more than one wave takes all places
+    const int most = gemv_ctas_per_sm(p.M), S = p.cluster ? p.split : 1, sms = device_sms();
+    const int need = ctas_per_sm_for(n_desc / S, S, most, sms), cap = need ? need : most;
+    // fp16 form, short parts of a launch that leaves SMs idle in any case: starting under the kernel in front is worth more (1,024 x 5,120
+    // IQ4_XS at 32 rows 7.8 / 7.6 us, 5,120 x 1,280 7.0 / 6.7)
+    const int apart = cap < most && !(fp16 && p.nb <= 6 * p.split) ? cap : 0;
     const int stage_bytes = p.wbytes_max + (p.M <= 4 ? gq_stage_xbytes<1, 2>() : 8 * mt * GQ_X_ROW + 32 * mt), red1 = mt == 8 ? 0 : GQ_CONSUMER_WARPS * mt * 512;
     const auto resident = [&](int stages, int red, int most) { return resident_ctas(stages * stage_bytes + 64 + 8 * GQ_CONSUMER_WARPS + p.cb_bytes + red, most); };
     // split-K in a cluster: the push form of the reduction needs a scratch slot per other split in every CTA; it is used when that
@@ -1439,11 +1486,11 @@ static int launch_grouped(GemvParams &p, int run_info, int64_t n_desc, cudaStrea
         p.stages = resident(4, red, cap) >= cap ? 4 : 3;
     }
     switch (mt) {
-        case 1: return p.M <= 4 ? launch_gemv8_m8<2>(p, n_desc, st, (run_info >> 17) & 31) : launch_gemv8_m8<1>(p, n_desc, st, (run_info >> 17) & 31);
-        case 2: return launch_gemv<2, 3, 1, 0>(p, n_desc, st);
-        case 3: return launch_gemv<3, 2, 0, 0>(p, n_desc, st);
-        case 4: return launch_gemv<4, 2, 0, 0>(p, n_desc, st);
-        default: return launch_gemv<8, 2, 0, 0>(p, n_desc, st);
+        case 1: return p.M <= 4 ? launch_gemv8_m8<2>(p, n_desc, apart, st, (run_info >> 17) & 31) : launch_gemv8_m8<1>(p, n_desc, apart, st, (run_info >> 17) & 31);
+        case 2: return launch_gemv<2, 3, 1, 0>(p, n_desc, apart, st);
+        case 3: return launch_gemv<3, 2, 0, 0>(p, n_desc, apart, st);
+        case 4: return launch_gemv<4, 2, 0, 0>(p, n_desc, apart, st);
+        default: return launch_gemv<8, 2, 0, 0>(p, n_desc, apart, st);
     }
 }
 

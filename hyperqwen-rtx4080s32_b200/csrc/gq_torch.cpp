@@ -95,13 +95,12 @@ class Run {
     }
 
   private:
+    // the table of a split, or of the largest below it that there is (split 1 always is)
     int index_of(int64_t split) const {
-        int one = 0;
-        for (size_t i = 0; i < splits_.size(); ++i) {
-            if (splits_[i] == split) return (int)i;
-            if (splits_[i] == 1) one = (int)i;
-        }
-        return one;
+        int best = -1;
+        for (size_t i = 0; i < splits_.size(); ++i)
+            if (splits_[i] <= split && (best < 0 || splits_[i] > splits_[best])) best = (int)i;
+        return best < 0 ? 0 : best;
     }
     static PyObject *none() { Py_RETURN_NONE; }
 

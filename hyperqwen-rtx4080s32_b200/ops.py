@@ -463,6 +463,11 @@ def prefill_gemm(x: torch.Tensor, packed: torch.Tensor, desc1: torch.Tensor, n_t
     return out
 
 
+def _table_split(s: int, desc_splits: Sequence[int]) -> int:
+    """The split of the table to use: s, or the largest below it that the run was prepared with (split 1 always is)."""
+    return s if s in desc_splits else max([t for t in desc_splits if t < s], default=1)
+
+
 def mul_mat_tiles_grouped_pre(x: torch.Tensor, pre, packed: torch.Tensor, descs: list[torch.Tensor], desc_splits: list[int],
                               tiles: list[torch.Tensor], n_outs: list[int], weight_types: list[int], nb: int, block_bytes: int) -> torch.Tensor:
     """mul_mat_tiles_grouped of pre(x): up to 16 rows the op is folded into the grouped launch's activation
@@ -472,9 +477,7 @@ def mul_mat_tiles_grouped_pre(x: torch.Tensor, pre, packed: torch.Tensor, descs:
         return mul_mat_tiles_grouped(pre.unfused(x), packed, descs, desc_splits, tiles, n_outs, weight_types, nb, block_bytes)
     n_total = sum(int(n) for n in n_outs)
     n_tiles = sum(-(-int(n) // 64) for n in n_outs)
-    s = grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sm_count(x.device))
-    if s not in desc_splits:
-        s = 1
+    s = _table_split(grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sm_count(x.device)), desc_splits)
     ar = _FUSED_AR
     if ar is not None:
         if pre.kind != 1 or not (m <= ar.max_m and n_total <= ar.max_n_total and s <= 8 and all(int(n) % 2 == 0 for n in n_outs)):
@@ -499,9 +502,7 @@ def mul_mat_tiles_grouped(x: torch.Tensor, packed: torch.Tensor, descs: list[tor
     # about 20 rows it is the faster one on the wide layers; whole calls in microseconds, grouped at 17 / 27 rows and tcgen05 at 64, whose time
     # hardly depends on them: 2 x 17408 x 5120 Q4_K 41 / 49 and 38, IQ3_S 52 / 60 and 53; 5120 x 5120 Q4_K 10.4 / 12.2 and 13.7.
     if m <= DECODE_MAX_ROWS:
-        s = grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sm_count(x.device))
-        if s not in desc_splits:
-            s = 1
+        s = _table_split(grouped_split_for(n_tiles, nb, m=m, block_bytes=block_bytes, sms=sm_count(x.device)), desc_splits)
         ar = _FUSED_AR
         if ar is not None and not (m <= ar.max_m and n_total <= ar.max_n_total and s <= 8 and all(int(n) % 2 == 0 for n in n_outs)):
             ar = None

@@ -96,7 +96,8 @@ int64_t gq_build_descs_device(int n_shards, const int32_t *types, const int64_t 
                               int32_t *desc_dev, void *stream);
 
 /* Split-K of a grouped launch: n_tiles output tiles, nb k-blocks, M batch rows (it matters whether there are up to 8, up to
- * 16 or more), avg_bytes_per_256 of the run, on a device with sm_count SMs.  Always in [1, nb] and at most 8 (the split then stays inside
+ * 16 or more), avg_bytes_per_256 of the run, on a device with sm_count SMs.  Up to 16 rows the split is chosen together with how many CTAs
+ * every SM is then held to.  Always in [1, nb] and at most 8 (the split then stays inside
  * one thread-block cluster); any other value in [1, nb] is also valid for the calls below.
  * Reference: grouped_split_for (gguf-plugin/gluon/tiles_grouped.py:209-250), re-derived for 148 SMs. */
 int gq_split_for(int64_t n_tiles, int64_t nb, int64_t M, int avg_bytes_per_256, int sm_count);

@@ -1,0 +1,46 @@
+"""How many CTAs of a grouped launch an SM is held to: launches of one, two, three and four to an SM and of more than a wave, with and without
+a split, in each of the kernel's forms."""
+import numpy as np
+import pytest
+import torch
+
+from hyperqwen_rtx4080s32_b200 import formats as F
+from hyperqwen_rtx4080s32_b200 import ops, synth
+from hyperqwen_rtx4080s32_b200.linear import GGUFLinear
+from oracle import oracle
+
+TOL = 6e-3      # bf16 output rounding (2^-8 of the value) plus fp32 accumulation
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t", [F.Q4_K, F.IQ2_S, F.Q8_0])
+@pytest.mark.parametrize("tiles, nb", [(2, 3), (13, 16), (14, 16), (21, 8), (68, 5), (80, 4), (113, 4), (136, 6), (150, 3), (280, 2), (560, 2), (640, 1)])
+def test_launches_of_every_density(t, tiles, nb):
+    n, k = 64 * tiles - 5, 256 * nb
+    raw = synth.random_blocks(n, k, t, seed=tiles, device="cuda")
+    lin = GGUFLinear(k, [n])
+    lin.load_shard(raw, t)
+    lin.finalize()
+    cols = np.unique(np.concatenate([np.arange(0, n, 977), np.arange(63, n, 64 * 41), [n - 1]]))
+    pick = torch.from_numpy(cols).cuda()
+    rows = raw[pick].cpu().numpy()
+    for m in (1, 4, 8, 16, 20, 32):
+        x = synth.activations(m, k, device="cuda")
+        y = lin(x)
+        assert oracle.rel_err(y[:, pick].float().cpu().numpy(), oracle.matmul_f64(x.float().cpu().numpy(), rows, t)) < TOL, m
+        assert torch.equal(y, lin(x))
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+def test_the_split_leaves_no_part_empty_and_follows_the_tile_width(m):
+    for nb in (1, 2, 5, 8, 17, 20, 68):
+        for tiles in (1, 4, 15, 16, 56, 80, 112, 136, 148, 272, 544, 593, 3880):
+            splits = [ops.grouped_split_for(tiles, nb, m=m, block_bytes=b, sms=148) for b in (84, 144, 210, 272)]
+            assert all(1 <= s <= min(nb, 8) for s in splits) and splits[0] == splits[1] and splits[2] == splits[3]
+            assert m > 8 or nb < 8 or splits[2] <= max(1, nb // 3) or tiles * splits[2] <= 3 * 148
+
+
+def test_a_run_prepared_with_other_splits_uses_the_nearest_below():
+    assert [ops._table_split(s, [1, 3, 6]) for s in (1, 2, 3, 5, 6, 8)] == [1, 1, 3, 3, 6, 6]
+    assert ops._table_split(2, [6]) == 1
