@@ -307,66 +307,129 @@ __global__ void __launch_bounds__(32 * GQ_PREP_WARPS) prep_x_kernel(const __nv_b
     prep_store<FORM>(v, kb, m, M, xt, lane);
 }
 
-// RMSNorm (with the residual add) in front of the layer: grid (batch rows, k-blocks / 8).  Every CTA sums the squares of
-// its whole row (a few KB from L2), then each warp converts one k-block.
-__global__ void __launch_bounds__(32 * GQ_PREP_WARPS) prep_x_norm_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int M, uint8_t *__restrict__ xt,
-                                                                           int *status, const PreOp pre) {
-    __shared__ float red[GQ_PREP_WARPS];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, m = blockIdx.x;
+// eight bf16 values as they are, wherever they start
+__device__ __forceinline__ uint4 load8_raw(const __nv_bfloat16 *p) {
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) return __ldg(reinterpret_cast<const uint4 *>(p));
+    const unsigned short *h = reinterpret_cast<const unsigned short *>(p);
+    return make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16, h[4] | (uint32_t)h[5] << 16, h[6] | (uint32_t)h[7] << 16);
+}
+__device__ __forceinline__ void unpack8(const uint4 &raw, float (&v)[8]) {
+    const uint32_t r[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { v[2 * j] = __uint_as_float(r[j] << 16); v[2 * j + 1] = __uint_as_float(r[j] & 0xffff0000u); }
+}
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) { return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7])); }
+__device__ __forceinline__ void store8_raw(__nv_bfloat16 *p, const uint4 &o) {
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+        *reinterpret_cast<uint4 *>(p) = o;
+    } else {
+        unsigned short *h = reinterpret_cast<unsigned short *>(p);
+        const uint32_t r[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { h[2 * j] = (unsigned short)r[j]; h[2 * j + 1] = (unsigned short)(r[j] >> 16); }
+    }
+}
+
+// RMSNorm (with the residual add) in front of the layer, one CTA per batch row: x, residual and weight are requested together and stay in registers,
+// as bf16, between the sum of squares and the scaling, two k-blocks to a warp (of rows beyond 64 k-blocks the rest is read again).
+// PREP: into the integer form's workspace (up to GQ_GEMV8_MAX_ROWS rows), a warp to a k-block where they last; else as bf16 to `out`, two to a warp.
+// Bound by its latency chain at few rows (one trip to memory, two reductions, the stores), by HBM at many.  With a CTA to eight k-blocks that each
+// summed the whole row and read its own part again, 13 rows of 5,120 took 0.5 to 1 us longer; torch's operations at 24 rows take 32 us more than this,
+// at 2,048 rows 80 to 100.
+#define GQ_NORM_MAX_WARPS 32
+#define GQ_NORM_KEEP 2
+template <bool PREP>
+__global__ void __launch_bounds__(32 * GQ_NORM_MAX_WARPS) norm_rows_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int M, uint8_t *__restrict__ xt, int *status,
+                                                                           __nv_bfloat16 *__restrict__ out, int64_t ldo, const PreOp pre) {
+    __shared__ float red[GQ_NORM_MAX_WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, m = blockIdx.x, nb = pre.K / GQ_QK;
     pdl_trigger();
     pdl_wait();
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status = 0;
+    if (PREP && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
     const __nv_bfloat16 *row = x + (int64_t)m * ldx;
     const __nv_bfloat16 *res = pre.residual ? pre.residual + (int64_t)m * pre.ld_res : nullptr;
-    float ss = 0.0f;
-#pragma unroll 4
-    for (int c = threadIdx.x; c < pre.K / 8; c += 32 * GQ_PREP_WARPS) {
-        float a[8];
-        load8(row + 8 * c, a);
+    // the k-block's values after the add, rounded to bf16
+    const auto load = [&](int kb) {
+        const int64_t col = (int64_t)kb * GQ_QK + 8 * lane;
+        uint4 z = load8_raw(row + col);
         if (res) {
-            float r[8];
-            load8(res + 8 * c, r);
+            float a[8], r[8];
+            unpack8(load8_raw(res + col), r);
+            unpack8(z, a);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) a[j] = bf16_round(a[j] + r[j]);
+            for (int j = 0; j < 8; ++j) a[j] += r[j];
+            z = pack8(a);
         }
+        return z;
+    };
+    const auto squares = [](const uint4 &z, float s) {
+        float a[8];
+        unpack8(z, a);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ss = fmaf(a[j], a[j], ss);
+        for (int j = 0; j < 8; ++j) s = fmaf(a[j], a[j], s);
+        return s;
+    };
+    const auto use = [&](int kb, const uint4 &z, float rs, const uint4 &w) {
+        const int64_t col = (int64_t)kb * GQ_QK + 8 * lane;
+        if (res) store8_raw(pre.residual_out + (int64_t)m * pre.ld_res + col, z);
+        float v[8], u[8];
+        unpack8(z, v);
+        unpack8(w, u);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = bf16_round(v[j] * rs) * u[j];
+        if constexpr (PREP) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = bf16_round(v[j]);
+            prep8_store(v, kb, m, M, xt, lane);
+        } else {
+            store8_raw(out + (int64_t)m * ldo + col, pack8(v));
+        }
+    };
+    uint4 z[GQ_NORM_KEEP], w[GQ_NORM_KEEP];
+#pragma unroll
+    for (int i = 0; i < GQ_NORM_KEEP; ++i) {
+        const int kb = warp + i * warps;
+        z[i] = w[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (kb < nb) { z[i] = load(kb); w[i] = load8_raw(pre.weight + (int64_t)kb * GQ_QK + 8 * lane); }
     }
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < GQ_NORM_KEEP; ++i) ss = squares(z[i], ss);
+    for (int kb = warp + GQ_NORM_KEEP * warps; kb < nb; kb += warps) ss = squares(load(kb), ss);
 #pragma unroll
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if (lane == 0) red[warp] = ss;
     __syncthreads();
-    ss = 0.0f;
+    ss = lane < warps ? red[lane] : 0.0f;
 #pragma unroll
-    for (int i = 0; i < GQ_PREP_WARPS; ++i) ss += red[i];
+    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const float rs = rsqrtf(ss / (float)pre.K + pre.eps);
-    const int kb = blockIdx.y * GQ_PREP_WARPS + warp;
-    if (kb < pre.K / GQ_QK) {
-        const int64_t col = (int64_t)kb * GQ_QK + 8 * lane;
-        float v[8], w[8];
-        load8(row + col, v);
-        load8(pre.weight + col, w);
-        if (res) {
-            float r[8];
-            load8(res + col, r);
-            uint4 z;
-            __nv_bfloat162 *zb = reinterpret_cast<__nv_bfloat162 *>(&z);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = bf16_round(v[j] + r[j]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) zb[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-            __nv_bfloat16 *zo = pre.residual_out + (int64_t)m * pre.ld_res + col;
-            if ((reinterpret_cast<uintptr_t>(zo) & 15) == 0) {
-                *reinterpret_cast<uint4 *>(zo) = z;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) zo[j] = __float2bfloat16_rn(v[j]);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = bf16_round(bf16_round(v[j] * rs) * w[j]);
-        prep8_store(v, kb, m, M, xt, lane);
+    for (int i = 0; i < GQ_NORM_KEEP; ++i) {
+        const int kb = warp + i * warps;
+        if (kb < nb) use(kb, z[i], rs, w[i]);
     }
+    for (int kb = warp + GQ_NORM_KEEP * warps; kb < nb; kb += warps) use(kb, load(kb), rs, load8_raw(pre.weight + (int64_t)kb * GQ_QK + 8 * lane));
+}
+
+// silu(in[:, :K]) * in[:, K:2K] as bf16, for batches whose preparation does not fold it: eight elements to a thread, bound by HBM at many rows
+// (torch's two operations: 5 us more at 24 rows of 4,352, 40 at 2,048)
+__global__ void __launch_bounds__(256) silu_mul_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int K, __nv_bfloat16 *__restrict__ out, int64_t ldo) {
+    pdl_trigger();
+    pdl_wait();
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    if (c >= K) return;
+    const __nv_bfloat16 *xr = x + (int64_t)blockIdx.y * ldx + c;
+    float v[8], u[8];
+    load8(xr, v);
+    load8(xr + K, u);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = bf16_round(v[j] / (1.0f + expf(-v[j]))) * u[j];
+    store8_raw(out + (int64_t)blockIdx.y * ldo + c, pack8(v));
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -1447,8 +1510,9 @@ static int launch_prep(const __nv_bfloat16 *x, int64_t rows, int64_t K, int64_t 
     cfg.gridDim = dim3((unsigned)(K / GQ_QK), (unsigned)((rows + GQ_PREP_WARPS - 1) / GQ_PREP_WARPS)); cfg.blockDim = dim3(32 * GQ_PREP_WARPS);
     const PreOp po = pre ? *pre : PreOp{};
     if (po.kind == GQ_PRE_ADD_RMSNORM) {
-        cfg.gridDim = dim3((unsigned)rows, (unsigned)((K / GQ_QK + GQ_PREP_WARPS - 1) / GQ_PREP_WARPS));
-        GQ_CUDA(cudaLaunchKernelEx(&cfg, prep_x_norm_kernel, x, ldx, (int)rows, xt, status, po));
+        const int64_t nb = K / GQ_QK;
+        cfg.gridDim = dim3((unsigned)rows); cfg.blockDim = dim3(32 * (unsigned)(nb < GQ_NORM_MAX_WARPS ? nb : GQ_NORM_MAX_WARPS));
+        GQ_CUDA(cudaLaunchKernelEx(&cfg, norm_rows_kernel<true>, x, ldx, (int)rows, xt, status, (__nv_bfloat16 *)nullptr, (int64_t)0, po));
     } else {
         auto *kern = po.kind == GQ_PRE_SILU_MUL ? prep_x_kernel<GQ_PRE_SILU_MUL, 1> : form ? prep_x_kernel<GQ_PRE_NONE, 1> : prep_x_kernel<GQ_PRE_NONE, 0>;
         GQ_CUDA(cudaLaunchKernelEx(&cfg, kern, x, ldx, (int)rows, xt, status, po));
@@ -1569,16 +1633,8 @@ extern "C" int gq_gemv_grouped(const void *x_dev, int64_t M, int64_t K, int64_t 
                                   workspace_bytes, stream, 7);
 }
 
-// ---- the same call with the op in front of the layer folded into the activation preparation -----------------
-// pre_op GQ_PRE_SILU_MUL: x_dev is the [M, 2K] output of gate_up_proj (ldx >= 2K), the layer multiplies
-// silu(x[:, :K]) * x[:, K:].  GQ_PRE_ADD_RMSNORM: x_dev is [M, K]; norm_weight [K]; residual_in / residual_out [M, ld_res]
-// both or neither (distinct memory: every warp of a row reads the whole old residual).  1..GQ_GEMV8_MAX_ROWS rows.
-extern "C" int gq_gemv_grouped_pre(const void *x_dev, int64_t M, int64_t K, int64_t ldx, int pre_op, const void *norm_weight_dev,
-                                   const void *residual_in_dev, void *residual_out_dev, int64_t ld_res, float eps, const void *packed_dev,
-                                   const int32_t *desc_dev, int64_t n_desc, int split, int run_info, void *y_dev, int64_t ldy,
-                                   int64_t n_total, void *workspace_dev, int64_t workspace_bytes, void *stream) {
-    if (M < 0 || M > GQ_GEMV8_MAX_ROWS) return GQ_ERR_SHAPE;
-    PreOp po{};
+static int make_pre_op(PreOp &po, int64_t K, int64_t ldx, int pre_op, const void *norm_weight_dev, const void *residual_in_dev, void *residual_out_dev, int64_t ld_res,
+                       float eps) {
     po.kind = pre_op; po.K = (int)K; po.eps = eps;
     if (pre_op == GQ_PRE_SILU_MUL) {
         if (ldx < 2 * K) return GQ_ERR_ARG;
@@ -1591,6 +1647,54 @@ extern "C" int gq_gemv_grouped_pre(const void *x_dev, int64_t M, int64_t K, int6
     } else if (pre_op != GQ_PRE_NONE) {
         return GQ_ERR_ARG;
     }
+    return GQ_OK;
+}
+
+// the op by itself, for batches of more rows than the preparation folds
+extern "C" int gq_pre_op(const void *x_dev, int64_t M, int64_t K, int64_t ldx, int pre_op, const void *norm_weight_dev, const void *residual_in_dev,
+                         void *residual_out_dev, int64_t ld_res, float eps, void *out_dev, int64_t ldo, void *stream) {
+    if (M < 0 || K <= 0 || K % GQ_QK || K > 0x3fffffff) return GQ_ERR_SHAPE;
+    if (pre_op != GQ_PRE_SILU_MUL && pre_op != GQ_PRE_ADD_RMSNORM) return GQ_ERR_ARG;
+    if (M == 0) return GQ_OK;
+    if (!x_dev || !out_dev || ldo < K || ldx < K || (((uintptr_t)x_dev | (uintptr_t)out_dev | (uintptr_t)residual_in_dev | (uintptr_t)residual_out_dev) & 1)) return GQ_ERR_ARG;
+    PreOp po{};
+    if (int rc = make_pre_op(po, K, ldx, pre_op, norm_weight_dev, residual_in_dev, residual_out_dev, ld_res, eps)) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.stream = (cudaStream_t)stream; cfg.attrs = attr; cfg.numAttrs = 1;
+    if (pre_op == GQ_PRE_ADD_RMSNORM) {
+        if (M > 0x7fffffff) return GQ_ERR_LIMIT;
+        // two k-blocks to a warp where there are rows for every SM (more CTAs to it), else one
+        const int64_t nb = K / GQ_QK, warps = M > device_sms() ? (nb + 1) / 2 : nb;
+        cfg.gridDim = dim3((unsigned)M); cfg.blockDim = dim3(32 * (unsigned)(warps < GQ_NORM_MAX_WARPS ? warps : GQ_NORM_MAX_WARPS));
+        GQ_CUDA(cudaLaunchKernelEx(&cfg, norm_rows_kernel<false>, (const __nv_bfloat16 *)x_dev, ldx, (int)M, (uint8_t *)nullptr, (int *)nullptr,
+                                   (__nv_bfloat16 *)out_dev, ldo, po));
+        GQ_LAUNCHED();
+        return GQ_OK;
+    }
+    // a row over CTAs of equal size, whole warps (a grid has 65,535 rows of CTAs)
+    const unsigned parts = (unsigned)((K / 8 + 255) / 256), threads = (unsigned)((K / 8 + 32 * parts - 1) / (32 * parts)) * 32;
+    for (int64_t m = 0; m < M; m += 65535) {
+        cfg.gridDim = dim3(parts, (unsigned)(M - m < 65535 ? M - m : 65535)); cfg.blockDim = dim3(threads);
+        GQ_CUDA(cudaLaunchKernelEx(&cfg, silu_mul_kernel, (const __nv_bfloat16 *)x_dev + m * ldx, ldx, (int)K, (__nv_bfloat16 *)out_dev + m * ldo, ldo));
+        GQ_LAUNCHED();
+    }
+    return GQ_OK;
+}
+
+// ---- the same call with the op in front of the layer folded into the activation preparation -----------------
+// pre_op GQ_PRE_SILU_MUL: x_dev is the [M, 2K] output of gate_up_proj (ldx >= 2K), the layer multiplies
+// silu(x[:, :K]) * x[:, K:].  GQ_PRE_ADD_RMSNORM: x_dev is [M, K]; norm_weight [K]; residual_in / residual_out [M, ld_res]
+// both or neither (distinct memory: every warp of a row reads the whole old residual).  1..GQ_GEMV8_MAX_ROWS rows.
+extern "C" int gq_gemv_grouped_pre(const void *x_dev, int64_t M, int64_t K, int64_t ldx, int pre_op, const void *norm_weight_dev,
+                                   const void *residual_in_dev, void *residual_out_dev, int64_t ld_res, float eps, const void *packed_dev,
+                                   const int32_t *desc_dev, int64_t n_desc, int split, int run_info, void *y_dev, int64_t ldy,
+                                   int64_t n_total, void *workspace_dev, int64_t workspace_bytes, void *stream) {
+    if (M < 0 || M > GQ_GEMV8_MAX_ROWS) return GQ_ERR_SHAPE;
+    PreOp po{};
+    if (int rc = make_pre_op(po, K, ldx, pre_op, norm_weight_dev, residual_in_dev, residual_out_dev, ld_res, eps)) return rc;
     return gemv_grouped_impl(x_dev, M, K, ldx, packed_dev, desc_dev, n_desc, split, run_info, y_dev, ldy, n_total, workspace_dev,
                              workspace_bytes, stream, 7, nullptr, 0, nullptr, &po);
 }

@@ -114,7 +114,6 @@ class Run {
         else { if (!x.is_contiguous()) return none(); for (int64_t i = 0; i + 1 < nd; ++i) m *= x.size(i); }
         if (m <= 0 || n_total_ == 0 || ldx < width) return none();
         if (pre) {
-            if (m > pre_rows_) return none();
             if (pre == 2) {
                 if (!plain_cuda(*weight, device_) || weight->scalar_type() != at::kBFloat16 || weight->numel() != K_ || !weight->is_contiguous()) return none();
                 if ((residual == nullptr) != (residual_out == nullptr)) return none();
@@ -126,8 +125,8 @@ class Run {
                 }
             }
         }
-        const bool wide = m > decode_rows_;
-        if (wide && ((ldx & 7) || (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15))) return none();
+        const bool wide = m > decode_rows_, apart = pre && m > pre_rows_;       // apart: the op is a launch of its own
+        if (wide && !apart && ((ldx & 7) || (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15))) return none();
         at::Tensor y;
         Status status;
         {
@@ -143,18 +142,27 @@ class Run {
     Status launch(const at::Tensor &x, int64_t m, int64_t ldx, int pre, const at::Tensor *weight, const at::Tensor *residual,
                   const at::Tensor *residual_out, float eps, at::Tensor &y) const {
         const bool wide = m > decode_rows_;
+        const void *in = x.data_ptr();
+        c10::DataPtr pre_out;
         c10::cuda::CUDAGuard guard((c10::DeviceIndex)device_);
         void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device_).stream();
         at::DimVector sizes(x.sizes().begin(), x.sizes().end());
         sizes.back() = n_total_;
         y = at::detail::empty_cuda(sizes, at::kBFloat16, x.device(), c10::nullopt);
         auto *alloc = c10::cuda::CUDACachingAllocator::get();
+        if (pre && m > pre_rows_) {
+            pre_out = alloc->allocate((size_t)(m * K_ * 2));
+            const int rc = gq_pre_op(in, m, K_, ldx, pre, weight ? weight->data_ptr() : nullptr, residual ? residual->data_ptr() : nullptr,
+                                     residual_out ? residual_out->data_ptr() : nullptr, residual ? residual->stride(0) : 0, eps, pre_out.get(), K_, stream);
+            if (rc < 0) return {rc, "gq_pre_op"};
+            in = pre_out.get(); ldx = K_; pre = 0;
+        }
         if (wide) {
             const int64_t n_desc = descs_[one_].size(0), need = gq_prefill_workspace_bytes(m, K_, n_total_, n_desc);
             if (need < 0) return {need, "gq_prefill_workspace_bytes"};
             c10::DataPtr ws = alloc->allocate((size_t)need + 1024);
             const uintptr_t base = (reinterpret_cast<uintptr_t>(ws.get()) + 1023) & ~(uintptr_t)1023;
-            return {gq_gemm_prefill(x.data_ptr(), m, K_, ldx, packed_.data_ptr(), (const int32_t *)descs_[one_].data_ptr(), n_desc, info_, y.data_ptr(),
+            return {gq_gemm_prefill(in, m, K_, ldx, packed_.data_ptr(), (const int32_t *)descs_[one_].data_ptr(), n_desc, info_, y.data_ptr(),
                                     n_total_, n_total_, (void *)base, need, stream), "gq_gemm_prefill"};
         }
         const int i = by_rows_[m];
@@ -169,7 +177,7 @@ class Run {
                                         (const int32_t *)d.data_ptr(), d.size(0), split, info_, y.data_ptr(), n_total_, n_total_, ws.get(), need, stream),
                     "gq_gemv_grouped_pre"};
         // 15: nobody reads this workspace's status word, so a small launch may do without the preparation kernel
-        return {gq_gemv_grouped_phases(x.data_ptr(), m, K_, ldx, packed_.data_ptr(), (const int32_t *)d.data_ptr(), d.size(0), split, info_,
+        return {gq_gemv_grouped_phases(in, m, K_, ldx, packed_.data_ptr(), (const int32_t *)d.data_ptr(), d.size(0), split, info_,
                                        y.data_ptr(), n_total_, n_total_, ws.get(), need, stream, 15), "gq_gemv_grouped"};
     }
 

@@ -356,7 +356,7 @@ class PreAddRMSNorm:
         return v.to(t.dtype) * self.weight
 
 
-PRE_MAX_ROWS = 16     # the folded ops live in the integer form's preparation
+PRE_MAX_ROWS = 16     # the folded ops live in the integer form's preparation; above, the op is a launch of its own (gq_pre_op, by the native path)
 
 
 def grouped_gemm(x: torch.Tensor, packed: torch.Tensor, desc: torch.Tensor, split: int, wtypes: Sequence[int], n_total: int,

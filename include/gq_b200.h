@@ -178,6 +178,11 @@ int gq_gemv_grouped_pre(const void *x_dev, int64_t M, int64_t K, int64_t ldx, in
                         const int32_t *desc_dev, int64_t n_desc, int split, int run_info, void *y_dev, int64_t ldy, int64_t n_total,
                         void *workspace_dev, int64_t workspace_bytes, void *stream);
 
+/* The op in front of a layer by itself, at any number of rows (gq_gemv_grouped_pre folds it up to 16): out_dev, bf16 [M, ldo], receives what the
+ * layer multiplies; the arguments are those of gq_gemv_grouped_pre and K is a multiple of 256.  One launch, the arithmetic of the folded form. */
+int gq_pre_op(const void *x_dev, int64_t M, int64_t K, int64_t ldx, int pre_op, const void *norm_weight_dev, const void *residual_in_dev,
+              void *residual_out_dev, int64_t ld_res, float eps, void *out_dev, int64_t ldo, void *stream);
+
 /* gq_gemv_grouped without a workspace argument, for callers that cannot allocate device memory at the
  * point of the call — a plugin op running where the framework's allocator is off limits (inside another
  * library's callback, under a fixed memory plan, or in a process that handed all of its device memory to a
