@@ -1923,9 +1923,9 @@ struct PrefillPlan {
 static PrefillPlan prefill_shape(int64_t M, int64_t tiles) {
     PrefillPlan p;
     const int64_t rows = (M + tiles - 1) / tiles;
-    p.tiles = (int)tiles;
     p.wide = rows > 256;
     p.N = (int)(p.wide ? (rows + 31) & ~31 : (rows + 15) & ~15);
+    p.tiles = (int)((M + p.N - 1) / p.N);       // (the steps of N may make the last of many tiles superfluous: each has a row of the batch)
     p.sets = p.N <= 128 ? 1 : 2;
     p.split = 1;
     return p;
@@ -1942,12 +1942,14 @@ static PrefillPlan prefill_plan(int64_t n_desc, int64_t M, int64_t nb, int sms) 
     double best_cost = 1e300;
     for (int64_t tiles = (M + 383) / 384; tiles <= (M + 255) / 256; ++tiles) {
         PrefillPlan p = prefill_shape(M, tiles);
-        const int64_t slots = p.sets == 1 ? 2 * (int64_t)sms : sms, ctas = prefill_ctas(n_desc, p) * tiles;
+        const int64_t ctas = prefill_ctas(n_desc, p) * p.tiles;
         const double mma = 7.8 * p.N + 300.0, decode = p.sets == 1 ? 4200.0 : 2700.0, per_kb = mma > decode ? mma : decode;
         for (int S = 1; S * p.sets <= 8 && (S == 1 || (int64_t)S * 4 <= nb); ++S) {
-            // clusters leave some slots unused
-            const int64_t usable = slots * (100 - 3 * (S - 1)) / 100;
-            const int64_t waves = (ctas * S + usable - 1) / usable;
+            // clusters of a unit's parts that the GPU holds side by side: of CTAs short of the last places (ctas_per_sm_for), of pairs, one
+            // CTA to an SM, all (32 of 33 and 14 of 15 run as one wave; 34 of two pairs, 8,704 x 5,120 Q4_K at 300 rows, took 55 us where 34
+            // whole pairs take 31)
+            const int64_t held = cluster_places(p.sets == 1 ? 2 : 1, S * p.sets, sms) * (p.sets == 1 && S > 1 ? 93 : 100), clusters = ctas / p.sets * 100;
+            const int64_t waves = (clusters + held - 1) / held;
             const double cost = (double)waves * ((double)((nb + S - 1) / S) * per_kb + 5000.0 + 25.0 * p.N + (S > 1 ? 6000.0 : 0.0));
             if (cost < best_cost * (1.0 - 1e-9)) { best_cost = cost; best = p; best.split = S; }
         }

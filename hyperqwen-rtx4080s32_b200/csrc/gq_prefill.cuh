@@ -243,6 +243,9 @@ __device__ __forceinline__ void pf_store8(const PrefillParams &p, const float (&
     }
 }
 
+// batch rows of tile mt that enter the MMAs: all N, of the last tile those that the batch has, in steps of 16 (517 rows are tiles of 288 and 240)
+__host__ __device__ inline int pf_rows(int M, int N, int mt) { const int left = (M - mt * N + 15) & ~15; return left < N ? left : N; }
+
 template <int SETS, bool WIDE, int SL>
 __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_prefill_kernel(const __grid_constant__ PrefillParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -264,6 +267,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
     // grid (CG * split, units, batch tiles): a cluster is the parts of one unit, CG groups of two tiles each
     const int half = (int)blockIdx.x % CG, part = (int)blockIdx.x / CG, unit = blockIdx.y, mt = blockIdx.z;
     const int kb0 = (int)((uint32_t)(part * p.nb) / (uint32_t)p.split), nkb = (int)((uint32_t)((part + 1) * p.nb) / (uint32_t)p.split) - kb0;
+    const int rows = SETS == 1 ? N : pf_rows(p.M, N, mt);        // of the batch tile, those that are multiplied (one set: all, up to 15 past the batch)
     const uint32_t leader = (uint32_t)(part * CG);       // cluster rank of the CTA that issues the pair's MMAs
     __shared__ __align__(16) float s_ex[SETS == 1 ? 128 : 384];
 
@@ -371,8 +375,9 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
     } else if (warp == DEQ + 2) {
         // ---- MMA issuer: the warp waits as one and a thread chosen by elect.sync issues, so that addresses and descriptors
         // stay in uniform registers (issued from a `lane == 0` branch an MMA cost the thread a hundred cycles) ----
-        const int nmma = WIDE ? N >> 1 : N;           // an MMA takes up to 256 batch rows: the wide tile is two of them
-        const uint32_t idesc = umma_idesc(128 * CG, nmma);
+        // an MMA takes up to 256 batch rows: the wide tile is two of them, of a last tile's rows the second has what is left, if anything
+        const int nmma = WIDE ? N >> 1 : N, n0 = rows < nmma ? rows : nmma, n1 = rows - n0;
+        const uint32_t idesc = umma_idesc(128 * CG, n0), idesc1 = umma_idesc(128 * CG, n1);
         const uint16_t ctas = (uint16_t)(3u << leader);
         const uint64_t bdesc0 = umma_desc(smem_u32(smem));
         const uint32_t bstep = (uint32_t)bbytes >> 4, bwrap = bstep * (uint32_t)p.bstages;
@@ -394,7 +399,8 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
                     for (int kk = 0; kk < 4; ++kk) {
                         const uint32_t acc = (j > 0 || kk > 0) ? 1u : (uint32_t)(kb > 0);
                         umma_ts_f16<CG>(tmem, ta + 32 * j + 8 * kk, bd + 2 * kk, idesc, acc);
-                        if constexpr (WIDE) umma_ts_f16<CG>(tmem + nmma, ta + 32 * j + 8 * kk, bd + 8 / CG * nmma + 2 * kk, idesc, acc);      // 128 bytes a row
+                        if constexpr (WIDE)
+                            if (n1 > 0) umma_ts_f16<CG>(tmem + nmma, ta + 32 * j + 8 * kk, bd + 8 / CG * nmma + 2 * kk, idesc1, acc);      // 128 bytes a row
                     }
                     // the slot and the activation stage may be overwritten once these MMAs have read them
                     if (j % SL == SL - 1) umma_commit<CG>(j == 3 && kb + 1 == nkb ? done : free + j / SL, ctas);
@@ -445,7 +451,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
     if (p.split == 1) {
         if (warp < DEQ && ok) {
 #pragma unroll 1
-            for (int c = 8 * e; c < N; c += 8 * (DEQ / 4)) {
+            for (int c = 8 * e; c < rows; c += 8 * (DEQ / 4)) {
                 uint32_t a[8];
                 tmem_ld_32x32b_x8(td + c, a);
                 const float4 e0 = *reinterpret_cast<const float4 *>(s_ex + c), e1 = *reinterpret_cast<const float4 *>(s_ex + c + 4);
@@ -460,13 +466,13 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
     } else {
         // columns [r ch, (r + 1) ch) are summed and stored by the CTA of part r; slot s of its buffer is part s's share, as
         // [ch / 4][128 rows] of four columns each: 16-byte stores and loads, one per lane side by side
-        const int S = p.split, ch = ((N + S - 1) / S + 7) & ~7;
+        const int S = p.split, ch = ((rows + S - 1) / S + 7) & ~7;
         float4 *buf = reinterpret_cast<float4 *>(smem);
         cluster_sync_all();                 // every CTA of the cluster has finished with its rings
         if (warp < DEQ) {
             const uint32_t mine = smem_u32(buf) + (uint32_t)(part * (ch >> 2) * 128 + feat) * 16;
 #pragma unroll 1
-            for (int c = 8 * e; c < N; c += 8 * (DEQ / 4)) {
+            for (int c = 8 * e; c < rows; c += 8 * (DEQ / 4)) {
                 uint32_t a[8];
                 tmem_ld_32x32b_x8(td + c, a);
                 const int r = c / ch;
@@ -479,7 +485,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
         }
         const bool any_bad = __syncthreads_or(!ok);
         cluster_sync_all();
-        const int c1 = (part + 1) * ch < N ? (part + 1) * ch : N;
+        const int c1 = (part + 1) * ch < rows ? (part + 1) * ch : rows;
         if (warp < DEQ && !any_bad) {
 #pragma unroll 1
             for (int c = part * ch + 8 * e; c < c1; c += 8 * (DEQ / 4)) {
@@ -540,9 +546,11 @@ __device__ __forceinline__ float amax8(const uint4 &v) {
 __global__ void __launch_bounds__(GQ_PF_PREP_THREADS, GQ_PF_PREP_CTAS) prep_x_prefill_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int K, int M, int N, int nmma,
                                                                             float *__restrict__ ex, uint8_t *__restrict__ xp, int *status) {
     __shared__ float red[GQ_PF_PREP_THREADS / 32], peers[8];
-    const int part = blockIdx.y, parts = gridDim.y, m = blockIdx.x, n = m % N, nvec = K >> 3, hn = nmma >> 1;
-    const int r = nmma ? (n % nmma) / hn * (N >> 1) + n / nmma * hn + n % hn : n;
-    uint8_t *dst = xp + (int64_t)(m / N) * (K / 64) * (N * 128) + r * 128;
+    const int part = blockIdx.y, parts = gridDim.y, m = blockIdx.x, mt = m / N, n = m - mt * N, nvec = K >> 3;
+    // of a pair's tile each MMA (rows [0, nmma) and the rest) has its first half in the first CTA
+    const int rows = pf_rows(M, N, mt), second = nmma && n >= nmma, in = second ? n - nmma : n, of = !nmma ? 0 : second ? rows - nmma : rows < nmma ? rows : nmma;
+    const int r = !nmma || n >= rows ? n : in / (of >> 1) * (N >> 1) + (second ? nmma >> 1 : 0) + in % (of >> 1);
+    uint8_t *dst = xp + (int64_t)mt * (K / 64) * (N * 128) + r * 128;
     const int phase = r & 7;
     if (parts > 1) cluster_arrive_relaxed();      // collected before the first store into another CTA: by then it runs
     pdl_trigger();    // the kernel behind this one may start fetching weights
@@ -550,8 +558,9 @@ __global__ void __launch_bounds__(GQ_PF_PREP_THREADS, GQ_PF_PREP_CTAS) prep_x_pr
     if (m == 0 && part == 0 && threadIdx.x == 0) *status = 0;
     const int first = part * GQ_PF_PREP_THREADS + threadIdx.x, step = parts * GQ_PF_PREP_THREADS;       // the thread's chunks of the row
     const auto put = [&](int c, const uint4 &o) { *reinterpret_cast<uint4 *>(dst + (int64_t)(c >> 3) * (N * 128) + (((c & 7) ^ phase) << 4)) = o; };
+    if (n >= rows) return;      // no MMA reads it
     if (m >= M) {
-        // rows past the batch inside the last tile: zeros (their outputs are never stored)
+        // rows past the batch among the last 16: zeros (their outputs are never stored)
         for (int c = first; c < nvec; c += step) put(c, make_uint4(0, 0, 0, 0));
         return;
     }
