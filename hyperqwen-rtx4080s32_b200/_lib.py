@@ -35,6 +35,7 @@ SIGNATURES = {
     "gq_build_descs_device": (_i64, [_i32, _vp, _vp, _i64, _i32, _vp, _vp, _vp]),
     "gq_split_for": (_i32, [_i64, _i64, _i64, _i32, _i32]),
     "gq_run_info": (_i32, [_i32, _vp]),
+    "gq_run_order": (_i32, [_i32, _vp, _vp]),
     "gq_workspace_bytes": (_i64, [_i64, _i64, _i64, _i32]),
     "gq_gemv_grouped": (_i32, [_vp, _i64, _i64, _i64, _vp, _vp, _i64, _i32, _i32, _vp, _i64, _i64, _vp, _i64, _vp]),
     "gq_gemv_grouped_phases": (_i32, [_vp, _i64, _i64, _i64, _vp, _vp, _i64, _i32, _i32, _vp, _i64, _i64, _vp, _i64, _vp, _i32]),

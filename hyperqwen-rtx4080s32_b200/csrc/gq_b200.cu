@@ -465,6 +465,7 @@ struct GemvParams {
     int64_t ldy, n_total;
     int wbytes_max;      // largest tile bytes in the launch (stage stride of the weight buffers)
     int cb_bytes;                    // shared-memory bytes of the codebook-table region (0: the run has no codebook type)
+    int reverse;         // 1: tiles from the last to the first
     int cluster;         // 1: the `split` CTAs of a tile form a thread-block cluster and reduce through shared memory
     int cluster_push;    // 1: the others store their accumulators into slots of the split-0 CTA's shared memory (one cluster barrier)
     const __nv_bfloat16 *x;  // FORM 2, one row: the activations themselves, converted by the producer warp (null: xt is prepared)
@@ -806,7 +807,9 @@ __global__ void __launch_bounds__(32 * (GQ_CONSUMER_WARPS + 1), MINB) gemv_group
     uint32_t *grid_s = reinterpret_cast<uint32_t *>(parts + GQ_CONSUMER_WARPS);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int32_t *d = p.desc + (int64_t)blockIdx.x * GQ_DESC_WORDS;
+    // the table row: the tile (and of a cluster, which is one, the part), perhaps counted from the last
+    const int row = p.reverse ? (int)((gridDim.x - 1 - blockIdx.x) / (unsigned)p.split) * p.split + (int)(blockIdx.x % (unsigned)p.split) : (int)blockIdx.x;
+    const int32_t *d = p.desc + (int64_t)row * GQ_DESC_WORDS;
     const int64_t off = (int64_t)d[0] * 16;
     const int type = ONLY ? ONLY : d[1];
     const int col0 = d[2], nvalid = d[3], kb0 = d[4], kb1 = d[5], split_idx = d[6];
@@ -1499,6 +1502,42 @@ extern "C" int gq_run_info(int n_shards, const int32_t *types) {
     return maxb | ((cb ? 1 : 0) << 16) | (single << 17) | (cb << 22);
 }
 
+// A run's tiles may be worked on from the last to the first.  Which types first: the CTAs of an SM are neighbours of the launch's order, and those
+// that start last, on the SMs that the kernel in front leaves last or in what is left of a wave, should be the quick ones.  2 x 17,408 x 5,120 with
+// the slower type first / second: IQ3_S and Q4_K at 1 / 8 rows 28.6 / 33.5 and 31.4 / 36.2 us, at 64 52.3 / 54.4; IQ3_S and Q2_K 29.6 / 32.7, 32.7 / 36.1
+// and 50.9 / 53.4.  From 9 to 32 rows, of one and a quarter to two waves, neither order is the better one (IQ3_S and Q4_K at 13 rows 46.2 / 40.0), nor is
+// it with CTA pairs.  Costs: 17,408 x 5,120 at 8 rows, 34,816 x 5,120 at 64, in tenths of a microsecond.
+static int order_cost(int type, bool tcgen05) {
+    switch (type) {
+        case GQ_Q4_0: return tcgen05 ? 348 : 123; case GQ_Q5_0: return tcgen05 ? 484 : 175; case GQ_Q8_0: return tcgen05 ? 400 : 212;
+        case GQ_Q2_K: return tcgen05 ? 394 : 117; case GQ_Q3_K: return tcgen05 ? 457 : 159; case GQ_Q4_K: return tcgen05 ? 380 : 124;
+        case GQ_Q5_K: return tcgen05 ? 469 : 151; case GQ_Q6_K: return tcgen05 ? 435 : 179; case GQ_IQ4_NL: return tcgen05 ? 456 : 176;
+        case GQ_IQ3_S: return tcgen05 ? 529 : 170; case GQ_IQ4_XS: return tcgen05 ? 487 : 191; case GQ_IQ3_XXS: return tcgen05 ? 598 : 204;
+        case GQ_IQ2_XXS: return tcgen05 ? 598 : 196; case GQ_IQ2_XS: return tcgen05 ? 617 : 221; case GQ_IQ2_S: return tcgen05 ? 588 : 213;
+        default: return tcgen05 ? 567 : 220;
+    }
+}
+extern "C" int gq_run_order(int n_shards, const int32_t *types, const int64_t *n_outs) {
+    if (n_shards <= 0 || !types || !n_outs) return GQ_ERR_ARG;
+    int64_t tiles = 0;
+    for (int i = 0; i < n_shards; ++i) {
+        if (!gq_type_bytes(types[i])) return GQ_ERR_TYPE;
+        if (n_outs[i] < 0) return GQ_ERR_SHAPE;
+        tiles += (n_outs[i] + 63) / 64;
+    }
+    int flags = 0;
+    for (int form = 0; form < 2; ++form) {
+        // what the first and the second half of the tiles cost
+        double first = 0.0, second = 0.0, at = 0.0;
+        for (int i = 0; i < n_shards; ++i) {
+            const double n = (double)((n_outs[i] + 63) / 64), mid = 0.5 * (double)tiles, in = at + n <= mid ? n : at >= mid ? 0.0 : mid - at, c = order_cost(types[i], form == 1);
+            first += in * c; second += (n - in) * c; at += n;
+        }
+        if (second > 1.03 * first) flags |= GQ_ORDER_8 << form;
+    }
+    return flags;
+}
+
 // the activation preparation of `rows` batch rows (form 1: integer, 0: fp16, which has no folded op: the entry points end those at
 // GQ_GEMV8_MAX_ROWS)
 static int launch_prep(const __nv_bfloat16 *x, int64_t rows, int64_t K, int64_t ldx, uint8_t *xt, int *status, int form, const PreOp *pre, cudaStream_t st) {
@@ -1535,6 +1574,8 @@ static int launch_grouped(GemvParams &p, int run_info, int64_t n_desc, cudaStrea
     // as many CTAs to an SM as the launch needs and no more (gq_split_for); a launch of more than one wave takes all places
     const int most = gemv_ctas_per_sm(p.M), S = p.cluster ? p.split : 1, sms = device_sms();
     const int need = ctas_per_sm_for(n_desc / S, S, most, sms), cap = need ? need : most;
+    // (a launch that leaves a tenth of its places empty is as fast or faster in its own order: q, k, v of 5,120 + 2 x 1,024 rows)
+    if (n_desc * 10 < 9 * (int64_t)cap * sms) p.reverse = 0;
     // fp16 form, short parts of a launch that leaves SMs idle in any case: starting under the kernel in front is worth more (1,024 x 5,120
     // IQ4_XS at 32 rows 7.8 / 7.6 us, 5,120 x 1,280 7.0 / 6.7)
     const int apart = cap < most && !(fp16 && p.nb <= 6 * p.split) ? cap : 0;
@@ -1597,6 +1638,7 @@ static int gemv_grouped_impl(const void *x_dev, int64_t M, int64_t K, int64_t ld
         p.wbytes_max = 64 * maxb;   // every stage can hold a tile of any shard of the run
         p.cb_bytes = gq_cb_region_max((run_info >> 22) & 63);
         p.cluster = cluster;
+        p.reverse = M <= 8 && (run_info & GQ_ORDER_8) && !ar && n_desc % split == 0 ? 1 : 0;      // (launch_grouped has the last word)
         p.x = direct ? (const __nv_bfloat16 *)x_dev : nullptr;
         p.pf_ptr = (next_packed_dev && next_bytes > 0 && !((uintptr_t)next_packed_dev & 15)) ? (const uint8_t *)next_packed_dev : nullptr;
         p.pf_bytes = next_bytes;
@@ -1997,7 +2039,7 @@ extern "C" int64_t gq_prefill_workspace_bytes(int64_t M, int64_t K, int64_t n_to
 }
 
 template <int SETS, bool WIDE, int SL>
-static int launch_prefill_kernel(PrefillParams &p, const PrefillPlan &pl, int smem, cudaStream_t st) {
+static int launch_prefill_kernel(PrefillParams &p, const PrefillPlan &pl, int smem, bool reverse, cudaStream_t st) {
     if (int rc = allow_smem<gemm_prefill_kernel<SETS, WIDE, SL>>(smem)) return rc;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
@@ -2016,6 +2058,7 @@ static int launch_prefill_kernel(PrefillParams &p, const PrefillPlan &pl, int sm
     for (int64_t d = 0; d < n_desc; d += step, p.desc += step * GQ_DESC_WORDS) {
         p.n_desc = (int)(n_desc - d < step ? n_desc - d : step);
         cfg.gridDim = dim3((unsigned)(pl.split * SETS), (unsigned)(prefill_ctas(p.n_desc, pl) / SETS), (unsigned)pl.tiles);
+        p.unit0 = reverse ? (int)cfg.gridDim.y - 1 : 0; p.unit_step = reverse ? -1 : 1;
         GQ_CUDA(cudaLaunchKernelEx(&cfg, gemm_prefill_kernel<SETS, WIDE, SL>, p));
         GQ_LAUNCHED();
     }
@@ -2023,7 +2066,7 @@ static int launch_prefill_kernel(PrefillParams &p, const PrefillPlan &pl, int sm
 }
 
 template <int SETS, bool WIDE>
-static int launch_prefill(PrefillParams &p, const PrefillPlan &pl, int maxb, int only, cudaStream_t st) {
+static int launch_prefill(PrefillParams &p, const PrefillPlan &pl, int maxb, int run_info, cudaStream_t st) {
     const int total = SETS == 1 ? GQ_PF_SMEM_1 : GQ_PF_SMEM_2, tables = gq_cb_region_sum(p.cb_mask), bbytes = pl.N * 128 / SETS;
     p.wstage_bytes = 128 * maxb;
     // the activation ring takes four slices (one k-block), the weight ring the rest; a run whose widest type leaves no two
@@ -2037,10 +2080,12 @@ static int launch_prefill(PrefillParams &p, const PrefillPlan &pl, int maxb, int
     if (p.wstages < 1) return GQ_ERR_LIMIT;
     left -= p.wstages * p.wstage_bytes + p.bstages * bbytes;
     while (p.bstages < GQ_PF_SLOTS * (WIDE ? 1 : SETS) && left >= bbytes) { ++p.bstages; left -= bbytes; }
+    const bool reverse = SETS == 1 && (run_info & GQ_ORDER_128);
     if constexpr (SETS == 1) {
-        if ((p.bstages == GQ_PF_SLOTS || p.cb_mask) && !(only == GQ_Q4_0 && pl.N > 64)) return launch_prefill_kernel<SETS, WIDE, 2>(p, pl, total, st);
+        if ((p.bstages == GQ_PF_SLOTS || p.cb_mask) && !(((run_info >> 17) & 31) == GQ_Q4_0 && pl.N > 64))
+            return launch_prefill_kernel<SETS, WIDE, 2>(p, pl, total, reverse, st);
     }
-    return launch_prefill_kernel<SETS, WIDE, 1>(p, pl, total, st);
+    return launch_prefill_kernel<SETS, WIDE, 1>(p, pl, total, reverse, st);
 }
 
 extern "C" int gq_gemm_prefill(const void *x_dev, int64_t M, int64_t K, int64_t ldx, const void *packed_dev, const int32_t *desc_dev,
@@ -2082,9 +2127,8 @@ extern "C" int gq_gemm_prefill(const void *x_dev, int64_t M, int64_t K, int64_t 
         GQ_CUDA(cudaLaunchKernelEx(&cfg, prep_x_prefill_kernel, (const __nv_bfloat16 *)x_dev, ldx, (int)K, (int)M, pl.N, pl.sets == 1 ? 0 : pl.wide ? pl.N / 2 : pl.N, ex, xp, status));
         GQ_LAUNCHED();
     }
-    const int only = (run_info >> 17) & 31;
-    if (pl.wide) return launch_prefill<2, true>(p, pl, maxb, only, st);
-    return pl.sets == 1 ? launch_prefill<1, false>(p, pl, maxb, only, st) : launch_prefill<2, false>(p, pl, maxb, only, st);
+    if (pl.wide) return launch_prefill<2, true>(p, pl, maxb, run_info, st);
+    return pl.sets == 1 ? launch_prefill<1, false>(p, pl, maxb, run_info, st) : launch_prefill<2, false>(p, pl, maxb, run_info, st);
 }
 
 extern "C" int gq_device_status(int clear, void *stream) {

@@ -57,6 +57,7 @@ struct PrefillParams {
     int M, nb, N;             // N: batch rows of a CTA's tile
     int *status;
     int split;                // CTAs of a cluster, each with its part of the k-blocks
+    int unit0, unit_step;     // one set: the first unit and +1, or the last and -1
     int wstages, bstages;     // ring depths
     int wstage_bytes;         // both tiles of the widest type of the run
     int cb_mask;              // the codebook types of the run (bit gq_cb_kind): their tables sit side by side in shared memory
@@ -265,7 +266,7 @@ __global__ void __launch_bounds__(32 * (8 * SETS + 3), SETS == 1 ? 2 : 1) gemm_p
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // grid (CG * split, units, batch tiles): a cluster is the parts of one unit, CG groups of two tiles each
-    const int half = (int)blockIdx.x % CG, part = (int)blockIdx.x / CG, unit = blockIdx.y, mt = blockIdx.z;
+    const int half = (int)blockIdx.x % CG, part = (int)blockIdx.x / CG, unit = SETS == 1 ? p.unit0 + p.unit_step * (int)blockIdx.y : (int)blockIdx.y, mt = blockIdx.z;
     const int kb0 = (int)((uint32_t)(part * p.nb) / (uint32_t)p.split), nkb = (int)((uint32_t)((part + 1) * p.nb) / (uint32_t)p.split) - kb0;
     const int rows = SETS == 1 ? N : pf_rows(p.M, N, mt);        // of the batch tile, those that are multiplied (one set: all, up to 15 past the batch)
     const uint32_t leader = (uint32_t)(part * CG);       // cluster rank of the CTA that issues the pair's MMAs

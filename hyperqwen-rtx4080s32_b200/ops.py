@@ -137,6 +137,17 @@ def run_info(wtypes: Sequence[int]) -> int:
     return _RUN_INFO[key]
 
 
+_RUN_ORDER: dict[tuple, int] = {}      # bounded by the merged layers a model has
+
+
+def run_order(wtypes: Sequence[int], n_outs: Sequence[int]) -> int:
+    """The flags of gq_run_order for a run's shards: which end of it a launch begins with."""
+    key = (tuple(wtypes), tuple(n_outs))
+    if key not in _RUN_ORDER:
+        _RUN_ORDER[key] = check(lib().gq_run_order(len(key[0]), _i32_array(key[0]), _i64_array(key[1])), "gq_run_order")
+    return _RUN_ORDER[key]
+
+
 def device_status(device=None, clear: bool = True) -> int:
     """The largest status code a kernel of the library reported on the device since it was last cleared (0: none;
     1: a bounded wait ran out and that call's output is incomplete; 2: bad shape).  Synchronises the stream."""
@@ -360,12 +371,12 @@ PRE_MAX_ROWS = 16     # the folded ops live in the integer form's preparation; a
 
 
 def grouped_gemm(x: torch.Tensor, packed: torch.Tensor, desc: torch.Tensor, split: int, wtypes: Sequence[int], n_total: int,
-                 out: torch.Tensor | None = None, workspace: torch.Tensor | None = None, phases: int = 7, allreduce=None, pre=None) -> torch.Tensor:
+                 out: torch.Tensor | None = None, workspace: torch.Tensor | None = None, phases: int = 7, allreduce=None, pre=None, order: int = 0) -> torch.Tensor:
     """One grouped launch for 1..64 rows: x bf16 [M, K] -> out bf16 [M, n_total] (out may be a column view).
     `workspace` (uint8, 256-byte aligned, at least gq_workspace_bytes) is allocated per call unless given;
     `phases` selects the launches (1 prepare activations, 2 grouped kernel, 4 partial sum); `allreduce` (a
     tp.FusedAllReduce) makes the output the sum over the tensor-parallel ranks; `pre` (PreSiluMul / PreAddRMSNorm,
-    up to 16 rows) folds the op in front of the layer into the activation preparation — x is then that op's input."""
+    up to 16 rows) folds the op in front of the layer into the activation preparation — x is then that op's input; `order`: flags of run_order."""
     _need_cuda(x, "x")
     if x.dtype != torch.bfloat16 or x.dim() != 2:
         raise GqError(f"x must be bf16 [M, K], got {x.dtype} {tuple(x.shape)}")
@@ -393,7 +404,7 @@ def grouped_gemm(x: torch.Tensor, packed: torch.Tensor, desc: torch.Tensor, spli
     if pre is not None and allreduce is not None:
         with torch.cuda.device(x.device):
             check(L.gq_gemv_grouped_allreduce_silu_mul(x.data_ptr(), m, k, x.stride(0), packed.data_ptr(), desc.data_ptr(), int(desc.shape[0]),
-                                                       int(split), run_info(wtypes), out.data_ptr(), out.stride(0), n_total, ws.data_ptr(),
+                                                       int(split), run_info(wtypes) | order, out.data_ptr(), out.stride(0), n_total, ws.data_ptr(),
                                                        ws.numel(), allreduce.rank, allreduce.world, allreduce.ptrs, allreduce.max_m,
                                                        allreduce.max_n_total, _stream_ptr(x)), "gq_gemv_grouped_allreduce_silu_mul")
         allreduce.used = True
@@ -410,13 +421,13 @@ def grouped_gemm(x: torch.Tensor, packed: torch.Tensor, desc: torch.Tensor, spli
             check(L.gq_gemv_grouped_pre(x.data_ptr(), m, k, x.stride(0), pre.kind, w.data_ptr() if w is not None else None,
                                         res.data_ptr() if res is not None else None, res_out.data_ptr() if res_out is not None else None,
                                         res.stride(0) if res is not None else 0, getattr(pre, "eps", 0.0), packed.data_ptr(), desc.data_ptr(),
-                                        int(desc.shape[0]), int(split), run_info(wtypes), out.data_ptr(), out.stride(0), n_total, ws.data_ptr(),
+                                        int(desc.shape[0]), int(split), run_info(wtypes) | order, out.data_ptr(), out.stride(0), n_total, ws.data_ptr(),
                                         ws.numel(), _stream_ptr(x)), "gq_gemv_grouped_pre")
         return out
     if allreduce is not None:
         with torch.cuda.device(x.device):
             check(L.gq_gemv_grouped_allreduce(x.data_ptr(), m, k, x.stride(0), packed.data_ptr(), desc.data_ptr(), int(desc.shape[0]), int(split),
-                                              run_info(wtypes), out.data_ptr(), out.stride(0), n_total, ws.data_ptr(), ws.numel(),
+                                              run_info(wtypes) | order, out.data_ptr(), out.stride(0), n_total, ws.data_ptr(), ws.numel(),
                                               allreduce.rank, allreduce.world, allreduce.ptrs, allreduce.max_m, allreduce.max_n_total,
                                               _stream_ptr(x)), "gq_gemv_grouped_allreduce")
         allreduce.used = True
@@ -425,18 +436,18 @@ def grouped_gemm(x: torch.Tensor, packed: torch.Tensor, desc: torch.Tensor, spli
     if nxt is not None:
         with torch.cuda.device(x.device):
             check(L.gq_gemv_grouped_prefetch(x.data_ptr(), m, k, x.stride(0), packed.data_ptr(), desc.data_ptr(), int(desc.shape[0]), int(split),
-                                             run_info(wtypes), out.data_ptr(), out.stride(0), n_total, ws.data_ptr(), ws.numel(), _stream_ptr(x),
+                                             run_info(wtypes) | order, out.data_ptr(), out.stride(0), n_total, ws.data_ptr(), ws.numel(), _stream_ptr(x),
                                              nxt[0], min(nxt[1], 96 << 20)), "gq_gemv_grouped_prefetch")
         return out
     with torch.cuda.device(x.device):
         check(L.gq_gemv_grouped_phases(x.data_ptr(), m, k, x.stride(0), packed.data_ptr(), desc.data_ptr(), int(desc.shape[0]), int(split),
-                                       run_info(wtypes), out.data_ptr(), out.stride(0), n_total, ws.data_ptr(), ws.numel(), _stream_ptr(x),
+                                       run_info(wtypes) | order, out.data_ptr(), out.stride(0), n_total, ws.data_ptr(), ws.numel(), _stream_ptr(x),
                                        int(phases)), "gq_gemv_grouped")
     return out
 
 
 def prefill_gemm(x: torch.Tensor, packed: torch.Tensor, desc1: torch.Tensor, n_total: int, out: torch.Tensor | None = None, *,
-                 wtypes: Sequence[int]) -> torch.Tensor:
+                 wtypes: Sequence[int], order: int = 0) -> torch.Tensor:
     """The large-batch path (tcgen05 dequant-GEMM): x bf16 [M, K] -> out bf16 [M, n_total]; desc1 is the run's
     split-1 descriptor table; wtypes the run's GGML types (they size the shared-memory tables)."""
     _need_cuda(x, "x")
@@ -456,7 +467,7 @@ def prefill_gemm(x: torch.Tensor, packed: torch.Tensor, desc1: torch.Tensor, n_t
         ws_bytes = check(L.gq_prefill_workspace_bytes(m, k, n_total, int(desc1.shape[0])), "gq_prefill_workspace_bytes")
     ws = torch.empty(ws_bytes + 1024, dtype=torch.uint8, device=x.device)
     base = (ws.data_ptr() + 1023) // 1024 * 1024
-    info = run_info(wtypes)
+    info = run_info(wtypes) | order
     with torch.cuda.device(x.device):
         check(L.gq_gemm_prefill(x.data_ptr(), m, k, x.stride(0), packed.data_ptr(), desc1.data_ptr(), int(desc1.shape[0]), info, out.data_ptr(),
                                 out.stride(0), n_total, base, ws_bytes, _stream_ptr(x)), "gq_gemm_prefill")
@@ -482,7 +493,7 @@ def mul_mat_tiles_grouped_pre(x: torch.Tensor, pre, packed: torch.Tensor, descs:
     if ar is not None:
         if pre.kind != 1 or not (m <= ar.max_m and n_total <= ar.max_n_total and s <= 8 and all(int(n) % 2 == 0 for n in n_outs)):
             return mul_mat_tiles_grouped(pre.unfused(x), packed, descs, desc_splits, tiles, n_outs, weight_types, nb, block_bytes)
-    return grouped_gemm(x, packed, descs[desc_splits.index(s)], s, weight_types, n_total, pre=pre, allreduce=ar)
+    return grouped_gemm(x, packed, descs[desc_splits.index(s)], s, weight_types, n_total, pre=pre, allreduce=ar, order=run_order(weight_types, n_outs))
 
 
 def mul_mat_tiles_grouped(x: torch.Tensor, packed: torch.Tensor, descs: list[torch.Tensor], desc_splits: list[int],
@@ -506,9 +517,9 @@ def mul_mat_tiles_grouped(x: torch.Tensor, packed: torch.Tensor, descs: list[tor
         ar = _FUSED_AR
         if ar is not None and not (m <= ar.max_m and n_total <= ar.max_n_total and s <= 8 and all(int(n) % 2 == 0 for n in n_outs)):
             ar = None
-        grouped_gemm(x, packed, descs[desc_splits.index(s)], s, weight_types, n_total, out=out, allreduce=ar)
+        grouped_gemm(x, packed, descs[desc_splits.index(s)], s, weight_types, n_total, out=out, allreduce=ar, order=run_order(weight_types, n_outs))
         return out
-    prefill_gemm(x, packed, descs[desc_splits.index(1)], n_total, out=out, wtypes=weight_types)
+    prefill_gemm(x, packed, descs[desc_splits.index(1)], n_total, out=out, wtypes=weight_types, order=run_order(weight_types, n_outs))
     return out
 
 

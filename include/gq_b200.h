@@ -112,6 +112,12 @@ int gq_split_for(int64_t n_tiles, int64_t nb, int64_t M, int avg_bytes_per_256, 
  * Reference: meta["max_rw"] and the NEW mask (gguf-plugin/gluon/tiles_grouped.py:181-202,1239-1265). */
 int gq_run_info(int n_shards, const int32_t *types);
 
+/* Flags for the run_info of a call, by the run's shards: work on the tiles from the last to the first, up to 8 rows (GQ_ORDER_8) or on the tcgen05 path
+ * up to 128 (GQ_ORDER_128), because the later ones take longer.  A hint for speed: the results are the same, and 0 is always right.  < 0 on error. */
+#define GQ_ORDER_8 (1 << 28)
+#define GQ_ORDER_128 (1 << 29)
+int gq_run_order(int n_shards, const int32_t *types, const int64_t *n_outs);
+
 /* ---- per call ---------------------------------------------------------------------------------- */
 
 /* Workspace bytes a call with these sizes needs (activation staging, split-K partials, status). */

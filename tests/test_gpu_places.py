@@ -44,3 +44,28 @@ def test_the_split_leaves_no_part_empty_and_follows_the_tile_width(m):
 def test_a_run_prepared_with_other_splits_uses_the_nearest_below():
     assert [ops._table_split(s, [1, 3, 6]) for s in (1, 2, 3, 5, 6, 8)] == [1, 1, 3, 3, 6, 6]
     assert ops._table_split(2, [6]) == 1
+
+
+@pytest.mark.parametrize("types, n_outs, flags", [([F.Q4_K], [640], 0), ([F.Q4_K, F.IQ3_S], [17408, 17408], 3), ([F.IQ3_S, F.Q4_K], [17408, 17408], 0),
+                                                  ([F.IQ3_S, F.IQ4_XS], [640, 640], 1), ([F.IQ4_XS, F.IQ3_S], [640, 640], 2), ([F.Q2_K, F.Q2_K], [64, 640], 0),
+                                                  ([F.Q4_K, F.IQ2_XS], [0, 64], 0), ([F.Q4_K, F.IQ2_XS], [17408, 64], 0)])
+def test_which_end_of_a_run_is_begun_with(types, n_outs, flags):
+    assert ops.run_order(types, n_outs) == flags << 28
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_outs, k", [([64 * 280, 64 * 270 - 7], 256), ([64 * 130 + 3, 64 * 140], 2560), ([70, 200, 130], 5120), ([64, 64 * 13], 256 * 17)])
+def test_a_run_begun_at_its_end_gives_the_same_bits(n_outs, k):
+    types = [F.Q4_K, F.IQ3_S, F.IQ2_XS][:len(n_outs)]
+    raws = [synth.random_blocks(n, k, t, seed=n, device="cuda") for n, t in zip(n_outs, types)]
+    packed, _, descs, splits, _, _ = ops.prepare_grouped_layer([ops.repack_tiles(r, n, t) for r, n, t in zip(raws, n_outs, types)], n_outs, types)
+    assert ops.run_order(types, n_outs) == 3 << 28
+    for m in (1, 4, 8, 16, 33, 64, 128, 200):
+        x = synth.activations(m, k, device="cuda")
+        for s, d in zip(splits, descs):
+            if m <= 64:
+                got = [ops.grouped_gemm(x, packed, d, s, types, sum(n_outs), order=o) for o in (0, 3 << 28)]
+                assert torch.equal(*got), (m, s)
+        got = [ops.prefill_gemm(x, packed, descs[splits.index(1)], sum(n_outs), wtypes=types, order=o) for o in (0, 3 << 28)]
+        assert torch.equal(*got), m
+    assert ops.device_status() == 0
