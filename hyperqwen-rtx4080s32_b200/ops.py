@@ -482,7 +482,7 @@ def _table_split(s: int, desc_splits: Sequence[int]) -> int:
 def mul_mat_tiles_grouped_pre(x: torch.Tensor, pre, packed: torch.Tensor, descs: list[torch.Tensor], desc_splits: list[int],
                               tiles: list[torch.Tensor], n_outs: list[int], weight_types: list[int], nb: int, block_bytes: int) -> torch.Tensor:
     """mul_mat_tiles_grouped of pre(x): up to 16 rows the op is folded into the grouped launch's activation
-    preparation; above, it runs as torch operations on the device in front of the usual call."""
+    preparation; above, it runs as torch operations in front of the usual call (the native path of a layer: as one kernel, gq_pre_op)."""
     m = int(x.shape[0])
     if m == 0 or m > PRE_MAX_ROWS:
         return mul_mat_tiles_grouped(pre.unfused(x), packed, descs, desc_splits, tiles, n_outs, weight_types, nb, block_bytes)
