@@ -26,7 +26,8 @@ def _native_only(lin, x, pre):
 @pytest.mark.parametrize("m", [1, 16, 17, 33, 300])
 def test_norm_of_rows_of_any_length(k, m):
     """Beside torch's operations: the mean square is summed in another order, so a normalised value that lies at a rounding edge of bf16 may round the
-    other way (one bit of 8): few of them, and no more."""
+    other way (one bit of 8): few of them, and no more.  One unit there is up to 2^-7 of the value; the products with the weight are each rounded
+    again, by up to 2^-8: 2^-6 in all."""
     lin, x = _layer(k), synth.activations(m, k, device="cuda")
     res = synth.activations(m, k, seed=5, device="cuda") * 3
     w = (1 + 0.1 * torch.randn(k, device="cuda")).to(torch.bfloat16)
@@ -43,7 +44,7 @@ def test_norm_of_rows_of_any_length(k, m):
             out = torch.empty_like(x) if residual is not None else None
             ops.check(ops.lib().gq_pre_op(x.data_ptr(), m, k, k, 2, w.data_ptr(), residual.data_ptr() if residual is not None else None,
                                           out.data_ptr() if out is not None else None, k, 1e-6, h.data_ptr(), k, torch.cuda.current_stream().cuda_stream), "gq_pre_op")
-            assert float((h != want).float().mean()) < 2e-3 and float(((h - want).abs() / want.abs().clamp_min(1e-20)).max()) <= 2.0 ** -7
+            assert float((h != want).float().mean()) < 2e-3 and float(((h - want).abs() / want.abs().clamp_min(1e-20)).max()) <= 2.0 ** -6
     assert ops.device_status() == 0
 
 
