@@ -1416,7 +1416,15 @@ extern "C" int gq_split_for(int64_t n_tiles, int64_t nb, int64_t M, int avg_byte
     }
     static const SplitCost costs[2] = {{{0.80, 1.08, 1.47, 1.95}, 0.72, 0.04, 1.67, 0.96, 0.32, 0.46}, {{0.90, 1.21, 1.80, 0.0}, 0.29, 0.033, 1.94, 0.64, 0.34, 0.67}};
     const SplitCost &c = costs[most == 4 ? 0 : 1];
-    double best = 1e300;
+    double best = 1e300, held = 0.0;
+    // 9 .. 16 rows: the largest split of one wave that leaves a CTA three k-blocks stays unless another is to save more than an eighth.  Below
+    // that, which types the launch behind finds on an SM counts for more (o_proj and down_proj before 34,816 x 5,120, whose 544 CTAs are a wave and
+    // a quarter): four / three parts, o + gate_up of IQ4_XS, IQ4_XS + IQ3_S
+    // 52.1 / 60.5 us, stacks of two blocks 191 / 199 to 199 / 189, where the single layers with three take 0.95 to 0.99 of the time.
+    int wave = 0;
+    if (most == 3)
+        for (int S = 1; S <= 8 && (S == 1 || S <= nb / 3); ++S)
+            if (S * n_tiles * 100 <= slots * (100 - 3 * (S - 1))) wave = S;
     for (int S = 1; S <= 8 && S <= nb; ++S) {
         const int r = ctas_per_sm_for(n_tiles, S, most, sm_count);
         const double kb = 0.5 * (double)((nb + S - 1) / S) + 0.5 * (double)nb / S;      // parts differ by one k-block
@@ -1428,9 +1436,10 @@ extern "C" int gq_split_for(int64_t n_tiles, int64_t nb, int64_t M, int avg_byte
         else if (S > 1 && n_tiles * S * 10 > slots * 14) continue;
         else cost = (double)n_tiles * (double)nb / sm_count * c.kb[most - 1] / most * c.work + kb * c.tail + c.start + c.crowd * (S - 1);
         cost += (S > 1 ? c.split : 0.0) + c.part * S;
+        if (S == wave) held = cost;
         if (cost < best * (1.0 - 1e-9)) { best = cost; s = S; }
     }
-    return s;
+    return 8.0 * best > 7.0 * held && held > 0.0 ? wave : s;
 }
 
 extern "C" int64_t gq_workspace_bytes(int64_t M, int64_t K, int64_t n_total, int split) {

@@ -41,6 +41,12 @@ def test_the_split_leaves_no_part_empty_and_follows_the_tile_width(m):
             assert m > 8 or nb < 8 or splits[2] <= max(1, nb // 3) or tiles * splits[2] <= 3 * 148
 
 
+@pytest.mark.parametrize("tiles, nb, split", [(112, 20, 3), (80, 20, 4), (80, 68, 4), (544, 20, 1), (80, 17, 3), (136, 20, 2), (272, 20, 1)])
+def test_9_to_16_rows_keep_the_split_of_one_wave_unless_another_saves_an_eighth(tiles, nb, split):
+    """The first four: q + k + v, o, down and gate + up of 5,120 x 17,408; the others: shards of them."""
+    assert [ops.grouped_split_for(tiles, nb, m=m, block_bytes=b, sms=148) for m in (9, 13, 16) for b in (84, 144, 272)] == [split] * 9
+
+
 def test_a_run_prepared_with_other_splits_uses_the_nearest_below():
     assert [ops._table_split(s, [1, 3, 6]) for s in (1, 2, 3, 5, 6, 8)] == [1, 1, 3, 3, 6, 6]
     assert ops._table_split(2, [6]) == 1
