@@ -307,9 +307,10 @@ __global__ void __launch_bounds__(32 * GQ_PREP_WARPS) prep_x_kernel(const __nv_b
     prep_store<FORM>(v, kb, m, M, xt, lane);
 }
 
-// eight bf16 values as they are, wherever they start
+// eight bf16 values as they are, wherever they start (CONST: nothing writes them while the kernel runs)
+template <bool CONST = true>
 __device__ __forceinline__ uint4 load8_raw(const __nv_bfloat16 *p) {
-    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) return __ldg(reinterpret_cast<const uint4 *>(p));
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) return CONST ? __ldg(reinterpret_cast<const uint4 *>(p)) : *reinterpret_cast<const uint4 *>(p);
     const unsigned short *h = reinterpret_cast<const unsigned short *>(p);
     return make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16, h[4] | (uint32_t)h[5] << 16, h[6] | (uint32_t)h[7] << 16);
 }
@@ -340,6 +341,8 @@ __device__ __forceinline__ void store8_raw(__nv_bfloat16 *p, const uint4 &o) {
 // Bound by its latency chain at few rows (one trip to memory, two reductions, the stores), by HBM at many.  With a CTA to eight k-blocks that each
 // summed the whole row and read its own part again, 13 rows of 5,120 took 0.5 to 1 us longer; torch's operations at 24 rows take 32 us more than this,
 // at 2,048 rows 80 to 100.
+// A thread reads and writes the same columns of its row, each before it writes it, so that the new residual may take the old one's place; the
+// entry point of the op by itself accepts that (the folded call never did).
 #define GQ_NORM_MAX_WARPS 32
 #define GQ_NORM_KEEP 2
 template <bool PREP>
@@ -358,7 +361,7 @@ __global__ void __launch_bounds__(32 * GQ_NORM_MAX_WARPS) norm_rows_kernel(const
         uint4 z = load8_raw(row + col);
         if (res) {
             float a[8], r[8];
-            unpack8(load8_raw(res + col), r);
+            unpack8(load8_raw<PREP>(res + col), r);
             unpack8(z, a);
 #pragma unroll
             for (int j = 0; j < 8; ++j) a[j] += r[j];
@@ -1684,15 +1687,16 @@ extern "C" int gq_gemv_grouped(const void *x_dev, int64_t M, int64_t K, int64_t 
                                   workspace_bytes, stream, 7);
 }
 
+// in_place: residual_out may be residual_in
 static int make_pre_op(PreOp &po, int64_t K, int64_t ldx, int pre_op, const void *norm_weight_dev, const void *residual_in_dev, void *residual_out_dev, int64_t ld_res,
-                       float eps) {
+                       float eps, bool in_place) {
     po.kind = pre_op; po.K = (int)K; po.eps = eps;
     if (pre_op == GQ_PRE_SILU_MUL) {
         if (ldx < 2 * K) return GQ_ERR_ARG;
     } else if (pre_op == GQ_PRE_ADD_RMSNORM) {
         if (!norm_weight_dev || ((uintptr_t)norm_weight_dev & 1)) return GQ_ERR_ARG;
         if ((residual_in_dev == nullptr) != (residual_out_dev == nullptr)) return GQ_ERR_ARG;
-        if (residual_in_dev && (residual_in_dev == residual_out_dev || ld_res < K)) return GQ_ERR_ARG;
+        if (residual_in_dev && ((residual_in_dev == residual_out_dev && !in_place) || ld_res < K)) return GQ_ERR_ARG;
         po.weight = (const __nv_bfloat16 *)norm_weight_dev;
         po.residual = (const __nv_bfloat16 *)residual_in_dev; po.residual_out = (__nv_bfloat16 *)residual_out_dev; po.ld_res = ld_res;
     } else if (pre_op != GQ_PRE_NONE) {
@@ -1709,7 +1713,7 @@ extern "C" int gq_pre_op(const void *x_dev, int64_t M, int64_t K, int64_t ldx, i
     if (M == 0) return GQ_OK;
     if (!x_dev || !out_dev || ldo < K || ldx < K || (((uintptr_t)x_dev | (uintptr_t)out_dev | (uintptr_t)residual_in_dev | (uintptr_t)residual_out_dev) & 1)) return GQ_ERR_ARG;
     PreOp po{};
-    if (int rc = make_pre_op(po, K, ldx, pre_op, norm_weight_dev, residual_in_dev, residual_out_dev, ld_res, eps)) return rc;
+    if (int rc = make_pre_op(po, K, ldx, pre_op, norm_weight_dev, residual_in_dev, residual_out_dev, ld_res, eps, true)) return rc;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1738,14 +1742,14 @@ extern "C" int gq_pre_op(const void *x_dev, int64_t M, int64_t K, int64_t ldx, i
 // ---- the same call with the op in front of the layer folded into the activation preparation -----------------
 // pre_op GQ_PRE_SILU_MUL: x_dev is the [M, 2K] output of gate_up_proj (ldx >= 2K), the layer multiplies
 // silu(x[:, :K]) * x[:, K:].  GQ_PRE_ADD_RMSNORM: x_dev is [M, K]; norm_weight [K]; residual_in / residual_out [M, ld_res]
-// both or neither (distinct memory: every warp of a row reads the whole old residual).  1..GQ_GEMV8_MAX_ROWS rows.
+// both or neither (the same memory is refused here; gq_pre_op takes it).  1..GQ_GEMV8_MAX_ROWS rows.
 extern "C" int gq_gemv_grouped_pre(const void *x_dev, int64_t M, int64_t K, int64_t ldx, int pre_op, const void *norm_weight_dev,
                                    const void *residual_in_dev, void *residual_out_dev, int64_t ld_res, float eps, const void *packed_dev,
                                    const int32_t *desc_dev, int64_t n_desc, int split, int run_info, void *y_dev, int64_t ldy,
                                    int64_t n_total, void *workspace_dev, int64_t workspace_bytes, void *stream) {
     if (M < 0 || M > GQ_GEMV8_MAX_ROWS) return GQ_ERR_SHAPE;
     PreOp po{};
-    if (int rc = make_pre_op(po, K, ldx, pre_op, norm_weight_dev, residual_in_dev, residual_out_dev, ld_res, eps)) return rc;
+    if (int rc = make_pre_op(po, K, ldx, pre_op, norm_weight_dev, residual_in_dev, residual_out_dev, ld_res, eps, false)) return rc;
     return gemv_grouped_impl(x_dev, M, K, ldx, packed_dev, desc_dev, n_desc, split, run_info, y_dev, ldy, n_total, workspace_dev,
                              workspace_bytes, stream, 7, nullptr, 0, nullptr, &po);
 }

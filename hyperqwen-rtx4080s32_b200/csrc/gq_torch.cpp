@@ -72,6 +72,16 @@ inline bool plain_tensor(const at::Tensor &t) {
 }
 inline bool plain_cuda(const at::Tensor &t, int device) { return plain_tensor(t) && t.get_device() == device && !t.requires_grad(); }
 
+// Whether two sets of bf16 rows may share memory: `cols` columns each, rows and row strides of their own.  Rows of one stride that lie beside each
+// other, as two column ranges of one buffer do, do not.
+inline bool may_overlap(const void *a, int64_t rows_a, int64_t ld_a, const void *b, int64_t rows_b, int64_t ld_b, int64_t cols) {
+    const int64_t pa = (int64_t)((uintptr_t)a / 2), pb = (int64_t)((uintptr_t)b / 2);
+    if (pa + (rows_a - 1) * ld_a + cols <= pb || pb + (rows_b - 1) * ld_b + cols <= pa) return false;
+    if (ld_a != ld_b) return true;
+    const int64_t off = ((pb - pa) % ld_a + ld_a) % ld_a;
+    return off < cols || ld_a - off < cols;
+}
+
 class Run {
   public:
     Run(at::Tensor packed, std::vector<at::Tensor> descs, std::vector<int64_t> splits, std::vector<int64_t> n_outs, std::vector<int64_t> types,
@@ -129,6 +139,13 @@ class Run {
             }
         }
         const bool wide = m > decode_rows_, apart = pre && m > pre_rows_;       // apart: the op is a launch of its own
+        if (apart && residual) {
+            // the new residual may take the old one's place; where it shares other memory that the kernel reads, the general path reads all of it first
+            const void *out = residual_out->data_ptr();
+            const int64_t ld = residual_out->stride(0);
+            if (ld < K_ || (out != residual->data_ptr() && may_overlap(out, m, ld, residual->data_ptr(), m, ld, K_)) ||
+                may_overlap(out, m, ld, x.data_ptr(), m, ldx, K_) || may_overlap(out, m, ld, weight->data_ptr(), 1, K_, K_)) return none();
+        }
         if (wide && !apart && ((ldx & 7) || (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15))) return none();
         at::Tensor y;
         Status status;

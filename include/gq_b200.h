@@ -185,7 +185,9 @@ int gq_gemv_grouped_pre(const void *x_dev, int64_t M, int64_t K, int64_t ldx, in
                         void *workspace_dev, int64_t workspace_bytes, void *stream);
 
 /* The op in front of a layer by itself, at any number of rows (gq_gemv_grouped_pre folds it up to 16): out_dev, bf16 [M, ldo], receives what the
- * layer multiplies; the arguments are those of gq_gemv_grouped_pre and K is a multiple of 256.  One launch, the arithmetic of the folded form. */
+ * layer multiplies; the arguments are those of gq_gemv_grouped_pre and K is a multiple of 256.  residual_out_dev may be residual_in_dev (the sum in
+ * place); otherwise what is written shares no memory with what is read.  One launch (silu_and_mul: one per 65,535 rows), the arithmetic of the folded
+ * form. */
 int gq_pre_op(const void *x_dev, int64_t M, int64_t K, int64_t ldx, int pre_op, const void *norm_weight_dev, const void *residual_in_dev,
               void *residual_out_dev, int64_t ld_res, float eps, void *out_dev, int64_t ldo, void *stream);
 

@@ -71,3 +71,37 @@ def test_more_rows_than_a_grid_has_and_refused_arguments():
     assert L.gq_pre_op(x.data_ptr(), 4, k, k, 2, None, None, None, 0, 0.0, out.data_ptr(), k, st) < 0           # no weight
     assert L.gq_pre_op(x.data_ptr(), 4, k + 1, 2 * k, 2, x.data_ptr(), None, None, 0, 0.0, out.data_ptr(), 2 * k, st) < 0
     assert L.gq_pre_op(x.data_ptr(), 4, k, k, 0, None, None, None, 0, 0.0, out.data_ptr(), k, st) < 0
+
+
+@pytest.mark.parametrize("k", [256, 5120, 16640])
+@pytest.mark.parametrize("m", [17, 24, 300])
+def test_the_new_residual_in_place_of_the_old_one(k, m):
+    """Above 16 rows, also of rows that are read again before they are written (K beyond 16,384), and in memory that the kernel may not share."""
+    lin, x = _layer(k), synth.activations(m, k, device="cuda")
+    old = synth.activations(m, k, seed=5, device="cuda") * 3
+    w = (1 + 0.1 * torch.randn(k, device="cuda")).to(torch.bfloat16)
+    apart = ops.PreAddRMSNorm(w, 1e-6, old)
+    want = _native_only(lin, x, apart)
+    pre = ops.PreAddRMSNorm(w, 1e-6, old.clone())
+    pre.residual_out = pre.residual
+    for y in (_native_only(lin, x, pre), None):
+        if y is None:                   # the same through the layer
+            pre.residual.copy_(old)
+            y = lin(x, pre=pre)
+        assert torch.equal(pre.residual, apart.residual_out) and torch.equal(y, want)
+    # beside each other in one buffer: the kernel; a row on, or over the input: read in full first
+    both = torch.empty(m, 2 * k, dtype=torch.bfloat16, device="cuda")
+    rows = torch.empty(m + 1, k, dtype=torch.bfloat16, device="cuda")
+    xc = x.clone()
+    for res, out, inp, native in ((both[:, :k], both[:, k:], x, True), (rows[:m], rows[1:], x, False), (old.clone(), xc, xc, False)):
+        res.copy_(old)
+        pre = ops.PreAddRMSNorm(w, 1e-6, res)
+        pre.residual_out = out
+        if native:
+            y = _native_only(lin, inp, pre)
+        else:
+            assert lin.gguf_native(lin.gguf_groups, inp, pre) is None
+            y = lin(inp, pre=pre)
+        assert torch.equal(pre.residual_out, apart.residual_out)
+        assert float((y.double() - want.double()).norm() / want.double().norm()) < 4e-3          # torch sums the mean square in another order
+    assert ops.device_status() == 0
