@@ -2003,7 +2003,9 @@ static PrefillPlan prefill_plan(int64_t n_desc, int64_t M, int64_t nb, int sms) 
             // clusters of a unit's parts that the GPU holds side by side: of CTAs short of the last places (ctas_per_sm_for), of pairs, one
             // CTA to an SM, all (32 of 33 and 14 of 15 run as one wave; 34 of two pairs, 8,704 x 5,120 Q4_K at 300 rows, took 55 us where 34
             // whole pairs take 31)
-            const int64_t held = cluster_places(p.sets == 1 ? 2 : 1, S * p.sets, sms) * (p.sets == 1 && S > 1 ? 93 : 100), clusters = ctas / p.sets * 100;
+            const int64_t places = cluster_places(p.sets == 1 ? 2 : 1, S * p.sets, sms);
+            if (places == 0 && S > 1) break;        // so few SMs hold no such cluster, and no larger one
+            const int64_t held = (places ? places : 1) * (p.sets == 1 && S > 1 ? 93 : 100), clusters = ctas / p.sets * 100;
             const int64_t waves = (clusters + held - 1) / held;
             const double cost = (double)waves * ((double)((nb + S - 1) / S) * per_kb + 5000.0 + 25.0 * p.N + (S > 1 ? 6000.0 : 0.0));
             if (cost < best_cost * (1.0 - 1e-9)) { best_cost = cost; best = p; best.split = S; }

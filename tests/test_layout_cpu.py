@@ -103,6 +103,21 @@ def test_split_policy_above_16_rows_is_one_rule_for_all_sizes(gq_lib, m, per_sm)
             assert gq_lib.gq_split_for(n_tiles, nb, m, 144, 148) == max(fits, default=1), (n_tiles, nb)
 
 
+def test_plans_and_splits_for_any_number_of_sms(gq_lib):
+    """sm_count is the caller's: a device too small for a cluster of eight gets a plan without one, and none at all is the default."""
+    from hyperqwen_rtx4080s32_b200 import ops
+
+    for sms in list(range(1, 161)) + [1000]:
+        for tiles, nb in [(1, 1), (5, 16), (80, 20), (80, 68), (544, 20)]:
+            for m in (33, 129, 300, 517, 2048):
+                p = ops.prefill_plan(m, 256 * nb, tiles, sms)
+                assert 1 <= p["split"] <= max(1, nb // 4) and p["split"] * p["sets"] <= 8 and (p["tiles"] - 1) * p["rows"] < m <= p["tiles"] * p["rows"]
+                assert sms > 1 or p["split"] == 1 or p["sets"] == 1
+            for m in (1, 8, 16, 17, 64):
+                assert 1 <= gq_lib.gq_split_for(tiles, nb, m, 144, sms) <= min(nb, 8)
+    assert ops.prefill_plan(300, 4096, 34, -1) == ops.prefill_plan(300, 4096, 34, 148) and gq_lib.gq_split_for(80, 20, 8, 144, 0) == gq_lib.gq_split_for(80, 20, 8, 144, 148)
+
+
 def test_a_run_is_prepared_for_any_row_counts():
     """The tables of exactly the splits that these row counts choose, and split 1; a count above the grouped kernel's limit is
     answered like the largest it takes."""
