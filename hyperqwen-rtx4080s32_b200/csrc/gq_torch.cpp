@@ -90,7 +90,7 @@ class Run {
           pre_rows_(pre_rows), device_(packed_.get_device()) {
         std::vector<int32_t> t32(types.begin(), types.end());
         raise_if(info_ = gq_run_info((int)t32.size(), t32.data()), "gq_run_info");
-        const int order = gq_run_order((int)t32.size(), t32.data(), n_outs.data());
+        const int order = t32.size() == n_outs.size() ? gq_run_order((int)t32.size(), t32.data(), n_outs.data()) : 0;      // a hint
         raise_if(order, "gq_run_order");
         info_ |= order;
         for (int64_t n : n_outs) n_total_ += n;

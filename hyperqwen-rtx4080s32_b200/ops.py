@@ -141,10 +141,11 @@ _RUN_ORDER: dict[tuple, int] = {}      # bounded by the merged layers a model ha
 
 
 def run_order(wtypes: Sequence[int], n_outs: Sequence[int]) -> int:
-    """The flags of gq_run_order for a run's shards: which end of it a launch begins with."""
+    """The flags of gq_run_order for a run's shards: which end of it a launch begins with.  A hint: none where the lists do not name the same
+    shards, or no rows at all."""
     key = (tuple(wtypes), tuple(n_outs))
     if key not in _RUN_ORDER:
-        _RUN_ORDER[key] = check(lib().gq_run_order(len(key[0]), _i32_array(key[0]), _i64_array(key[1])), "gq_run_order")
+        _RUN_ORDER[key] = 0 if len(key[0]) != len(key[1]) or not any(key[1]) else check(lib().gq_run_order(len(key[0]), _i32_array(key[0]), _i64_array(key[1])), "gq_run_order")
     return _RUN_ORDER[key]
 
 

@@ -59,6 +59,12 @@ def test_which_end_of_a_run_is_begun_with(types, n_outs, flags):
     assert ops.run_order(types, n_outs) == flags << 28
 
 
+@pytest.mark.parametrize("types, n_outs", [([], []), ([F.Q4_K, F.IQ2_XS], [64]), ([F.Q4_K], [64, 64]), ([F.Q4_K, 999], [0, 0])])
+def test_no_order_for_lists_that_name_no_run(types, n_outs):
+    """Calls of no rows, and lists of unequal length, were taken before there was an order: it is 0 there, and nothing is read past a list's end."""
+    assert ops.run_order(types, n_outs) == 0
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n_outs, k", [([64 * 280, 64 * 270 - 7], 256), ([64 * 130 + 3, 64 * 140], 2560), ([70, 200, 130], 5120), ([64, 64 * 13], 256 * 17)])
 def test_a_run_begun_at_its_end_gives_the_same_bits(n_outs, k):
