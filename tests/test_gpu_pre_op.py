@@ -105,3 +105,48 @@ def test_the_new_residual_in_place_of_the_old_one(k, m):
         assert torch.equal(pre.residual_out, apart.residual_out)
         assert float((y.double() - want.double()).norm() / want.double().norm()) < 4e-3          # torch sums the mean square in another order
     assert ops.device_status() == 0
+
+
+def _at_odd(t, at=3):
+    """The rows of t as a column view that starts at an odd element, in rows of odd stride, and the buffer around it."""
+    m, k = t.shape
+    buf = torch.full((m, k + 9), 7.0, dtype=torch.bfloat16, device="cuda")
+    buf[:, at:at + k].copy_(t)
+    return buf[:, at:at + k], buf
+
+
+def _untouched(buf, k):
+    return bool((buf[:, :3] == 7.0).all()) and bool((buf[:, 3 + k:] == 7.0).all())
+
+
+@pytest.mark.parametrize("k", [256, 5120, 16640])
+@pytest.mark.parametrize("m", [4, 17, 200])
+def test_norm_of_rows_that_start_anywhere(k, m):
+    """Whatever the alignment of the input, the weight and both residuals: the bits of aligned rows, nothing written beside them."""
+    lin, x = _layer(k), synth.activations(m, k, device="cuda")
+    old = synth.activations(m, k, seed=5, device="cuda") * 3
+    w = (1 + 0.1 * torch.randn(k, device="cuda")).to(torch.bfloat16)
+    aligned = ops.PreAddRMSNorm(w, 1e-6, old)
+    want, plain = _native_only(lin, x, aligned), _native_only(lin, x, ops.PreAddRMSNorm(w, 1e-6))
+    xo, wo = _at_odd(x, 2 if m <= ops.PRE_MAX_ROWS else 3)[0], _at_odd(w[None])[0][0]       # (folded, the first row begins at a multiple of four bytes)
+    pre = ops.PreAddRMSNorm(wo, 1e-6, _at_odd(old)[0])
+    pre.residual_out, buf = _at_odd(torch.zeros_like(old))
+    assert torch.equal(_native_only(lin, xo, pre), want)
+    assert torch.equal(pre.residual_out, aligned.residual_out) and _untouched(buf, k)
+    assert torch.equal(_native_only(lin, xo, ops.PreAddRMSNorm(wo, 1e-6)), plain)
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("k", [256, 2304, 16640])
+@pytest.mark.parametrize("m", [5, 200])
+def test_the_op_by_itself_writes_rows_that_start_anywhere(k, m):
+    st, call = torch.cuda.current_stream().cuda_stream, lambda *a: ops.check(ops.lib().gq_pre_op(*a), "gq_pre_op")
+    gu, w = synth.activations(m, 2 * k, device="cuda") * 4, (1 + 0.1 * torch.randn(k, device="cuda")).to(torch.bfloat16)
+    for op, args in ((1, (None, None, None, 0, 0.0)), (2, (w.data_ptr(), None, None, 0, 1e-6))):
+        want = torch.empty(m, k, dtype=torch.bfloat16, device="cuda")
+        call(gu.data_ptr(), m, k, 2 * k, op, *args, want.data_ptr(), k, st)
+        out, buf = _at_odd(torch.zeros_like(want))
+        call(gu.data_ptr(), m, k, 2 * k, op, *args, out.data_ptr(), buf.stride(0), st)
+        assert torch.equal(out, want) and _untouched(buf, k)
+        ref = ops.PreSiluMul().unfused(gu) if op == 1 else ops.PreAddRMSNorm(w, 1e-6).unfused(gu[:, :k])
+        assert float((want != ref).float().mean()) < (1e-9 if op == 1 else 2e-3)       # the norm: torch sums the mean square in another order
