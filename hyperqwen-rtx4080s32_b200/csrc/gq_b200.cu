@@ -337,8 +337,9 @@ __device__ __forceinline__ void store8_raw(__nv_bfloat16 *p, const uint4 &o) {
 
 // RMSNorm (with the residual add) in front of the layer, one CTA per batch row: x, residual and weight are requested together and stay in registers,
 // as bf16, between the sum of squares and the scaling, two k-blocks to a warp (of rows beyond 64 k-blocks the rest is read again).
-// PREP: into the integer form's workspace (up to GQ_GEMV8_MAX_ROWS rows), a warp to a k-block where they last; else as bf16 to `out`, two to a warp.
-// Bound by its latency chain at few rows (one trip to memory, two reductions, the stores), by HBM at many.  With a CTA to eight k-blocks that each
+// PREP: into the integer form's workspace (up to GQ_GEMV8_MAX_ROWS rows); else as bf16 to `out`.  A warp to a k-block where they last, two k-blocks
+// to a warp where there are more rows than SMs.  Bound by its latency chain at few rows (one trip to memory, two reductions, the stores), at many by
+// waiting for memory with six CTAs to an SM (2,048 rows of 5,120: 84 MB in 19.6 us from a cold cache).  With a CTA to eight k-blocks that each
 // summed the whole row and read its own part again, 13 rows of 5,120 took 0.5 to 1 us longer; torch's operations at 24 rows take 32 us more than this,
 // at 2,048 rows 80 to 100.
 // A thread reads and writes the same columns of its row, each before it writes it, so that the new residual may take the old one's place; the
@@ -419,8 +420,8 @@ __global__ void __launch_bounds__(32 * GQ_NORM_MAX_WARPS) norm_rows_kernel(const
     for (int kb = warp + GQ_NORM_KEEP * warps; kb < nb; kb += warps) use(kb, load(kb), rs, load8_raw(pre.weight + (int64_t)kb * GQ_QK + 8 * lane));
 }
 
-// silu(in[:, :K]) * in[:, K:2K] as bf16, for batches whose preparation does not fold it: eight elements to a thread, bound by HBM at many rows
-// (torch's two operations: 5 us more at 24 rows of 4,352, 40 at 2,048)
+// silu(in[:, :K]) * in[:, K:2K] as bf16, for batches whose preparation does not fold it: eight elements to a thread, at many rows bound by memory and
+// its own instructions alike (2,048 rows of 5,120: 63 MB in 17.2 us, SM 62 % busy; torch's two operations: 5 us more at 24 rows of 4,352, 40 at 2,048)
 __global__ void __launch_bounds__(256) silu_mul_kernel(const __nv_bfloat16 *__restrict__ x, int64_t ldx, int K, __nv_bfloat16 *__restrict__ out, int64_t ldo) {
     pdl_trigger();
     pdl_wait();
@@ -1378,7 +1379,8 @@ extern "C" int64_t gq_build_descs_device(int n_shards, const int32_t *types, con
 static int gemv_ctas_per_sm(int64_t M) { return M <= 8 ? 4 : M <= 16 ? 3 : 2; }
 
 // How many thread-block clusters of 1 .. 8 CTAs the GPU holds side by side with one to four CTAs to an SM (cudaOccupancyMaxActiveClusters on
-// 148 SMs: a cluster lies within one of the GPU's processing clusters, and what is left of each stays empty).
+// 148 SMs: a cluster lies within one of the GPU's processing clusters, and what is left of each stays empty).  Another chip may spread its SMs over
+// them differently: a launch planned as one wave may then take two, which costs time and changes no result.
 static int64_t cluster_places(int per_sm, int split, int sms) {
     static const short places[4][8] = {{148, 74, 45, 33, 26, 22, 15, 15}, {296, 148, 93, 71, 56, 45, 37, 33}, {444, 222, 142, 104, 82, 71, 56, 48},
                                        {592, 296, 187, 142, 112, 93, 78, 71}};
@@ -1423,7 +1425,8 @@ extern "C" int gq_split_for(int64_t n_tiles, int64_t nb, int64_t M, int avg_byte
     // 9 .. 16 rows: the largest split of one wave that leaves a CTA three k-blocks stays unless another is to save more than an eighth.  Below
     // that, which types the launch behind finds on an SM counts for more (o_proj and down_proj before 34,816 x 5,120, whose 544 CTAs are a wave and
     // a quarter): four / three parts, o + gate_up of IQ4_XS, IQ4_XS + IQ3_S
-    // 52.1 / 60.5 us, stacks of two blocks 191 / 199 to 199 / 189, where the single layers with three take 0.95 to 0.99 of the time.
+    // 52.1 / 60.5 us, stacks of two blocks 191 / 199 to 199 / 189, where the single layers with three take 0.95 to 0.99 of the time.  (That effect
+    // depends on the next launch, which is not known here; up to 8 rows the unsharded layers get the same splits either way.)
     int wave = 0;
     if (most == 3)
         for (int S = 1; S <= 8 && (S == 1 || S <= nb / 3); ++S)

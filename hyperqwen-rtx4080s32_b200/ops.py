@@ -528,7 +528,8 @@ def mul_mat_tiles_grouped(x: torch.Tensor, packed: torch.Tensor, descs: list[tor
 
 class NativeRun:
     """A packed run's calls without the torch dispatcher and ctypes (csrc/gq_torch.cpp): the same entry points of the C ABI,
-    chosen by the same rules.  Answers None for a call it does not take; the caller then goes through
+    chosen by the same rules, but for the op in front of a layer above PRE_MAX_ROWS rows, which is one launch here (gq_pre_op) and torch operations in
+    mul_mat_tiles_grouped_pre (the same roundings; the mean square is summed in another order).  Answers None for a call it does not take; the caller then goes through
     mul_mat_tiles_grouped.  Copies and pickles of the layer that holds one start without it."""
     __slots__ = ("group", "_run")
 

@@ -89,7 +89,7 @@ def test_add_rms_norm_folded_into_gate_up_proj(t, m, with_residual):
     assert ops.device_status() == 0
 
 
-def test_folded_ops_above_sixteen_rows_run_unfused_and_bad_arguments_are_refused():
+def test_silu_and_mul_above_sixteen_rows_equals_the_unfused_operations_and_bad_arguments_are_refused():
     k, n = 1024, 512
     lin, raws = make_layer([n], k, F.Q4_K, 8300)
     gu = synth.activations(24, 2 * k, device=dev())
@@ -98,7 +98,7 @@ def test_folded_ops_above_sixteen_rows_run_unfused_and_bad_arguments_are_refused
     x = synth.activations(4, k, device=dev())
     w = torch.ones(k, dtype=torch.bfloat16, device=dev())
     pre = ops.PreAddRMSNorm(w, 1e-6, residual=x.clone())
-    pre.residual_out = pre.residual                      # in place: refused, every warp of a row reads the old residual
+    pre.residual_out = pre.residual                      # in place: refused up to 16 rows (above, the op by itself takes it)
     with pytest.raises(ops.GqError):
         lin(x, pre=pre)
     packed, descs, splits = lin.gguf_groups[next(iter(lin.gguf_groups))][:3]
@@ -132,7 +132,7 @@ def test_lm_head_shape_and_embedding_lookup(t):
 
 def test_silu_and_mul_folded_into_the_fused_all_reduce_call_single_rank():
     """The row-parallel down_proj of a tensor-parallel block in one call (gq_gemv_grouped_allreduce_silu_mul), world size 1: bit-identical
-    to the folded call without the exchange; above 16 rows the op falls back to the unfused sequence."""
+    to the folded call without the exchange; above 16 rows the op runs in front of the call, as torch operations here and as one kernel there."""
     from hyperqwen_rtx4080s32_b200 import tp
 
     k, n = 2048, 512

@@ -86,8 +86,8 @@ def test_split_policy_bounds(gq_lib):
 
 
 def test_split_policy_on_the_decoder_shapes(gq_lib):
-    """148 SMs, four CTAs per SM: the largest split that leaves three k-blocks per CTA, fits a cluster of 8 and keeps
-    the launch in one wave with headroom for cluster placement."""
+    """Up to 8 rows the split of the least modelled time; for the unsharded layers, on 148 SMs of four CTAs, that is the largest one that leaves three
+    k-blocks to a CTA and the launch one wave.  (Parts may be shorter elsewhere.)"""
     got = {name: gq_lib.gq_split_for(tiles, nb, 8, 144, 148)
            for name, tiles, nb in [("q", 80, 20), ("qkv", 112, 20), ("gate", 272, 20), ("gate_up", 544, 20), ("down", 80, 68), ("kv", 16, 20)]}
     assert got == {"q": 6, "qkv": 4, "gate": 2, "gate_up": 1, "down": 6, "kv": 6}
